@@ -72,17 +72,21 @@ int launch_cross_generic_query_bwd(const __half* q, const float* s, const float*
 int launch_state_generic_bwd(const __half* k, const __half* v, const uint8_t* pad_mask, const float* d_s, const float* d_z,
                              __half* gk, __half* gv, int64_t T, int BH, int H, int K, int d, cudaStream_t st);
 
+// A chunk of 128 tokens costs a CTA about 7.3 us over forward and backward together; cutting a sequence of n chunks into
+// segments of m removes n - m of them from the serial chain and pays for the pre-pass and the two scans (about 24 us,
+// 10 of them in a forward alone).  Measured, forward + backward in us at (heads x batch, tokens), whole / cut to the shortest segments
+// that one wave of SMs holds: (8, 512) 36 / 37, (16, 600) 43 / 39, (36, 700) 50 / 50, (64, 1024) 67 / 69, (8, 1024) 64 / 38,
+// (72, 2000) 125 / 116, (36, 1531) 93 / 60, (8, 2048) 121 / 46, (4, 4096) 235 / 48, (32, 16384) 915 / 363.  A forward alone
+// at (8, 1024) takes 14 us either way and is slower cut below that, hence 6 chunks saved as the line.
 static CausalPlan plan_causal(int64_t T, int BH) {
-  CausalPlan p{1, ((T + kSegAlign - 1) / kSegAlign) * kSegAlign};
-  if (BH >= 120 || T < 1024) return p;
-  int64_t want = 148 / BH;                      // segments per head that still fit one wave of 148 SMs
-  int64_t maxseg = T / 512;                     // keep segments >= 512 tokens
-  int64_t n = want < maxseg ? want : maxseg;
-  if (n < 1) n = 1;
-  int64_t tseg = ((T + n - 1) / n + kSegAlign - 1) / kSegAlign * kSegAlign;
-  p.nseg = (int)((T + tseg - 1) / tseg);
-  p.tseg = tseg;
-  return p;
+  constexpr int64_t kSms = 148, kMinSaved = 6;
+  const int64_t n = (T + kSegAlign - 1) / kSegAlign;
+  const int64_t fit = kSms / BH;                // segments per head that still fit one wave
+  if (fit >= 2 && n >= 2) {
+    const int64_t s = fit < n ? fit : n, m = (n + s - 1) / s;
+    if (n - m >= kMinSaved) return CausalPlan{(int)((n + m - 1) / m), m * kSegAlign};
+  }
+  return CausalPlan{1, n * kSegAlign};
 }
 
 struct CausalWs {
@@ -120,22 +124,38 @@ __device__ __forceinline__ float* state_elem(float* s_seg, float* z_seg, size_t 
 }
 
 // In-place exclusive scan over the segment axis of s_seg [BH][nseg][K*d] and z_seg [BH][nseg][K] (forward or reverse
-// order), seeded with carry_s [BH][K*d] / carry_z [BH][K] (may be null).
-__global__ void scan_states_kernel(float* __restrict__ s_seg, float* __restrict__ z_seg, const float* __restrict__ carry_s,
-                                   const float* __restrict__ carry_z, int BH, int nseg, int reverse) {
+// order), seeded with carry_s [BH][K*d] / carry_z [BH][K] (may be null).  Four elements per thread.
+// Bound by latency, not by its few MB (all in L2): the loads of kScanBatch segments are issued together before the first
+// sum, where a load per step of the sum chained nseg memory latencies; and the kernel asks for the shared-memory
+// carve-out of the attention kernels around it, without which every SM drains and re-partitions its L1 twice per launch.
+// 36 x 2 states: 19 -> 3.6 us.
+constexpr int kScanBatch = 8, kScanThreads = 128;
+
+__global__ void __launch_bounds__(kScanThreads)
+scan_states_kernel(float* __restrict__ s_seg, float* __restrict__ z_seg, const float* __restrict__ carry_s,
+                   const float* __restrict__ carry_z, int BH, int nseg, int reverse) {
   sm100::pdl_wait();
   sm100::pdl_launch_dependents();
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (size_t)BH * kStateN) return;
-  const size_t bh = i / kStateN;
-  const int e = (int)(i % kStateN);
-  float run = 0.f;
-  if (carry_s) run = e < kK * kD ? carry_s[bh * (kK * kD) + e] : carry_z[bh * kK + (e - kK * kD)];
-  for (int j = 0; j < nseg; ++j) {
-    float* p = state_elem(s_seg, z_seg, bh, nseg, reverse ? nseg - 1 - j : j, e);
-    const float t = *p;
-    *p = run;
-    run += t;
+  constexpr int kQuads = kStateN / 4, kSQuads = kK * kD / 4;
+  const unsigned i = blockIdx.x * kScanThreads + threadIdx.x;          // BH <= 65535: 2080 * BH fits 32 bits
+  const unsigned bh = i / kQuads, e = i % kQuads;
+  if (bh >= (unsigned)BH) return;
+  const bool is_s = e < kSQuads;
+  const int width = is_s ? kSQuads : kK / 4, col = is_s ? (int)e : (int)e - kSQuads;
+  float4* base = reinterpret_cast<float4*>(is_s ? s_seg : z_seg) + (size_t)bh * nseg * width + col;
+  const float4* carry = reinterpret_cast<const float4*>(is_s ? carry_s : carry_z);
+  float4 run = carry ? carry[(size_t)bh * width + col] : make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int j0 = 0; j0 < nseg; j0 += kScanBatch) {
+    float4 t[kScanBatch];
+#pragma unroll
+    for (int u = 0; u < kScanBatch; ++u)
+      if (j0 + u < nseg) t[u] = base[(size_t)(reverse ? nseg - 1 - (j0 + u) : j0 + u) * width];
+#pragma unroll
+    for (int u = 0; u < kScanBatch; ++u)
+      if (j0 + u < nseg) {
+        base[(size_t)(reverse ? nseg - 1 - (j0 + u) : j0 + u) * width] = run;
+        run.x += t[u].x; run.y += t[u].y; run.z += t[u].z; run.w += t[u].w;
+      }
   }
 }
 
@@ -195,7 +215,9 @@ static unsigned state_blocks(int BH) { return (unsigned)(((size_t)BH * kStateN +
 
 static int scan_launch(float* s_seg, float* z_seg, const float* carry_s, const float* carry_z, int BH, int nseg, int reverse,
                        cudaStream_t st) {
-  sm100::launch_pdl(scan_states_kernel, dim3(state_blocks(BH)), dim3(256), 0, st, s_seg, z_seg, carry_s, carry_z, BH, nseg, reverse);
+  cudaFuncSetAttribute(scan_states_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+  const unsigned blocks = (unsigned)(((size_t)BH * (kStateN / 4) + kScanThreads - 1) / kScanThreads);
+  sm100::launch_pdl(scan_states_kernel, dim3(blocks), dim3(kScanThreads), 0, st, s_seg, z_seg, carry_s, carry_z, BH, nseg, reverse);
   return check_launch("scan_states");
 }
 
