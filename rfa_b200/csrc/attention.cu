@@ -53,7 +53,21 @@ int launch_cross_query_bwd_tc(const __half* q, const float* s, const float* z, c
 int launch_cross_state_bwd_tc(const __half* k, const __half* v, const uint8_t* pad_mask, const float* d_s, const float* d_z,
                               __half* gk, __half* gv, int64_t T, int BH, int H, cudaStream_t st);
 
-// CUDA-core kernels for every other geometry (generic.cu)
+// chunked tensor-core kernels for other geometries (generic_mma.cu)
+int generic_chunk(int K, int d, int* ctas);
+int launch_causal_chunked_fwd(const __half* q, const __half* k, const __half* v, __half* out, const float* s_seg, const float* z_seg,
+                              float* s_out, float* z_out, float* den_out, int64_t T, int BH, int nseg, int64_t tseg, int K, int d,
+                              cudaStream_t st);
+int launch_causal_chunked_bwd_q(const __half* q, const __half* k, const __half* v, const __half* g, __half* gq, const float* s_seg,
+                                const float* z_seg, float* ws_den, float* ws_gz, int64_t T, int BH, int nseg, int64_t tseg, int K, int d,
+                                cudaStream_t st);
+int launch_causal_chunked_bwd_kv(const __half* q, const __half* k, const __half* v, const __half* g, __half* gk, __half* gv,
+                                 const float* ws_den, const float* ws_gz, const float* ds_seg, const float* dz_seg, int64_t T, int BH,
+                                 int nseg, int64_t tseg, int K, int d, cudaStream_t st);
+int launch_state_chunked(const __half* x, const __half* y, const uint8_t* pad_mask, const float* ws_den, const float* ws_gz, float* s,
+                         float* z, int64_t T, int BH, int H, int nseg, int64_t tseg, int K, int d, cudaStream_t st);
+
+// CUDA-core kernels for the geometries neither of them takes (generic.cu)
 bool generic_geometry_ok(int K, int d, bool two_states);
 int launch_causal_generic_fwd(const __half* q, const __half* k, const __half* v, __half* out, const float* s_in, const float* z_in,
                               float* s_out, float* z_out, float* den_out, int64_t T, int BH, int K, int d, cudaStream_t st);
@@ -78,15 +92,29 @@ int launch_state_generic_bwd(const __half* k, const __half* v, const uint8_t* pa
 // that one wave of SMs holds: (8, 512) 36 / 37, (16, 600) 43 / 39, (36, 700) 50 / 50, (64, 1024) 67 / 69, (8, 1024) 64 / 38,
 // (72, 2000) 125 / 116, (36, 1531) 93 / 60, (8, 2048) 121 / 46, (4, 4096) 235 / 48, (32, 16384) 915 / 363.  A forward alone
 // at (8, 1024) takes 14 us either way and is slower cut below that, hence 6 chunks saved as the line.
-static CausalPlan plan_causal(int64_t T, int BH) {
-  constexpr int64_t kSms = 148, kMinSaved = 6;
-  const int64_t n = (T + kSegAlign - 1) / kSegAlign;
-  const int64_t fit = kSms / BH;                // segments per head that still fit one wave
+constexpr int64_t kSms = 148;
+static CausalPlan cut_segments(int64_t T, int64_t chunk, int64_t fit, int64_t min_saved) {
+  const int64_t n = (T + chunk - 1) / chunk;
   if (fit >= 2 && n >= 2) {
     const int64_t s = fit < n ? fit : n, m = (n + s - 1) / s;
-    if (n - m >= kMinSaved) return CausalPlan{(int)((n + m - 1) / m), m * kSegAlign};
+    if (n - m >= min_saved) return CausalPlan{(int)((n + m - 1) / m), m * chunk};
   }
-  return CausalPlan{1, n * kSegAlign};
+  return CausalPlan{1, n * chunk};
+}
+static CausalPlan plan_causal(int64_t T, int BH) { return cut_segments(T, kSegAlign, kSms / BH, 6); }
+
+// Which kernels serve a geometry: the tcgen05 ones (K = 128, d = 64), the chunked ones of generic_mma.cu, or the
+// token-at-a-time ones of generic.cu.
+static bool is_tc(int K, int d) { return K == kK && d == kD; }
+static bool is_chunked(int K, int d) { return !is_tc(K, d) && generic_chunk(K, d, nullptr) > 0; }
+
+constexpr int64_t kChunkedMinSaved = 4;
+static CausalPlan plan_geometry(int64_t T, int BH, int K, int d) {
+  if (is_tc(K, d)) return plan_causal(T, BH);
+  int ctas = 1;
+  const int chunk = generic_chunk(K, d, &ctas);
+  if (!chunk) return CausalPlan{1, T};
+  return cut_segments(T, chunk, kSms * ctas / BH, kChunkedMinSaved);
 }
 
 struct CausalWs {
@@ -101,26 +129,26 @@ struct CausalWs {
 
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-static CausalWs carve_ws(void* base, int64_t T, int BH, const CausalPlan& p) {
+static CausalWs carve_ws(void* base, int64_t T, int BH, int K, int d, const CausalPlan& p) {
   CausalWs w;
   char* c = reinterpret_cast<char*>(base);
   size_t off = 0;
   auto take = [&](size_t n) { float* r = reinterpret_cast<float*>(c + off); off += align256(n * sizeof(float)); return r; };
   w.den = take((size_t)T * BH);
   w.gz = take((size_t)T * BH);
-  w.s_seg = take((size_t)BH * p.nseg * kK * kD);
-  w.z_seg = take((size_t)BH * p.nseg * kK);
-  w.ds_seg = take((size_t)BH * p.nseg * kK * kD);
-  w.dz_seg = take((size_t)BH * p.nseg * kK);
+  w.s_seg = take((size_t)BH * p.nseg * K * d);
+  w.z_seg = take((size_t)BH * p.nseg * K);
+  w.ds_seg = take((size_t)BH * p.nseg * K * d);
+  w.dz_seg = take((size_t)BH * p.nseg * K);
   w.bytes = off;
   return w;
 }
 
 constexpr int kStateN = kK * kD + kK;          // floats of one packed state [S (K*d) | z (K)]
 
-// element e of the packed state of (bh, segment): S and z live in two arrays
-__device__ __forceinline__ float* state_elem(float* s_seg, float* z_seg, size_t bh, int nseg, int sg, int e) {
-  return e < kK * kD ? s_seg + (bh * nseg + sg) * (size_t)(kK * kD) + e : z_seg + (bh * nseg + sg) * (size_t)kK + (e - kK * kD);
+// element e of the packed state of (bh, segment): S (ns floats) and z (nz floats) live in two arrays
+__device__ __forceinline__ const float* state_elem(const float* s_seg, const float* z_seg, int ns, int nz, size_t bh, int nseg, int sg, int e) {
+  return e < ns ? s_seg + (bh * nseg + sg) * (size_t)ns + e : z_seg + (bh * nseg + sg) * (size_t)nz + (e - ns);
 }
 
 // In-place exclusive scan over the segment axis of s_seg [BH][nseg][K*d] and z_seg [BH][nseg][K] (forward or reverse
@@ -133,15 +161,14 @@ constexpr int kScanBatch = 8, kScanThreads = 128;
 
 __global__ void __launch_bounds__(kScanThreads)
 scan_states_kernel(float* __restrict__ s_seg, float* __restrict__ z_seg, const float* __restrict__ carry_s,
-                   const float* __restrict__ carry_z, int BH, int nseg, int reverse) {
+                   const float* __restrict__ carry_z, int BH, int nseg, int reverse, unsigned s_quads, unsigned z_quads) {
   sm100::pdl_wait();
   sm100::pdl_launch_dependents();
-  constexpr int kQuads = kStateN / 4, kSQuads = kK * kD / 4;
-  const unsigned i = blockIdx.x * kScanThreads + threadIdx.x;          // BH <= 65535: 2080 * BH fits 32 bits
-  const unsigned bh = i / kQuads, e = i % kQuads;
+  const unsigned i = blockIdx.x * kScanThreads + threadIdx.x;          // BH <= 65535, a state < 57 K floats: fits 32 bits
+  const unsigned bh = i / (s_quads + z_quads), e = i % (s_quads + z_quads);
   if (bh >= (unsigned)BH) return;
-  const bool is_s = e < kSQuads;
-  const int width = is_s ? kSQuads : kK / 4, col = is_s ? (int)e : (int)e - kSQuads;
+  const bool is_s = e < s_quads;
+  const unsigned width = is_s ? s_quads : z_quads, col = is_s ? e : e - s_quads;
   float4* base = reinterpret_cast<float4*>(is_s ? s_seg : z_seg) + (size_t)bh * nseg * width + col;
   const float4* carry = reinterpret_cast<const float4*>(is_s ? carry_s : carry_z);
   float4 run = carry ? carry[(size_t)bh * width + col] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -161,19 +188,18 @@ scan_states_kernel(float* __restrict__ s_seg, float* __restrict__ z_seg, const f
 
 // Sum over the segment axis -> packed [BH][K*d + K] and / or the two plain arrays tot_s [BH][K*d], tot_z [BH][K].
 __global__ void total_states_kernel(const float* __restrict__ s_seg, const float* __restrict__ z_seg, float* __restrict__ packed,
-                                    float* __restrict__ tot_s, float* __restrict__ tot_z, int BH, int nseg) {
+                                    float* __restrict__ tot_s, float* __restrict__ tot_z, int BH, int nseg, int ns, int nz) {
   sm100::pdl_wait();
   sm100::pdl_launch_dependents();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (size_t)BH * kStateN) return;
-  const size_t bh = i / kStateN;
-  const int e = (int)(i % kStateN);
+  if (i >= (size_t)BH * (ns + nz)) return;
+  const size_t bh = i / (ns + nz);
+  const int e = (int)(i % (ns + nz));
   float sum = 0.f;
-  for (int j = 0; j < nseg; ++j)
-    sum += *state_elem(const_cast<float*>(s_seg), const_cast<float*>(z_seg), bh, nseg, j, e);
+  for (int j = 0; j < nseg; ++j) sum += *state_elem(s_seg, z_seg, ns, nz, bh, nseg, j, e);
   if (packed) packed[i] = sum;
   if (tot_s) {
-    if (e < kK * kD) tot_s[bh * (kK * kD) + e] = sum; else tot_z[bh * kK + (e - kK * kD)] = sum;
+    if (e < ns) tot_s[bh * ns + e] = sum; else tot_z[bh * nz + (e - ns)] = sum;
   }
 }
 
@@ -197,9 +223,6 @@ __global__ void scan_gathered_kernel(const float* __restrict__ gathered, int wor
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-// Which kernels serve a geometry: the tensor-core ones (K = 128, d = 64) or the generic CUDA-core ones.
-static bool is_tc(int K, int d) { return K == kK && d == kD; }
-
 static int check_geometry(const char* what, int64_t T, int BH, int K, int d, bool generic_allowed = true, bool two_states = false) {
   RFA_REQUIRE(T >= 0 && BH > 0, RFA_EINVAL, "%s: T=%lld BH=%d", what, (long long)T, BH);
   RFA_REQUIRE(BH <= 65535, RFA_EUNSUPPORTED, "%s: BH=%d exceeds 65535", what, BH);
@@ -214,29 +237,32 @@ static int check_geometry(const char* what, int64_t T, int BH, int K, int d, boo
 static unsigned state_blocks(int BH) { return (unsigned)(((size_t)BH * kStateN + 255) / 256); }
 
 static int scan_launch(float* s_seg, float* z_seg, const float* carry_s, const float* carry_z, int BH, int nseg, int reverse,
-                       cudaStream_t st) {
+                       int K, int d, cudaStream_t st) {
   cudaFuncSetAttribute(scan_states_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
-  const unsigned blocks = (unsigned)(((size_t)BH * (kStateN / 4) + kScanThreads - 1) / kScanThreads);
-  sm100::launch_pdl(scan_states_kernel, dim3(blocks), dim3(kScanThreads), 0, st, s_seg, z_seg, carry_s, carry_z, BH, nseg, reverse);
+  const unsigned blocks = (unsigned)(((size_t)BH * ((K * d + K) / 4) + kScanThreads - 1) / kScanThreads);
+  sm100::launch_pdl(scan_states_kernel, dim3(blocks), dim3(kScanThreads), 0, st, s_seg, z_seg, carry_s, carry_z, BH, nseg, reverse,
+                    (unsigned)(K * d / 4), (unsigned)(K / 4));
   return check_launch("scan_states");
 }
 
 static int total_launch(const float* s_seg, const float* z_seg, float* packed, float* tot_s, float* tot_z, int BH, int nseg,
-                        cudaStream_t st) {
-  sm100::launch_pdl(total_states_kernel, dim3(state_blocks(BH)), dim3(256), 0, st, s_seg, z_seg, packed, tot_s, tot_z, BH, nseg);
+                        int K, int d, cudaStream_t st) {
+  sm100::launch_pdl(total_states_kernel, dim3((unsigned)(((size_t)BH * (K * d + K) + 255) / 256)), dim3(256), 0, st, s_seg, z_seg, packed,
+                    tot_s, tot_z, BH, nseg, K * d, K);
   return check_launch("total_states");
 }
 
 // Per-segment sums of k (x) v and k -> ws.s_seg / ws.z_seg (one CTA per (batch, head, segment)).
-static int segment_partials(const __half* k, const __half* v, const CausalWs& ws, const CausalPlan& p, int64_t T, int BH,
+static int segment_partials(const __half* k, const __half* v, const CausalWs& ws, const CausalPlan& p, int64_t T, int BH, int K, int d,
                             cudaStream_t st) {
+  if (!is_tc(K, d)) return launch_state_chunked(k, v, nullptr, nullptr, nullptr, ws.s_seg, ws.z_seg, T, BH, 1, p.nseg, p.tseg, K, d, st);
   return launch_cross_state_fwd_tc(k, v, nullptr, ws.s_seg, ws.z_seg, T, BH, 1, p.nseg, p.tseg, st);
 }
 
-static int check_ws(const char* what, void* workspace, size_t bytes, int64_t T, int BH, const CausalPlan& p, CausalWs* out) {
+static int check_ws(const char* what, void* workspace, size_t bytes, int64_t T, int BH, int K, int d, const CausalPlan& p, CausalWs* out) {
   RFA_REQUIRE(workspace, RFA_EWORKSPACE, "%s: workspace is null", what);
   RFA_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 255u) == 0, RFA_EALIGN, "%s: workspace must be 256-byte aligned", what);
-  *out = carve_ws(workspace, T, BH, p);
+  *out = carve_ws(workspace, T, BH, K, d, p);
   RFA_REQUIRE(bytes >= out->bytes, RFA_EWORKSPACE, "%s: workspace has %zu bytes, %zu needed", what, bytes, out->bytes);
   return 0;
 }
@@ -247,12 +273,8 @@ using namespace rfa;
 
 extern "C" size_t rfa_causal_workspace_bytes(int64_t T, int BH, int K, int d) {
   if (T < 0 || BH <= 0) return 0;
-  if (!is_tc(K, d)) {                     // generic geometry: one run per sequence, only the two per-token scalars
-    if (!generic_geometry_ok(K, d, false)) return 0;
-    return carve_ws(nullptr, T, BH, CausalPlan{1, T}).bytes;
-  }
-  const CausalPlan p = plan_causal(T, BH);
-  return carve_ws(nullptr, T, BH, p).bytes;
+  if (!is_tc(K, d) && !generic_geometry_ok(K, d, false)) return 0;
+  return carve_ws(nullptr, T, BH, K, d, plan_geometry(T, BH, K, d)).bytes;
 }
 
 // ---- forward ---------------------------------------------------------------------------------------------------
@@ -267,7 +289,7 @@ extern "C" int rfa_causal_fwd_staged(const void* q, const void* k, const void* v
   RFA_REQUIRE(aligned16(q) && aligned16(k) && aligned16(v) && aligned16(out) && aligned16(s_in) && aligned16(z_in) &&
                   aligned16(s_out) && aligned16(z_out), RFA_EALIGN, "causal_fwd: 16-byte alignment required");
   RFA_REQUIRE((ws_has & ~RFA_WS_PARTIALS) == 0, RFA_EINVAL, "causal_fwd: ws_has may only name RFA_WS_PARTIALS (got %d)", ws_has);
-  const CausalPlan p = is_tc(K, d) ? plan_causal(T, BH) : CausalPlan{1, T};
+  CausalPlan p = plan_geometry(T, BH, K, d);
   cudaStream_t st = as_stream(stream);
   const float *s_seg = s_in, *z_seg = z_in;
   if (T == 0) {
@@ -282,23 +304,30 @@ extern "C" int rfa_causal_fwd_staged(const void* q, const void* k, const void* v
     }
     return check_launch("causal_fwd(T=0)");
   }
-  if (!is_tc(K, d)) {
+  const bool chunked = is_chunked(K, d);
+  if (!is_tc(K, d) && !chunked) {
     CausalWs gws{};
     if (save_den)
-      if (int e = check_ws("causal_fwd", workspace, workspace_bytes, T, BH, p, &gws)) return e;
+      if (int e = check_ws("causal_fwd", workspace, workspace_bytes, T, BH, K, d, p, &gws)) return e;
     return launch_causal_generic_fwd((const __half*)q, (const __half*)k, (const __half*)v, (__half*)out, s_in, z_in, s_out, z_out,
                                      save_den ? gws.den : nullptr, T, BH, K, d, st);
   }
+  // a plain forward of these geometries asks for no workspace: without one the sequences stay whole
+  if (chunked && !save_den && (!workspace || ((uintptr_t)workspace & 255u) || workspace_bytes < carve_ws(nullptr, T, BH, K, d, p).bytes))
+    p = CausalPlan{1, cut_segments(T, kSegAlign, 1, 0).tseg};
   CausalWs ws{};
   if (p.nseg > 1 || save_den)
-    if (int e = check_ws("causal_fwd", workspace, workspace_bytes, T, BH, p, &ws)) return e;
+    if (int e = check_ws("causal_fwd", workspace, workspace_bytes, T, BH, K, d, p, &ws)) return e;
   if (p.nseg > 1) {
-    if (!(ws_has & RFA_WS_PARTIALS))
-      if (int e = segment_partials((const __half*)k, (const __half*)v, ws, p, T, BH, st)) return e;
-    if (int e = scan_launch(ws.s_seg, ws.z_seg, s_in, z_in, BH, p.nseg, 0, st)) return e;
+    if (!(ws_has & RFA_WS_PARTIALS) || chunked)      // (rfa_causal_shard_total, which leaves them, is not built for these)
+      if (int e = segment_partials((const __half*)k, (const __half*)v, ws, p, T, BH, K, d, st)) return e;
+    if (int e = scan_launch(ws.s_seg, ws.z_seg, s_in, z_in, BH, p.nseg, 0, K, d, st)) return e;
     s_seg = ws.s_seg;
     z_seg = ws.z_seg;
   }
+  if (chunked)
+    return launch_causal_chunked_fwd((const __half*)q, (const __half*)k, (const __half*)v, (__half*)out, s_seg, z_seg, s_out, z_out,
+                                     save_den ? ws.den : nullptr, T, BH, p.nseg, p.tseg, K, d, st);
   return launch_causal_fwd_tc((const __half*)q, (const __half*)k, (const __half*)v, (__half*)out, s_seg, z_seg, s_out,
                               z_out, save_den ? ws.den : nullptr, T, BH, p.nseg, p.tseg, st);
 }
@@ -334,7 +363,7 @@ extern "C" int rfa_causal_fwd_fused(const void* x_q, const void* x_k, const void
   }
   CausalWs ws{};
   if (save_den)      // the denominators go where a later backward on the same T, BH expects them
-    if (int e = check_ws("causal_fwd_fused", workspace, workspace_bytes, T, BH, plan_causal(T, BH), &ws)) return e;
+    if (int e = check_ws("causal_fwd_fused", workspace, workspace_bytes, T, BH, kK, kD, plan_causal(T, BH), &ws)) return e;
   return launch_causal_fwd_fused_tc((const __half*)x_q, (const __half*)x_k, (const __half*)v, w, row_mask, (__half*)out, s_in, z_in,
                                     s_out, z_out, save_den ? ws.den : nullptr, T, BH, H, scale, st);
 }
@@ -361,9 +390,9 @@ extern "C" int rfa_causal_shard_total(const void* k, const void* v, float* total
   }
   const CausalPlan p = plan_causal(T, BH);
   CausalWs ws;
-  if (int e = check_ws("causal_shard_total", workspace, workspace_bytes, T, BH, p, &ws)) return e;
-  if (int e = segment_partials((const __half*)k, (const __half*)v, ws, p, T, BH, st)) return e;
-  return total_launch(ws.s_seg, ws.z_seg, total_packed, nullptr, nullptr, BH, p.nseg, st);
+  if (int e = check_ws("causal_shard_total", workspace, workspace_bytes, T, BH, K, d, p, &ws)) return e;
+  if (int e = segment_partials((const __half*)k, (const __half*)v, ws, p, T, BH, K, d, st)) return e;
+  return total_launch(ws.s_seg, ws.z_seg, total_packed, nullptr, nullptr, BH, p.nseg, K, d, st);
 }
 
 extern "C" int rfa_exclusive_scan_gathered(const float* gathered, int world, int rank, int reverse, float* s_out, float* z_out,
@@ -390,7 +419,7 @@ static int bwd_q_impl(const void* q, const void* k, const void* v, const void* g
   RFA_REQUIRE((ws_has & ~(RFA_WS_STATES | RFA_WS_DEN)) == 0, RFA_EINVAL,
               "causal_bwd_q: ws_has may only name RFA_WS_STATES and RFA_WS_DEN (got %d)", ws_has);
   RFA_REQUIRE(!(ws_has & RFA_WS_DEN) || out, RFA_EINVAL, "causal_bwd_q: RFA_WS_DEN needs the forward's output as well");
-  const CausalPlan p = is_tc(K, d) ? plan_causal(T, BH) : CausalPlan{1, T};
+  const CausalPlan p = plan_geometry(T, BH, K, d);
   cudaStream_t st = as_stream(stream);
   const bool want_tot = ds_tot != nullptr || dtotal_packed != nullptr;
   if (T == 0) {
@@ -402,21 +431,30 @@ static int bwd_q_impl(const void* q, const void* k, const void* v, const void* g
     return check_launch("causal_bwd_q(T=0)");
   }
   CausalWs ws;
-  if (int e = check_ws("causal_bwd_q", workspace, workspace_bytes, T, BH, p, &ws)) return e;
-  if (!is_tc(K, d))      // the generic sweep recomputes (it does not use a saved output) and writes the totals itself
+  if (int e = check_ws("causal_bwd_q", workspace, workspace_bytes, T, BH, K, d, p, &ws)) return e;
+  const bool chunked = is_chunked(K, d);
+  if (!is_tc(K, d) && !chunked)      // the generic sweep recomputes (it does not use a saved output) and writes the totals itself
     return launch_causal_generic_bwd_q((const __half*)q, (const __half*)k, (const __half*)v, (const __half*)g, (__half*)gq, s_in,
                                        z_in, ws.den, ws.gz, ds_tot, dz_tot, T, BH, K, d, st);
   const float *s_seg = s_in, *z_seg = z_in;
   if (p.nseg > 1) {
     if (!(ws_has & RFA_WS_STATES)) {    // the states entering each segment: partial sums, then an exclusive scan
-      if (int e = segment_partials((const __half*)k, (const __half*)v, ws, p, T, BH, st)) return e;
-      if (int e = scan_launch(ws.s_seg, ws.z_seg, s_in, z_in, BH, p.nseg, 0, st)) return e;
+      if (int e = segment_partials((const __half*)k, (const __half*)v, ws, p, T, BH, K, d, st)) return e;
+      if (int e = scan_launch(ws.s_seg, ws.z_seg, s_in, z_in, BH, p.nseg, 0, K, d, st)) return e;
     }
     s_seg = ws.s_seg;
     z_seg = ws.z_seg;
   }
   const bool want_dseg = p.nseg > 1 || want_tot;
-  if (ws_has & RFA_WS_DEN) {
+  if (chunked) {          // recomputes out and its denominators in fp32; the totals are a state reduction of q with g / den
+    if (int e = launch_causal_chunked_bwd_q((const __half*)q, (const __half*)k, (const __half*)v, (const __half*)g, (__half*)gq, s_seg,
+                                            z_seg, ws.den, ws.gz, T, BH, p.nseg, p.tseg, K, d, st))
+      return e;
+    if (want_dseg)
+      if (int e = launch_state_chunked((const __half*)q, (const __half*)g, nullptr, ws.den, ws.gz, ws.ds_seg, ws.dz_seg, T, BH, 1, p.nseg,
+                                       p.tseg, K, d, st))
+        return e;
+  } else if (ws_has & RFA_WS_DEN) {
     if (int e = launch_causal_bwd_q_saved_tc((const __half*)q, (const __half*)k, (const __half*)v, (const __half*)g,
                                              (const __half*)out, ws.den, (__half*)gq, s_seg, z_seg, ws.gz,
                                              want_dseg ? ws.ds_seg : nullptr, want_dseg ? ws.dz_seg : nullptr, T, BH, p.nseg,
@@ -429,7 +467,7 @@ static int bwd_q_impl(const void* q, const void* k, const void* v, const void* g
       return e;
   }
   if (want_tot)   // this shard's own total, before any carry is known
-    return total_launch(ws.ds_seg, ws.dz_seg, dtotal_packed, ds_tot, dz_tot, BH, p.nseg, st);
+    return total_launch(ws.ds_seg, ws.dz_seg, dtotal_packed, ds_tot, dz_tot, BH, p.nseg, K, d, st);
   return 0;
 }
 
@@ -459,19 +497,23 @@ extern "C" int rfa_causal_bwd_kv(const void* q, const void* k, const void* v, co
   RFA_REQUIRE(aligned16(q) && aligned16(k) && aligned16(v) && aligned16(g) && aligned16(gk) && aligned16(gv) &&
                   aligned16(ds_in) && aligned16(dz_in), RFA_EALIGN, "causal_bwd_kv: 16-byte alignment required");
   if (T == 0) return 0;
-  const CausalPlan p = is_tc(K, d) ? plan_causal(T, BH) : CausalPlan{1, T};
+  const CausalPlan p = plan_geometry(T, BH, K, d);
   cudaStream_t st = as_stream(stream);
   CausalWs ws;
-  if (int e = check_ws("causal_bwd_kv", workspace, workspace_bytes, T, BH, p, &ws)) return e;
-  if (!is_tc(K, d))
+  if (int e = check_ws("causal_bwd_kv", workspace, workspace_bytes, T, BH, K, d, p, &ws)) return e;
+  const bool chunked = is_chunked(K, d);
+  if (!is_tc(K, d) && !chunked)
     return launch_causal_generic_bwd_kv((const __half*)q, (const __half*)k, (const __half*)v, (const __half*)g, (__half*)gk,
                                         (__half*)gv, ws.den, ws.gz, ds_in, dz_in, T, BH, K, d, st);
   const float *ds_seg = ds_in, *dz_seg = dz_in;
   if (p.nseg > 1) {   // segment totals left by the forward-direction sweep -> reverse exclusive scan seeded with the carry
-    if (int e = scan_launch(ws.ds_seg, ws.dz_seg, ds_in, dz_in, BH, p.nseg, 1, st)) return e;
+    if (int e = scan_launch(ws.ds_seg, ws.dz_seg, ds_in, dz_in, BH, p.nseg, 1, K, d, st)) return e;
     ds_seg = ws.ds_seg;
     dz_seg = ws.dz_seg;
   }
+  if (chunked)
+    return launch_causal_chunked_bwd_kv((const __half*)q, (const __half*)k, (const __half*)v, (const __half*)g, (__half*)gk, (__half*)gv,
+                                        ws.den, ws.gz, ds_seg, dz_seg, T, BH, p.nseg, p.tseg, K, d, st);
   return launch_causal_bwd_kv_tc((const __half*)q, (const __half*)k, (const __half*)v, (const __half*)g, (__half*)gk,
                                  (__half*)gv, ws.den, ws.gz, ds_seg, dz_seg, T, BH, p.nseg, p.tseg, st);
 }
@@ -508,6 +550,8 @@ extern "C" int rfa_cross_state_fwd(const void* phi_k, const void* v, const uint8
     cudaMemsetAsync(z, 0, (size_t)BH * K * sizeof(float), as_stream(stream));
     return check_launch("rfa_cross_state_fwd(T=0)");
   }
+  if (is_chunked(K, d))
+    return launch_state_chunked((const __half*)phi_k, (const __half*)v, pad_mask, nullptr, nullptr, s, z, T, BH, H, 1, T, K, d, as_stream(stream));
   if (!is_tc(K, d))
     return launch_state_generic_fwd((const __half*)phi_k, (const __half*)v, pad_mask, s, z, T, BH, H, 1, T, K, d, as_stream(stream));
   const int64_t tseg = ((T + kSegAlign - 1) / kSegAlign) * kSegAlign;
@@ -532,6 +576,9 @@ extern "C" int rfa_state_partials(const void* phi_k, const void* v, float* s_par
     cudaMemsetAsync(z_part, 0, (size_t)BH * nseg * K * sizeof(float), as_stream(stream));
     return check_launch("rfa_state_partials(T=0)");
   }
+  if (is_chunked(K, d))
+    return launch_state_chunked((const __half*)phi_k, (const __half*)v, nullptr, nullptr, nullptr, s_part, z_part, T, BH, 1, nseg,
+                                rfa_state_partials_run_length(T, nseg), K, d, as_stream(stream));
   if (!is_tc(K, d))
     return launch_state_generic_fwd((const __half*)phi_k, (const __half*)v, nullptr, s_part, z_part, T, BH, 1, nseg,
                                     rfa_state_partials_run_length(T, nseg), K, d, as_stream(stream));

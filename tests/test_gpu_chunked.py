@@ -1,0 +1,72 @@
+"""The chunked kernels of the geometries other than K = 128, d = 64 (csrc/generic_mma.cu) against the PyTorch twins in fp64.
+
+Results are fp16, so that a correct one is within half a unit in the last place of the fp64 value: 2^-11 = 4.9e-4 relative at
+worst, 2.9e-4 in the 2-norm of evenly spread significands; the gate is 4e-4 in the 2-norm.  Below fp16's smallest normal number
+that is an absolute error instead, and gq of a first token whose denominator is out of the clamp is exactly zero, two
+terms of about 0.05 that cancel in 22 bits: three spacings of 6e-8 are allowed to every element.  The carried state is fp32 sums
+of exact products, a chunk's from zero: 2e-6."""
+import ctypes
+
+import pytest
+import torch
+
+from rfa_b200.rfa import RFA
+
+pytestmark = pytest.mark.gpu
+
+GEOMETRIES = [(64, 32), (96, 40), (128, 128), (256, 128), (72, 24), (8, 8), (512, 64)]      # chunks of 64, 32 and 16 tokens
+
+
+def inputs(T, BH, K, d, seed):
+    gen = torch.Generator().manual_seed(seed)
+    q, k = (torch.rand(T, BH, K, generator=gen) * 0.3 - 0.1 for _ in range(2))
+    return [t.half() for t in (q, k, torch.randn(T, BH, d, generator=gen), torch.randn(T, BH, d, generator=gen))]
+
+
+def rel(a, b, spacing=0.0):
+    return float((a.detach().cpu().double() - b).norm() - 3 * spacing * b.numel() ** 0.5) / max(float(b.norm()), 1e-30)
+
+
+@pytest.mark.parametrize("K,d", GEOMETRIES)
+@pytest.mark.parametrize("T,BH", [(1, 1), (15, 3), (64, 2), (65, 2), (131, 2), (700, 2)])
+def test_chunked_kernels_against_fp64(dev, K, d, T, BH):
+    q, k, v, g = inputs(T, BH, K, d, K + d + T)
+    want = RFA.forward_torch(*(t.double() for t in (q, k, v)))
+    grads = RFA.backward_torch(*(t.double() for t in (q, k, v, g)))
+    leaves = [t.to(dev).requires_grad_() for t in (q, k, v)]
+    out = RFA.apply(*leaves)
+    out.backward(g.to(dev))
+    assert rel(out, want, 2.0 ** -24) < 4e-4
+    for name, leaf, ref in zip("qkv", leaves, grads):
+        assert rel(leaf.grad, ref, 2.0 ** -24) < 4e-4, name
+
+
+@pytest.mark.parametrize("K,d", [(64, 32), (96, 40), (256, 128)])
+@pytest.mark.parametrize("T", [40, 700])
+def test_state_out_and_a_forward_without_workspace(dev, K, d, T):
+    from rfa_b200 import _lib, ops
+    q, k, v, _ = (t.to(dev) for t in inputs(T, 2, K, d, 5))
+    out, s, z = ops.causal_fwd(q, k, v, return_state=True)
+    kd, vd = k.cpu().double(), v.cpu().double()
+    assert rel(s, torch.einsum("tbk,tbd->bkd", kd, vd)) < 2e-6 and rel(z, kd.sum(0)) < 2e-6
+    bare = torch.empty_like(out)                       # no workspace: sequences stay whole
+    assert _lib.load().rfa_causal_fwd(*(t.data_ptr() for t in (q, k, v, bare)), None, None, None, None, None,
+                                      ctypes.c_size_t(0), T, 2, K, d, _lib.stream_of(q)) == 0
+    assert rel(bare, out.cpu().double()) < 4e-4
+
+
+@pytest.mark.parametrize("which", [0, 1, 2])
+def test_no_token_sees_a_later_non_finite_one(dev, which):
+    """A chunk's masked products multiply zeros with the tokens they mask; an infinity there must not reach earlier outputs."""
+    T, cut, K, d = 60, 37, 64, 32
+    ins = inputs(T, 2, K, d, 9)
+    clean = RFA.forward_cuda(*(t.to(dev) for t in ins[:3]))
+    ins[which][cut, :, 3] = float("inf")
+    q, k, v, g = (t.to(dev) for t in ins)
+    out = RFA.forward_cuda(q, k, v)
+    assert torch.equal(out[:cut], clean[:cut])
+    gq, _, _ = RFA.backward_cuda(q, k, v, g)
+    assert torch.isfinite(gq[:cut]).all()
+    if which == 0:       # q of a token reaches the key gradients of itself and of earlier tokens only
+        _, gk, gv = RFA.backward_cuda(q, k, v, g)
+        assert torch.isfinite(gk[cut + 1:]).all() and torch.isfinite(gv[cut + 1:]).all()
