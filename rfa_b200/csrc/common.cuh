@@ -81,40 +81,6 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
-// Block-wide register-tiled product over shared-memory operands:
-//   C(i,j) = sum_{l<L} A(i,l) * B(l,j),  i < M, j < N
-// Each thread owns TM x TN outputs with interleaved rows/columns
-// (i = tm + ii*M/TM, j = tn + jj*N/TN) so neighbouring threads touch neighbouring
-// shared-memory words.  la/lb read one operand element, st receives (i, j, value).
-template <int TM, int TN, class LA, class LB, class ST>
-__device__ __forceinline__ void tile_gemm(int M, int N, int L, LA la, LB lb, ST st) {
-  const int tiles_m = M / TM, tiles_n = N / TN;
-  for (int tile = threadIdx.x; tile < tiles_m * tiles_n; tile += blockDim.x) {
-    const int tm = tile / tiles_n, tn = tile - tm * tiles_n;
-    float acc[TM][TN];
-#pragma unroll
-    for (int ii = 0; ii < TM; ++ii)
-#pragma unroll
-      for (int jj = 0; jj < TN; ++jj) acc[ii][jj] = 0.f;
-#pragma unroll 4
-    for (int l = 0; l < L; ++l) {
-      float a[TM], b[TN];
-#pragma unroll
-      for (int ii = 0; ii < TM; ++ii) a[ii] = la(tm + ii * tiles_m, l);
-#pragma unroll
-      for (int jj = 0; jj < TN; ++jj) b[jj] = lb(l, tn + jj * tiles_n);
-#pragma unroll
-      for (int ii = 0; ii < TM; ++ii)
-#pragma unroll
-        for (int jj = 0; jj < TN; ++jj) acc[ii][jj] = fmaf(a[ii], b[jj], acc[ii][jj]);
-    }
-#pragma unroll
-    for (int ii = 0; ii < TM; ++ii)
-#pragma unroll
-      for (int jj = 0; jj < TN; ++jj) st(tm + ii * tiles_m, tn + jj * tiles_n, acc[ii][jj]);
-  }
-}
-
 #endif  // __CUDACC__
 
 }  // namespace rfa

@@ -3,115 +3,125 @@
 //   n = |x|_2,  xh = x / (n + 1e-3),  u = W_h xh,  phi = scale * [sin u | cos u]
 // (upstream utils.py:100-120, one pass instead of norm/div/einsum/sin/cos/cat/mul).
 // x [rows,H,d], W [H,D,d] fp32, phi [rows,H,2D].  One CTA owns one head and walks
-// tiles of R rows with that head's W resident in shared memory; each x element is
-// read once and each phi element written once with 16-byte accesses.
+// tiles of 64 rows with that head's W resident in shared memory; each x element is
+// read once and each phi element written once.
 #include "common.cuh"
 
 namespace rfa {
 
-constexpr int kFmThreads = 256;
+constexpr int kFmThreads = 256, kFmRows = 64;
+// Bound by fp32 arithmetic at 64 x 64 (3 of 4 products' FMAs are in the backward) and by memory at 32 x 32.  The products are
+// register tiles of 4 x 4 fed by 16-byte shared-memory reads (8 reads, 12 wavefronts, per 64 FMAs and warp; one 4-byte
+// read per operand element kept the load/store unit busy twice as long as the FMA pipe), and what follows a product
+// happens in its registers: the sines and cosines of u go straight to phi, g_u straight to the operand of the next two
+// products, and x_hat . g_xh is taken as sum_j g_u[j] u[j], which is at hand, not as a pass over g_xh.
+//
+// A thread owns rows rg + 16 i (rg = tid / 16) and columns 4 (tid % 16) .. + 3 of each block of 64 columns.  Pitches are
+// the width + 4: rows one apart are 4 banks apart and stay 16-byte aligned.
+constexpr int kFmI = kFmRows / 16;
 
 struct FmSmem {
-  float* W;    // [D][d+1]
-  float* X;    // [R][d+1]   normalised rows
-  float* U;    // [R][LU]    projections / reused for g_xh
-  float* GU;   // [R][LU]    (backward)
-  float* GW;   // [D][d+1]   (backward, optional)
-  float* nrm;  // [R]
+  float* Wt;   // [d][D + 4]   W transposed
+  float* X;    // [64][d + 4]  normalised rows
+  float* nrm;  // [64]
+  float* W;    // [D][d + 4]   (backward)
+  float* GU;   // [64][D + 4]  (backward)
+  float* c2;   // [64]         (backward) x_hat . g_xh
 };
-
-// row stride of the U / GU buffers: they hold [R][D] projections and later [R][d] g_xh
-__host__ __device__ inline int fm_ldu(int D, int d) { return (D > d ? D : d) + 1; }
-
-__host__ __device__ inline size_t fm_smem_floats(int R, int D, int d, bool bwd, bool gw) {
-  const int LU = fm_ldu(D, d);
-  size_t n = (size_t)D * (d + 1) + (size_t)R * (d + 1) + (size_t)R * LU + R;
-  if (bwd) n += (size_t)R * LU;
-  if (bwd && gw) n += (size_t)D * (d + 1);
-  return n;
+__host__ __device__ inline size_t fm_smem_floats(int D, int d, bool bwd) {
+  const size_t fwd = (size_t)d * (D + 4) + (size_t)kFmRows * (d + 4) + kFmRows;
+  return bwd ? fwd + (size_t)D * (d + 4) + (size_t)kFmRows * (D + 4) + kFmRows : fwd;
 }
-
-__device__ __forceinline__ FmSmem fm_carve(float* base, int R, int D, int d, bool bwd, bool gw) {
-  const int LU = fm_ldu(D, d);
+__device__ __forceinline__ FmSmem fm_carve(float* base, int D, int d) {
   FmSmem s;
-  s.W = base;
-  s.X = s.W + D * (d + 1);
-  s.U = s.X + R * (d + 1);
-  s.nrm = s.U + R * LU;
-  s.GU = s.nrm + R;
-  s.GW = s.GU + (bwd ? R * LU : 0);
+  s.Wt = base;
+  s.X = s.Wt + d * (D + 4);
+  s.nrm = s.X + kFmRows * (d + 4);
+  s.W = s.nrm + kFmRows;
+  s.GU = s.W + D * (d + 4);
+  s.c2 = s.GU + kFmRows * (D + 4);
   return s;
 }
 
-// Load + normalise R rows of this head into s.X (zero rows past the end).
+// Load + normalise 64 rows of this head into s.X (zero rows past the end): 16 lanes per row, all of a thread's loads issued
+// before the first sum.
 template <typename TX>
-__device__ __forceinline__ void fm_load_rows(const FmSmem& s, const TX* __restrict__ x, int64_t row0,
-                                             int64_t rows, int R, int H, int h, int d) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int r = warp; r < R; r += kFmThreads / 32) {
-    const int64_t row = row0 + r;
-    float ss = 0.f;
-    if (row < rows) {
-      const TX* src = x + ((size_t)row * H + h) * d;
-      for (int i = lane; i < d; i += 32) {
-        float t = to_f(src[i]);
-        s.X[r * (d + 1) + i] = t;
-        ss = fmaf(t, t, ss);
-      }
-    } else {
-      for (int i = lane; i < d; i += 32) s.X[r * (d + 1) + i] = 0.f;
+__device__ __forceinline__ void fm_load_rows(const FmSmem& s, const TX* __restrict__ x, int64_t row0, int64_t rows, int H, int h, int d) {
+  const int rg = threadIdx.x >> 4, c = (threadIdx.x & 15) * 4;
+  float4 v[kFmI][2];
+#pragma unroll
+  for (int i = 0; i < kFmI; ++i)
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int64_t row = row0 + rg + 16 * i;
+      v[i][u] = row < rows && c + 64 * u < d ? load4(x + ((size_t)row * H + h) * d + c + 64 * u) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    ss = warp_sum(ss);
-    const float n = sqrtf(ss);
-    const float inv = 1.f / (n + kNormEps);
-    for (int i = lane; i < d; i += 32) s.X[r * (d + 1) + i] *= inv;
-    if (lane == 0) s.nrm[r] = n;
+#pragma unroll
+  for (int i = 0; i < kFmI; ++i) {
+    float ss = 0.f;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) ss = fmaf(v[i][u].x, v[i][u].x, fmaf(v[i][u].y, v[i][u].y, fmaf(v[i][u].z, v[i][u].z, fmaf(v[i][u].w, v[i][u].w, ss))));
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    const float n = sqrtf(ss), inv = 1.f / (n + kNormEps);
+    const int r = rg + 16 * i;
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      if (c + 64 * u < d)
+        store4(s.X + r * (d + 4) + c + 64 * u, make_float4(v[i][u].x * inv, v[i][u].y * inv, v[i][u].z * inv, v[i][u].w * inv));
+    if (c == 0) s.nrm[r] = n;
+  }
+}
+__device__ __forceinline__ void fm_axpy(float (&acc)[4], float a, float4 b) {
+  acc[0] = fmaf(a, b.x, acc[0]); acc[1] = fmaf(a, b.y, acc[1]); acc[2] = fmaf(a, b.z, acc[2]); acc[3] = fmaf(a, b.w, acc[3]);
+}
+// acc[i][.] = sum_l A[rg + 16 i][l] B[l][col .. col + 3]
+__device__ __forceinline__ void fm_product(float (&acc)[kFmI][4], const float* A, int pa, const float* B, int pb, int L, int rg, int col) {
+#pragma unroll
+  for (int i = 0; i < kFmI; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[i][e] = 0.f;
+#pragma unroll 2
+  for (int l = 0; l < L; l += 4) {
+    float4 a[kFmI];
+#pragma unroll
+    for (int i = 0; i < kFmI; ++i) a[i] = load4(A + (rg + 16 * i) * pa + l);
+    const float4 b0 = load4(B + l * pb + col), b1 = load4(B + (l + 1) * pb + col), b2 = load4(B + (l + 2) * pb + col), b3 = load4(B + (l + 3) * pb + col);
+#pragma unroll
+    for (int i = 0; i < kFmI; ++i) {
+      fm_axpy(acc[i], a[i].x, b0); fm_axpy(acc[i], a[i].y, b1); fm_axpy(acc[i], a[i].z, b2); fm_axpy(acc[i], a[i].w, b3);
+    }
   }
 }
 
 template <typename TX, typename TP>
-__global__ void __launch_bounds__(kFmThreads)
+__global__ void __launch_bounds__(kFmThreads, 4)
 feature_map_fwd_kernel(const TX* __restrict__ x, const float* __restrict__ w, const uint8_t* __restrict__ row_mask,
-                       TP* __restrict__ phi, int64_t rows, int H, int d, int D, float scale, int R) {
+                       TP* __restrict__ phi, int64_t rows, int H, int d, int D, float scale) {
   extern __shared__ __align__(16) float fm_smem[];
-  const FmSmem s = fm_carve(fm_smem, R, D, d, false, false);
-  const int LU = fm_ldu(D, d);
-  const int h = blockIdx.y;
+  const FmSmem s = fm_carve(fm_smem, D, d);
+  const int h = blockIdx.y, rg = threadIdx.x >> 4, cg = (threadIdx.x & 15) * 4;
   const float* wh = w + (size_t)h * D * d;
-  for (int i = threadIdx.x; i < D * d; i += kFmThreads) s.W[(i / d) * (d + 1) + (i % d)] = wh[i];
-  const int64_t ntiles = (rows + R - 1) / R;
+  for (int i = threadIdx.x; i < D * d; i += kFmThreads) s.Wt[(i % d) * (D + 4) + i / d] = wh[i];
+  const int64_t ntiles = (rows + kFmRows - 1) / kFmRows;
   for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int64_t row0 = tile * R;
+    const int64_t row0 = tile * kFmRows;
     __syncthreads();
-    fm_load_rows(s, x, row0, rows, R, H, h, d);
+    fm_load_rows(s, x, row0, rows, H, h, d);
     __syncthreads();
-    tile_gemm<4, 4>(R, D, d,
-                    [&](int r, int l) { return s.X[r * (d + 1) + l]; },
-                    [&](int l, int j) { return s.W[j * (d + 1) + l]; },
-                    [&](int r, int j, float v) { s.U[r * LU + j] = v; });
-    __syncthreads();
-    const int groups = D / 8;
-    for (int idx = threadIdx.x; idx < R * groups; idx += kFmThreads) {
-      const int r = idx / groups, j0 = (idx % groups) * 8;
-      const int64_t row = row0 + r;
-      if (row >= rows) continue;
-      float sn[8], cs[8];
-      const float sc_row = (row_mask && row_mask[row]) ? 0.f : scale;     // a masked row gets all-zero features
+    for (int col = cg; col < D; col += 64) {
+      float u[kFmI][4];
+      fm_product(u, s.X, d + 4, s.Wt, D + 4, d, rg, col);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        sincosf(s.U[r * LU + j0 + e], &sn[e], &cs[e]);
-        sn[e] *= sc_row;
-        cs[e] *= sc_row;
-      }
-      TP* dst = phi + ((size_t)row * H + h) * 2 * D + j0;
-      if constexpr (sizeof(TP) == 2) {
-        store8(dst, sn);
-        store8(dst + D, cs);
-      } else {
-        store4(dst, make_float4(sn[0], sn[1], sn[2], sn[3]));
-        store4(dst + 4, make_float4(sn[4], sn[5], sn[6], sn[7]));
-        store4(dst + D, make_float4(cs[0], cs[1], cs[2], cs[3]));
-        store4(dst + D + 4, make_float4(cs[4], cs[5], cs[6], cs[7]));
+      for (int i = 0; i < kFmI; ++i) {
+        const int64_t row = row0 + rg + 16 * i;
+        if (row >= rows) continue;
+        const float sc = (row_mask && row_mask[row]) ? 0.f : scale;     // a masked row gets all-zero features
+        float4 sn, cs;
+        sincosf(u[i][0], &sn.x, &cs.x); sincosf(u[i][1], &sn.y, &cs.y); sincosf(u[i][2], &sn.z, &cs.z); sincosf(u[i][3], &sn.w, &cs.w);
+        TP* dst = phi + ((size_t)row * H + h) * 2 * D + col;
+        store4(dst, make_float4(sn.x * sc, sn.y * sc, sn.z * sc, sn.w * sc));
+        store4(dst + D, make_float4(cs.x * sc, cs.y * sc, cs.z * sc, cs.w * sc));
       }
     }
   }
@@ -119,75 +129,99 @@ feature_map_fwd_kernel(const TX* __restrict__ x, const float* __restrict__ w, co
 
 // Backward.  With g_u = scale * (g_sin * cos u - g_cos * sin u):
 //   g_xh = W^T g_u;  g_x = g_xh / (n + eps) - xh * (xh . g_xh) / n;  g_W += g_u (x) xh
-template <typename TX, typename TG, typename TO>
-__global__ void __launch_bounds__(kFmThreads)
-feature_map_bwd_kernel(const TX* __restrict__ x, const float* __restrict__ w, const uint8_t* __restrict__ row_mask,
-                       const TG* __restrict__ g_phi, TO* __restrict__ g_x, float* __restrict__ g_w,
-                       int64_t rows, int H, int d, int D, float scale, int R) {
+// GWT: 4 x 4 tiles of g_W per thread (D d <= 4096 GWT), summed per 64 rows from zero and kept in registers over the tiles.
+template <typename T, int GWT>
+__global__ void __launch_bounds__(kFmThreads, GWT == 1 ? 2 : 1)
+feature_map_bwd_kernel(const T* __restrict__ x, const float* __restrict__ w, const uint8_t* __restrict__ row_mask,
+                       const T* __restrict__ g_phi, T* __restrict__ g_x, float* __restrict__ g_w,
+                       int64_t rows, int H, int d, int D, float scale) {
   extern __shared__ __align__(16) float fm_smem[];
-  const bool want_gw = g_w != nullptr;
-  const FmSmem s = fm_carve(fm_smem, R, D, d, true, want_gw);
-  const int LU = fm_ldu(D, d);
-  const int h = blockIdx.y;
+  const FmSmem s = fm_carve(fm_smem, D, d);
+  const int h = blockIdx.y, rg = threadIdx.x >> 4, cg = (threadIdx.x & 15) * 4;
   const float* wh = w + (size_t)h * D * d;
   for (int i = threadIdx.x; i < D * d; i += kFmThreads) {
-    s.W[(i / d) * (d + 1) + (i % d)] = wh[i];
-    if (want_gw) s.GW[(i / d) * (d + 1) + (i % d)] = 0.f;
+    const int j = i / d, l = i - j * d;
+    s.Wt[l * (D + 4) + j] = s.W[j * (d + 4) + l] = wh[i];
   }
-  const int64_t ntiles = (rows + R - 1) / R;
+  float gw[GWT][16];
+#pragma unroll
+  for (int k = 0; k < GWT; ++k)
+#pragma unroll
+    for (int e = 0; e < 16; ++e) gw[k][e] = 0.f;
+  const int wt = d / 4, ntw = g_w ? (D / 4) * wt : 0;
+  const int64_t ntiles = (rows + kFmRows - 1) / kFmRows;
   for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int64_t row0 = tile * R;
+    const int64_t row0 = tile * kFmRows;
     __syncthreads();
-    fm_load_rows(s, x, row0, rows, R, H, h, d);
+    fm_load_rows(s, x, row0, rows, H, h, d);
     __syncthreads();
-    tile_gemm<4, 4>(R, D, d,
-                    [&](int r, int l) { return s.X[r * (d + 1) + l]; },
-                    [&](int l, int j) { return s.W[j * (d + 1) + l]; },
-                    [&](int r, int j, float v) { s.U[r * LU + j] = v; });
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < R * D; idx += kFmThreads) {
-      const int r = idx / D, j = idx % D;
-      const int64_t row = row0 + r;
-      float gu = 0.f;
-      if (row < rows && !(row_mask && row_mask[row])) {     // a masked row's features are constants: no gradient
-        float sn, cs;
-        sincosf(s.U[r * LU + j], &sn, &cs);
-        const TG* gp = g_phi + ((size_t)row * H + h) * 2 * D;
-        gu = scale * (to_f(gp[j]) * cs - to_f(gp[D + j]) * sn);
+    float dot[kFmI];
+#pragma unroll
+    for (int i = 0; i < kFmI; ++i) dot[i] = 0.f;
+    for (int col = cg; col < D; col += 64) {
+      float u[kFmI][4];
+      fm_product(u, s.X, d + 4, s.Wt, D + 4, d, rg, col);
+#pragma unroll
+      for (int i = 0; i < kFmI; ++i) {
+        const int64_t row = row0 + rg + 16 * i;
+        float4 gu = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (row < rows && !(row_mask && row_mask[row])) {     // a masked row's features are constants: no gradient
+          const T* gp = g_phi + ((size_t)row * H + h) * 2 * D + col;
+          const float4 gs = load4(gp), gc = load4(gp + D);
+          float sn, cs;
+          sincosf(u[i][0], &sn, &cs); gu.x = scale * (gs.x * cs - gc.x * sn);
+          sincosf(u[i][1], &sn, &cs); gu.y = scale * (gs.y * cs - gc.y * sn);
+          sincosf(u[i][2], &sn, &cs); gu.z = scale * (gs.z * cs - gc.z * sn);
+          sincosf(u[i][3], &sn, &cs); gu.w = scale * (gs.w * cs - gc.w * sn);
+        }
+        dot[i] = fmaf(gu.x, u[i][0], fmaf(gu.y, u[i][1], fmaf(gu.z, u[i][2], fmaf(gu.w, u[i][3], dot[i]))));
+        store4(s.GU + (rg + 16 * i) * (D + 4) + col, gu);
       }
-      s.GU[r * LU + j] = gu;
+    }
+#pragma unroll
+    for (int i = 0; i < kFmI; ++i) {
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) dot[i] += __shfl_xor_sync(0xffffffffu, dot[i], o);
+      if (cg == 0) s.c2[rg + 16 * i] = dot[i];
     }
     __syncthreads();
-    // g_xh -> s.U (projections no longer needed)
-    tile_gemm<4, 4>(R, d, D,
-                    [&](int r, int l) { return s.GU[r * LU + l]; },
-                    [&](int l, int i) { return s.W[l * (d + 1) + i]; },
-                    [&](int r, int i, float v) { s.U[r * LU + i] = v; });
-    if (want_gw)
-      tile_gemm<4, 4>(D, d, R,
-                      [&](int j, int l) { return s.GU[l * LU + j]; },
-                      [&](int l, int i) { return s.X[l * (d + 1) + i]; },
-                      [&](int j, int i, float v) { s.GW[j * (d + 1) + i] += v; });
-    __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int r = warp; r < R; r += kFmThreads / 32) {
-      const int64_t row = row0 + r;
-      if (row >= rows) continue;
-      float dot = 0.f;
-      for (int i = lane; i < d; i += 32) dot = fmaf(s.X[r * (d + 1) + i], s.U[r * LU + i], dot);
-      dot = warp_sum(dot);
-      const float n = s.nrm[r];
-      const float inv = 1.f / (n + kNormEps);
-      const float c2 = n > 0.f ? dot / n : 0.f;
-      TO* dst = g_x + ((size_t)row * H + h) * d;
-      for (int i = lane; i < d; i += 32)
-        dst[i] = from_f<TO>(s.U[r * LU + i] * inv - s.X[r * (d + 1) + i] * c2);
+    for (int col = cg; col < d; col += 64) {
+      float gx[kFmI][4];
+      fm_product(gx, s.GU, D + 4, s.W, d + 4, D, rg, col);
+#pragma unroll
+      for (int i = 0; i < kFmI; ++i) {
+        const int r = rg + 16 * i;
+        const int64_t row = row0 + r;
+        if (row >= rows) continue;
+        const float n = s.nrm[r], inv = 1.f / (n + kNormEps), c2 = n > 0.f ? s.c2[r] / n : 0.f;
+        const float4 xh = load4(s.X + r * (d + 4) + col);
+        store4(g_x + ((size_t)row * H + h) * d + col, make_float4(gx[i][0] * inv - xh.x * c2, gx[i][1] * inv - xh.y * c2,
+                                                                  gx[i][2] * inv - xh.z * c2, gx[i][3] * inv - xh.w * c2));
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < GWT; ++k) {
+      const int id = threadIdx.x + k * kFmThreads;
+      if (id < ntw) {
+        const float *pa = s.GU + (id / wt) * 4, *pb = s.X + (id % wt) * 4;
+        float acc[4][4] = {};
+#pragma unroll 4
+        for (int r = 0; r < kFmRows; ++r) {
+          const float4 a = load4(pa + r * (D + 4)), b = load4(pb + r * (d + 4));
+          fm_axpy(acc[0], a.x, b); fm_axpy(acc[1], a.y, b); fm_axpy(acc[2], a.z, b); fm_axpy(acc[3], a.w, b);
+        }
+#pragma unroll
+        for (int e = 0; e < 16; ++e) gw[k][e] += acc[e >> 2][e & 3];
+      }
     }
   }
-  if (want_gw) {
-    __syncthreads();
-    float* gwh = g_w + (size_t)h * D * d;
-    for (int i = threadIdx.x; i < D * d; i += kFmThreads) atomicAdd(gwh + i, s.GW[(i / d) * (d + 1) + (i % d)]);
+  float* gwh = g_w ? g_w + (size_t)h * D * d : nullptr;
+#pragma unroll
+  for (int k = 0; k < GWT; ++k) {
+    const int id = threadIdx.x + k * kFmThreads;
+    if (id < ntw)
+#pragma unroll
+      for (int e = 0; e < 16; ++e) atomicAdd(gwh + ((id / wt) * 4 + (e >> 2)) * d + (id % wt) * 4 + (e & 3), gw[k][e]);
   }
 }
 
@@ -208,21 +242,17 @@ static int fm_check(const void* x, const float* w, int64_t rows, int H, int d, i
   return 0;
 }
 
-static int fm_pick_rows(int D, int d, bool bwd, bool gw, size_t* bytes) {
-  for (int R = 64; R >= 16; R >>= 1) {
-    size_t b = fm_smem_floats(R, D, d, bwd, gw) * sizeof(float);
-    if (b <= 200 * 1024) { *bytes = b; return R; }
-  }
-  return 0;
-}
-
-static int fm_grid_x(int64_t ntiles, int H) {
+// CTAs per head, so that the grid is one wave of the `ctas` that an SM holds
+static int fm_grid_x(int64_t rows, int H, int ctas) {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  int64_t want = (2LL * sms + H - 1) / H;   // about two CTAs per SM over all heads
-  if (want < 1) want = 1;
+  const int64_t ntiles = (rows + kFmRows - 1) / kFmRows, fit = (int64_t)ctas * sms / H, want = fit < 1 ? 1 : fit;
   return (int)(ntiles < want ? ntiles : want);
+}
+static int fm_ctas(size_t smem, int most) {
+  const int n = (int)(227 * 1024 / (smem + 1024));
+  return n < 1 ? 1 : n < most ? n : most;
 }
 
 }  // namespace rfa
@@ -242,15 +272,13 @@ extern "C" int rfa_feature_map_fwd_masked(const void* x, int x_dtype, const floa
     return launch_feature_map_fwd_tc((const __half*)x, w, row_mask, (__half*)phi, nullptr, nullptr, nullptr, rows, H, scale, sms,
                                      as_stream(stream));
   }
-  size_t smem = 0;
-  const int R = fm_pick_rows(D, d, false, false, &smem);
-  RFA_REQUIRE(R > 0, RFA_EUNSUPPORTED, "feature_map_fwd: shared memory budget exceeded");
-  dim3 grid(fm_grid_x((rows + R - 1) / R, H), H);
+  const size_t smem = fm_smem_floats(D, d, false) * sizeof(float);      // 100 KB at most (D, d <= 128)
+  const dim3 grid(fm_grid_x(rows, H, fm_ctas(smem, 4)), H);
   cudaStream_t st = as_stream(stream);
 #define RFA_LAUNCH(TX, TP)                                                                         \
   do {                                                                                             \
     cudaFuncSetAttribute(feature_map_fwd_kernel<TX, TP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-    feature_map_fwd_kernel<TX, TP><<<grid, kFmThreads, smem, st>>>((const TX*)x, w, row_mask, (TP*)phi, rows, H, d, D, scale, R); \
+    feature_map_fwd_kernel<TX, TP><<<grid, kFmThreads, smem, st>>>((const TX*)x, w, row_mask, (TP*)phi, rows, H, d, D, scale); \
   } while (0)
   if (x_dtype == RFA_F16 && phi_dtype == RFA_F16) RFA_LAUNCH(__half, __half);
   else if (x_dtype == RFA_F32 && phi_dtype == RFA_F32) RFA_LAUNCH(float, float);
@@ -283,21 +311,22 @@ extern "C" int rfa_feature_map_bwd_masked(const void* x, int x_dtype, const floa
     return launch_feature_map_bwd_tc((const __half*)x, w, row_mask, (const __half*)g_phi, (__half*)g_x, nullptr, nullptr, nullptr,
                                      nullptr, g_w, rows, H, scale, sms, as_stream(stream));
   }
-  size_t smem = 0;
-  const int R = fm_pick_rows(D, d, true, g_w != nullptr, &smem);
-  RFA_REQUIRE(R > 0, RFA_EUNSUPPORTED, "feature_map_bwd: shared memory budget exceeded");
-  dim3 grid(fm_grid_x((rows + R - 1) / R, H), H);
+  const size_t smem = fm_smem_floats(D, d, true) * sizeof(float);       // 199 KB at most (D, d <= 128)
+  const bool small = D * d <= 4096;
+  const dim3 grid(fm_grid_x(rows, H, fm_ctas(smem, small ? 2 : 1)), H);
   cudaStream_t st = as_stream(stream);
-#define RFA_LAUNCH(T)                                                                              \
+#define RFA_LAUNCH1(T, GWT)                                                                        \
   do {                                                                                             \
-    cudaFuncSetAttribute(feature_map_bwd_kernel<T, T, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-    feature_map_bwd_kernel<T, T, T><<<grid, kFmThreads, smem, st>>>((const T*)x, w, row_mask, (const T*)g_phi, (T*)g_x, g_w, \
-                                                                    rows, H, d, D, scale, R);      \
+    cudaFuncSetAttribute(feature_map_bwd_kernel<T, GWT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    feature_map_bwd_kernel<T, GWT><<<grid, kFmThreads, smem, st>>>((const T*)x, w, row_mask, (const T*)g_phi, (T*)g_x, g_w, rows, H, d, \
+                                                                   D, scale);                      \
   } while (0)
+#define RFA_LAUNCH(T) do { if (small) RFA_LAUNCH1(T, 1); else RFA_LAUNCH1(T, 4); } while (0)
   if (x_dtype == RFA_F16) RFA_LAUNCH(__half);
   else if (x_dtype == RFA_F32) RFA_LAUNCH(float);
   else return fail(RFA_EUNSUPPORTED, "feature_map_bwd: bad dtype %d", x_dtype);
 #undef RFA_LAUNCH
+#undef RFA_LAUNCH1
   return check_launch("rfa_feature_map_bwd");
 }
 

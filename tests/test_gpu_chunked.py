@@ -70,3 +70,26 @@ def test_no_token_sees_a_later_non_finite_one(dev, which):
     if which == 0:       # q of a token reaches the key gradients of itself and of earlier tokens only
         _, gk, gv = RFA.backward_cuda(q, k, v, g)
         assert torch.isfinite(gk[cut + 1:]).all() and torch.isfinite(gv[cut + 1:]).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("rows,H,D,d", [(1, 2, 64, 64), (63, 2, 32, 32), (130, 3, 48, 40), (65, 2, 128, 128), (500, 1, 8, 128), (90, 2, 72, 8)])
+def test_feature_map_of_any_width_against_fp64(dev, dtype, rows, H, D, d):
+    """csrc/feature_map.cu: 64-row tiles, column blocks of 64, with remainders of both.  fp32: sums of d (D) products, 4e-7 per
+    result and 2e-6 for the gradient of the matrices (a sum over rows); fp16: the results' rounding, 4e-4."""
+    from rfa_b200.utils import random_project
+    gen = torch.Generator().manual_seed(rows + D)
+    x, w = torch.randn(rows, 1, H, d, generator=gen).to(dtype), torch.randn(H, D, d, generator=gen)
+    g = torch.randn(rows, 1, H, 2 * D, generator=gen).to(dtype)
+    xd, wd = x.double().requires_grad_(), w.double().requires_grad_()
+    u = torch.einsum("tbhd,hkd->tbhk", xd / (xd.norm(dim=-1, keepdim=True) + 1e-3), wd)
+    ref = 0.1 * torch.cat([u.sin(), u.cos()], dim=-1)
+    ref.backward(g.double())
+    xg, wg = x.to(dev).requires_grad_(), w.to(dev).requires_grad_()
+    phi = random_project(x=xg, random_matrices=wg)
+    phi.backward(g.to(dev))
+    half = dtype == torch.float16
+    tc = half and (D, d) == (64, 64)              # the tensor-core kernel, with fp16 operands
+    assert rel(phi, ref.detach()) < (2e-3 if tc else 4e-4 if half else 4e-7)
+    assert rel(xg.grad, xd.grad) < (2e-3 if tc else 4e-4 if half else 1e-6)
+    assert rel(wg.grad, wd.grad) < (2e-3 if tc else 2e-6)
