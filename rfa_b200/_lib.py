@@ -80,6 +80,23 @@ def load() -> C.CDLL:
     return lib
 
 
+_native_module = None
+
+
+def native():
+    """The tensor-level calls (``csrc/torch_ops.cpp``), loaded once; raise loudly if they are absent."""
+    global _native_module
+    if _native_module is None:
+        load()
+        try:
+            from . import _native
+        except ImportError as e:
+            raise ImportError(f"rfa_b200/_native.so is missing or was built for another torch ({e}). rfa_b200 has no fallback "
+                              "path: build it with `python -m rfa_b200.build`.") from e
+        _native_module = _native
+    return _native_module
+
+
 def last_error() -> str:
     return load().rfa_last_error().decode("utf-8", "replace")
 

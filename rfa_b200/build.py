@@ -1,4 +1,5 @@
-"""Build the C-ABI shared library ``rfa_b200/csrc/librfa_b200.so`` with nvcc for sm_100a.
+"""Build the C-ABI shared library ``rfa_b200/csrc/librfa_b200.so`` with nvcc for sm_100a, and ``rfa_b200/_native.so``, the
+tensor-level calls over it (``csrc/torch_ops.cpp``, against this interpreter's torch).
 
     python -m rfa_b200.build [--force] [--verbose]
 
@@ -17,6 +18,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(CSRC, "librfa_b200.so")
+NATIVE_SRC, NATIVE = os.path.join(CSRC, "torch_ops.cpp"), os.path.join(HERE, "_native.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -66,6 +68,25 @@ def compile_one(src: str, verbose: bool) -> str:
     return obj
 
 
+def build_native() -> str:
+    """The torch extension module: links the C-ABI library beside it (found through its own path)."""
+    if stale(NATIVE, [NATIVE_SRC, os.path.join(os.path.dirname(HERE), "include", "rfa_b200.h")]):
+        import sysconfig
+
+        import torch
+        from torch.utils.cpp_extension import include_paths
+        root = os.path.dirname(torch.__file__)
+        cuda = os.path.dirname(os.path.dirname(os.path.realpath(nvcc())))
+        incs = [*include_paths(), sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+        cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+               *[f"-I{i}" for i in incs], NATIVE_SRC, "-o", NATIVE, "-L" + CSRC, "-l:librfa_b200.so", "-L" + os.path.join(root, "lib"),
+               "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN/csrc"]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError("building _native.so failed:\n" + r.stdout + r.stderr)
+    return NATIVE
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     srcs = sources()
     if force:
@@ -79,6 +100,9 @@ def build(force: bool = False, verbose: bool = False) -> str:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError("link failed:\n" + r.stdout + r.stderr)
+    if force and os.path.exists(NATIVE):
+        os.remove(NATIVE)
+    build_native()
     return LIB
 
 

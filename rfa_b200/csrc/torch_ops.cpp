@@ -1,0 +1,378 @@
+// The tensor-level calls of ops.py over the C ABI: check, allocate outputs and workspace, pass pointers and the current
+// stream, turn status codes into exceptions.  No arithmetic happens here.
+//
+// In C++ because the passes of a small model are bound by this code: through ctypes a call of the causal path cost 30 to 40 us
+// of interpreter time around kernels of 10 to 20 us (checks, device guard, argument conversion, the status words), here a few.
+// Errors keep their Python types: AssertionError for shapes, TypeError for dtypes, ValueError for refused arguments,
+// RuntimeError for device trouble.
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/extension.h>
+
+#include <atomic>
+#include <string>
+#include <tuple>
+
+#include "../../include/rfa_b200.h"
+
+namespace py = pybind11;
+using at::Tensor;
+using OptTensor = std::optional<Tensor>;
+
+namespace {
+
+[[noreturn]] void raise(PyObject* type, const std::string& msg) {
+  PyErr_SetString(type, msg.c_str());
+  throw py::error_already_set();
+}
+std::string dtype_name(const Tensor& t) { return py::str(py::cast(t).attr("dtype")).cast<std::string>(); }
+std::string shape_name(const Tensor& t) { return py::str(py::cast(t).attr("shape")).cast<std::string>(); }
+
+void require_cuda(const Tensor& t) {
+  if (!t.is_cuda())
+    raise(PyExc_RuntimeError, "rfa_b200 kernels take CUDA tensors only (there is no CPU path); got a " + t.device().str() + " tensor");
+}
+void* ptr(const Tensor& t) {
+  require_cuda(t);
+  if (!t.is_contiguous()) raise(PyExc_ValueError, "rfa_b200: tensor must be contiguous");
+  return t.data_ptr();
+}
+void* ptr(const OptTensor& t) { return t ? ptr(*t) : nullptr; }
+float* fptr(const Tensor& t) { return static_cast<float*>(ptr(t)); }
+float* fptr(const OptTensor& t) { return static_cast<float*>(ptr(t)); }
+const uint8_t* bptr(const OptTensor& t) { return static_cast<const uint8_t*>(ptr(t)); }
+
+int dtype_code(const Tensor& t) {
+  if (t.scalar_type() == at::kHalf) return RFA_F16;
+  if (t.scalar_type() == at::kFloat) return RFA_F32;
+  raise(PyExc_TypeError, "rfa_b200: unsupported dtype " + dtype_name(t) + " (fp16 and fp32 only)");
+}
+template <class... T>
+void require_half(const T&... ts) {
+  for (const Tensor* t : {&ts...})
+    if (t->scalar_type() != at::kHalf) raise(PyExc_TypeError, "rfa_b200: this kernel is fp16-only, got " + dtype_name(*t));
+}
+void require(bool ok, const std::string& msg = "") {
+  if (!ok) raise(PyExc_AssertionError, msg);
+}
+void rank(const Tensor& t, int64_t n) {
+  if (t.dim() != n) raise(PyExc_ValueError, "rfa_b200: expected a tensor of " + std::to_string(n) + " dimensions, got " + shape_name(t));
+}
+int64_t rows_of(const Tensor& x, int64_t H, int64_t d) {
+  if (H * d == 0) raise(PyExc_ZeroDivisionError, "rfa_b200: the matrices are empty");
+  return x.numel() / (H * d);
+}
+std::string shapes(const Tensor& a, const Tensor& b) { return "(" + shape_name(a) + ", " + shape_name(b) + ")"; }
+
+int64_t status_error(int status, const char* what) {
+  if (status == 0) {      // a bounded wait of an earlier kernel ran out: synchronise and clear, so that it is reported once
+    const int code = rfa_status_peek();
+    rfa_debug_status();
+    raise(PyExc_RuntimeError, std::string("rfa_b200: a bounded wait inside a kernel launched before or by ") + what + " ran out (site code " +
+                                  std::to_string(code) + "); results computed since are invalid");
+  }
+  raise(status < 0 && status != RFA_EDEVICE ? PyExc_ValueError : PyExc_RuntimeError,
+        std::string(what) + " failed with status " + std::to_string(status) + ": " + rfa_last_error());
+}
+void check(int status, const char* what) {
+  if (status != 0 || rfa_status_peek() != 0) status_error(status, what);
+}
+
+// Makes the tensor's device current for the call and, on first use of a device, switches on the status mirror.
+struct Call {
+  c10::cuda::CUDAGuard guard;
+  rfa_stream_t stream;
+  explicit Call(const Tensor& t) : guard((require_cuda(t), t.device())) {
+    static std::atomic<bool> watched[64];
+    const int i = t.device().index();
+    stream = c10::cuda::getCurrentCUDAStream(i).stream();
+    if (i >= 64 || !watched[i].load(std::memory_order_acquire)) {
+      const int s = rfa_status_mirror_enable();
+      if (s != 0) raise(PyExc_RuntimeError, "rfa_status_mirror_enable failed with status " + std::to_string(s) + ": " + rfa_last_error());
+      watched[i].store(true, std::memory_order_release);
+    }
+  }
+};
+
+Tensor fresh(at::IntArrayRef shape, const Tensor& like, at::ScalarType dtype) { return at::empty(shape, like.options().dtype(dtype).requires_grad(false)); }
+Tensor fresh_zeros(at::IntArrayRef shape, const Tensor& like) { return at::zeros(shape, like.options().dtype(at::kFloat).requires_grad(false)); }
+Tensor fresh_like(const Tensor& t) { return fresh(t.sizes(), t, t.scalar_type()); }
+Tensor f32(const Tensor& t) { return t.contiguous().to(at::kFloat); }
+OptTensor f32(const OptTensor& t) { return t ? OptTensor(f32(*t)) : t; }
+
+Tensor workspace(int64_t T, int64_t BH, int64_t K, int64_t d, const Tensor& like) {
+  const int64_t n = static_cast<int64_t>(rfa_causal_workspace_bytes(T, static_cast<int>(BH), static_cast<int>(K), static_cast<int>(d)));
+  return fresh({std::max<int64_t>(n, 256)}, like, at::kByte);
+}
+
+// A mask as bytes, non-zero = masked.  Booleans are taken as they are.
+OptTensor mask_bytes(const OptTensor& mask, int64_t n, const Tensor& like) {
+  if (!mask) return mask;
+  Tensor m = mask->to(like.device()).reshape({-1});
+  if (m.scalar_type() != at::kBool) m = m.ne(0);
+  m = m.contiguous();
+  require(m.numel() == n, "(" + std::to_string(m.numel()) + ", " + std::to_string(n) + ")");
+  return m;
+}
+
+// ---- feature map ---------------------------------------------------------------------------------------------------------
+void check_feature_shapes(const Tensor& x, const Tensor& w) {
+  rank(w, 3);
+  require(x.dim() >= 2 && x.size(-2) == w.size(0) && x.size(-1) == w.size(2), shapes(x, w));
+}
+Tensor phi_like(const Tensor& x, const Tensor& w, at::ScalarType dtype) {
+  auto shape = x.sizes().vec();
+  shape.back() = 2 * w.size(1);
+  return fresh(shape, x, dtype);
+}
+
+Tensor feature_map_fwd(Tensor x, Tensor w, double scale, std::optional<at::ScalarType> out_dtype, const OptTensor& row_mask) {
+  check_feature_shapes(x, w);
+  x = x.contiguous();
+  w = f32(w);
+  const int64_t H = w.size(0), D = w.size(1), d = w.size(2), rows = rows_of(x, H, d);
+  Tensor phi = phi_like(x, w, out_dtype.value_or(x.scalar_type()));
+  const OptTensor m = mask_bytes(row_mask, rows, x);
+  Call c(x);
+  check(rfa_feature_map_fwd_masked(ptr(x), dtype_code(x), fptr(w), bptr(m), ptr(phi), dtype_code(phi), rows, H, d, D, scale, c.stream),
+        "rfa_feature_map_fwd");
+  return phi;
+}
+
+std::tuple<Tensor, OptTensor> feature_map_bwd(Tensor x, Tensor w, Tensor g_phi, double scale, bool need_gw, const OptTensor& row_mask) {
+  rank(w, 3);
+  x = x.contiguous();
+  w = f32(w);
+  g_phi = g_phi.contiguous().to(x.scalar_type());
+  const int64_t H = w.size(0), D = w.size(1), d = w.size(2), rows = rows_of(x, H, d);
+  Tensor g_x = fresh_like(x);
+  OptTensor g_w;
+  if (need_gw) g_w = fresh_zeros({H, D, d}, x);
+  const OptTensor m = mask_bytes(row_mask, rows, x);
+  Call c(x);
+  check(rfa_feature_map_bwd_masked(ptr(x), dtype_code(x), fptr(w), bptr(m), ptr(g_phi), dtype_code(g_phi), ptr(g_x), dtype_code(g_x), fptr(g_w),
+                                   rows, H, d, D, scale, c.stream),
+        "rfa_feature_map_bwd");
+  return {g_x, g_w};
+}
+
+std::tuple<Tensor, Tensor> feature_map_fwd_pair(Tensor a, Tensor b, Tensor w, double scale, const OptTensor& mask_a, const OptTensor& mask_b) {
+  require(a.sizes() == b.sizes(), shapes(a, b));
+  check_feature_shapes(a, w);
+  require_half(a, b);
+  a = a.contiguous(); b = b.contiguous();
+  w = f32(w);
+  const int64_t H = w.size(0), D = w.size(1), d = w.size(2), rows = rows_of(a, H, d);
+  Tensor pa = phi_like(a, w, at::kHalf), pb = fresh_like(pa);
+  const OptTensor ma = mask_bytes(mask_a, rows, a), mb = mask_bytes(mask_b, rows, a);
+  Call c(a);
+  check(rfa_feature_map_fwd_pair(ptr(a), ptr(b), fptr(w), bptr(ma), bptr(mb), ptr(pa), ptr(pb), rows, H, d, D, scale, c.stream),
+        "rfa_feature_map_fwd_pair");
+  return {pa, pb};
+}
+
+std::tuple<Tensor, Tensor, OptTensor> feature_map_bwd_pair(Tensor a, Tensor b, Tensor w, Tensor g_a, Tensor g_b, double scale, bool need_gw,
+                                                           const OptTensor& mask_a, const OptTensor& mask_b) {
+  rank(w, 3);
+  require_half(a, b);
+  a = a.contiguous(); b = b.contiguous();
+  w = f32(w);
+  g_a = g_a.contiguous().to(at::kHalf); g_b = g_b.contiguous().to(at::kHalf);
+  const int64_t H = w.size(0), D = w.size(1), d = w.size(2), rows = rows_of(a, H, d);
+  Tensor gxa = fresh_like(a), gxb = fresh_like(b);
+  OptTensor g_w;
+  if (need_gw) g_w = fresh_zeros({H, D, d}, a);
+  const OptTensor ma = mask_bytes(mask_a, rows, a), mb = mask_bytes(mask_b, rows, a);
+  Call c(a);
+  check(rfa_feature_map_bwd_pair(ptr(a), ptr(b), fptr(w), bptr(ma), bptr(mb), ptr(g_a), ptr(g_b), ptr(gxa), ptr(gxb), fptr(g_w), rows, H, d, D,
+                                 scale, c.stream),
+        "rfa_feature_map_bwd_pair");
+  return {gxa, gxb, g_w};
+}
+
+// ---- causal --------------------------------------------------------------------------------------------------------------
+std::tuple<Tensor, OptTensor, OptTensor> causal_fwd(Tensor q, Tensor k, Tensor v, const OptTensor& s_in, const OptTensor& z_in, bool return_state) {
+  require_half(q, k, v);
+  rank(q, 3);
+  require(v.dim() >= 2 && k.sizes() == q.sizes() && v.size(0) == q.size(0) && v.size(1) == q.size(1));
+  q = q.contiguous(); k = k.contiguous(); v = v.contiguous();
+  const int64_t T = q.size(0), BH = q.size(1), K = q.size(2), d = v.size(-1);
+  Tensor out = fresh({T, BH, d}, q, at::kHalf);
+  const OptTensor s = f32(s_in), z = f32(z_in);
+  if (T == 0) {      // nothing to launch (empty tensors have no address); the state passes through
+    if (!return_state) return {out, std::nullopt, std::nullopt};
+    if (!s) return {out, fresh_zeros({BH, K, d}, q), fresh_zeros({BH, K}, q)};
+    return {out, s->clone(), z->clone()};
+  }
+  OptTensor s_out, z_out;
+  if (return_state) {
+    s_out = fresh({BH, K, d}, q, at::kFloat);
+    z_out = fresh({BH, K}, q, at::kFloat);
+  }
+  Tensor ws = workspace(T, BH, K, d, q);
+  Call c(q);
+  check(rfa_causal_fwd(ptr(q), ptr(k), ptr(v), ptr(out), fptr(s), fptr(z), fptr(s_out), fptr(z_out), ptr(ws), ws.numel(), T, BH, K, d, c.stream),
+        "rfa_causal_fwd");
+  return {out, s_out, z_out};
+}
+
+std::tuple<Tensor, Tensor> causal_fwd_saved(Tensor q, Tensor k, Tensor v, const OptTensor& s_in, const OptTensor& z_in, const OptTensor& kept,
+                                            int ws_has) {
+  require_half(q, k, v);
+  rank(q, 3);
+  q = q.contiguous(); k = k.contiguous(); v = v.contiguous();
+  const int64_t T = q.size(0), BH = q.size(1), K = q.size(2), d = v.size(-1);
+  Tensor out = fresh({T, BH, d}, q, at::kHalf);
+  if (T == 0) return {out, fresh({256}, q, at::kByte)};
+  Tensor ws = kept ? *kept : workspace(T, BH, K, d, q);
+  Call c(q);
+  check(rfa_causal_fwd_staged(ptr(q), ptr(k), ptr(v), ptr(out), fptr(s_in), fptr(z_in), nullptr, nullptr, ptr(ws), ws.numel(), T, BH, K, d,
+                              kept ? ws_has & RFA_WS_PARTIALS : 0, 1, c.stream),
+        "rfa_causal_fwd_staged");
+  return {out, ws};
+}
+
+std::tuple<Tensor, Tensor, Tensor> causal_bwd_saved(Tensor q, Tensor k, Tensor v, Tensor g, Tensor out, const Tensor& ws, int ws_has,
+                                                    const OptTensor& s_in, const OptTensor& z_in) {
+  require_half(q, k, v, g, out);
+  rank(q, 3);
+  q = q.contiguous(); k = k.contiguous(); v = v.contiguous(); g = g.contiguous(); out = out.contiguous();
+  const int64_t T = q.size(0), BH = q.size(1), K = q.size(2), d = v.size(-1);
+  Tensor gq = fresh_like(q), gk = fresh_like(k), gv = fresh_like(v);
+  if (T == 0) return {gq, gk, gv};
+  Call c(q);
+  check(rfa_causal_bwd_saved(ptr(q), ptr(k), ptr(v), ptr(g), ptr(out), ptr(gq), ptr(gk), ptr(gv), fptr(s_in), fptr(z_in), nullptr, nullptr,
+                             ptr(ws), ws.numel(), T, BH, K, d, ws_has, c.stream),
+        "rfa_causal_bwd_saved");
+  return {gq, gk, gv};
+}
+
+std::tuple<Tensor, OptTensor, OptTensor, OptTensor> causal_fwd_fused(Tensor xq, Tensor xk, Tensor v, Tensor w, double scale, const OptTensor& row_mask,
+                                                                     const OptTensor& s_in, const OptTensor& z_in, bool return_state, bool save_den) {
+  require_half(xq, xk, v);
+  rank(xq, 4);
+  xq = xq.contiguous(); xk = xk.contiguous(); v = v.contiguous();
+  w = f32(w);
+  const int64_t T = xq.size(0), B = xq.size(1), H = xq.size(2), d = xq.size(3), BH = B * H, D = w.size(-2);
+  Tensor out = fresh({T, BH, d}, xq, at::kHalf);
+  const OptTensor m = mask_bytes(row_mask, T * B, xq);
+  OptTensor s_out, z_out, ws;
+  if (return_state) {
+    s_out = fresh({BH, 2 * D, d}, xq, at::kFloat);
+    z_out = fresh({BH, 2 * D}, xq, at::kFloat);
+  }
+  if (save_den) ws = workspace(std::max<int64_t>(T, 1), BH, 2 * D, d, xq);
+  Call c(xq);
+  check(rfa_causal_fwd_fused(ptr(xq), ptr(xk), ptr(v), fptr(w), bptr(m), scale, ptr(out), fptr(s_in), fptr(z_in), fptr(s_out), fptr(z_out), ptr(ws),
+                             ws ? ws->numel() : 0, T, B, H, d, D, save_den ? 1 : 0, c.stream),
+        "rfa_causal_fwd_fused");
+  return {out, s_out, z_out, ws};
+}
+
+// ---- cross ---------------------------------------------------------------------------------------------------------------
+std::tuple<Tensor, Tensor> cross_state_fwd(Tensor phi_k, Tensor v, const OptTensor& pad) {
+  require_half(phi_k, v);
+  rank(phi_k, 4);
+  phi_k = phi_k.contiguous(); v = v.contiguous();
+  const int64_t T = phi_k.size(0), B = phi_k.size(1), H = phi_k.size(2), K = phi_k.size(3), d = v.size(-1);
+  const OptTensor m = mask_bytes(pad, B * T, phi_k);
+  Tensor s = fresh({B, H, K, d}, phi_k, at::kFloat), z = fresh({B, H, K}, phi_k, at::kFloat);
+  Call c(phi_k);
+  check(rfa_cross_state_fwd(ptr(phi_k), ptr(v), bptr(m), fptr(s), fptr(z), T, B, H, K, d, c.stream), "rfa_cross_state_fwd");
+  return {s, z};
+}
+
+std::tuple<Tensor, Tensor> cross_state_bwd(Tensor phi_k, Tensor v, const OptTensor& pad, Tensor d_s, Tensor d_z) {
+  rank(phi_k, 4);
+  phi_k = phi_k.contiguous(); v = v.contiguous();
+  d_s = f32(d_s); d_z = f32(d_z);
+  const int64_t T = phi_k.size(0), B = phi_k.size(1), H = phi_k.size(2), K = phi_k.size(3), d = v.size(-1);
+  const OptTensor m = mask_bytes(pad, B * T, phi_k);
+  Tensor g_k = fresh_like(phi_k), g_v = fresh_like(v);
+  Call c(phi_k);
+  check(rfa_cross_state_bwd(ptr(phi_k), ptr(v), bptr(m), fptr(d_s), fptr(d_z), ptr(g_k), ptr(g_v), T, B, H, K, d, c.stream), "rfa_cross_state_bwd");
+  return {g_k, g_v};
+}
+
+Tensor cross_query_fwd(Tensor phi_q, Tensor s, Tensor z) {
+  require_half(phi_q);
+  rank(phi_q, 4);
+  phi_q = phi_q.contiguous();
+  s = f32(s); z = f32(z);
+  const int64_t T = phi_q.size(0), B = phi_q.size(1), H = phi_q.size(2), K = phi_q.size(3), d = s.size(-1);
+  Tensor out = fresh({T, B, H, d}, phi_q, at::kHalf);
+  Call c(phi_q);
+  check(rfa_cross_query_fwd(ptr(phi_q), fptr(s), fptr(z), ptr(out), T, B * H, K, d, c.stream), "rfa_cross_query_fwd");
+  return out;
+}
+
+std::tuple<Tensor, Tensor, Tensor> cross_query_bwd(Tensor phi_q, Tensor s, Tensor z, Tensor g) {
+  require_half(phi_q, g);
+  rank(phi_q, 4);
+  phi_q = phi_q.contiguous(); g = g.contiguous();
+  s = f32(s); z = f32(z);
+  const int64_t T = phi_q.size(0), B = phi_q.size(1), H = phi_q.size(2), K = phi_q.size(3), d = s.size(-1);
+  Tensor g_q = fresh_like(phi_q), d_s = fresh_like(s), d_z = fresh_like(z);
+  Call c(phi_q);
+  check(rfa_cross_query_bwd(ptr(phi_q), fptr(s), fptr(z), ptr(g), ptr(g_q), fptr(d_s), fptr(d_z), T, B * H, K, d, c.stream), "rfa_cross_query_bwd");
+  return {g_q, d_s, d_z};
+}
+
+// ---- decode --------------------------------------------------------------------------------------------------------------
+Tensor decode_out(const char* what, const Tensor& v, const OptTensor& out) {
+  if (!out) return fresh(v.sizes(), v, v.scalar_type());
+  if (out->scalar_type() != v.scalar_type() || !out->is_contiguous())
+    raise(PyExc_TypeError, std::string(what) + ": out must be contiguous and of v's dtype");
+  return *out;
+}
+void check_state(const char* what, const char* inputs, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& s, const Tensor& z) {
+  if (q.scalar_type() != k.scalar_type() || k.scalar_type() != v.scalar_type() || s.scalar_type() != z.scalar_type())
+    raise(PyExc_TypeError, std::string(what) + ": " + inputs + ", v must share a dtype and so must s, z (got " + dtype_name(q) + ", " + dtype_name(k) +
+                               ", " + dtype_name(v) + "; " + dtype_name(s) + ", " + dtype_name(z) + ")");
+  if (!s.is_contiguous() || !z.is_contiguous())
+    raise(PyExc_ValueError, std::string(what) + ": state tensors must be contiguous (they are updated in place)");
+}
+
+Tensor decode_step(Tensor phi_q, Tensor phi_k, Tensor v, const Tensor& s, const Tensor& z, const OptTensor& out_) {
+  rank(phi_q, 3);
+  const int64_t B = phi_q.size(0), H = phi_q.size(1), K = phi_q.size(2), d = v.size(-1);
+  phi_q = phi_q.contiguous(); phi_k = phi_k.contiguous(); v = v.contiguous();
+  check_state("decode_step", "phi_q, phi_k", phi_q, phi_k, v, s, z);
+  Tensor out = out_ ? decode_out("decode_step", v, out_) : fresh({B, H, d}, v, v.scalar_type());
+  Call c(v);
+  check(rfa_decode_step(ptr(phi_q), ptr(phi_k), ptr(v), dtype_code(v), ptr(s), ptr(z), dtype_code(s), ptr(out), B * H, K, d, c.stream),
+        "rfa_decode_step");
+  return out;
+}
+
+Tensor decode_step_fused(Tensor q, Tensor k, Tensor v, const Tensor& w, double scale, const Tensor& s, const Tensor& z, const OptTensor& out_) {
+  rank(q, 3);
+  const int64_t B = q.size(0), H = q.size(1), d = q.size(2), D = w.size(1);
+  q = q.contiguous(); k = k.contiguous(); v = v.contiguous();
+  if (w.scalar_type() != at::kFloat || !w.is_contiguous()) raise(PyExc_ValueError, "decode_step_fused: w must be a contiguous fp32 [H,D,d] tensor");
+  check_state("decode_step_fused", "q, k", q, k, v, s, z);
+  Tensor out = out_ ? decode_out("decode_step_fused", v, out_) : fresh({B, H, d}, v, v.scalar_type());
+  Call c(v);
+  check(rfa_decode_step_fused(ptr(q), ptr(k), ptr(v), dtype_code(v), fptr(w), scale, ptr(s), ptr(z), dtype_code(s), ptr(out), B * H, H, D, d, c.stream),
+        "rfa_decode_step_fused");
+  return out;
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_native, m) {
+  m.def("feature_map_fwd", &feature_map_fwd);
+  m.def("feature_map_bwd", &feature_map_bwd);
+  m.def("feature_map_fwd_pair", &feature_map_fwd_pair);
+  m.def("feature_map_bwd_pair", &feature_map_bwd_pair);
+  m.def("causal_fwd", &causal_fwd);
+  m.def("causal_fwd_saved", &causal_fwd_saved);
+  m.def("causal_bwd_saved", &causal_bwd_saved);
+  m.def("causal_fwd_fused", &causal_fwd_fused);
+  m.def("cross_state_fwd", &cross_state_fwd);
+  m.def("cross_state_bwd", &cross_state_bwd);
+  m.def("cross_query_fwd", &cross_query_fwd);
+  m.def("cross_query_bwd", &cross_query_bwd);
+  m.def("decode_step", &decode_step);
+  m.def("decode_step_fused", &decode_step_fused);
+}

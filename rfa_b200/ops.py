@@ -1,6 +1,8 @@
 """Tensor-level wrappers over the C ABI: allocate outputs, pass raw pointers and
 the current stream, turn status codes into exceptions.  No arithmetic happens
-here; every function launches kernels from ``librfa_b200.so``.
+here; every function launches kernels from ``librfa_b200.so``.  The calls of the
+forward, backward and decoding paths are in ``csrc/torch_ops.cpp``; the rest go
+through ctypes.
 """
 from __future__ import annotations
 
@@ -10,7 +12,7 @@ import torch
 from torch import Tensor
 
 from . import _lib
-from ._lib import check, dtype_code, ptr, require_half, stream_of
+from ._lib import check, dtype_code, native, ptr, require_half, stream_of
 
 K_BUILT, D_BUILT = 128, 64      # geometry the attention kernels are built for
 
@@ -44,46 +46,16 @@ def _workspace(T: int, BH: int, K: int, d: int, like: Tensor) -> Tuple[Tensor, i
 
 
 # --------------------------------------------------------------------------- feature map
-def _row_mask(row_mask: Optional[Tensor], rows: int, dev) -> Optional[Tensor]:
-    if row_mask is None:
-        return None
-    m = (row_mask.to(device=dev).reshape(-1) != 0).to(torch.uint8).contiguous()
-    assert m.numel() == rows, (m.numel(), rows)
-    return m
-
-
 def feature_map_fwd(x: Tensor, w: Tensor, scale: float, out_dtype: Optional[torch.dtype] = None,
                     row_mask: Optional[Tensor] = None) -> Tensor:
     """x [..., H, d], w [H, D, d] fp32 -> phi [..., H, 2D].  row_mask (one entry per leading index, non-zero = masked):
     those rows get all-zero features."""
-    H, D, d = w.shape
-    assert x.shape[-2] == H and x.shape[-1] == d, (x.shape, w.shape)
-    x = x.contiguous()
-    w = w.contiguous().float()
-    phi = torch.empty(*x.shape[:-1], 2 * D, dtype=out_dtype or x.dtype, device=x.device)
-    rows = x.numel() // (H * d)
-    m = _row_mask(row_mask, rows, x.device)
-    with _guard(x):
-        check(_lib.load().rfa_feature_map_fwd_masked(ptr(x), dtype_code(x), ptr(w), ptr(m), ptr(phi), dtype_code(phi),
-                                                     rows, H, d, D, float(scale), stream_of(x)), "rfa_feature_map_fwd")
-    return phi
+    return native().feature_map_fwd(x, w, scale, out_dtype, row_mask)
 
 
 def feature_map_bwd(x: Tensor, w: Tensor, g_phi: Tensor, scale: float, need_gw: bool,
                     row_mask: Optional[Tensor] = None) -> Tuple[Tensor, Optional[Tensor]]:
-    H, D, d = w.shape
-    x = x.contiguous()
-    w = w.contiguous().float()
-    g_phi = g_phi.contiguous().to(x.dtype)
-    g_x = torch.empty_like(x)
-    g_w = torch.zeros(H, D, d, dtype=torch.float32, device=x.device) if need_gw else None
-    rows = x.numel() // (H * d)
-    m = _row_mask(row_mask, rows, x.device)
-    with _guard(x):
-        check(_lib.load().rfa_feature_map_bwd_masked(ptr(x), dtype_code(x), ptr(w), ptr(m), ptr(g_phi), dtype_code(g_phi),
-                                                     ptr(g_x), dtype_code(g_x), ptr(g_w), rows, H, d, D, float(scale),
-                                                     stream_of(x)), "rfa_feature_map_bwd")
-    return g_x, g_w
+    return native().feature_map_bwd(x, w, g_phi, scale, need_gw, row_mask)
 
 
 def feature_map_pair_supported(x_a: Tensor, x_b: Tensor, w: Tensor) -> bool:
@@ -95,38 +67,13 @@ def feature_map_pair_supported(x_a: Tensor, x_b: Tensor, w: Tensor) -> bool:
 def feature_map_fwd_pair(x_a: Tensor, x_b: Tensor, w: Tensor, scale: float, row_mask_a: Optional[Tensor] = None,
                          row_mask_b: Optional[Tensor] = None) -> Tuple[Tensor, Tensor]:
     """phi of x_a and of x_b (same shape [..., H, 64], fp16; w [H, 64, 64]) in one launch."""
-    H, D, d = w.shape
-    assert x_a.shape == x_b.shape and x_a.shape[-2] == H and x_a.shape[-1] == d, (x_a.shape, x_b.shape, w.shape)
-    require_half(x_a, x_b)
-    x_a, x_b = x_a.contiguous(), x_b.contiguous()
-    w = w.contiguous().float()
-    phi_a = torch.empty(*x_a.shape[:-1], 2 * D, dtype=torch.float16, device=x_a.device)
-    phi_b = torch.empty_like(phi_a)
-    rows = x_a.numel() // (H * d)
-    ma, mb = _row_mask(row_mask_a, rows, x_a.device), _row_mask(row_mask_b, rows, x_a.device)
-    with _guard(x_a):
-        check(_lib.load().rfa_feature_map_fwd_pair(ptr(x_a), ptr(x_b), ptr(w), ptr(ma), ptr(mb), ptr(phi_a), ptr(phi_b), rows, H, d, D,
-                                                   float(scale), stream_of(x_a)), "rfa_feature_map_fwd_pair")
-    return phi_a, phi_b
+    return native().feature_map_fwd_pair(x_a, x_b, w, scale, row_mask_a, row_mask_b)
 
 
 def feature_map_bwd_pair(x_a: Tensor, x_b: Tensor, w: Tensor, g_phi_a: Tensor, g_phi_b: Tensor, scale: float, need_gw: bool,
                          row_mask_a: Optional[Tensor] = None, row_mask_b: Optional[Tensor] = None):
     """Backward of ``feature_map_fwd_pair``: (g_x_a, g_x_b, g_w) with g_w the sum of both arrays' contributions (or None)."""
-    H, D, d = w.shape
-    require_half(x_a, x_b)
-    x_a, x_b = x_a.contiguous(), x_b.contiguous()
-    w = w.contiguous().float()
-    g_phi_a, g_phi_b = g_phi_a.contiguous().to(torch.float16), g_phi_b.contiguous().to(torch.float16)
-    g_x_a, g_x_b = torch.empty_like(x_a), torch.empty_like(x_b)
-    g_w = torch.zeros(H, D, d, dtype=torch.float32, device=x_a.device) if need_gw else None
-    rows = x_a.numel() // (H * d)
-    ma, mb = _row_mask(row_mask_a, rows, x_a.device), _row_mask(row_mask_b, rows, x_a.device)
-    with _guard(x_a):
-        check(_lib.load().rfa_feature_map_bwd_pair(ptr(x_a), ptr(x_b), ptr(w), ptr(ma), ptr(mb), ptr(g_phi_a), ptr(g_phi_b), ptr(g_x_a),
-                                                   ptr(g_x_b), ptr(g_w), rows, H, d, D, float(scale), stream_of(x_a)),
-              "rfa_feature_map_bwd_pair")
-    return g_x_a, g_x_b, g_w
+    return native().feature_map_bwd_pair(x_a, x_b, w, g_phi_a, g_phi_b, scale, need_gw, row_mask_a, row_mask_b)
 
 
 def gather_random_matrices(bank: Tensor, picks: Tensor, sigma: Optional[Tensor] = None,
@@ -153,26 +100,7 @@ def gather_random_matrices(bank: Tensor, picks: Tensor, sigma: Optional[Tensor] 
 def causal_fwd(q: Tensor, k: Tensor, v: Tensor, s_in: Optional[Tensor] = None, z_in: Optional[Tensor] = None,
                return_state: bool = False):
     """q,k [T,BH,K], v [T,BH,d] fp16 -> out [T,BH,d] (and the final state when asked)."""
-    require_half(q, k, v)
-    T, BH, K = q.shape
-    d = v.shape[-1]
-    assert k.shape == q.shape and v.shape[:2] == q.shape[:2]
-    q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-    out = torch.empty(T, BH, d, dtype=torch.float16, device=q.device)
-    if s_in is not None:
-        s_in, z_in = s_in.contiguous().float(), z_in.contiguous().float()
-    if T == 0:      # nothing to launch (empty tensors have no address); the state passes through
-        if not return_state:
-            return out
-        if s_in is None:
-            return out, torch.zeros(BH, K, d, device=q.device), torch.zeros(BH, K, device=q.device)
-        return out, s_in.clone(), z_in.clone()
-    s_out = torch.empty(BH, K, d, dtype=torch.float32, device=q.device) if return_state else None
-    z_out = torch.empty(BH, K, dtype=torch.float32, device=q.device) if return_state else None
-    ws, n = _workspace(T, BH, K, d, q)
-    with _guard(q):
-        check(_lib.load().rfa_causal_fwd(ptr(q), ptr(k), ptr(v), ptr(out), ptr(s_in), ptr(z_in), ptr(s_out),
-                                         ptr(z_out), ptr(ws), n, T, BH, K, d, stream_of(q)), "rfa_causal_fwd")
+    out, s_out, z_out = native().causal_fwd(q, k, v, s_in, z_in, return_state)
     return (out, s_out, z_out) if return_state else out
 
 
@@ -202,21 +130,8 @@ def causal_fwd_saved(q: Tensor, k: Tensor, v: Tensor, s_in: Optional[Tensor] = N
     """Forward that keeps what the backward can reuse.  Returns (out, workspace, ws_has): the workspace then holds the
     raw denominators and, when the sequence is cut into segments, the states entering each of them.  ``ws`` / ``ws_has``
     hand in a workspace that ``shard_total`` has already filled for the same k, v."""
-    require_half(q, k, v)
-    T, BH, K = q.shape
-    d = v.shape[-1]
-    q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-    out = torch.empty(T, BH, d, dtype=torch.float16, device=q.device)
-    if T == 0:
-        return out, torch.empty(256, dtype=torch.uint8, device=q.device), 0
-    if ws is None:
-        ws, _ = _workspace(T, BH, K, d, q)
-        ws_has = 0
-    with _guard(q):
-        check(_lib.load().rfa_causal_fwd_staged(ptr(q), ptr(k), ptr(v), ptr(out), ptr(s_in), ptr(z_in), None, None,
-                                                ptr(ws), ws.numel(), T, BH, K, d, ws_has & _lib.WS_PARTIALS, 1, stream_of(q)),
-              "rfa_causal_fwd_staged")
-    return out, ws, _lib.WS_STATES | _lib.WS_DEN
+    out, ws = native().causal_fwd_saved(q, k, v, s_in, z_in, ws, ws_has)
+    return out, ws, (_lib.WS_STATES | _lib.WS_DEN if q.shape[0] else 0)
 
 
 def fused_forward_supported(x: Tensor, w: Tensor) -> bool:
@@ -234,25 +149,7 @@ def causal_fwd_fused(x_q: Tensor, x_k: Tensor, v: Tensor, w: Tensor, scale: floa
     scale * [sin | cos]((W x) / (|x| + 1e-3)) of q and k are formed inside the kernel.  row_mask [T, B] (or [T * B]) marks
     padded keys.  Returns out [T, B*H, 64] and, as asked, the final state (s, z) and the workspace holding the raw
     denominators for ``causal_bwd_saved(..., ws_has=WS_DEN)``: (out[, s, z][, ws])."""
-    require_half(x_q, x_k, v)
-    T, B, H, d = x_q.shape
-    D = w.shape[-2]
-    x_q, x_k, v = x_q.contiguous(), x_k.contiguous(), v.contiguous()
-    w = w.contiguous().float()
-    BH = B * H
-    out = torch.empty(T, BH, d, dtype=torch.float16, device=x_q.device)
-    m = _row_mask(row_mask, T * B, x_q.device)
-    s_out = z_out = None
-    if return_state:
-        s_out = torch.empty(BH, 2 * D, d, dtype=torch.float32, device=x_q.device)
-        z_out = torch.empty(BH, 2 * D, dtype=torch.float32, device=x_q.device)
-    ws = None
-    if save_den:
-        ws, _ = _workspace(max(T, 1), BH, 2 * D, d, x_q)
-    with _guard(x_q):
-        check(_lib.load().rfa_causal_fwd_fused(ptr(x_q), ptr(x_k), ptr(v), ptr(w), ptr(m), float(scale), ptr(out), ptr(s_in),
-                                               ptr(z_in), ptr(s_out), ptr(z_out), ptr(ws), ws.numel() if ws is not None else 0,
-                                               T, B, H, d, D, 1 if save_den else 0, stream_of(x_q)), "rfa_causal_fwd_fused")
+    out, s_out, z_out, ws = native().causal_fwd_fused(x_q, x_k, v, w, scale, row_mask, s_in, z_in, return_state, save_den)
     res = (out,)
     if return_state:
         res += (s_out, z_out)
@@ -264,18 +161,7 @@ def causal_fwd_fused(x_q: Tensor, x_k: Tensor, v: Tensor, w: Tensor, scale: floa
 def causal_bwd_saved(q: Tensor, k: Tensor, v: Tensor, g: Tensor, out: Tensor, ws: Tensor, ws_has: int,
                      s_in: Optional[Tensor] = None, z_in: Optional[Tensor] = None):
     """Backward from the forward's output and kept workspace (``causal_fwd_saved``)."""
-    require_half(q, k, v, g, out)
-    T, BH, K = q.shape
-    d = v.shape[-1]
-    q, k, v, g, out = q.contiguous(), k.contiguous(), v.contiguous(), g.contiguous(), out.contiguous()
-    gq, gk, gv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-    if T == 0:
-        return gq, gk, gv
-    with _guard(q):
-        check(_lib.load().rfa_causal_bwd_saved(ptr(q), ptr(k), ptr(v), ptr(g), ptr(out), ptr(gq), ptr(gk), ptr(gv), ptr(s_in),
-                                               ptr(z_in), None, None, ptr(ws), ws.numel(), T, BH, K, d, ws_has, stream_of(q)),
-              "rfa_causal_bwd_saved")
-    return gq, gk, gv
+    return native().causal_bwd_saved(q, k, v, g, out, ws, ws_has, s_in, z_in)
 
 
 def shard_total(k: Tensor, v: Tensor, packed: Optional[Tensor] = None):
@@ -364,26 +250,9 @@ def causal_bwd_kv(q, k, v, g, ds_in, dz_in, ws: Tensor):
 
 
 # --------------------------------------------------------------------------- cross
-def _mask_bytes(pad_mask: Optional[Tensor], B: int, T: int, dev) -> Optional[Tensor]:
-    if pad_mask is None:
-        return None
-    m = pad_mask.to(device=dev).reshape(B, T)
-    return (m != 0).to(torch.uint8).contiguous()
-
-
 def cross_state_fwd(phi_k: Tensor, v: Tensor, pad_mask: Optional[Tensor]) -> Tuple[Tensor, Tensor]:
     """phi_k [T,B,H,K], v [T,B,H,d] fp16, pad_mask [B,T] (non-zero = pad) -> s [B,H,K,d], z [B,H,K] fp32."""
-    require_half(phi_k, v)
-    T, B, H, K = phi_k.shape
-    d = v.shape[-1]
-    phi_k, v = phi_k.contiguous(), v.contiguous()
-    m = _mask_bytes(pad_mask, B, T, phi_k.device)
-    s = torch.empty(B, H, K, d, dtype=torch.float32, device=phi_k.device)
-    z = torch.empty(B, H, K, dtype=torch.float32, device=phi_k.device)
-    with _guard(phi_k):
-        check(_lib.load().rfa_cross_state_fwd(ptr(phi_k), ptr(v), ptr(m), ptr(s), ptr(z), T, B, H, K, d,
-                                              stream_of(phi_k)), "rfa_cross_state_fwd")
-    return s, z
+    return native().cross_state_fwd(phi_k, v, pad_mask)
 
 
 def state_total(phi_k: Tensor, v: Tensor) -> Tuple[Tensor, Tensor]:
@@ -406,89 +275,28 @@ def state_total(phi_k: Tensor, v: Tensor) -> Tuple[Tensor, Tensor]:
 
 
 def cross_state_bwd(phi_k: Tensor, v: Tensor, pad_mask: Optional[Tensor], d_s: Tensor, d_z: Tensor):
-    T, B, H, K = phi_k.shape
-    d = v.shape[-1]
-    phi_k, v = phi_k.contiguous(), v.contiguous()
-    m = _mask_bytes(pad_mask, B, T, phi_k.device)
-    d_s, d_z = d_s.contiguous().float(), d_z.contiguous().float()
-    g_k, g_v = torch.empty_like(phi_k), torch.empty_like(v)
-    with _guard(phi_k):
-        check(_lib.load().rfa_cross_state_bwd(ptr(phi_k), ptr(v), ptr(m), ptr(d_s), ptr(d_z), ptr(g_k), ptr(g_v),
-                                              T, B, H, K, d, stream_of(phi_k)), "rfa_cross_state_bwd")
-    return g_k, g_v
+    return native().cross_state_bwd(phi_k, v, pad_mask, d_s, d_z)
 
 
 def cross_query_fwd(phi_q: Tensor, s: Tensor, z: Tensor) -> Tensor:
     """phi_q [T,B,H,K] fp16, s [B,H,K,d], z [B,H,K] fp32 -> out [T,B,H,d] fp16."""
-    require_half(phi_q)
-    T, B, H, K = phi_q.shape
-    d = s.shape[-1]
-    phi_q = phi_q.contiguous()
-    s, z = s.contiguous().float(), z.contiguous().float()
-    out = torch.empty(T, B, H, d, dtype=torch.float16, device=phi_q.device)
-    with _guard(phi_q):
-        check(_lib.load().rfa_cross_query_fwd(ptr(phi_q), ptr(s), ptr(z), ptr(out), T, B * H, K, d,
-                                              stream_of(phi_q)), "rfa_cross_query_fwd")
-    return out
+    return native().cross_query_fwd(phi_q, s, z)
 
 
 def cross_query_bwd(phi_q: Tensor, s: Tensor, z: Tensor, g: Tensor):
-    require_half(phi_q, g)
-    T, B, H, K = phi_q.shape
-    d = s.shape[-1]
-    phi_q, g = phi_q.contiguous(), g.contiguous()
-    s, z = s.contiguous().float(), z.contiguous().float()
-    g_q = torch.empty_like(phi_q)
-    d_s, d_z = torch.empty_like(s), torch.empty_like(z)
-    with _guard(phi_q):
-        check(_lib.load().rfa_cross_query_bwd(ptr(phi_q), ptr(s), ptr(z), ptr(g), ptr(g_q), ptr(d_s), ptr(d_z),
-                                              T, B * H, K, d, stream_of(phi_q)), "rfa_cross_query_bwd")
-    return g_q, d_s, d_z
+    return native().cross_query_bwd(phi_q, s, z, g)
 
 
 # --------------------------------------------------------------------------- decode
 def decode_step(phi_q: Tensor, phi_k: Tensor, v: Tensor, s: Tensor, z: Tensor, out: Optional[Tensor] = None) -> Tensor:
     """One token, state updated IN PLACE.  phi_q,phi_k [B,H,K], v [B,H,d]; s [B,H,K,d], z [B,H,K]."""
-    B, H, K = phi_q.shape
-    d = v.shape[-1]
-    phi_q, phi_k, v = phi_q.contiguous(), phi_k.contiguous(), v.contiguous()
-    if not (s.is_contiguous() and z.is_contiguous()):
-        raise ValueError("decode_step: state tensors must be contiguous (they are updated in place)")
-    if not (phi_q.dtype == phi_k.dtype == v.dtype) or s.dtype != z.dtype:
-        raise TypeError(f"decode_step: phi_q, phi_k, v must share a dtype and so must s, z (got {phi_q.dtype}, {phi_k.dtype}, "
-                        f"{v.dtype}; {s.dtype}, {z.dtype})")
-    if out is None:
-        out = torch.empty(B, H, d, dtype=v.dtype, device=v.device)
-    elif out.dtype != v.dtype or not out.is_contiguous():
-        raise TypeError("decode_step: out must be contiguous and of v's dtype")
-    with _guard(v):
-        check(_lib.load().rfa_decode_step(ptr(phi_q), ptr(phi_k), ptr(v), dtype_code(v), ptr(s), ptr(z), dtype_code(s),
-                                          ptr(out), B * H, K, d, stream_of(v)), "rfa_decode_step")
-    return out
+    return native().decode_step(phi_q, phi_k, v, s, z, out)
 
 
 def decode_step_fused(q: Tensor, k: Tensor, v: Tensor, w: Tensor, scale: float, s: Tensor, z: Tensor,
                       out: Optional[Tensor] = None) -> Tensor:
     """One token from raw q,k [B,H,d]; w [H,D,d] fp32 contiguous; state updated IN PLACE."""
-    B, H, d = q.shape
-    D = w.shape[1]
-    q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-    if w.dtype != torch.float32 or not w.is_contiguous():
-        raise ValueError("decode_step_fused: w must be a contiguous fp32 [H,D,d] tensor")
-    if not (q.dtype == k.dtype == v.dtype) or s.dtype != z.dtype:
-        raise TypeError(f"decode_step_fused: q, k, v must share a dtype and so must s, z (got {q.dtype}, {k.dtype}, {v.dtype}; "
-                        f"{s.dtype}, {z.dtype})")
-    if not (s.is_contiguous() and z.is_contiguous()):
-        raise ValueError("decode_step_fused: state tensors must be contiguous (they are updated in place)")
-    if out is None:
-        out = torch.empty(B, H, d, dtype=v.dtype, device=v.device)
-    elif out.dtype != v.dtype or not out.is_contiguous():
-        raise TypeError("decode_step_fused: out must be contiguous and of v's dtype")
-    with _guard(v):
-        check(_lib.load().rfa_decode_step_fused(ptr(q), ptr(k), ptr(v), dtype_code(v), ptr(w), float(scale), ptr(s),
-                                                ptr(z), dtype_code(s), ptr(out), B * H, H, D, d, stream_of(v)),
-              "rfa_decode_step_fused")
-    return out
+    return native().decode_step_fused(q, k, v, w, scale, s, z, out)
 
 
 class CrossDecodeStates:
