@@ -53,6 +53,12 @@ int launch_cross_query_bwd_tc(const __half* q, const float* s, const float* z, c
 int launch_cross_state_bwd_tc(const __half* k, const __half* v, const uint8_t* pad_mask, const float* d_s, const float* d_z,
                               __half* gk, __half* gv, int64_t T, int BH, int H, cudaStream_t st);
 
+// sequences of one chunk with no state carried (causal_short.cu)
+int causal_short_max();
+int launch_causal_short_fwd(const __half* q, const __half* k, const __half* v, __half* out, float* den_out, int64_t T, int BH, cudaStream_t st);
+int launch_causal_short_bwd(const __half* q, const __half* k, const __half* v, const __half* g, const __half* out, const float* den, __half* gq,
+                            __half* gk, __half* gv, int64_t T, int BH, cudaStream_t st);
+
 // chunked tensor-core kernels for other geometries (generic_mma.cu)
 int generic_chunk(int K, int d, int* ctas);
 int launch_causal_chunked_fwd(const __half* q, const __half* k, const __half* v, __half* out, const float* s_seg, const float* z_seg,
@@ -325,6 +331,8 @@ extern "C" int rfa_causal_fwd_staged(const void* q, const void* k, const void* v
     s_seg = ws.s_seg;
     z_seg = ws.z_seg;
   }
+  if (is_tc(K, d) && T <= causal_short_max() && !s_in && !s_out)
+    return launch_causal_short_fwd((const __half*)q, (const __half*)k, (const __half*)v, (__half*)out, save_den ? ws.den : nullptr, T, BH, st);
   if (chunked)
     return launch_causal_chunked_fwd((const __half*)q, (const __half*)k, (const __half*)v, (__half*)out, s_seg, z_seg, s_out, z_out,
                                      save_den ? ws.den : nullptr, T, BH, p.nseg, p.tseg, K, d, st);
@@ -532,6 +540,18 @@ extern "C" int rfa_causal_bwd_saved(const void* q, const void* k, const void* v,
                                     void* gq, void* gk, void* gv, const float* s_in, const float* z_in,
                                     const float* ds_in, const float* dz_in, void* workspace, size_t workspace_bytes,
                                     int64_t T, int BH, int K, int d, int ws_has, rfa_stream_t stream) {
+  if (is_tc(K, d) && T > 0 && T <= causal_short_max() && !s_in && !z_in && !ds_in && !dz_in && (ws_has & RFA_WS_DEN)) {
+    if (int e = check_geometry("causal_bwd_saved", T, BH, K, d)) return e;
+    RFA_REQUIRE(q && k && v && g && out && gq && gk && gv, RFA_EINVAL, "causal_bwd_saved: null pointer");
+    RFA_REQUIRE(aligned16(q) && aligned16(k) && aligned16(v) && aligned16(g) && aligned16(out) && aligned16(gq) && aligned16(gk) && aligned16(gv),
+                RFA_EALIGN, "causal_bwd_saved: 16-byte alignment required");
+    RFA_REQUIRE((ws_has & ~(RFA_WS_STATES | RFA_WS_DEN)) == 0, RFA_EINVAL,
+                "causal_bwd_saved: ws_has may only name RFA_WS_STATES and RFA_WS_DEN (got %d)", ws_has);
+    CausalWs ws;
+    if (int e = check_ws("causal_bwd_saved", workspace, workspace_bytes, T, BH, K, d, plan_causal(T, BH), &ws)) return e;
+    return launch_causal_short_bwd((const __half*)q, (const __half*)k, (const __half*)v, (const __half*)g, (const __half*)out, ws.den, (__half*)gq,
+                                   (__half*)gk, (__half*)gv, T, BH, as_stream(stream));
+  }
   if (int e = rfa_causal_bwd_q_staged(q, k, v, g, out, gq, s_in, z_in, nullptr, workspace, workspace_bytes, T, BH, K, d, ws_has, stream))
     return e;
   return rfa_causal_bwd_kv(q, k, v, g, gk, gv, ds_in, dz_in, workspace, workspace_bytes, T, BH, K, d, stream);

@@ -1,0 +1,53 @@
+"""Sequences of one chunk on their own kernels (csrc/causal_short.cu): against the oracle, and against the general kernels, which
+the same call reaches when a state is asked for (forward) or the sweeps are called one by one (backward).
+
+Gates: the oracle's 2e-3 / 1e-2 of the other parity tests; between the two paths, whose operands are rounded alike and whose
+fp32 sums differ in order, a rounding of the fp16 result (2^-11 relative at worst) and of the operands that a sum's last
+bit tips: 6e-4 in the 2-norm."""
+import pytest
+import torch
+
+from conftest import assert_close
+from oracle import rfa_oracle as O
+from rfa_b200 import _lib, ops
+
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    return float((a.double() - b.double()).norm() / b.double().norm().clamp_min(1e-30))
+
+
+@pytest.mark.parametrize("scale", [0.3, 3.0])          # denominators in the clamp, and far out of it
+@pytest.mark.parametrize("T", [1, 2, 15, 16, 17, 33, 45, 64, 65, 100, 127, 128, 129])
+def test_short_sequences(dev, T, scale):
+    BH = 3
+    gen = torch.Generator().manual_seed(T)
+    q, k = ((torch.rand(T, BH, 128, generator=gen) * scale - 0.1).half() for _ in range(2))
+    v, g = (torch.randn(T, BH, 64, generator=gen).half() for _ in range(2))
+    f = [t.float() for t in (q, k, v)]
+    want, grads = O.causal_forward(*f), O.causal_backward(*f, g.float())
+    q, k, v, g = (t.to(dev) for t in (q, k, v, g))
+    out, ws, has = ops.causal_fwd_saved(q, k, v)
+    got = ops.causal_bwd_saved(q, k, v, g, out, ws, has)
+    rows = 1e-2 * max(1.0, float(want.abs().max()))
+    assert_close(out, want, "out", mabs=rows)
+    # one token out of the clamp has out = v whatever q and k are: its gq and gk are zero, two equal terms of g . out inv z (at most 64 * 16 *
+    # 3 / 100 = 30) whose fp16 operands differ by 2^-11 each: 3e-2, and nothing relative
+    zero = T == 1 and scale > 1
+    for name, a, b in zip(("gq", "gk", "gv"), got, grads):
+        if zero and name != "gv":
+            assert float(a.abs().max()) < 3e-2
+            continue
+        assert_close(a, b, name, mabs=1e-2 * max(1.0, float(b.abs().max())))
+    assert torch.equal(ops.causal_fwd(q, k, v), out)
+    # the general path on the same inputs and the same saved output
+    general, _, _ = ops.causal_fwd(q, k, v, return_state=True)
+    assert rel(out, general) < 6e-4
+    ws2 = ws.clone()
+    gq, _ = ops.causal_bwd_q_staged(q, k, v, g, out, None, None, ws2, _lib.WS_DEN, want_total=False)
+    gk, gv = ops.causal_bwd_kv(q, k, v, g, None, None, ws2)
+    for name, a, b in zip(("gq", "gk", "gv"), got, (gq, gk, gv)):
+        if zero and name != "gv":
+            continue
+        assert rel(a, b) < 6e-4, name
