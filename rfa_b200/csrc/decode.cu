@@ -5,7 +5,8 @@
 // exactly once with 16-byte (fp32) / 8-byte (fp16) accesses; a warp covers whole
 // 128-byte lines.  One CTA per (batch, head); HBM-bound: 2*K*d*sizeof(state)
 // bytes per head per token.
-#include "common.cuh"
+#define RFA_TC_FAMILY 9
+#include "tc_common.cuh"
 
 namespace rfa {
 
@@ -257,12 +258,185 @@ cross_decode_kernel(const TIn* __restrict__ phi_q, const float* const* __restric
   }
 }
 
+// ===========================================================================
+// The fused step for many heads (D = d = 64): a persistent CTA per SM streams its share of the states through shared memory.
+//
+// With one CTA per head, 7 of them on an SM load half of their state, compute features while nothing is in flight, load the
+// rest and store: 57 us for the 275 MB of 4096 fp32 heads (4.8 TB/s).  Here every head's state, z, q, k and v arrive by bulk
+// copies into one of six stages, two per group of 128 threads, so that a group's next head is on its way while it works
+// on one, and leave by a bulk store that its producer warp waits for before it refills the stage.  Heads are taken in order
+// of h, so that a thread's half row of W_h stays in registers from one head to the next.
+// ===========================================================================
+namespace dst {
+constexpr int kGroups = 3, kStages = 2, kThreads_ = kGroups * 128 + kGroups * 32;
+constexpr int kProj = 64;
+template <typename TIn, typename TState> struct Layout {
+  static constexpr uint32_t S = 0, Z = kK * kD * sizeof(TState), Q = Z + kK * sizeof(TState), Kv = Q + kD * sizeof(TIn), V = Kv + kD * sizeof(TIn),
+                            Bytes = V + kD * sizeof(TIn), Stage = (Bytes + 127) / 128 * 128;
+  // per group, fp32: xq, xk [64], pq, pk [128], acc [4][64], den [4]
+  static constexpr uint32_t Work = kGroups * kStages * Stage, WorkStride = (2 * 64 + 2 * 128 + 4 * 64 + 4) * 4;
+  static constexpr uint32_t Bar = Work + kGroups * WorkStride, Smem = Bar + kGroups * kStages * 2 * 8;
+};
+static_assert(Layout<float, float>::Smem <= 227 * 1024, "decode: shared memory");
+}  // namespace dst
+
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void bulk_store(void* dst, const void* src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(src)), "r"(bytes) : "memory");
+}
+// barrier of a group's 128 threads that also tells whether `ok` holds for all of them (so that they leave together)
+__device__ __forceinline__ bool group_sync_and(int grp, bool ok) {
+  uint32_t all;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %2, 0;\n\tbarrier.cta.red.and.pred q, %1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+               : "=r"(all) : "r"(grp + 1), "r"((uint32_t)ok) : "memory");
+  return all != 0;
+}
+__device__ __forceinline__ void group_sync(int grp) { asm volatile("bar.sync %0, 128;" ::"r"(grp + 1) : "memory"); }
+
+template <typename TIn, typename TState>
+__global__ void __launch_bounds__(dst::kThreads_, 1)
+decode_stream_fused_kernel(const TIn* __restrict__ q, const TIn* __restrict__ k, const TIn* __restrict__ v, const float* __restrict__ w,
+                           float scale, TState* __restrict__ S, TState* __restrict__ z, TIn* __restrict__ out, int BH, int H) {
+  using namespace dst;
+  using L = Layout<TIn, TState>;
+  extern __shared__ __align__(128) unsigned char ds_raw[];
+  uint64_t* full = reinterpret_cast<uint64_t*>(ds_raw + L::Bar);      // [group][stage]: a head has landed
+  uint64_t* done = full + kGroups * kStages;                          // [group][stage]: its new state is in the stage
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, B = BH / H;
+  const bool producer = warp >= kGroups * 4;
+  const int grp = producer ? warp - kGroups * 4 : warp >> 2;
+  const int first = (int)((int64_t)blockIdx.x * BH / gridDim.x), last = (int)((int64_t)(blockIdx.x + 1) * BH / gridDim.x);
+  const int n_items = (last - first - grp + kGroups - 1) / kGroups;   // items first + grp, + kGroups, ... (<= 0: none)
+  auto head = [&](int n) { const int i = first + grp + n * kGroups; return (size_t)(i % B) * H + i / B; };
+  auto stage = [&](int n) { return ds_raw + (grp * kStages + (n & 1)) * L::Stage; };
+  if (tid == 0) {
+    for (int i = 0; i < kGroups * kStages; ++i) { mbar_init(&full[i], 1); mbar_init(&done[i], 128); }
+    mbar_fence_init();
+  }
+  __syncthreads();
+  full += grp * kStages;
+  done += grp * kStages;
+
+  if (producer) {
+    if (lane == 0) {
+      auto load = [&](int n) {
+        if (n >= n_items) return;
+        const size_t bh = head(n);
+        unsigned char* st = stage(n);
+        uint64_t* bar = &full[n & 1];
+        mbar_arrive_expect_tx(bar, L::Bytes);
+        bulk_load(st + L::Q, q + bh * kD, kD * sizeof(TIn), bar);
+        bulk_load(st + L::Kv, k + bh * kD, kD * sizeof(TIn), bar);
+        bulk_load(st + L::V, v + bh * kD, kD * sizeof(TIn), bar);
+        bulk_load(st + L::S, S + bh * (kK * kD), kK * kD * sizeof(TState), bar);
+        bulk_load(st + L::Z, z + bh * kK, kK * sizeof(TState), bar);
+      };
+      load(0);
+      load(1);
+      for (int n = 0; n < n_items; ++n) {
+        if (!mbar_wait(&done[n & 1], (n >> 1) & 1)) { tc_fail(1); break; }
+        const size_t bh = head(n);
+        unsigned char* st = stage(n);
+        bulk_store(S + bh * (kK * kD), st + L::S, kK * kD * sizeof(TState));
+        bulk_store(z + bh * kK, st + L::Z, kK * sizeof(TState));
+        tma_store_commit();
+        if (n + 2 < n_items) tma_store_wait_read<0>();       // the stage has been read out
+        load(n + 2);
+      }
+      tma_store_wait<0>();
+    }
+    return;
+  }
+
+  float* work = reinterpret_cast<float*>(ds_raw + L::Work + grp * L::WorkStride);
+  float *xq = work, *xk = xq + 64, *pq = xk + 64, *pk = pq + 128, *red = pk + 128, *dens = red + 256;
+  const int gt = tid & 127, gw = gt >> 5, j = gt >> 1, half = gt & 1;
+  float4 wr[8];                      // half a row of W_h: columns 4 (2 i + half) .. + 3
+  int wh = -1;
+  for (int n = 0; n < n_items; ++n) {
+    const size_t bh = head(n);
+    unsigned char* st = stage(n);
+    const int h = (int)(bh % H);
+    if (h != wh) {
+      const float4* src = reinterpret_cast<const float4*>(w + ((size_t)h * kProj + j) * kD) + half;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) wr[i] = __ldg(src + 2 * i);
+      wh = h;
+    }
+    const bool ok = mbar_wait(&full[n & 1], (n >> 1) & 1);
+    if (!ok) tc_fail(2);
+    if (gw < 2) {                    // warp 0 normalises q, warp 1 k
+      const TIn* src = reinterpret_cast<const TIn*>(st + (gw == 0 ? L::Q : L::Kv));
+      const float a = to_f(src[lane]), b = to_f(src[lane + 32]);
+      const float inv = 1.f / (sqrtf(warp_sum(fmaf(a, a, b * b))) + kNormEps);
+      float* dst = gw == 0 ? xq : xk;
+      dst[lane] = a * inv;
+      dst[lane + 32] = b * inv;
+    }
+    if (!group_sync_and(grp, ok)) break;
+    float uq = 0.f, uk = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float4 a = load4(xq + 8 * i + 4 * half), b = load4(xk + 8 * i + 4 * half);
+      uq = fmaf(wr[i].x, a.x, uq); uq = fmaf(wr[i].y, a.y, uq); uq = fmaf(wr[i].z, a.z, uq); uq = fmaf(wr[i].w, a.w, uq);
+      uk = fmaf(wr[i].x, b.x, uk); uk = fmaf(wr[i].y, b.y, uk); uk = fmaf(wr[i].z, b.z, uk); uk = fmaf(wr[i].w, b.w, uk);
+    }
+    uq += __shfl_xor_sync(0xffffffffu, uq, 1);
+    uk += __shfl_xor_sync(0xffffffffu, uk, 1);
+    {
+      float sn, cs;
+      sincosf(half ? uk : uq, &sn, &cs);
+      float* dst = half ? pk : pq;   // features are handed over in the I/O precision, as the unfused path does
+      dst[j] = to_f(from_f<TIn>(scale * sn));
+      dst[kProj + j] = to_f(from_f<TIn>(scale * cs));
+    }
+    group_sync(grp);
+    {
+      TState* zs = reinterpret_cast<TState*>(st + L::Z);
+      const float zn = to_f(zs[gt]) + pk[gt];
+      zs[gt] = from_f<TState>(zn);
+      const float part = warp_sum(pq[gt] * zn);
+      if (lane == 0) dens[gw] = part;
+    }
+    const int c = gt & 15, r0 = gt >> 4;
+    const float4 v4 = load4(reinterpret_cast<const TIn*>(st + L::V) + 4 * c);
+    TState* Sc = reinterpret_cast<TState*>(st + L::S) + 4 * c;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int u = 0; u < kK / 8; ++u) {
+      const int kk = r0 + 8 * u;
+      const float a = pk[kk], b = pq[kk];
+      float4 t = load4(Sc + kk * kD);
+      t.x = fmaf(a, v4.x, t.x); t.y = fmaf(a, v4.y, t.y); t.z = fmaf(a, v4.z, t.z); t.w = fmaf(a, v4.w, t.w);
+      store4(Sc + kk * kD, t);
+      acc.x = fmaf(b, t.x, acc.x); acc.y = fmaf(b, t.y, acc.y); acc.z = fmaf(b, t.z, acc.z); acc.w = fmaf(b, t.w, acc.w);
+    }
+    fence_async_smem();              // the new state, before the bulk store reads it
+    mbar_arrive(&done[n & 1]);
+    acc.x += __shfl_xor_sync(0xffffffffu, acc.x, 16); acc.y += __shfl_xor_sync(0xffffffffu, acc.y, 16);
+    acc.z += __shfl_xor_sync(0xffffffffu, acc.z, 16); acc.w += __shfl_xor_sync(0xffffffffu, acc.w, 16);
+    if (lane < 16) store4(red + gw * 64 + 4 * c, acc);
+    group_sync(grp);
+    if (gt < 16) {
+      const float4 a = load4(red + 4 * gt), b = load4(red + 64 + 4 * gt), e = load4(red + 128 + 4 * gt), f = load4(red + 192 + 4 * gt);
+      const float inv = 1.f / fmaxf((dens[0] + dens[1]) + (dens[2] + dens[3]), kEps);
+      store4(out + bh * kD + 4 * gt, make_float4(((a.x + b.x) + (e.x + f.x)) * inv, ((a.y + b.y) + (e.y + f.y)) * inv,
+                                                 ((a.z + b.z) + (e.z + f.z)) * inv, ((a.w + b.w) + (e.w + f.w)) * inv));
+    }
+  }
+}
+
 static int check_decode_dtypes(const char* what, int in_dtype, int state_dtype) {
   const bool ok = (in_dtype == RFA_F16 && (state_dtype == RFA_F32 || state_dtype == RFA_F16)) ||
                   (in_dtype == RFA_F32 && state_dtype == RFA_F32);
   RFA_REQUIRE(ok, RFA_EUNSUPPORTED, "%s: unsupported dtype pair in=%d state=%d", what, in_dtype, state_dtype);
   return 0;
 }
+
+constexpr int kStreamMinHeads = 7 * 148;
 
 static int check_decode_geometry(int BH, int K, int d) {
   RFA_REQUIRE(BH > 0 && K > 0 && d > 0, RFA_EINVAL, "decode: BH=%d K=%d d=%d must be positive", BH, K, d);
@@ -313,6 +487,25 @@ extern "C" int rfa_decode_step_fused(const void* q, const void* k, const void* v
   const int K = 2 * D;
   const size_t smem = kDecodeThreads * sizeof(float4) + (2 * K + 3 * d + 4 + 2 * D) * sizeof(float);
   cudaStream_t st = as_stream(stream);
+  // more heads than one wave of one-head CTAs (7 on each of 148 SMs) and the width it is built for: the streaming kernel.
+  if (D == dst::kProj && d == kD && BH % H == 0 && BH > kStreamMinHeads) {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+#define RFA_LAUNCH(TI, TS)                                                                                                       \
+  do {                                                                                                                           \
+    const cudaError_t e = cudaFuncSetAttribute(decode_stream_fused_kernel<TI, TS>, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
+                                               (int)dst::Layout<TI, TS>::Smem);                                                  \
+    if (e != cudaSuccess) return fail((int)e, "decode_fused: cannot reserve shared memory: %s", cudaGetErrorString(e));          \
+    decode_stream_fused_kernel<TI, TS><<<sms, dst::kThreads_, dst::Layout<TI, TS>::Smem, st>>>(                                  \
+        (const TI*)q, (const TI*)k, (const TI*)v, w, scale, (TS*)s, (TS*)z, (TI*)out, BH, H);                                    \
+  } while (0)
+    if (in_dtype == RFA_F16 && state_dtype == RFA_F32) RFA_LAUNCH(__half, float);
+    else if (in_dtype == RFA_F16) RFA_LAUNCH(__half, __half);
+    else RFA_LAUNCH(float, float);
+#undef RFA_LAUNCH
+    return check_launch("rfa_decode_step_fused (streaming)");
+  }
 #define RFA_LAUNCH(TI, TS)                                                                        \
   decode_step_fused_kernel<TI, TS><<<BH, kDecodeThreads, smem, st>>>(                             \
       (const TI*)q, (const TI*)k, (const TI*)v, w, scale, (TS*)s, (TS*)z, (TI*)out, H, D, d)
@@ -339,3 +532,7 @@ extern "C" int rfa_cross_decode_step(const void* phi_q, int in_dtype, const floa
     cross_decode_kernel<float><<<grid, kDecodeThreads, smem, as_stream(stream)>>>((const float*)phi_q, s_ptrs, z_ptrs, (float*)out, BH, K, d);
   return check_launch("rfa_cross_decode_step");
 }
+
+namespace rfa {
+RFA_TC_UNIT(decode)
+}  // namespace rfa

@@ -51,3 +51,20 @@ def test_short_sequences(dev, T, scale):
         if zero and name != "gv":
             continue
         assert rel(a, b) < 6e-4, name
+
+
+@pytest.mark.parametrize("state_dtype,in_dtype", [(torch.float32, torch.float16), (torch.float16, torch.float16), (torch.float32, torch.float32)])
+@pytest.mark.parametrize("B,H", [(130, 8), (41, 27)])          # just over one wave of the one-head-per-CTA kernel; heads that split unevenly
+def test_decode_of_many_heads(dev, state_dtype, in_dtype, B, H):
+    """The streaming kernel against the general one, which the same call reaches for half of the batch at a time.  A projection
+    summed in another order may round a feature to the neighbouring fp16 number (2^-11): 1e-3."""
+    gen = torch.Generator().manual_seed(B)
+    rnd = lambda *s: torch.randn(*s, generator=gen).to(dev)
+    w, (q, k, v) = rnd(H, 64, 64), (rnd(B, H, 64).to(in_dtype) for _ in range(3))
+    s, z = (rnd(B, H, 128, 64) * 0.1).to(state_dtype), (rnd(B, H, 128) * 0.1 + 1.0).to(state_dtype)
+    s1, z1, s2, z2 = s.clone(), z.clone(), s.clone(), z.clone()
+    outs = [ops.decode_step_fused(q, k, v, w, 0.1, s1, z1) for _ in range(2)]
+    for i in range(2):
+        halves = [ops.decode_step_fused(q[a], k[a], v[a], w, 0.1, s2[a], z2[a]) for a in (slice(0, B // 2), slice(B // 2, B))]
+        assert rel(outs[i], torch.cat(halves)) < 1e-3
+    assert rel(s1, s2) < 1e-3 and rel(z1, z2) < 1e-3
