@@ -34,7 +34,7 @@ int launch_causal_fwd_fused_tc(const __half* xq, const __half* xk, const __half*
 // forward-direction sweep from the forward's saved output and raw denominators (causal_bwd_q_saved_tc.cu)
 int launch_causal_bwd_q_saved_tc(const __half* q, const __half* k, const __half* v, const __half* g, const __half* out,
                                  const float* den_raw, __half* gq, const float* s_seg, const float* z_seg, float* ws_gz,
-                                 float* ds_seg, float* dz_seg, int64_t T, int BH, int nseg, int64_t tseg, cudaStream_t st);
+                                 float* ds_seg, float* dz_seg, int first_dseg, int64_t T, int BH, int nseg, int64_t tseg, cudaStream_t st);
 // tensor-core backward, forward-direction sweep (causal_bwd_tc.cu)
 int launch_causal_bwd_q_tc(const __half* q, const __half* k, const __half* v, const __half* g, __half* gq,
                            const float* s_seg, const float* z_seg, float* ws_den, float* ws_gz, float* ds_seg,
@@ -46,7 +46,7 @@ int launch_causal_bwd_kv_tc(const __half* q, const __half* k, const __half* v, c
 
 // tensor-core state reduction and cross-attention kernels (cross_tc.cu)
 int launch_cross_state_fwd_tc(const __half* k, const __half* v, const uint8_t* pad_mask, float* s, float* z, int64_t T, int BH,
-                              int H, int nseg, int64_t tseg, cudaStream_t st);
+                              int H, int nseg, int64_t tseg, int runs, cudaStream_t st);
 int launch_cross_query_fwd_tc(const __half* q, const float* s, const float* z, __half* out, int64_t T, int BH, cudaStream_t st);
 int launch_cross_query_bwd_tc(const __half* q, const float* s, const float* z, const __half* g, __half* gq, float* d_s, float* d_z,
                               int64_t T, int BH, cudaStream_t st);
@@ -71,7 +71,7 @@ int launch_causal_chunked_bwd_kv(const __half* q, const __half* k, const __half*
                                  const float* ws_den, const float* ws_gz, const float* ds_seg, const float* dz_seg, int64_t T, int BH,
                                  int nseg, int64_t tseg, int K, int d, cudaStream_t st);
 int launch_state_chunked(const __half* x, const __half* y, const uint8_t* pad_mask, const float* ws_den, const float* ws_gz, float* s,
-                         float* z, int64_t T, int BH, int H, int nseg, int64_t tseg, int K, int d, cudaStream_t st);
+                         float* z, int64_t T, int BH, int H, int nseg, int64_t tseg, int runs, int K, int d, cudaStream_t st);
 
 // CUDA-core kernels for the geometries neither of them takes (generic.cu)
 bool generic_geometry_ok(int K, int d, bool two_states);
@@ -182,12 +182,12 @@ scan_states_kernel(float* __restrict__ s_seg, float* __restrict__ z_seg, const f
     float4 t[kScanBatch];
 #pragma unroll
     for (int u = 0; u < kScanBatch; ++u)
-      if (j0 + u < nseg) t[u] = base[(size_t)(reverse ? nseg - 1 - (j0 + u) : j0 + u) * width];
+      if (j0 + u < nseg - 1) t[u] = base[(size_t)(reverse ? nseg - 1 - (j0 + u) : j0 + u) * width];
 #pragma unroll
     for (int u = 0; u < kScanBatch; ++u)
       if (j0 + u < nseg) {
         base[(size_t)(reverse ? nseg - 1 - (j0 + u) : j0 + u) * width] = run;
-        run.x += t[u].x; run.y += t[u].y; run.z += t[u].z; run.w += t[u].w;
+        if (j0 + u < nseg - 1) { run.x += t[u].x; run.y += t[u].y; run.z += t[u].z; run.w += t[u].w; }   // the last one's sum enters nothing
       }
   }
 }
@@ -258,11 +258,12 @@ static int total_launch(const float* s_seg, const float* z_seg, float* packed, f
   return check_launch("total_states");
 }
 
-// Per-segment sums of k (x) v and k -> ws.s_seg / ws.z_seg (one CTA per (batch, head, segment)).
+// Per-segment sums of k (x) v and k -> ws.s_seg / ws.z_seg (one CTA per (batch, head, segment)), of the first `runs` segments:
+// no state enters a segment from the last one on, so that only a total needs all of them.
 static int segment_partials(const __half* k, const __half* v, const CausalWs& ws, const CausalPlan& p, int64_t T, int BH, int K, int d,
-                            cudaStream_t st) {
-  if (!is_tc(K, d)) return launch_state_chunked(k, v, nullptr, nullptr, nullptr, ws.s_seg, ws.z_seg, T, BH, 1, p.nseg, p.tseg, K, d, st);
-  return launch_cross_state_fwd_tc(k, v, nullptr, ws.s_seg, ws.z_seg, T, BH, 1, p.nseg, p.tseg, st);
+                            int runs, cudaStream_t st) {
+  if (!is_tc(K, d)) return launch_state_chunked(k, v, nullptr, nullptr, nullptr, ws.s_seg, ws.z_seg, T, BH, 1, p.nseg, p.tseg, runs, K, d, st);
+  return launch_cross_state_fwd_tc(k, v, nullptr, ws.s_seg, ws.z_seg, T, BH, 1, p.nseg, p.tseg, runs, st);
 }
 
 static int check_ws(const char* what, void* workspace, size_t bytes, int64_t T, int BH, int K, int d, const CausalPlan& p, CausalWs* out) {
@@ -326,7 +327,7 @@ extern "C" int rfa_causal_fwd_staged(const void* q, const void* k, const void* v
     if (int e = check_ws("causal_fwd", workspace, workspace_bytes, T, BH, K, d, p, &ws)) return e;
   if (p.nseg > 1) {
     if (!(ws_has & RFA_WS_PARTIALS) || chunked)      // (rfa_causal_shard_total, which leaves them, is not built for these)
-      if (int e = segment_partials((const __half*)k, (const __half*)v, ws, p, T, BH, K, d, st)) return e;
+      if (int e = segment_partials((const __half*)k, (const __half*)v, ws, p, T, BH, K, d, p.nseg - 1, st)) return e;
     if (int e = scan_launch(ws.s_seg, ws.z_seg, s_in, z_in, BH, p.nseg, 0, K, d, st)) return e;
     s_seg = ws.s_seg;
     z_seg = ws.z_seg;
@@ -399,7 +400,7 @@ extern "C" int rfa_causal_shard_total(const void* k, const void* v, float* total
   const CausalPlan p = plan_causal(T, BH);
   CausalWs ws;
   if (int e = check_ws("causal_shard_total", workspace, workspace_bytes, T, BH, K, d, p, &ws)) return e;
-  if (int e = segment_partials((const __half*)k, (const __half*)v, ws, p, T, BH, K, d, st)) return e;
+  if (int e = segment_partials((const __half*)k, (const __half*)v, ws, p, T, BH, K, d, p.nseg, st)) return e;
   return total_launch(ws.s_seg, ws.z_seg, total_packed, nullptr, nullptr, BH, p.nseg, K, d, st);
 }
 
@@ -447,7 +448,7 @@ static int bwd_q_impl(const void* q, const void* k, const void* v, const void* g
   const float *s_seg = s_in, *z_seg = z_in;
   if (p.nseg > 1) {
     if (!(ws_has & RFA_WS_STATES)) {    // the states entering each segment: partial sums, then an exclusive scan
-      if (int e = segment_partials((const __half*)k, (const __half*)v, ws, p, T, BH, K, d, st)) return e;
+      if (int e = segment_partials((const __half*)k, (const __half*)v, ws, p, T, BH, K, d, p.nseg - 1, st)) return e;
       if (int e = scan_launch(ws.s_seg, ws.z_seg, s_in, z_in, BH, p.nseg, 0, K, d, st)) return e;
     }
     s_seg = ws.s_seg;
@@ -460,13 +461,13 @@ static int bwd_q_impl(const void* q, const void* k, const void* v, const void* g
       return e;
     if (want_dseg)
       if (int e = launch_state_chunked((const __half*)q, (const __half*)g, nullptr, ws.den, ws.gz, ws.ds_seg, ws.dz_seg, T, BH, 1, p.nseg,
-                                       p.tseg, K, d, st))
+                                       p.tseg, p.nseg, K, d, st))
         return e;
   } else if (ws_has & RFA_WS_DEN) {
     if (int e = launch_causal_bwd_q_saved_tc((const __half*)q, (const __half*)k, (const __half*)v, (const __half*)g,
                                              (const __half*)out, ws.den, (__half*)gq, s_seg, z_seg, ws.gz,
-                                             want_dseg ? ws.ds_seg : nullptr, want_dseg ? ws.dz_seg : nullptr, T, BH, p.nseg,
-                                             p.tseg, st))
+                                             want_dseg ? ws.ds_seg : nullptr, want_dseg ? ws.dz_seg : nullptr, want_tot ? 0 : 1, T, BH,
+                                             p.nseg, p.tseg, st))
       return e;
   } else {
     if (int e = launch_causal_bwd_q_tc((const __half*)q, (const __half*)k, (const __half*)v, (const __half*)g,
@@ -571,11 +572,11 @@ extern "C" int rfa_cross_state_fwd(const void* phi_k, const void* v, const uint8
     return check_launch("rfa_cross_state_fwd(T=0)");
   }
   if (is_chunked(K, d))
-    return launch_state_chunked((const __half*)phi_k, (const __half*)v, pad_mask, nullptr, nullptr, s, z, T, BH, H, 1, T, K, d, as_stream(stream));
+    return launch_state_chunked((const __half*)phi_k, (const __half*)v, pad_mask, nullptr, nullptr, s, z, T, BH, H, 1, T, 1, K, d, as_stream(stream));
   if (!is_tc(K, d))
     return launch_state_generic_fwd((const __half*)phi_k, (const __half*)v, pad_mask, s, z, T, BH, H, 1, T, K, d, as_stream(stream));
   const int64_t tseg = ((T + kSegAlign - 1) / kSegAlign) * kSegAlign;
-  return launch_cross_state_fwd_tc((const __half*)phi_k, (const __half*)v, pad_mask, s, z, T, BH, H, 1, tseg, as_stream(stream));
+  return launch_cross_state_fwd_tc((const __half*)phi_k, (const __half*)v, pad_mask, s, z, T, BH, H, 1, tseg, 1, as_stream(stream));
 }
 
 extern "C" int64_t rfa_state_partials_run_length(int64_t T, int nseg) {
@@ -598,12 +599,12 @@ extern "C" int rfa_state_partials(const void* phi_k, const void* v, float* s_par
   }
   if (is_chunked(K, d))
     return launch_state_chunked((const __half*)phi_k, (const __half*)v, nullptr, nullptr, nullptr, s_part, z_part, T, BH, 1, nseg,
-                                rfa_state_partials_run_length(T, nseg), K, d, as_stream(stream));
+                                rfa_state_partials_run_length(T, nseg), nseg, K, d, as_stream(stream));
   if (!is_tc(K, d))
     return launch_state_generic_fwd((const __half*)phi_k, (const __half*)v, nullptr, s_part, z_part, T, BH, 1, nseg,
                                     rfa_state_partials_run_length(T, nseg), K, d, as_stream(stream));
   return launch_cross_state_fwd_tc((const __half*)phi_k, (const __half*)v, nullptr, s_part, z_part, T, BH, 1, nseg,
-                                   rfa_state_partials_run_length(T, nseg), as_stream(stream));
+                                   rfa_state_partials_run_length(T, nseg), nseg, as_stream(stream));
 }
 
 extern "C" int rfa_cross_state_bwd(const void* phi_k, const void* v, const uint8_t* pad_mask, const float* d_s,

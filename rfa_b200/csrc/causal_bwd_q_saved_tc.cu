@@ -51,7 +51,7 @@ causal_bwd_q_saved_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __g
                              const __half* __restrict__ out_ptr, const float* __restrict__ den_raw,
                              __half* __restrict__ gq_ptr,
                              const float* __restrict__ s_seg, const float* __restrict__ z_seg,
-                             float* __restrict__ ws_gz, float* __restrict__ ds_seg, float* __restrict__ dz_seg,
+                             float* __restrict__ ws_gz, float* __restrict__ ds_seg, float* __restrict__ dz_seg, int first_dseg,
                              int64_t T, int BH, int nseg, int64_t tseg) {
   using L = BsLayout<WANT_DSEG>;
   extern __shared__ __align__(1024) unsigned char bs_raw[];
@@ -70,6 +70,7 @@ causal_bwd_q_saved_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __g
   const int64_t t_begin = seg * tseg, t_end = min(T, t_begin + tseg);
   const int nchunk = (int)((t_end - t_begin + kTC - 1) / kTC);
   const size_t slot = (size_t)bh * nseg + seg;
+  const bool dseg = WANT_DSEG && seg >= first_dseg;     // this segment's reverse total is wanted: q is read
   const float* s_in = s_seg ? s_seg + slot * kK * kD : nullptr;
   const float* z_in = z_seg ? z_seg + slot * kK : nullptr;
 
@@ -116,10 +117,10 @@ causal_bwd_q_saved_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __g
         mbar_arrive_expect_tx(fv, 2 * kBox);
         tma_load_3d(base + L::G, &tm_g, fv, 0, bh, t0);
         tma_load_3d(base + L::V, &tm_v, fv, 0, bh, t0);
-        mbar_arrive_expect_tx(fk, (WANT_DSEG ? 4 : 2) * kBox);
+        mbar_arrive_expect_tx(fk, (dseg ? 4 : 2) * kBox);
         tma_load_3d(base + L::K, &tm_k, fk, 0, bh, t0);
         tma_load_3d(base + L::K + kBox, &tm_k, fk, 64, bh, t0);
-        if (WANT_DSEG) {
+        if (dseg) {
           tma_load_3d(base + L::Q, &tm_q, fk, 0, bh, t0);
           tma_load_3d(base + L::Q + kBox, &tm_q, fk, 64, bh, t0);
         }
@@ -173,7 +174,7 @@ causal_bwd_q_saved_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __g
         if (c > 0 && !mbar_wait(&bars[sDQFree], (c - 1) & 1)) { tc_fail(5); break; }
         tc_fence_after_sync();
         umma_chain_ss<4, kStepK, kBlockK, kStepK, kBlockK>(lead, tmem + bsColDQ, dGk + so, dSk + st * kTile, idKK, 0);     // dQ = gs S_prev^T
-        if (WANT_DSEG)                                                                      // dSseg += Q^T gs
+        if (dseg)                                                                           // dSseg += Q^T gs
           umma_chain_ss<8, kStepMN, kBlockMN, kStepMN, kBlockMN>(lead, tmem + bsColDS, dQm + so, dGm + so, idMM64, c > 0 ? 1u : 0u);
         if (!mbar_wait(&bars[sDA16 + st], (c >> 1) & 1)) { tc_fail(6); break; }
         tc_fence_after_sync();
@@ -251,11 +252,11 @@ causal_bwd_q_saved_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __g
       if (WANT_DSEG) {                             // dzseg += Q^T gz: needs every row's gz and the staged Q tile
         if (!mbar_wait(&bars[sG + st], (c >> 1) & 1)) { tc_fail(11); break; }
         if (!mbar_wait(&bars[sFullK + st], (c >> 1) & 1)) { tc_fail(12); break; }
-        dz_acc += column_sum2(sm + st * L::Stage + L::Q, quarter, lane, rg_buf + st * 128);
+        if (dseg) dz_acc += column_sum2(sm + st * L::Stage + L::Q, quarter, lane, rg_buf + st * 128);
         mbar_arrive(&bars[sEmpty + st]);
       }
     }
-    if (WANT_DSEG) dz_seg[slot * kK + row] = dz_acc;       // (zero when the run has no tokens)
+    if (dseg) dz_seg[slot * kK + row] = dz_acc;       // (zero when the run has no tokens)
   } else if (warp >= 10) {
     // ------------------------------------------------------------------ pack/state group: dA -> masked fp16; z, S export
     const int quarter = warp & 3;
@@ -411,7 +412,7 @@ causal_bwd_q_saved_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __g
         }
       }
     }
-    if (ok && WANT_DSEG) {
+    if (ok && dseg) {
       uint32_t r[64];
       if (nchunk > 0) {
         tmem_ld32(tmem + lane_addr + bsColDS, r);      // the wait on sDQ of the last chunk ordered the last dSseg product
@@ -436,10 +437,11 @@ causal_bwd_q_saved_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __g
 
 // ---------------------------------------------------------------------------
 // out [T][BH][d] and den_raw [BH][T] are the forward's saved results; ds_seg / dz_seg non-null = also write each segment's
-// reverse-state total (then q is read).
+// reverse-state total (then q is read), from segment first_dseg on: no reverse state enters a segment from the first one, so
+// that only the whole run's total needs that.  (32 heads x 131072 tokens in four segments: a quarter of q's 1.07 GB.)
 int launch_causal_bwd_q_saved_tc(const __half* q, const __half* k, const __half* v, const __half* g, const __half* out,
                                  const float* den_raw, __half* gq, const float* s_seg, const float* z_seg, float* ws_gz,
-                                 float* ds_seg, float* dz_seg, int64_t T, int BH, int nseg, int64_t tseg, cudaStream_t st) {
+                                 float* ds_seg, float* dz_seg, int first_dseg, int64_t T, int BH, int nseg, int64_t tseg, cudaStream_t st) {
   const bool want = ds_seg != nullptr;
   CUtensorMap tq, tk, tv, tg, tgq;
   if (make_tmap_rows(&tq, want ? q : k, T, BH, kK, kTC) || make_tmap_rows(&tk, k, T, BH, kK, kTC) ||
@@ -452,13 +454,13 @@ int launch_causal_bwd_q_saved_tc(const __half* q, const __half* k, const __half*
     e = cudaFuncSetAttribute(causal_bwd_q_saved_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return fail((int)e, "causal_bwd_q_saved: cannot reserve %u bytes of shared memory: %s", smem, cudaGetErrorString(e));
     launch_pdl(causal_bwd_q_saved_tc_kernel<true>, dim3(BH, nseg), dim3(kBsThreads), smem, st, tq, tk, tv, tg, tgq, out, den_raw, gq, s_seg, z_seg,
-               ws_gz, ds_seg, dz_seg, T, BH, nseg, tseg);
+               ws_gz, ds_seg, dz_seg, first_dseg, T, BH, nseg, tseg);
   } else {
     constexpr uint32_t smem = BsLayout<false>::Smem;
     e = cudaFuncSetAttribute(causal_bwd_q_saved_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return fail((int)e, "causal_bwd_q_saved: cannot reserve %u bytes of shared memory: %s", smem, cudaGetErrorString(e));
     launch_pdl(causal_bwd_q_saved_tc_kernel<false>, dim3(BH, nseg), dim3(kBsThreads), smem, st, tq, tk, tv, tg, tgq, out, den_raw, gq, s_seg, z_seg,
-               ws_gz, ds_seg, dz_seg, T, BH, nseg, tseg);
+               ws_gz, ds_seg, dz_seg, first_dseg, T, BH, nseg, tseg);
   }
   return check_launch("rfa_causal_bwd_q_saved");
 }

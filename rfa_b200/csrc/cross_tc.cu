@@ -603,8 +603,9 @@ static int x_opt_in(Kern kern, uint32_t bytes, const char* what) {
   return 0;
 }
 
+// runs: how many of the nseg runs of tokens to reduce, from the first
 int launch_cross_state_fwd_tc(const __half* k, const __half* v, const uint8_t* pad_mask, float* s, float* z, int64_t T, int BH,
-                              int H, int nseg, int64_t tseg, cudaStream_t st) {
+                              int H, int nseg, int64_t tseg, int runs, cudaStream_t st) {
   CUtensorMap tk, tv;
   const int r1 = make_tmap_rows(&tk, k, T, BH, kK, kTC), r2 = make_tmap_rows(&tv, v, T, BH, kD, kTC);
   if (r1 || r2)
@@ -613,12 +614,12 @@ int launch_cross_state_fwd_tc(const __half* k, const __half* v, const uint8_t* p
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if ((int64_t)BH * nseg > sms) {            // more CTAs than SMs: two per SM, two stages each
+  if ((int64_t)BH * runs > sms) {            // more CTAs than SMs: two per SM, two stages each
     if (int e = x_opt_in(cross_state_fwd_tc_kernel<2>, xs::L<2>::kSmem, "cross_state_fwd")) return e;
-    launch_pdl(cross_state_fwd_tc_kernel<2>, dim3(BH, nseg), kXThreads, xs::L<2>::kSmem, st, tk, tv, pad_mask, s, z, T, BH, H, nseg, tseg);
+    launch_pdl(cross_state_fwd_tc_kernel<2>, dim3(BH, runs), kXThreads, xs::L<2>::kSmem, st, tk, tv, pad_mask, s, z, T, BH, H, nseg, tseg);
   } else {
     if (int e = x_opt_in(cross_state_fwd_tc_kernel<4>, xs::L<4>::kSmem, "cross_state_fwd")) return e;
-    launch_pdl(cross_state_fwd_tc_kernel<4>, dim3(BH, nseg), kXThreads, xs::L<4>::kSmem, st, tk, tv, pad_mask, s, z, T, BH, H, nseg, tseg);
+    launch_pdl(cross_state_fwd_tc_kernel<4>, dim3(BH, runs), kXThreads, xs::L<4>::kSmem, st, tk, tv, pad_mask, s, z, T, BH, H, nseg, tseg);
   }
   return check_launch("rfa_cross_state_fwd");
 }

@@ -630,17 +630,17 @@ gm_causal_bwd_kv_kernel(const __half* __restrict__ q, const __half* __restrict__
 
 // ===========================================================================================================================
 // state reduction over runs of tokens: sum x (x) y, sum x (padded keys left out), or with ws_den / ws_gz the reverse one,
-// sum x (x) (inv y), sum gz x.  grid (BH, nseg)
+// sum x (x) (inv y), sum gz x.  grid (BH, runs <= nseg)
 // ===========================================================================================================================
 template <int C, int STAGES, bool WEIGHTED>
 __global__ void __launch_bounds__(kGmThreads)
 gm_state_kernel(const __half* __restrict__ x, const __half* __restrict__ y, const uint8_t* __restrict__ pad_mask,
                 const float* __restrict__ ws_den, const float* __restrict__ ws_gz, float* __restrict__ s_out, float* __restrict__ z_out,
-                int64_t T, int BH, int H, int64_t tseg, int K, int d) {
+                int64_t T, int BH, int H, int nseg, int64_t tseg, int K, int d) {
   extern __shared__ __align__(16) unsigned char gm_raw[];
   const GmLayout L = gm_layout(C, K, d, STAGES, 1, 1, 0, kGmRowsState);
   float *S = (float*)(gm_raw + L.S), *z = (float*)(gm_raw + L.z), *inv = (float*)(gm_raw + L.row), *gz = inv + C;
-  const int bh = blockIdx.x, seg = blockIdx.y, nseg = gridDim.y;
+  const int bh = blockIdx.x, seg = blockIdx.y;
   const int64_t t_begin = seg * tseg, t_end = min(T, t_begin + tseg);
   const int nchunk = t_end > t_begin ? (int)((t_end - t_begin + C - 1) / C) : 0;
   const size_t slot = (size_t)bh * nseg + seg;
@@ -747,14 +747,14 @@ int launch_causal_chunked_bwd_kv(const __half* q, const __half* k, const __half*
 #undef RFA_GM_CALL
 }
 
-// ws_den / ws_gz null: sums of k (x) v and k; else of q (x) (g / den) and gz q
+// the first `runs` of nseg runs of tokens; ws_den / ws_gz null: sums of k (x) v and k; else of q (x) (g / den) and gz q
 int launch_state_chunked(const __half* x, const __half* y, const uint8_t* pad_mask, const float* ws_den, const float* ws_gz, float* s,
-                         float* z, int64_t T, int BH, int H, int nseg, int64_t tseg, int K, int d, cudaStream_t st) {
+                         float* z, int64_t T, int BH, int H, int nseg, int64_t tseg, int runs, int K, int d, cudaStream_t st) {
 #define RFA_GM_CALL(C, N)                                                                                                             \
   return ws_den ? gm_launch(gm_state_kernel<C, N, true>, "state reduction (chunked)", gm_layout(C, K, d, N, 1, 1, 0, kGmRowsState).total, \
-                            dim3(BH, nseg), st, x, y, pad_mask, ws_den, ws_gz, s, z, T, BH, H, tseg, K, d)                             \
+                            dim3(BH, runs), st, x, y, pad_mask, ws_den, ws_gz, s, z, T, BH, H, nseg, tseg, K, d)                             \
                 : gm_launch(gm_state_kernel<C, N, false>, "state reduction (chunked)", gm_layout(C, K, d, N, 1, 1, 0, kGmRowsState).total, \
-                            dim3(BH, nseg), st, x, y, pad_mask, ws_den, ws_gz, s, z, T, BH, H, tseg, K, d)
+                            dim3(BH, runs), st, x, y, pad_mask, ws_den, ws_gz, s, z, T, BH, H, nseg, tseg, K, d)
   RFA_GM_DISPATCH(gm_shape(K, d), RFA_GM_CALL);
 #undef RFA_GM_CALL
 }
