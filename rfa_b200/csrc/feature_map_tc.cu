@@ -15,7 +15,9 @@ constexpr uint32_t kX = 0, kStage = kBox, kW = 2 * kStage, kOut = kW + 8192, kBa
 enum { bFull = 0, bEmpty = 2, bU = 4, bUFree = 6, bEpi = 8, bNum = 9 };
 }
 
-__global__ void __launch_bounds__(fm::kThreads_, 2)
+// Three CTAs per SM (73 KB and 96 registers a thread): a tile's chain -- load, product, sines, store -- is latency, and twelve
+// epilogue warps hide more of it than eight.
+__global__ void __launch_bounds__(fm::kThreads_, 3)
 feature_map_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_phi,
                           const __grid_constant__ CUtensorMap tm_x2, const __grid_constant__ CUtensorMap tm_phi2,
                           const float* __restrict__ w, const uint8_t* __restrict__ row_mask, const uint8_t* __restrict__ row_mask2,
@@ -41,14 +43,20 @@ feature_map_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid
     for (int i = 0; i < 2; ++i) { mbar_init(&bars[bFull + i], 1); mbar_init(&bars[bEmpty + i], 129); mbar_init(&bars[bU + i], 1); mbar_init(&bars[bUFree + i], 128); }
     mbar_init(&bars[bEpi], 128);
     mbar_fence_init();
-    // the first tiles are requested before the rest of the prologue (W_h, tensor memory), which their flight then hides
+    tma_prefetch_desc(&tm_x); tma_prefetch_desc(&tm_phi);
+  }
+  if (warp == 1) { tmem_alloc(tmem_slot, 128); tmem_relinquish(); }
+  __syncthreads();              // tensor memory is allocated before the next kernel's CTAs may ask for theirs
+  pdl_wait();                   // everything above may overlap the tail of the previous kernel in the stream
+  pdl_launch_dependents();
+  if (tid == 0) {
+    // the first tiles are requested before W_h is read and converted, which their flight then hides
     for (int i = 0; i < 2 && i < ntile; ++i) {
       int which;
       const int row0 = tile_row0(i, which);
       mbar_arrive_expect_tx(&bars[bFull + i], kBox);
       tma_load_3d(sm + kX + i * kStage, which ? &tm_x2 : &tm_x, &bars[bFull + i], 0, h, row0);
     }
-    tma_prefetch_desc(&tm_phi);
   }
   // W_h as an fp16 K-major operand tile [64 rows j][64 i]
   for (int i = tid; i < 64 * 8; i += kThreads_) {
@@ -60,7 +68,6 @@ feature_map_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid
     *reinterpret_cast<uint4*>(sm + kW + row_chunk1(j, ch)) = u;
   }
   fence_async_smem();
-  if (warp == 1) { tmem_alloc(tmem_slot, 128); tmem_relinquish(); }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -171,11 +178,11 @@ int launch_feature_map_fwd_tc(const __half* x, const float* w, const uint8_t* ro
   cudaError_t e = cudaFuncSetAttribute(feature_map_fwd_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fm::kSmem);
   if (e != cudaSuccess) return fail((int)e, "feature_map_fwd: cannot reserve %u bytes of shared memory: %s", fm::kSmem, cudaGetErrorString(e));
   const int64_t ntile = (rows + kTC - 1) / kTC * (pair ? 2 : 1);
-  int64_t gx = 2LL * sms / H;                    // two CTAs per SM, and never more CTAs than fit at once
+  int64_t gx = 3LL * sms / H;                    // three CTAs per SM, and never more CTAs than fit at once
   if (gx > ntile) gx = ntile;
   if (gx < 1) gx = 1;
-  feature_map_fwd_tc_kernel<<<dim3((unsigned)gx, H), fm::kThreads_, fm::kSmem, st>>>(tx, tp, tx2, tp2, w, row_mask, row_mask2, rows, H,
-                                                                                     scale, pair);
+  launch_pdl(feature_map_fwd_tc_kernel, dim3((unsigned)gx, H), dim3(fm::kThreads_), fm::kSmem, st, tx, tp, tx2, tp2, w, row_mask, row_mask2,
+             rows, H, scale, pair);
   return check_launch("rfa_feature_map_fwd");
 }
 
@@ -246,7 +253,14 @@ feature_map_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid
     }
     mbar_init(&bars[bEpi], 128); mbar_init(&bars[bDone], 1);
     mbar_fence_init();
-    // the first tiles are requested before the rest of the prologue (W_h, tensor memory), which their flight then hides
+    tma_prefetch_desc(&tm_x); tma_prefetch_desc(&tm_gp); tma_prefetch_desc(&tm_gx);
+  }
+  if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  __syncthreads();              // tensor memory is allocated before the next kernel's CTAs may ask for theirs
+  pdl_wait();
+  pdl_launch_dependents();
+  if (tid == 0) {
+    // the first tiles are requested before W_h is read and converted, which their flight then hides
     for (int i = 0; i < kRing && i < ntile; ++i) {
       int which;
       const int row0 = tile_row0(i, which);
@@ -256,7 +270,6 @@ feature_map_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid
       tma_load_3d(base + kGP, which ? &tm_gp2 : &tm_gp, &bars[bFull + i], 0, h, row0);
       tma_load_3d(base + kGP + kBox, which ? &tm_gp2 : &tm_gp, &bars[bFull + i], 64, h, row0);
     }
-    tma_prefetch_desc(&tm_gx);
   }
   // W_h as two fp16 K-major operand tiles: [j][i] and its transpose [i][j]
   for (int idx = tid; idx < 64 * 8; idx += kThreads_) {
@@ -272,7 +285,6 @@ feature_map_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid
       *reinterpret_cast<__half*>(sm + kWt + sw128_offset(ch * 8 + e, j)) = __float2half_rn(v[e]);
   }
   fence_async_smem();
-  if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -491,8 +503,8 @@ int launch_feature_map_bwd_tc(const __half* x, const float* w, const uint8_t* ro
   int64_t gx = sms / H;                          // one CTA per SM (shared memory): never more CTAs than SMs, or a second wave runs
   if (gx > ntile) gx = ntile;
   if (gx < 1) gx = 1;
-  feature_map_bwd_tc_kernel<<<dim3((unsigned)gx, H), fmb::kThreads_, fmb::kSmem, st>>>(tx, tg, to, tx2, tg2, to2, w, g_w, row_mask,
-                                                                                        row_mask2, rows, H, scale, pair);
+  launch_pdl(feature_map_bwd_tc_kernel, dim3((unsigned)gx, H), dim3(fmb::kThreads_), fmb::kSmem, st, tx, tg, to, tx2, tg2, to2, w, g_w, row_mask,
+             row_mask2, rows, H, scale, pair);
   return check_launch("rfa_feature_map_bwd");
 }
 
