@@ -225,6 +225,18 @@ class CausalAttention(nn.Module):
     def _heads(self, t: Tensor) -> Tensor:
         return t.contiguous().view(t.size(0), t.size(1), self.num_heads, self.head_dim)
 
+    def _decode_step(self, q: Tensor, k: Tensor, v: Tensor, w: Tensor, saved_state: Dict[str, Optional[Tensor]]) -> Tensor:
+        """One token from the raw per-head vectors [bsz, num_heads, head_dim]: ``incremental_rfa`` with the feature map inside
+        the kernel, the state updated in place."""
+        s, z = saved_state.get("prev_s"), saved_state.get("prev_z")
+        assert (s is None) == (z is None)
+        if s is None:
+            s = torch.zeros(*q.shape[:2], 2 * w.size(1), q.size(2), device=v.device, dtype=torch.float32)
+            z = torch.zeros(*q.shape[:2], 2 * w.size(1), device=v.device, dtype=torch.float32)
+        attn = ops.decode_step_fused(q, k, v, w.float().contiguous(), SCALE, s, z)
+        saved_state["prev_s"], saved_state["prev_z"] = s, z
+        return attn
+
     def forward(self, x: Tensor, random_matrices: Tensor, key_padding_mask: Optional[Tensor] = None,
                 attn_mask: Optional[Tensor] = None,
                 saved_state: Optional[Dict[str, Optional[Tensor]]] = None) -> Tensor:
@@ -246,6 +258,12 @@ class CausalAttention(nn.Module):
             # request (fuse_feature_map), because the backward then has to form the features again
             attn = fused_causal_rfa(q=q, k=k, v=v, random_matrices=w, key_padding_mask=key_padding_mask)
             return self.out_proj(attn.to(x.dtype))
+        if saved_state is not None and not (torch.is_grad_enabled() and any(
+                t is not None and t.requires_grad for t in (q, k, v, w, saved_state.get("prev_s"), saved_state.get("prev_z")))) \
+                and ops.decode_fused_supported(q, w):
+            assert tgt_len == 1
+            attn = self._decode_step(q[0], k[0], v[0], w, saved_state)
+            return self.out_proj(attn.reshape(1, bsz, embed_dim).to(x.dtype))
         # the padding mask of the kernel path is applied inside the feature map of k (no separate pass over phi_k)
         fused_mask = key_padding_mask if (saved_state is None and self.cuda_causal_rfa) else None
         phi_q, phi_k = random_project_pair(x_a=q, x_b=k, random_matrices=w, key_padding_mask_b=fused_mask)

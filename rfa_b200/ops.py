@@ -299,6 +299,14 @@ def decode_step_fused(q: Tensor, k: Tensor, v: Tensor, w: Tensor, scale: float, 
     return native().decode_step_fused(q, k, v, w, scale, s, z, out)
 
 
+def decode_fused_supported(q: Tensor, w: Tensor) -> bool:
+    """Whether one token can go through ``decode_step_fused`` wherever ``feature_map_fwd`` and ``decode_step`` would take it:
+    CUDA, fp16 or fp32, head_dim 4 * 2^m and both widths multiples of 8 up to 128 (the feature map's reach)."""
+    D, d = w.shape[-2:]
+    return (q.is_cuda and q.dtype in (torch.float16, torch.float32) and d in (8, 16, 32, 64, 128) and D % 8 == 0 and D <= 128
+            and w.dim() == 3 and w.shape[0] == q.shape[-2] and d == q.shape[-1])
+
+
 class CrossDecodeStates:
     """The cross-attention states of all layers of a decoder, gathered once per sequence for ``cross_decode_step``:
     device arrays of pointers to each layer's ``s [B,H,K,d]`` and ``z [B,H,K]`` (fp32, contiguous).  The states are

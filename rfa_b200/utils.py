@@ -138,8 +138,10 @@ def sample_effective_matrices(*, num_layers: int, num_heads: int, random_matrice
 def build_random_matrices(random_matrices: Tensor, tau: float, sigma: Optional[Tensor] = None,
                           reparam_proj: bool = False) -> Tensor:
     """Effective projection ``sigma * W / tau`` (``sigma`` [H,1,d] only when reparam_proj)."""
-    w = sigma * random_matrices if reparam_proj else random_matrices
-    return w / tau
+    if not reparam_proj:
+        return random_matrices / tau
+    w = sigma * random_matrices
+    return w if tau == 1 else w / tau          # x / 1 is x, and a launch
 
 
 def _normalize(x: Tensor) -> Tuple[Tensor, Tensor]:

@@ -68,3 +68,27 @@ def test_decode_of_many_heads(dev, state_dtype, in_dtype, B, H):
         halves = [ops.decode_step_fused(q[a], k[a], v[a], w, 0.1, s2[a], z2[a]) for a in (slice(0, B // 2), slice(B // 2, B))]
         assert rel(outs[i], torch.cat(halves)) < 1e-3
     assert rel(s1, s2) < 1e-3 and rel(z1, z2) < 1e-3
+
+
+@pytest.mark.parametrize("head_dim,proj_dim,dtype", [(64, 64, torch.float16), (32, 32, torch.float16), (128, 128, torch.float32), (24, 32, torch.float16)])
+def test_layer_decode_step_against_the_differentiable_path(dev, head_dim, proj_dim, dtype):
+    """One token through the layer: with gradients recorded it goes through feature map and causal kernel, without through the
+    fused decoding step (head_dim 24 is none of its widths, and of no decoding kernel's: refused in both forms)."""
+    from rfa_b200 import CausalAttention
+    torch.manual_seed(0)
+    layer = CausalAttention(embed_dim=4 * head_dim, num_heads=4, head_dim=head_dim, proj_dim=proj_dim, tau=0.5).to(dev).to(dtype)
+    w = torch.randn(4, proj_dim, head_dim, device=dev, dtype=dtype)
+    plain, recorded = {}, {}
+    for _ in range(3):
+        x = torch.randn(1, 3, 4 * head_dim, device=dev, dtype=dtype)
+        y = layer(x, w, saved_state=recorded)
+        recorded = {k: t.detach() for k, t in recorded.items()}
+        with torch.no_grad():
+            if head_dim == 24:
+                with pytest.raises(ValueError, match="head_dim"):
+                    layer(x, w, saved_state=plain)
+                continue
+            assert rel(layer(x, w, saved_state=plain), y) < 4e-3
+    if head_dim != 24:
+        assert rel(plain["prev_s"], recorded["prev_s"]) < 2e-3 and rel(plain["prev_z"], recorded["prev_z"]) < 2e-3
+        assert plain["prev_s"].dtype == torch.float32
