@@ -114,13 +114,15 @@ static CausalPlan plan_causal(int64_t T, int BH) { return cut_segments(T, kSegAl
 static bool is_tc(int K, int d) { return K == kK && d == kD; }
 static bool is_chunked(int K, int d) { return !is_tc(K, d) && generic_chunk(K, d, nullptr) > 0; }
 
-constexpr int64_t kChunkedMinSaved = 4;
 static CausalPlan plan_geometry(int64_t T, int BH, int K, int d) {
   if (is_tc(K, d)) return plan_causal(T, BH);
   int ctas = 1;
   const int chunk = generic_chunk(K, d, &ctas);
   if (!chunk) return CausalPlan{1, T};
-  return cut_segments(T, chunk, kSms * ctas / BH, kChunkedMinSaved);
+  // A chunk takes these kernels 20 us and more, a cut's pre-pass and scans 15: any cut that one wave holds.  Forward + backward in
+  // us at (K, d, heads x batch, tokens), whole / cut: (64, 32, 32, 200) 109 / 47, (128, 128, 32, 200) 361 / 137,
+  // (256, 128, 8, 128) 357 / 152, (64, 32, 8, 512) 217 / 46.
+  return cut_segments(T, chunk, kSms * ctas / BH, 1);
 }
 
 struct CausalWs {

@@ -4,8 +4,8 @@
 // d % 8 == 0, cuda/forward.cu:150-153); what does not fit stays on the token-at-a-time kernels of generic.cu.  Those keep
 // every number in fp32, and so do these: the state, the weights and the gradients' partial sums are fp32 in registers and
 // shared memory, and a product with such an operand is two mma.sync m16n8k8 tf32 products, of its leading 11 bits and
-// of the rest (hi = rna_tf32(x), lo = x - hi: 22 bits together); fp16 inputs are exact in tf32, so a product of two inputs is
-// one.  tf32 also has fp32's exponent range, which an fp16 split would not.  tcgen05's kind::tf32 would need operands
+// of the rest (hi = x rounded to tf32, lo = x - hi: 22 bits together); fp16 inputs are exact in tf32.  A product of two inputs is
+// one, and goes to m16n8k16 f16 with its operands straight from ldmatrix.  tf32 also has fp32's exponent range, which an fp16 split would not.  tcgen05's kind::tf32 would need operands
 // padded to its tiles and swizzled and the splits written back to shared memory; at these widths (32 to 256) the warps'
 // fragments read straight from fp32 tiles cost less.
 //
@@ -28,7 +28,7 @@
 
 namespace rfa {
 
-constexpr int kGmThreads = 256, kGmWarps = 8;
+constexpr int kGmRegs = 80;      // three CTAs of 256 threads on an SM, or one of 512
 
 __host__ __device__ inline int gm_round16(int x) { return (x + 15) & ~15; }
 
@@ -72,27 +72,37 @@ __device__ __forceinline__ void gm_commit() { asm volatile("cp.async.commit_grou
 template <int N>
 __device__ __forceinline__ void gm_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
+// f(row, first column) of this thread's 16-byte pieces of a tile of C rows of `width` halves; one division for all of them
+template <class F>
+__device__ __forceinline__ void gm_each16(int C, int width, F f) {
+  const int w8 = width >> 3, dr = blockDim.x / w8, dc = blockDim.x - dr * w8;
+  int r = threadIdx.x / w8, c = threadIdx.x - r * w8;
+  while (r < C) {
+    f(r, c * 8);
+    r += dr;
+    c += dc;
+    if (c >= w8) { c -= w8; ++r; }
+  }
+}
 // C rows of `width` halves, token t0 + r of sequence bh; rows from `valid` on, and masked ones, come out as zeros
 __device__ __forceinline__ void gm_load(__half* dst, int pitch, const __half* src, int C, int width, int64_t t0, int valid, int BH,
                                         int bh, const uint8_t* mrow) {
-  const int w8 = width >> 3, n = C * w8;
-  for (int i = threadIdx.x; i < n; i += kGmThreads) {
-    const int r = i / w8, c = i - r * w8;
+  const size_t row = (size_t)BH * width;
+  src += ((size_t)t0 * BH + bh) * width;
+  gm_each16(C, width, [&](int r, int c) {
     const bool live = r < valid && !(mrow && mrow[t0 + r]);
-    gm_cp16(dst + r * pitch + c * 8, src + (live ? ((size_t)(t0 + r) * BH + bh) * width + c * 8 : 0), live);
-  }
+    gm_cp16(dst + r * pitch + c, src + (live ? r * row + c : 0), live);
+  });
 }
 // has any of this thread's own chunks of the tile a non-finite value?  (after its cp.async have landed)
 __device__ __forceinline__ bool gm_odd(const __half* tile, int pitch, int C, int width) {
-  const int w8 = width >> 3, n = C * w8;
   bool odd = false;
-  for (int i = threadIdx.x; i < n; i += kGmThreads) {
-    const int r = i / w8, c = i - r * w8;
-    const uint4 u = *reinterpret_cast<const uint4*>(tile + r * pitch + c * 8);
+  gm_each16(C, width, [&](int r, int c) {
+    const uint4 u = *reinterpret_cast<const uint4*>(tile + r * pitch + c);
     const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
     for (int e = 0; e < 4; ++e) odd |= (w[e] & 0x7C00u) == 0x7C00u || (w[e] & 0x7C000000u) == 0x7C000000u;
-  }
+  });
   return odd;
 }
 
@@ -102,44 +112,145 @@ __device__ __forceinline__ void gm_mma(float (&c)[4], const uint32_t (&a)[4], ui
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// Rounding by integer: the conversion unit takes a quarter of the ALU's rate.  The mma drops the low 13 bits of lo.
 __device__ __forceinline__ void gm_split(float x, uint32_t& hi, uint32_t& lo) {
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(x));
-  const float h = __uint_as_float(hi);
-  lo = __float_as_uint(fabsf(h) == CUDART_INF_F ? 0.f : x - h);          // inf stays inf
+  hi = (__float_as_uint(x) + 0x1000u) & 0xFFFFE000u;
+  lo = __float_as_uint(x - __uint_as_float(hi)) + 0x1000u;
+  if (!(fabsf(x) < CUDART_INF_F)) { hi = __float_as_uint(x); lo = 0u; }      // infinities and NaN stay what they are
+}
+__device__ __forceinline__ void gm_mma16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void gm_ldsm(uint32_t (&r)[4], const __half* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
+}
+__device__ __forceinline__ void gm_ldsm_t(uint32_t (&r)[4], const __half* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
+}
+// The lane's row and column offset for the four 8 x 8 blocks of a 16 x 16 fragment: A by rows or B by rows of the inner index
+// (trans) take `a`, B by rows of its columns or A by rows of the inner index (trans) take `b`.
+__device__ __forceinline__ int gm_off_a(int lane, int pitch) { return (lane & 15) * pitch + (lane >> 4) * 8; }
+__device__ __forceinline__ int gm_off_b(int lane, int pitch) { return ((lane & 7) + (lane >> 4) * 8) * pitch + ((lane >> 3) & 1) * 8; }
+// acc (16 x 16, rows i0, columns j0) = X Y^T of two fp16 tiles stored along the inner index, `width` (rounded up to 16: zeros) long
+__device__ __forceinline__ void gm_exact(float (&acc)[2][4], GmTile x, int i0, GmTile y, int j0, int width) {
+  const int lane = threadIdx.x & 31;
+  const __half *pa = x.p + i0 * x.pitch + gm_off_a(lane, x.pitch), *pb = y.p + j0 * y.pitch + gm_off_b(lane, y.pitch);
+#pragma unroll 4
+  for (int l = 0; l < width; l += 16) {
+    uint32_t a[4], b[4];
+    gm_ldsm(a, pa + l);
+    gm_ldsm(b, pb + l);
+    gm_mma16(acc[0], a, b[0], b[1]);
+    gm_mma16(acc[1], a, b[2], b[3]);
+  }
 }
 
-// acc (16 x 8 NT, rows i0.., columns j0..) += sum over l in [l0, l1) of A(i, l) B(l, j).  la(i, l) -> A(i, l), A(i, l + 1) and
-// lb(l, j) -> B(l, j), B(l + 1, j) for even l.  The sum's order is free, so that slots t and t + 4 of a fragment's inner index
-// stand for l = 2t and 2t + 1: a pair is one 4- or 8-byte read where the operand is stored along l.  SA / SB: the operand is
-// not exact in tf32 and goes in two parts (never both).
-template <int NT, bool SA, bool SB, class LA, class LB>
-__device__ __forceinline__ void gm_product(float (&acc)[NT][4], int i0, int j0, int nt, int l0, int l1, LA la, LB lb) {
-  static_assert(!(SA && SB), "one split operand at most");
-  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+// acc (16 x 8 NT) += sum over l in [l0, l1) of A(i, l) B(l, j), one operand exact in tf32 and the other (SPLIT_A: A, else B) in two
+// parts.  The sum's order is free, so that slots t and t + 4 of a fragment's inner index stand for l = 2t and 2t + 1: a pair is one
+// 8-byte read of an fp32 operand stored along l, and one 8 x 8 block of ldmatrix (two halves a lane) of an fp16 operand,
+// whichever way it is stored (trans).  fa(l, a): A at rows g, g + 8 of column l + 2t, then of l + 2t + 1.  fb(l, b): b[n] = B at rows
+// l + 2t, l + 2t + 1 of column g of the n-th block of 8.
+template <int NT, bool SPLIT_A, class FA, class FB>
+__device__ __forceinline__ void gm_product(float (&acc)[NT][4], int nt, int l0, int l1, FA fa, FB fb) {
 #pragma unroll 2
   for (int l = l0; l < l1; l += 8) {
-    const float2 x = la(i0 + g, l + 2 * t), y = la(i0 + g + 8, l + 2 * t);
+    float x[4];
+    float2 b[NT];
+    fa(l, x);
+    fb(l, b);
     uint32_t a[4], al[4];
-    if (SA) {
-      gm_split(x.x, a[0], al[0]); gm_split(y.x, a[1], al[1]); gm_split(x.y, a[2], al[2]); gm_split(y.y, a[3], al[3]);
-    } else {
-      a[0] = __float_as_uint(x.x); a[1] = __float_as_uint(y.x); a[2] = __float_as_uint(x.y); a[3] = __float_as_uint(y.y);
-    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (SPLIT_A) gm_split(x[e], a[e], al[e]);
+      else a[e] = __float_as_uint(x[e]);
 #pragma unroll
     for (int n = 0; n < NT; ++n)
       if (n < nt) {
-        const float2 b = lb(l + 2 * t, j0 + 8 * n + g);
-        if (SB) {
+        if (SPLIT_A) {
+          gm_mma(acc[n], al, __float_as_uint(b[n].x), __float_as_uint(b[n].y));
+          gm_mma(acc[n], a, __float_as_uint(b[n].x), __float_as_uint(b[n].y));
+        } else {
           uint32_t h0, l0_, h1, l1_;
-          gm_split(b.x, h0, l0_); gm_split(b.y, h1, l1_);
+          gm_split(b[n].x, h0, l0_); gm_split(b[n].y, h1, l1_);
           gm_mma(acc[n], a, l0_, l1_);
           gm_mma(acc[n], a, h0, h1);
-        } else {
-          if (SA) gm_mma(acc[n], al, __float_as_uint(b.x), __float_as_uint(b.y));
-          gm_mma(acc[n], a, __float_as_uint(b.x), __float_as_uint(b.y));
         }
       }
   }
+}
+// operand readers for it
+__device__ __forceinline__ void gm_ldsm2(uint32_t (&r)[2], const __half* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
+}
+__device__ __forceinline__ void gm_ldsm2_t(uint32_t (&r)[2], const __half* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
+}
+__device__ __forceinline__ float2 gm_f2(uint32_t u) { return __half22float2(*reinterpret_cast<const __half2*>(&u)); }
+__device__ __forceinline__ void gm_pairs(float (&a)[4], float2 x, float2 y) { a[0] = x.x; a[1] = y.x; a[2] = x.y; a[3] = y.y; }
+// A = 16 rows of an fp16 tile from row i0
+__device__ __forceinline__ auto gm_a_rows(GmTile x, int i0) {
+  const int lane = threadIdx.x & 31;
+  const __half* p = x.p + (i0 + (lane & 15)) * x.pitch;
+  return [=](int l, float (&a)[4]) { uint32_t r[2]; gm_ldsm2(r, p + l); gm_pairs(a, gm_f2(r[0]), gm_f2(r[1])); };
+}
+// A = 16 columns of an fp16 tile from column i0, transposed
+__device__ __forceinline__ auto gm_a_cols(GmTile x, int i0) {
+  const int lane = threadIdx.x & 31, pitch = x.pitch;
+  const __half* p = x.p + (lane & 7) * pitch + i0 + ((lane >> 3) & 1) * 8;
+  return [=](int l, float (&a)[4]) { uint32_t r[2]; gm_ldsm2_t(r, p + l * pitch); gm_pairs(a, gm_f2(r[0]), gm_f2(r[1])); };
+}
+// A = 16 rows / columns (transposed) of an fp32 array
+__device__ __forceinline__ auto gm_a_frows(const float* s, int pitch, int i0) {
+  const int lane = threadIdx.x & 31;
+  const float *p = s + (i0 + (lane >> 2)) * pitch + 2 * (lane & 3), *q = p + 8 * pitch;
+  return [=](int l, float (&a)[4]) { gm_pairs(a, *reinterpret_cast<const float2*>(p + l), *reinterpret_cast<const float2*>(q + l)); };
+}
+__device__ __forceinline__ auto gm_a_fcols(const float* s, int pitch, int i0) {
+  const int lane = threadIdx.x & 31;
+  const float* p = s + 2 * (lane & 3) * pitch + i0 + (lane >> 2);
+  return [=](int l, float (&a)[4]) { const float* u = p + l * pitch; a[0] = u[0]; a[1] = u[8]; a[2] = u[pitch]; a[3] = u[pitch + 8]; };
+}
+// B = nt blocks of 8 columns of an fp16 tile from column j0 (blocks from nt on are not read)
+template <int NT>
+__device__ __forceinline__ auto gm_b_cols(GmTile y, int j0, int nt) {
+  const int lane = threadIdx.x & 31, pitch = y.pitch, blk = (lane >> 3) & (NT - 1);
+  const __half* p = y.p + (lane & 7) * pitch + j0 + (blk < nt ? blk * 8 : 0);
+  return [=](int l, float2 (&b)[NT]) {
+    if constexpr (NT == 4) {
+      uint32_t r[4];
+      gm_ldsm_t(r, p + l * pitch);
+#pragma unroll
+      for (int n = 0; n < 4; ++n) b[n] = gm_f2(r[n]);
+    } else {
+      uint32_t r[2];
+      gm_ldsm2_t(r, p + l * pitch);
+      b[0] = gm_f2(r[0]); b[1] = gm_f2(r[1]);
+    }
+  };
+}
+// B = columns from j0 of an fp32 array / of its transpose
+template <int NT>
+__device__ __forceinline__ auto gm_b_fcols(const float* s, int pitch, int j0, int nt) {
+  const int lane = threadIdx.x & 31;
+  const float* p = s + 2 * (lane & 3) * pitch + j0 + (lane >> 2);
+  return [=](int l, float2 (&b)[NT]) {
+    const float* u = p + l * pitch;
+#pragma unroll
+    for (int n = 0; n < NT; ++n) b[n] = n < nt ? make_float2(u[8 * n], u[pitch + 8 * n]) : make_float2(0.f, 0.f);
+  };
+}
+template <int NT>
+__device__ __forceinline__ auto gm_b_frows(const float* s, int pitch, int j0, int nt) {
+  const int lane = threadIdx.x & 31;
+  const float* p = s + (j0 + (lane >> 2)) * pitch + 2 * (lane & 3);
+  return [=](int l, float2 (&b)[NT]) {
+#pragma unroll
+    for (int n = 0; n < NT; ++n) b[n] = n < nt ? *reinterpret_cast<const float2*>(p + 8 * n * pitch + l) : make_float2(0.f, 0.f);
+  };
 }
 // The same product where A is triangular (SA) and B holds a non-finite value: element by element, only over the l that
 // ok(i, l) admits.
@@ -167,7 +278,7 @@ __device__ __forceinline__ void gm_zero(float (&acc)[NT][4]) {
 #pragma unroll
     for (int e = 0; e < 4; ++e) acc[n][e] = 0.f;
 }
-// operand readers
+// single elements of operands
 __device__ __forceinline__ float2 gm_row(GmTile x, int i, int l) {          // fp16 tile stored along l: x[i][l], x[i][l + 1]
   return __half22float2(*reinterpret_cast<const __half2*>(x.p + i * x.pitch + l));
 }
@@ -183,18 +294,24 @@ __device__ __forceinline__ float gm_quad(float v) {
 
 // ---- shared steps ------------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void gm_state_in(float* S, float* z, const GmLayout& L, const float* s_in, const float* z_in, int K, int d) {
-  for (int e = threadIdx.x; e < L.Kp * d; e += kGmThreads) {
+  for (int e = threadIdx.x; e < L.Kp * d; e += blockDim.x) {
     const int kk = e / d, n = e - kk * d;
     S[kk * L.ps + n] = s_in && kk < K ? s_in[(size_t)kk * d + n] : 0.f;
   }
-  for (int i = threadIdx.x; i < L.Kp; i += kGmThreads) z[i] = z_in && i < K ? z_in[i] : 0.f;
+  for (int i = threadIdx.x; i < L.Kp; i += blockDim.x) z[i] = z_in && i < K ? z_in[i] : 0.f;
 }
 __device__ __forceinline__ void gm_state_out(const float* S, const float* z, const GmLayout& L, float* s_out, float* z_out, int K, int d) {
-  for (int e = threadIdx.x; e < K * d; e += kGmThreads) {
+  for (int e = threadIdx.x; e < K * d; e += blockDim.x) {
     const int kk = e / d, n = e - kk * d;
     s_out[e] = S[kk * L.ps + n];
   }
-  for (int i = threadIdx.x; i < K; i += kGmThreads) z_out[i] = z[i];
+  for (int i = threadIdx.x; i < K; i += blockDim.x) z_out[i] = z[i];
+}
+// zero the pad columns that gm_exact reads, once: the loads never touch them
+__device__ __forceinline__ void gm_pad(GmTile tile, int C, int width) {
+  const int w = gm_round16(width) - width;         // 0 or 8
+  if (w)
+    for (int i = threadIdx.x; i < C; i += blockDim.x) *reinterpret_cast<uint4*>(const_cast<__half*>(tile.p) + i * tile.pitch + width) = make_uint4(0, 0, 0, 0);
 }
 // S += X^T (wy Y), z += X^T wz over a chunk: summed in registers from zero, then added to the fp32 state with one rounding.
 // WEIGHTED: per-row factors inv (of Y) and gz (of z); else 1.
@@ -202,20 +319,47 @@ template <int C, bool WEIGHTED>
 __device__ __forceinline__ void gm_update(float* S, float* z, const GmLayout& L, GmTile x, GmTile y, const float* inv, const float* gz, int d) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int ng = (d + 8 + 15) / 16, mt = L.Kp / 16;                 // columns d..d+7 stand for z (only d is used)
-  for (int w = warp; w < mt * ng; w += kGmWarps) {
+  for (int w = warp; w < mt * ng; w += blockDim.x >> 5) {
     const int i0 = (w / ng) * 16, j0 = (w % ng) * 16, nt = min(2, (d + 8 - j0) / 8);
     float acc[2][4];
     gm_zero(acc);
-    gm_product<2, false, WEIGHTED>(acc, i0, j0, nt, 0, C, [&](int i, int l) { return gm_col(x, l, i); },
-                                   [&](int l, int j) {
-                                     if (j < d) {
-                                       float2 b = gm_col(y, l, j);
-                                       if (WEIGHTED) { b.x *= inv[l]; b.y *= inv[l + 1]; }
-                                       return b;
-                                     }
-                                     if (j > d) return make_float2(0.f, 0.f);
-                                     return WEIGHTED ? make_float2(gz[l], gz[l + 1]) : make_float2(1.f, 1.f);
-                                   });
+    if constexpr (WEIGHTED) {
+      const auto cols = gm_b_cols<2>(y, min(j0, d - 8), min(2, (d - j0) / 8));       // the z block is overwritten below
+      const auto weighted = [&](int l, float2(&b)[2]) {
+        cols(l, b);
+        const float2 wi = gm_frow(inv, 0, 0, l + 2 * t), wz = gm_frow(gz, 0, 0, l + 2 * t);
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+          if (j0 + 8 * n < d) { b[n].x *= wi.x; b[n].y *= wi.y; }
+          else b[n] = g == 0 ? wz : make_float2(0.f, 0.f);
+      };
+      const auto rows = gm_a_cols(x, i0);
+      for (int l = 0; l < C; l += 16) {        // as below
+        float part[2][4];
+        gm_zero(part);
+        gm_product<2, false>(part, nt, l, l + 16, rows, weighted);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { acc[0][e] += part[0][e]; acc[1][e] += part[1][e]; }
+      }
+    } else {
+      const __half *pa = x.p + i0 + gm_off_b(lane, x.pitch), *pb = y.p + j0 + gm_off_a(lane, y.pitch);
+      const uint32_t ones = g == 0 ? 0x3C003C00u : 0u;         // column d of the z block
+#pragma unroll
+      for (int l = 0; l < C; l += 16) {
+        uint32_t a[4], b[4];
+        gm_ldsm_t(a, pa + l * x.pitch);
+        if (j0 < d) gm_ldsm_t(b, pb + l * y.pitch);
+        else b[0] = b[1] = ones;
+        if (j0 + 8 >= d) b[2] = b[3] = ones;
+        // 16 tokens summed from zero, the sums rounded to nearest: the accumulator inside an mma truncates
+        float part[2][4];
+        gm_zero(part);
+        gm_mma16(part[0], a, b[0], b[1]);
+        if (nt > 1) gm_mma16(part[1], a, b[2], b[3]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { acc[0][e] += part[0][e]; acc[1][e] += part[1][e]; }
+      }
+    }
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
       const int j = j0 + 8 * n + 2 * t;
@@ -253,7 +397,7 @@ __device__ __forceinline__ void gm_store2(__half* p, float a, float b) { *reinte
 // forward.  grid (BH, nseg); s_seg / z_seg: the state entering each segment (null = zero)
 // ===========================================================================================================================
 template <int C, int STAGES>
-__global__ void __launch_bounds__(kGmThreads)
+__global__ void __maxnreg__(kGmRegs)
 gm_causal_fwd_kernel(const __half* __restrict__ q, const __half* __restrict__ k, const __half* __restrict__ v, __half* __restrict__ out,
                      const float* __restrict__ s_seg, const float* __restrict__ z_seg, float* __restrict__ s_out, float* __restrict__ z_out,
                      float* __restrict__ den_out, int64_t T, int BH, int64_t tseg, int K, int d) {
@@ -280,6 +424,8 @@ gm_causal_fwd_kernel(const __half* __restrict__ q, const __half* __restrict__ k,
     }
     gm_commit();
   };
+  for (int s = 0; s < STAGES; ++s)
+    for (int i = 0; i < 3; ++i) gm_pad(tile(s, i), C, i < 2 ? K : d);
   load(0);
   gm_state_in(S, z, L, s_seg ? s_seg + slot * K * d : nullptr, z_seg ? z_seg + slot * K : nullptr, K, d);
   for (int c = 0; c < nchunk; ++c) {
@@ -290,13 +436,12 @@ gm_causal_fwd_kernel(const __half* __restrict__ q, const __half* __restrict__ k,
     const bool odd = __syncthreads_or(gm_odd(tv.p, tv.pitch, C, d)) != 0;
     // P = tril(Q K^T), its row sums per 16 columns, q . z
     constexpr int MT = C / 16;
-    for (int w = warp; w < MT * MT; w += kGmWarps) {
+    for (int w = warp; w < MT * MT; w += blockDim.x >> 5) {
       const int mi = w / MT, ni = w % MT, i0 = mi * 16, j0 = ni * 16;
       if (ni > mi) continue;
       float acc[2][4];
       gm_zero(acc);
-      gm_product<2, false, false>(acc, i0, j0, 2, 0, K, [&](int i, int l) { return gm_row(tq, i, l); },
-                                  [&](int l, int j) { return gm_row(tk, j, l); });
+      gm_exact(acc, tq, i0, tk, j0, K);
       float r0 = 0.f, r1 = 0.f;
 #pragma unroll
       for (int n = 0; n < 2; ++n) {
@@ -317,16 +462,15 @@ gm_causal_fwd_kernel(const __half* __restrict__ q, const __half* __restrict__ k,
     __syncthreads();
     // out = (P V + Q S) / max(raw, 1)
     const int ng = (d + 15) / 16;
-    for (int w = warp; w < MT * ng; w += kGmWarps) {
+    for (int w = warp; w < MT * ng; w += blockDim.x >> 5) {
       const int mi = w / ng, i0 = mi * 16, j0 = (w % ng) * 16, nt = min(2, (d - j0) / 8);
       float acc[2][4];
       gm_zero(acc);
       auto la = [=](int i, int l) { return gm_frow(P, pp, i, l); };
       auto lb = [=](int l, int j) { return gm_col(tv, l, j); };
       if (odd) gm_product_masked<2>(acc, i0, j0, nt, 0, i0 + 16, la, lb, [](int i, int l) { return l <= i; });
-      else gm_product<2, true, false>(acc, i0, j0, nt, 0, i0 + 16, la, lb);
-      gm_product<2, false, true>(acc, i0, j0, nt, 0, K, [&](int i, int l) { return gm_row(tq, i, l); },
-                                 [&](int l, int j) { return gm_fcol(S, L.ps, l, j); });
+      else gm_product<2, true>(acc, nt, 0, i0 + 16, gm_a_frows(P, pp, i0), gm_b_cols<2>(tv, j0, nt));
+      gm_product<2, false>(acc, nt, 0, K, gm_a_rows(tq, i0), gm_b_fcols<2>(S, L.ps, j0, nt));
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         const int i = i0 + g + 8 * r;
@@ -356,7 +500,7 @@ gm_causal_fwd_kernel(const __half* __restrict__ q, const __half* __restrict__ k,
 // backward, sweep 1: gq, raw denominators, gz
 // ===========================================================================================================================
 template <int C, int STAGES>
-__global__ void __launch_bounds__(kGmThreads)
+__global__ void __maxnreg__(kGmRegs)
 gm_causal_bwd_q_kernel(const __half* __restrict__ q, const __half* __restrict__ k, const __half* __restrict__ v, const __half* __restrict__ gr,
                        __half* __restrict__ gq, const float* __restrict__ s_seg, const float* __restrict__ z_seg,
                        float* __restrict__ ws_den, float* __restrict__ ws_gz, int64_t T, int BH, int64_t tseg, int K, int d) {
@@ -386,6 +530,8 @@ gm_causal_bwd_q_kernel(const __half* __restrict__ q, const __half* __restrict__ 
     }
     gm_commit();
   };
+  for (int s = 0; s < STAGES; ++s)
+    for (int i = 0; i < 4; ++i) gm_pad(tile(s, i), C, i < 2 ? K : d);
   load(0);
   gm_state_in(S, z, L, s_seg ? s_seg + slot * K * d : nullptr, z_seg ? z_seg + slot * K : nullptr, K, d);
   for (int c = 0; c < nchunk; ++c) {
@@ -395,15 +541,13 @@ gm_causal_bwd_q_kernel(const __half* __restrict__ q, const __half* __restrict__ 
     const int valid = (int)min((int64_t)C, t_end - t0);
     const bool odd = __syncthreads_or(gm_odd(tk.p, tk.pitch, C, K)) != 0;
     // G = g V^T on and below the diagonal; per 16 columns the row sums of P and of P o G
-    for (int w = warp; w < MT * MT; w += kGmWarps) {
+    for (int w = warp; w < MT * MT; w += blockDim.x >> 5) {
       const int mi = w / MT, ni = w % MT, i0 = mi * 16, j0 = ni * 16;
       if (ni > mi) continue;
       float p[2][4], a[2][4];
       gm_zero(p); gm_zero(a);
-      gm_product<2, false, false>(p, i0, j0, 2, 0, K, [&](int i, int l) { return gm_row(tq, i, l); },
-                                  [&](int l, int j) { return gm_row(tk, j, l); });
-      gm_product<2, false, false>(a, i0, j0, 2, 0, d, [&](int i, int l) { return gm_row(tg, i, l); },
-                                  [&](int l, int j) { return gm_row(tv, j, l); });
+      gm_exact(p, tq, i0, tk, j0, K);
+      gm_exact(a, tg, i0, tv, j0, d);
       float r[2] = {0.f, 0.f}, s[2] = {0.f, 0.f};
 #pragma unroll
       for (int n = 0; n < 2; ++n)
@@ -425,12 +569,11 @@ gm_causal_bwd_q_kernel(const __half* __restrict__ q, const __half* __restrict__ 
       }
     }
     // W = g S^T: the row sums of Q o W per 32 features
-    for (int w = warp; w < MT * kg; w += kGmWarps) {
+    for (int w = warp; w < MT * kg; w += blockDim.x >> 5) {
       const int i0 = (w / kg) * 16, gi = w % kg, j0 = gi * 32, nt = min(4, (K - j0) / 8);
       float a[4][4];
       gm_zero(a);
-      gm_product<4, false, true>(a, i0, j0, nt, 0, d, [&](int i, int l) { return gm_row(tg, i, l); },
-                                 [&](int l, int j) { return gm_frow(S, L.ps, j, l); });
+      gm_product<4, false>(a, nt, 0, d, gm_a_rows(tg, i0), gm_b_frows<4>(S, L.ps, j0, nt));
       float s[2] = {0.f, 0.f};
 #pragma unroll
       for (int n = 0; n < 4; ++n)
@@ -460,12 +603,11 @@ gm_causal_bwd_q_kernel(const __half* __restrict__ q, const __half* __restrict__ 
     }
     __syncthreads();
     // gq = inv W + tril(inv G + gz) K + gz z
-    for (int w = warp; w < MT * kg; w += kGmWarps) {
+    for (int w = warp; w < MT * kg; w += blockDim.x >> 5) {
       const int i0 = (w / kg) * 16, j0 = (w % kg) * 32, nt = min(4, (K - j0) / 8);
       float a[4][4];
       gm_zero(a);
-      gm_product<4, false, true>(a, i0, j0, nt, 0, d, [&](int i, int l) { return gm_row(tg, i, l); },
-                                 [&](int l, int j) { return gm_frow(S, L.ps, j, l); });
+      gm_product<4, false>(a, nt, 0, d, gm_a_rows(tg, i0), gm_b_frows<4>(S, L.ps, j0, nt));
 #pragma unroll
       for (int n = 0; n < 4; ++n)
 #pragma unroll
@@ -476,7 +618,8 @@ gm_causal_bwd_q_kernel(const __half* __restrict__ q, const __half* __restrict__ 
       };
       auto lb = [=](int l, int j) { return gm_col(tk, l, j); };
       if (odd) gm_product_masked<4>(a, i0, j0, nt, 0, i0 + 16, la, lb, [](int i, int l) { return l <= i; });
-      else gm_product<4, true, false>(a, i0, j0, nt, 0, i0 + 16, la, lb);
+      else gm_product<4, true>(a, nt, 0, i0 + 16, [&](int l, float(&u)[4]) { gm_pairs(u, la(i0 + g, l + 2 * t), la(i0 + g + 8, l + 2 * t)); },
+                               gm_b_cols<4>(tk, j0, nt));
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         const int i = i0 + g + 8 * r;
@@ -510,7 +653,7 @@ __device__ __forceinline__ void gm_row_scalars(float* inv, float* gz, const floa
 // backward, sweep 2 (chunks in reverse): gk, gv
 // ===========================================================================================================================
 template <int C, int STAGES>
-__global__ void __launch_bounds__(kGmThreads)
+__global__ void __maxnreg__(kGmRegs)
 gm_causal_bwd_kv_kernel(const __half* __restrict__ q, const __half* __restrict__ k, const __half* __restrict__ v, const __half* __restrict__ gr,
                         __half* __restrict__ gk, __half* __restrict__ gv, const float* __restrict__ ws_den, const float* __restrict__ ws_gz,
                         const float* __restrict__ ds_seg, const float* __restrict__ dz_seg, int64_t T, int BH, int64_t tseg, int K, int d) {
@@ -540,6 +683,8 @@ gm_causal_bwd_kv_kernel(const __half* __restrict__ q, const __half* __restrict__
     }
     gm_commit();
   };
+  for (int s = 0; s < STAGES; ++s)
+    for (int i = 0; i < 4; ++i) gm_pad(tile(s, i), C, i < 2 ? K : d);
   load(nchunk - 1);
   gm_state_in(S, z, L, ds_seg ? ds_seg + slot * K * d : nullptr, dz_seg ? dz_seg + slot * K : nullptr, K, d);
   for (int c = nchunk - 1; c >= 0; --c) {
@@ -550,15 +695,13 @@ gm_causal_bwd_kv_kernel(const __half* __restrict__ q, const __half* __restrict__
     const GmTile tq = tile(c, 0), tk = tile(c, 1), tv = tile(c, 2), tg = tile(c, 3);
     const bool odd = __syncthreads_or(gm_odd(tq.p, tq.pitch, C, K) || gm_odd(tg.p, tg.pitch, C, d)) != 0;
     // P' = inv tril(Q K^T), D = tril(inv g V^T + gz)
-    for (int w = warp; w < MT * MT; w += kGmWarps) {
+    for (int w = warp; w < MT * MT; w += blockDim.x >> 5) {
       const int mi = w / MT, ni = w % MT, i0 = mi * 16, j0 = ni * 16;
       if (ni > mi) continue;
       float p[2][4], a[2][4];
       gm_zero(p); gm_zero(a);
-      gm_product<2, false, false>(p, i0, j0, 2, 0, K, [&](int i, int l) { return gm_row(tq, i, l); },
-                                  [&](int l, int j) { return gm_row(tk, j, l); });
-      gm_product<2, false, false>(a, i0, j0, 2, 0, d, [&](int i, int l) { return gm_row(tg, i, l); },
-                                  [&](int l, int j) { return gm_row(tv, j, l); });
+      gm_exact(p, tq, i0, tk, j0, K);
+      gm_exact(a, tg, i0, tv, j0, d);
 #pragma unroll
       for (int n = 0; n < 2; ++n) {
 #pragma unroll
@@ -577,7 +720,7 @@ gm_causal_bwd_kv_kernel(const __half* __restrict__ q, const __half* __restrict__
     __syncthreads();
     // gk = D^T Q + V dS^T + dz   and   gv = P'^T g + K dS
     const int ng = (d + 15) / 16;
-    for (int w = warp; w < MT * (kg + ng); w += kGmWarps) {
+    for (int w = warp; w < MT * (kg + ng); w += blockDim.x >> 5) {
       if (w < MT * kg) {
         const int i0 = (w / kg) * 16, j0 = (w % kg) * 32, nt = min(4, (K - j0) / 8);
         float a[4][4];
@@ -585,9 +728,8 @@ gm_causal_bwd_kv_kernel(const __half* __restrict__ q, const __half* __restrict__
         auto la = [=](int i, int l) { return gm_fcol(D, pp, l, i); };
         auto lb = [=](int l, int j) { return gm_col(tq, l, j); };
         if (odd) gm_product_masked<4>(a, i0, j0, nt, i0, C, la, lb, [](int i, int l) { return l >= i; });
-        else gm_product<4, true, false>(a, i0, j0, nt, i0, C, la, lb);
-        gm_product<4, false, true>(a, i0, j0, nt, 0, d, [&](int i, int l) { return gm_row(tv, i, l); },
-                                   [&](int l, int j) { return gm_frow(S, L.ps, j, l); });
+        else gm_product<4, true>(a, nt, i0, C, gm_a_fcols(D, pp, i0), gm_b_cols<4>(tq, j0, nt));
+        gm_product<4, false>(a, nt, 0, d, gm_a_rows(tv, i0), gm_b_frows<4>(S, L.ps, j0, nt));
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
           const int i = i0 + g + 8 * r;
@@ -607,9 +749,8 @@ gm_causal_bwd_kv_kernel(const __half* __restrict__ q, const __half* __restrict__
         auto la = [=](int i, int l) { return gm_fcol(P, pp, l, i); };
         auto lb = [=](int l, int j) { return gm_col(tg, l, j); };
         if (odd) gm_product_masked<2>(a, i0, j0, nt, i0, C, la, lb, [](int i, int l) { return l >= i; });
-        else gm_product<2, true, false>(a, i0, j0, nt, i0, C, la, lb);
-        gm_product<2, false, true>(a, i0, j0, nt, 0, K, [&](int i, int l) { return gm_row(tk, i, l); },
-                                   [&](int l, int j) { return gm_fcol(S, L.ps, l, j); });
+        else gm_product<2, true>(a, nt, i0, C, gm_a_fcols(P, pp, i0), gm_b_cols<2>(tg, j0, nt));
+        gm_product<2, false>(a, nt, 0, K, gm_a_rows(tk, i0), gm_b_fcols<2>(S, L.ps, j0, nt));
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
           const int i = i0 + g + 8 * r;
@@ -633,7 +774,7 @@ gm_causal_bwd_kv_kernel(const __half* __restrict__ q, const __half* __restrict__
 // sum x (x) (inv y), sum gz x.  grid (BH, runs <= nseg)
 // ===========================================================================================================================
 template <int C, int STAGES, bool WEIGHTED>
-__global__ void __launch_bounds__(kGmThreads)
+__global__ void __maxnreg__(kGmRegs)
 gm_state_kernel(const __half* __restrict__ x, const __half* __restrict__ y, const uint8_t* __restrict__ pad_mask,
                 const float* __restrict__ ws_den, const float* __restrict__ ws_gz, float* __restrict__ s_out, float* __restrict__ z_out,
                 int64_t T, int BH, int H, int nseg, int64_t tseg, int K, int d) {
@@ -683,14 +824,19 @@ static uint32_t gm_need(int C, int stages, int K, int d) {
   const uint32_t a = gm_layout(C, K, d, stages, 2, 2, 1, gm_rows_bwd_q(C, K)).total, b = gm_layout(C, K, d, stages, 2, 2, 2, kGmRowsKv).total;
   return a > b ? a : b;
 }
-struct GmShape { int C, stages; };
+struct GmShape { int C, stages, ctas, threads; };
 // The longest chunk that fits, two stages before one: a longer chunk shares the state's products and the barriers among
-// more tokens.  C = 0: nothing fits.
+// more tokens.  C = 0: nothing fits.  A chunk's phases are chains of latencies, so that an SM wants 16 warps or more: from several
+// CTAs of 256 threads (up to 3), or from one of 512 where the state leaves room for one (K = 256, d = 128, 64 heads x 512
+// tokens, backward: 740 us with 256).
 static GmShape gm_shape(int K, int d) {
   for (int C : {64, 32, 16})
     for (int stages : {2, 1})
-      if (gm_need(C, stages, K, d) <= kGmSmemMax) return GmShape{C, stages};
-  return GmShape{0, 0};
+      if (const uint32_t need = gm_need(C, stages, K, d); need <= kGmSmemMax) {
+        const int n = (int)(kGmSmemMax / (need + 1024));
+        return GmShape{C, stages, n < 1 ? 1 : n > 3 ? 3 : n, n < 2 ? 512 : 256};
+      }
+  return GmShape{0, 0, 0, 0};
 }
 
 // Tokens per chunk of the chunked kernels for this geometry, 0 when it does not fit them; *ctas = how many of their CTAs
@@ -698,18 +844,15 @@ static GmShape gm_shape(int K, int d) {
 int generic_chunk(int K, int d, int* ctas) {
   if (K <= 0 || d <= 0 || K % 8 || d % 8 || K > 1024 || d > 1024) return 0;
   const GmShape s = gm_shape(K, d);
-  if (s.C && ctas) {
-    const int n = (int)(kGmSmemMax / (gm_need(s.C, s.stages, K, d) + 1024));
-    *ctas = n < 1 ? 1 : n > 3 ? 3 : n;
-  }
+  if (ctas) *ctas = s.ctas;
   return s.C;
 }
 
 template <class KERNEL, class... Args>
-static int gm_launch(KERNEL kernel, const char* what, uint32_t smem, dim3 grid, cudaStream_t st, Args... args) {
+static int gm_launch(KERNEL kernel, const char* what, int threads, uint32_t smem, dim3 grid, cudaStream_t st, Args... args) {
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return fail((int)e, "%s: cannot reserve %u bytes of shared memory: %s", what, smem, cudaGetErrorString(e));
-  kernel<<<grid, kGmThreads, smem, st>>>(args...);
+  kernel<<<grid, threads, smem, st>>>(args...);
   return check_launch(what);
 }
 #define RFA_GM_DISPATCH(shape, CALL)                                  \
@@ -723,7 +866,7 @@ static int gm_launch(KERNEL kernel, const char* what, uint32_t smem, dim3 grid, 
 int launch_causal_chunked_fwd(const __half* q, const __half* k, const __half* v, __half* out, const float* s_seg, const float* z_seg,
                               float* s_out, float* z_out, float* den_out, int64_t T, int BH, int nseg, int64_t tseg, int K, int d,
                               cudaStream_t st) {
-#define RFA_GM_CALL(C, N) return gm_launch(gm_causal_fwd_kernel<C, N>, "rfa_causal_fwd (chunked)", gm_layout(C, K, d, N, 2, 1, 1, gm_rows_fwd(C)).total, \
+#define RFA_GM_CALL(C, N) return gm_launch(gm_causal_fwd_kernel<C, N>, "rfa_causal_fwd (chunked)", gs_.threads, gm_layout(C, K, d, N, 2, 1, 1, gm_rows_fwd(C)).total, \
                                            dim3(BH, nseg), st, q, k, v, out, s_seg, z_seg, s_out, z_out, den_out, T, BH, tseg, K, d)
   RFA_GM_DISPATCH(gm_shape(K, d), RFA_GM_CALL);
 #undef RFA_GM_CALL
@@ -732,7 +875,7 @@ int launch_causal_chunked_fwd(const __half* q, const __half* k, const __half* v,
 int launch_causal_chunked_bwd_q(const __half* q, const __half* k, const __half* v, const __half* g, __half* gq, const float* s_seg,
                                 const float* z_seg, float* ws_den, float* ws_gz, int64_t T, int BH, int nseg, int64_t tseg, int K, int d,
                                 cudaStream_t st) {
-#define RFA_GM_CALL(C, N) return gm_launch(gm_causal_bwd_q_kernel<C, N>, "rfa_causal_bwd_q (chunked)", gm_layout(C, K, d, N, 2, 2, 1, gm_rows_bwd_q(C, K)).total, \
+#define RFA_GM_CALL(C, N) return gm_launch(gm_causal_bwd_q_kernel<C, N>, "rfa_causal_bwd_q (chunked)", gs_.threads, gm_layout(C, K, d, N, 2, 2, 1, gm_rows_bwd_q(C, K)).total, \
                                            dim3(BH, nseg), st, q, k, v, g, gq, s_seg, z_seg, ws_den, ws_gz, T, BH, tseg, K, d)
   RFA_GM_DISPATCH(gm_shape(K, d), RFA_GM_CALL);
 #undef RFA_GM_CALL
@@ -741,7 +884,7 @@ int launch_causal_chunked_bwd_q(const __half* q, const __half* k, const __half* 
 int launch_causal_chunked_bwd_kv(const __half* q, const __half* k, const __half* v, const __half* g, __half* gk, __half* gv,
                                  const float* ws_den, const float* ws_gz, const float* ds_seg, const float* dz_seg, int64_t T, int BH,
                                  int nseg, int64_t tseg, int K, int d, cudaStream_t st) {
-#define RFA_GM_CALL(C, N) return gm_launch(gm_causal_bwd_kv_kernel<C, N>, "rfa_causal_bwd_kv (chunked)", gm_layout(C, K, d, N, 2, 2, 2, kGmRowsKv).total, \
+#define RFA_GM_CALL(C, N) return gm_launch(gm_causal_bwd_kv_kernel<C, N>, "rfa_causal_bwd_kv (chunked)", gs_.threads, gm_layout(C, K, d, N, 2, 2, 2, kGmRowsKv).total, \
                                            dim3(BH, nseg), st, q, k, v, g, gk, gv, ws_den, ws_gz, ds_seg, dz_seg, T, BH, tseg, K, d)
   RFA_GM_DISPATCH(gm_shape(K, d), RFA_GM_CALL);
 #undef RFA_GM_CALL
@@ -751,9 +894,9 @@ int launch_causal_chunked_bwd_kv(const __half* q, const __half* k, const __half*
 int launch_state_chunked(const __half* x, const __half* y, const uint8_t* pad_mask, const float* ws_den, const float* ws_gz, float* s,
                          float* z, int64_t T, int BH, int H, int nseg, int64_t tseg, int runs, int K, int d, cudaStream_t st) {
 #define RFA_GM_CALL(C, N)                                                                                                             \
-  return ws_den ? gm_launch(gm_state_kernel<C, N, true>, "state reduction (chunked)", gm_layout(C, K, d, N, 1, 1, 0, kGmRowsState).total, \
+  return ws_den ? gm_launch(gm_state_kernel<C, N, true>, "state reduction (chunked)", gs_.threads, gm_layout(C, K, d, N, 1, 1, 0, kGmRowsState).total, \
                             dim3(BH, runs), st, x, y, pad_mask, ws_den, ws_gz, s, z, T, BH, H, nseg, tseg, K, d)                             \
-                : gm_launch(gm_state_kernel<C, N, false>, "state reduction (chunked)", gm_layout(C, K, d, N, 1, 1, 0, kGmRowsState).total, \
+                : gm_launch(gm_state_kernel<C, N, false>, "state reduction (chunked)", gs_.threads, gm_layout(C, K, d, N, 1, 1, 0, kGmRowsState).total, \
                             dim3(BH, runs), st, x, y, pad_mask, ws_den, ws_gz, s, z, T, BH, H, nseg, tseg, K, d)
   RFA_GM_DISPATCH(gm_shape(K, d), RFA_GM_CALL);
 #undef RFA_GM_CALL

@@ -64,7 +64,9 @@ def test_no_token_sees_a_later_non_finite_one(dev, which):
     ins[which][cut, :, 3] = float("inf")
     q, k, v, g = (t.to(dev) for t in ins)
     out = RFA.forward_cuda(q, k, v)
-    assert torch.equal(out[:cut], clean[:cut])
+    assert torch.isfinite(out[:cut]).all()
+    # element by element where an infinity of v shares the chunk: fp32 sums in another order, a neighbouring fp16 number at most
+    assert ((out[:cut] - clean[:cut]).abs() <= 2.0 ** -10 * clean[:cut].abs() + 1e-6).all()
     gq, _, _ = RFA.backward_cuda(q, k, v, g)
     assert torch.isfinite(gq[:cut]).all()
     if which == 0:       # q of a token reaches the key gradients of itself and of earlier tokens only
