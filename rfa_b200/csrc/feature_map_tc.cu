@@ -206,11 +206,12 @@ constexpr uint32_t kX = 0, kGP = kBox, kStage = 3 * kBox;          // per stage:
 constexpr int kRing = 3;                       // staged tiles in flight: a stage lives through the tile's whole dependent chain
 constexpr uint32_t kGH = kRing * kStage;       // two gh tiles; the output staging tile follows them
 constexpr uint32_t kOut = kGH + 2 * kBox;
-constexpr uint32_t kW = kOut + kBox;           // W  as [j][i] (K-major, contraction over i)
+constexpr uint32_t kW = kOut + 2 * kBox;       // (two staging tiles)  W  as [j][i] (K-major, contraction over i)
 constexpr uint32_t kWt = kW + 8192;            // W^T as [i][j] (K-major, contraction over j)
-constexpr uint32_t kRn = kWt + 8192;           // float2 [kRing][128]: (inv, inv / |x|) of the tile's rows, one set per stage
-constexpr uint32_t kBarOff = kRn + kRing * 1024;
-constexpr uint32_t kSmem = kBarOff + 256 + 1024;
+constexpr uint32_t kRn = kWt + 8192;           // fp32 [kRing][128]: inv / |x| of the tile's rows, one set per stage
+constexpr uint32_t kBarOff = kRn + kRing * 512;
+constexpr uint32_t kSmem = kBarOff + 256;      // the base must come 1024-aligned (checked)
+static_assert(kSmem <= 227 * 1024, "feature_map_bwd: shared memory map");
 constexpr uint32_t cU = 0, cGX = 128, cGW = 256;
 enum { bFull = 0, bEmpty = 3, bU = 6, bUFree = 8, bGH = 10, bGHFree = 12, bGX = 14, bGXFree = 16, bEpi = 18, bDone = 19, bNum = 20 };
 static_assert(kRing == 3 && bNum * 8 + 4 <= 256, "feature_map_bwd: barrier block");
@@ -223,11 +224,15 @@ feature_map_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid
                           const float* __restrict__ w, float* __restrict__ g_w, const uint8_t* __restrict__ row_mask,
                           const uint8_t* __restrict__ row_mask2, int64_t rows, int H, float scale, int pair) {
   using namespace fmb;
-  extern __shared__ unsigned char fmb_raw[];
-  unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(fmb_raw) + 1023) & ~uintptr_t(1023));
+  extern __shared__ __align__(1024) unsigned char fmb_raw[];
+  unsigned char* sm = fmb_raw;
+  if (smem_u32(sm) & 1023u) {                    // swizzled tiles need a 1024-byte aligned base
+    if (threadIdx.x == 0) tc_fail(99);
+    return;
+  }
   uint64_t* bars = reinterpret_cast<uint64_t*>(sm + kBarOff);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + bNum);
-  float2* rn = reinterpret_cast<float2*>(sm + kRn);
+  float* rn = reinterpret_cast<float*>(sm + kRn);
   const uint32_t sbase = smem_u32(sm);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int h = blockIdx.y;
@@ -374,7 +379,7 @@ feature_map_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid
       mbar_arrive(&bars[bUFree + st]);
       // the gh tile of this parity was last read by the products of tile i - 2
       if (i >= 2 && !mbar_wait(&bars[bGHFree + st], ((i >> 1) + 1) & 1)) { tc_fail(18); break; }
-      if (half == 0) rn[sg * 128 + row] = make_float2(inv, n > 0.f ? inv / n : 0.f);      // read by group 2 before it releases the stage
+      if (half == 0) rn[sg * 128 + row] = n > 0.f ? inv / n : 0.f;      // read by group 2 before it releases the stage
       const float sc = scale_row * inv;
 #pragma unroll
       for (int c4 = 0; c4 < 4; ++c4) {
@@ -420,7 +425,7 @@ feature_map_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid
       tmem_ld_wait();
       tc_fence_before_sync();
       mbar_arrive(&bars[bGXFree + st]);
-      const float2 r2 = rn[sg * 128 + row];
+      const float inv_n = rn[sg * 128 + row];
       float dot = 0.f;
 #pragma unroll
       for (int ch = 0; ch < 8; ++ch) {
@@ -433,9 +438,10 @@ feature_map_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid
           dot = fmaf(f.y, __uint_as_float(gx[ch * 8 + 2 * e + 1]), dot);
         }
       }
-      const float c2 = dot * r2.y;                     // (x . gx') inv / |x|
-      if (i > 0) {                                     // the previous tile's store must have drained the staging tile
-        if (etid == 0) tma_store_wait_read<0>();
+      const float c2 = dot * inv_n;                    // (x . gx') inv / |x|
+      unsigned char* staging = sm + kOut + st * kBox;
+      if (i > 1) {                                     // the store before the previous one must have drained this staging tile
+        if (etid == 0) tma_store_wait_read<1>();
         if (!epi_sync(&bars[bEpi], epi_phase)) { tc_fail(22); ok = false; break; }
       }
 #pragma unroll
@@ -448,13 +454,13 @@ feature_map_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid
           const float2 f = unpack_half2(xw[e]);
           o[e] = pack_half2(__uint_as_float(gx[ch * 8 + 2 * e]) - f.x * c2, __uint_as_float(gx[ch * 8 + 2 * e + 1]) - f.y * c2);
         }
-        *reinterpret_cast<uint4*>(sm + kOut + row_chunk1(row, ch)) = make_uint4(o[0], o[1], o[2], o[3]);
+        *reinterpret_cast<uint4*>(staging + row_chunk1(row, ch)) = make_uint4(o[0], o[1], o[2], o[3]);
       }
       mbar_arrive(&bars[bEmpty + sg]);                 // this group's reads of the stage are done
       fence_async_smem();
       if (!epi_sync(&bars[bEpi], epi_phase)) { tc_fail(23); ok = false; break; }
       if (etid == 0) {
-        tma_store_3d(which ? &tm_gx2 : &tm_gx, sm + kOut, 0, h, row0);
+        tma_store_3d(which ? &tm_gx2 : &tm_gx, staging, 0, h, row0);
         tma_store_commit();
       }
     }
