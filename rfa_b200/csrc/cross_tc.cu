@@ -16,7 +16,7 @@
 
 namespace rfa {
 
-constexpr int kXThreads = 192;
+constexpr int kXThreads = 192, kXStoreThreads = kXThreads + 32;
 
 // every kernel: prologue shared by all roles
 #define RFA_X_PROLOGUE(NBARS, TMEM_COLS)                                                                          \
@@ -469,10 +469,13 @@ constexpr uint32_t kK_ = 0, kV_ = 2 * kBox, kStage = 3 * kBox, kS_ = 2 * kStage,
                    kSmem = 113 * 1024;
 static_assert(kBarOff + 128 <= kSmem, "cross_state_bwd: shared memory map exceeds half an SM");
 constexpr uint32_t cDK = 0, cDV = 128;
-enum { bFull = 0, bEmpty = 2, bReady = 4, bOut = 6, bFree = 7, bSt = 8, bEpi = 9, bNum = 10 };
+enum { bFull = 0, bEmpty = 2, bReady = 4, bStaged = 6, bOut = 8, bFree = 9, bSt = 10, bEpi = 11, bNum = 12 };
+// A seventh warp issues the stores and waits until their staging tiles -- the stage the inputs came in -- have been read out,
+// before it gives the stage back: under full memory traffic that takes a microsecond or more, which the epilogue warps spend
+// on the other stage's chunk (44.6 -> 42.9 us at 256 x 1024 keys; the query kernels gained nothing from it).
 }
 
-__global__ void __launch_bounds__(kXThreads, 2)
+__global__ void __launch_bounds__(kXStoreThreads, 2)
 cross_state_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                           const __grid_constant__ CUtensorMap tm_gk, const __grid_constant__ CUtensorMap tm_gv,
                           const uint8_t* __restrict__ pad_mask, const float* __restrict__ d_s, const float* __restrict__ d_z,
@@ -483,7 +486,7 @@ cross_state_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid
   const int bh = blockIdx.x;
   const int nchunk = (int)((T + kTC - 1) / kTC);
   if (tid == 0) {
-    for (int i = 0; i < 2; ++i) { mbar_init(&bars[bFull + i], 1); mbar_init(&bars[bEmpty + i], 1); mbar_init(&bars[bReady + i], 128); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&bars[bFull + i], 1); mbar_init(&bars[bEmpty + i], 1); mbar_init(&bars[bReady + i], 128); mbar_init(&bars[bStaged + i], 128); }
     mbar_init(&bars[bOut], 1); mbar_init(&bars[bFree], 128); mbar_init(&bars[bSt], 128); mbar_init(&bars[bEpi], 128);
     mbar_fence_init();
     tma_prefetch_desc(&tm_k); tma_prefetch_desc(&tm_v); tma_prefetch_desc(&tm_gk); tma_prefetch_desc(&tm_gv);
@@ -521,8 +524,23 @@ cross_state_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid
         umma_commit(&bars[bOut]);
       }
     }
+  } else if (warp == 6) {
+    if (lane == 0) {
+      for (int c = 0; c < nchunk; ++c) {
+        const int st = c & 1;
+        unsigned char* stage = sm + st * kStage;
+        if (!mbar_wait(&bars[bStaged + st], (c >> 1) & 1)) { tc_fail(48); break; }
+        tma_store_3d(&tm_gk, stage + kK_, 0, bh, c * kTC);
+        tma_store_3d(&tm_gk, stage + kK_ + kBox, 64, bh, c * kTC);
+        tma_store_3d(&tm_gv, stage + kV_, 0, bh, c * kTC);
+        tma_store_commit();
+        tma_store_wait_read<0>();
+        mbar_arrive(&bars[bEmpty + st]);
+      }
+      tma_store_wait<0>();
+    }
   } else {
-    const int quarter = warp & 3, row = quarter * 32 + lane, etid = tid - 64;
+    const int quarter = warp & 3, row = quarter * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
     const uint8_t* mrow = pad_mask ? pad_mask + (size_t)(bh / H) * T : nullptr;
     {
@@ -579,17 +597,8 @@ cross_state_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid
         }
       }
       fence_async_smem();
-      if (!epi_sync(&bars[bEpi], epi_phase)) { tc_fail(48); ok = false; break; }
-      if (etid == 0) {
-        tma_store_3d(&tm_gk, stage + kK_, 0, bh, c * kTC);
-        tma_store_3d(&tm_gk, stage + kK_ + kBox, 64, bh, c * kTC);
-        tma_store_3d(&tm_gv, stage + kV_, 0, bh, c * kTC);
-        tma_store_commit();
-        tma_store_wait_read<0>();
-        mbar_arrive(&bars[bEmpty + st]);
-      }
+      mbar_arrive(&bars[bStaged + st]);
     }
-    if (etid == 0) tma_store_wait<0>();
   }
   RFA_X_FINISH(256)
 }
@@ -650,7 +659,7 @@ int launch_cross_state_bwd_tc(const __half* k, const __half* v, const uint8_t* p
       make_tmap_rows(&tgk, gk, T, BH, kK, kTC) || make_tmap_rows(&tgv, gv, T, BH, kD, kTC))
     return fail(RFA_EDEVICE, "cross_state_bwd: cuTensorMapEncodeTiled failed or is unavailable");
   if (int e = x_opt_in(cross_state_bwd_tc_kernel, xk::kSmem, "cross_state_bwd")) return e;
-  launch_pdl(cross_state_bwd_tc_kernel, dim3(BH), kXThreads, xk::kSmem, st, tk, tv, tgk, tgv, pad_mask, d_s, d_z, T, BH, H);
+  launch_pdl(cross_state_bwd_tc_kernel, dim3(BH), kXStoreThreads, xk::kSmem, st, tk, tv, tgk, tgv, pad_mask, d_s, d_z, T, BH, H);
   return check_launch("rfa_cross_state_bwd");
 }
 
