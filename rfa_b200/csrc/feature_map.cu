@@ -160,20 +160,24 @@ feature_map_bwd_kernel(const T* __restrict__ x, const float* __restrict__ w, con
     for (int i = 0; i < kFmI; ++i) dot[i] = 0.f;
     for (int col = cg; col < D; col += 64) {
       float u[kFmI][4];
-      fm_product(u, s.X, d + 4, s.Wt, D + 4, d, rg, col);
+      float4 gs[kFmI], gc[kFmI];                              // asked for before the product, which their flight hides
 #pragma unroll
       for (int i = 0; i < kFmI; ++i) {
         const int64_t row = row0 + rg + 16 * i;
-        float4 gu = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (row < rows && !(row_mask && row_mask[row])) {     // a masked row's features are constants: no gradient
-          const T* gp = g_phi + ((size_t)row * H + h) * 2 * D + col;
-          const float4 gs = load4(gp), gc = load4(gp + D);
-          float sn, cs;
-          sincosf(u[i][0], &sn, &cs); gu.x = scale * (gs.x * cs - gc.x * sn);
-          sincosf(u[i][1], &sn, &cs); gu.y = scale * (gs.y * cs - gc.y * sn);
-          sincosf(u[i][2], &sn, &cs); gu.z = scale * (gs.z * cs - gc.z * sn);
-          sincosf(u[i][3], &sn, &cs); gu.w = scale * (gs.w * cs - gc.w * sn);
-        }
+        const bool live = row < rows && !(row_mask && row_mask[row]);     // a masked row's features are constants: no gradient
+        const T* gp = g_phi + ((size_t)row * H + h) * 2 * D + col;
+        gs[i] = live ? load4(gp) : make_float4(0.f, 0.f, 0.f, 0.f);
+        gc[i] = live ? load4(gp + D) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+      fm_product(u, s.X, d + 4, s.Wt, D + 4, d, rg, col);
+#pragma unroll
+      for (int i = 0; i < kFmI; ++i) {
+        float4 gu;
+        float sn, cs;
+        sincosf(u[i][0], &sn, &cs); gu.x = scale * (gs[i].x * cs - gc[i].x * sn);
+        sincosf(u[i][1], &sn, &cs); gu.y = scale * (gs[i].y * cs - gc[i].y * sn);
+        sincosf(u[i][2], &sn, &cs); gu.z = scale * (gs[i].z * cs - gc[i].z * sn);
+        sincosf(u[i][3], &sn, &cs); gu.w = scale * (gs[i].w * cs - gc[i].w * sn);
         dot[i] = fmaf(gu.x, u[i][0], fmaf(gu.y, u[i][1], fmaf(gu.z, u[i][2], fmaf(gu.w, u[i][3], dot[i]))));
         store4(s.GU + (rg + 16 * i) * (D + 4) + col, gu);
       }
