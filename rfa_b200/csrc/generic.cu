@@ -1,11 +1,12 @@
-// Causal and cross RFA for the geometries the tensor-core kernels are not built for (they are specialised for feature
-// width K = 128 and head dim d = 64): any K % 8 == 0, d % 8 == 0 whose fp32 state [K][d + 1] fits in shared memory.
+// Causal and cross RFA for the geometries neither the tcgen05 kernels (K = 128, d = 64) nor the chunked ones
+// (generic_mma.cu: the causal path and the state reduction, where a chunk's tiles fit beside the state) serve: any K % 8 == 0,
+// d % 8 == 0 whose fp32 state [K][d + 1] fits in shared memory.
 // Upstream's kernels accept any K % 16 == 0, d % 8 == 0 (cuda/forward.cu:150-153, cuda/backward.cu:560-562) and its
 // cross attention is einsums of any size (cross_attention.py:97-104, 266-269); these kernels keep that reach.
 //
 // They are plain CUDA-core kernels that walk the tokens of one (batch, head) sequence one at a time, as upstream's
 // do, with the state in shared memory in fp32 (upstream: fp16 registers): simple and exact rather than fast -- about
-// 0.4 us per token and CTA.  Math per token (rfa.py:57-64, 79-101):
+// 4 us per token and CTA.  Math per token (rfa.py:57-64, 79-101):
 //     S += k (x) v, z += k;  num = q^T S, raw = q . z, den = max(raw, 1);  out = num / den
 //     gs = g / den, gz = -(g . num) / den^2 * [raw > 1];  gq = S gs + gz z
 //     reverse: dS += q (x) gs, dz += q gz;  gk = dS v + dz;  gv = dS^T k
