@@ -20,7 +20,7 @@ enum { bFull = 0, bEmpty = 2, bU = 4, bUFree = 6, bEpi = 8, bNum = 9 };
 __global__ void __launch_bounds__(fm::kThreads_, 3)
 feature_map_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_phi,
                           const __grid_constant__ CUtensorMap tm_x2, const __grid_constant__ CUtensorMap tm_phi2,
-                          const float* __restrict__ w, const uint8_t* __restrict__ row_mask, const uint8_t* __restrict__ row_mask2,
+                          const __half* __restrict__ x, const __half* __restrict__ x2, const float* __restrict__ w, const uint8_t* __restrict__ row_mask, const uint8_t* __restrict__ row_mask2,
                           int64_t rows, int H, float scale, int pair) {
   using namespace fm;
   extern __shared__ unsigned char fm_raw[];
@@ -40,7 +40,7 @@ feature_map_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid
     return (pair ? (v >> 1) : v) * kTC;
   };
   if (tid == 0) {
-    for (int i = 0; i < 2; ++i) { mbar_init(&bars[bFull + i], 1); mbar_init(&bars[bEmpty + i], 129); mbar_init(&bars[bU + i], 1); mbar_init(&bars[bUFree + i], 128); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&bars[bFull + i], 1); mbar_init(&bars[bEmpty + i], 1); mbar_init(&bars[bU + i], 1); mbar_init(&bars[bUFree + i], 128); }
     mbar_init(&bars[bEpi], 128);
     mbar_fence_init();
     tma_prefetch_desc(&tm_x); tma_prefetch_desc(&tm_phi);
@@ -104,23 +104,41 @@ feature_map_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
     uint32_t epi_phase = 0;
     bool ok = true;
+    // The rows come from memory a second time (L2) for their norms, a tile ahead, and not from the staged tile: reads of a
+    // CTA's first tile right after its barrier, and even right after the product that used it, saw 16-byte pieces that had not
+    // landed (the product never did) -- rows off by a few percent in one launch of 300 at two CTAs per SM, in every third at
+    // three; what a neighbour's operand reads can hold back on shared memory is the likely reason, 3 us later all was well.
+    uint4 xr[8];
+    auto fetch = [&](int i) {
+      int which;
+      const int row0 = i < ntile ? tile_row0(i, which) : 0;
+      const __half* src = (i < ntile && which) ? x2 : x;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int64_t r = (int64_t)row0 + quarter * 32 + 4 * j + (lane >> 3);
+        xr[j] = i < ntile && r < rows ? __ldg(reinterpret_cast<const uint4*>(src + ((size_t)r * H + h) * 64) + (lane & 7)) : make_uint4(0, 0, 0, 0);
+      }
+    };
+    fetch(0);
     for (int i = 0; ok && i < ntile; ++i) {
       const int st = i & 1;
       int which;
       const int row0 = tile_row0(i, which);
       const uint8_t* mask = which ? row_mask2 : row_mask;
-      if (!mbar_wait(&bars[bFull + st], (i >> 1) & 1)) { tc_fail(4); ok = false; break; }
-      float ss = 0.f;                                  // |x|^2 of this thread's row
+      // |x|^2 of this thread's row: eight lanes hold each row that the warp fetched, four rows per fetch
+      float ss = 0.f;
 #pragma unroll
-      for (int ch = 0; ch < 8; ++ch) {
-        const uint4 u = *reinterpret_cast<const uint4*>(sm + kX + st * kStage + row_chunk1(row, ch));
-        float2 f;
-        f = unpack_half2(u.x); ss = fmaf(f.x, f.x, ss); ss = fmaf(f.y, f.y, ss);
-        f = unpack_half2(u.y); ss = fmaf(f.x, f.x, ss); ss = fmaf(f.y, f.y, ss);
-        f = unpack_half2(u.z); ss = fmaf(f.x, f.x, ss); ss = fmaf(f.y, f.y, ss);
-        f = unpack_half2(u.w); ss = fmaf(f.x, f.x, ss); ss = fmaf(f.y, f.y, ss);
+      for (int j = 0; j < 8; ++j) {
+        const uint32_t xw[4] = {xr[j].x, xr[j].y, xr[j].z, xr[j].w};
+        float t = 0.f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { const float2 f = unpack_half2(xw[e]); t = fmaf(f.x, f.x, t); t = fmaf(f.y, f.y, t); }
+        t += __shfl_xor_sync(0xffffffffu, t, 1);
+        t += __shfl_xor_sync(0xffffffffu, t, 2);
+        t += __shfl_xor_sync(0xffffffffu, t, 4);
+        t = __shfl_sync(0xffffffffu, t, (lane & 3) * 8);
+        if ((lane >> 2) == j) ss = t;
       }
-      mbar_arrive(&bars[bEmpty + st]);
       const float inv = 1.f / (sqrtf(ss) + kNormEps);
       if (!mbar_wait(&bars[bU + st], (i >> 1) & 1)) { tc_fail(5); ok = false; break; }
       tc_fence_after_sync();
@@ -151,6 +169,7 @@ feature_map_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid
         *reinterpret_cast<uint4*>(sm + kOut + row_chunk1(row, ch)) = a;            // sin block
         *reinterpret_cast<uint4*>(sm + kOut + kBox + row_chunk1(row, ch)) = b;     // cos block
       }
+      fetch(i + 1);
       fence_async_smem();
       if (!epi_sync(&bars[bEpi], epi_phase)) { tc_fail(7); ok = false; break; }
       if (etid == 0) {
@@ -181,7 +200,7 @@ int launch_feature_map_fwd_tc(const __half* x, const float* w, const uint8_t* ro
   int64_t gx = 3LL * sms / H;                    // three CTAs per SM, and never more CTAs than fit at once
   if (gx > ntile) gx = ntile;
   if (gx < 1) gx = 1;
-  launch_pdl(feature_map_fwd_tc_kernel, dim3((unsigned)gx, H), dim3(fm::kThreads_), fm::kSmem, st, tx, tp, tx2, tp2, w, row_mask, row_mask2,
+  launch_pdl(feature_map_fwd_tc_kernel, dim3((unsigned)gx, H), dim3(fm::kThreads_), fm::kSmem, st, tx, tp, tx2, tp2, x, pair ? x2 : x, w, row_mask, row_mask2,
              rows, H, scale, pair);
   return check_launch("rfa_feature_map_fwd");
 }
@@ -359,6 +378,8 @@ feature_map_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid
       // a masked row's features are constant zeros: no gradient flows through it
       const float scale_row = (mask && grow < rows && mask[grow]) ? 0.f : scale;
       if (!mbar_wait(&bars[bFull + sg], (i / kRing) & 1)) { tc_fail(16); break; }
+      if (!mbar_wait(&bars[bU + st], (i >> 1) & 1)) { tc_fail(17); break; }      // the norms after the product (see the forward)
+      tc_fence_after_sync();
       float ss = 0.f;                                  // |x|^2 of this thread's row
 #pragma unroll
       for (int ch = 0; ch < 8; ++ch) {
@@ -370,8 +391,6 @@ feature_map_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid
         f = unpack_half2(u.w); ss = fmaf(f.x, f.x, ss); ss = fmaf(f.y, f.y, ss);
       }
       const float n = sqrtf(ss), inv = 1.f / (n + kNormEps);
-      if (!mbar_wait(&bars[bU + st], (i >> 1) & 1)) { tc_fail(17); break; }
-      tc_fence_after_sync();
       uint32_t u[32];
       tmem_ld32(tmem + lane_addr + cU + st * 64 + half * 32, u);
       tmem_ld_wait();

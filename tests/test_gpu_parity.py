@@ -581,3 +581,18 @@ def test_feature_map_pair_equals_two_single_launches(dev, rows, B, H, masked):
     # against the oracle as well (float64 reference of the analytic gradient)
     want_a, want_wa = O.random_project_backward(xa.float().cpu(), w.cpu(), ga.float().cpu(), 0.1)
     assert_close(gxa, want_a, "g_x (pair, first array)")
+
+
+def test_feature_map_is_bit_stable(dev):
+    """Repeated launches on the same inputs: the rows' norms must come from the tile that has landed, never from what the
+    stage held before (a launch in three went wrong in a few rows of a CTA's first tile when they were read too early)."""
+    from rfa_b200 import ops
+    gen = torch.Generator().manual_seed(0)
+    w = torch.randn(16, 64, 64, generator=gen).to(dev)
+    x = torch.randn(1024, 16, 16, 64, generator=gen).half().to(dev)
+    g = torch.randn(1024, 16, 16, 128, generator=gen).half().to(dev)
+    first, grad = ops.feature_map_fwd(x, w, 0.1), ops.feature_map_bwd(x, w, g, 0.1, True)[0]
+    for _ in range(60):
+        pa, pb = ops.feature_map_fwd_pair(x, x, w, 0.1)
+        single, gx = ops.feature_map_fwd(x, w, 0.1), ops.feature_map_bwd(x, w, g, 0.1, True)[0]
+        assert torch.equal(pa, first) and torch.equal(pb, first) and torch.equal(single, first) and torch.equal(gx, grad)
