@@ -40,7 +40,7 @@ feature_map_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid
     return (pair ? (v >> 1) : v) * kTC;
   };
   if (tid == 0) {
-    for (int i = 0; i < 2; ++i) { mbar_init(&bars[bFull + i], 1); mbar_init(&bars[bEmpty + i], 1); mbar_init(&bars[bU + i], 1); mbar_init(&bars[bUFree + i], 128); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&bars[bFull + i], 1); mbar_init(&bars[bEmpty + i], 129); mbar_init(&bars[bU + i], 1); mbar_init(&bars[bUFree + i], 128); }
     mbar_init(&bars[bEpi], 128);
     mbar_fence_init();
     tma_prefetch_desc(&tm_x); tma_prefetch_desc(&tm_phi);
@@ -104,44 +104,55 @@ feature_map_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
     uint32_t epi_phase = 0;
     bool ok = true;
-    // The rows come from memory a second time (L2) for their norms, a tile ahead, and not from the staged tile: reads of a
-    // CTA's first tile right after its barrier, and even right after the product that used it, saw 16-byte pieces that had not
-    // landed (the product never did) -- rows off by a few percent in one launch of 300 at two CTAs per SM, in every third at
-    // three; what a neighbour's operand reads can hold back on shared memory is the likely reason, 3 us later all was well.
-    uint4 xr[8];
-    auto fetch = [&](int i) {
+    // The rows of a CTA's first tile come from memory a second time (L2) for their norms, not from the staged tile: reads of it
+    // right after its barrier, and even right after the product that used it, saw 16-byte pieces that had not landed (the
+    // product never did) -- rows off by a few percent in one launch of 300 at two CTAs per SM, in every third at three, always in
+    // the first tile; what a neighbour's operand reads can hold back on shared memory is the likely reason, 3 us later all was
+    // well.  Later tiles land while the tile before them is worked on and are read after their product.  (All tiles from
+    // memory: 24.4 us a launch of 16384 x 16 rows, the first one only 21.4, none 20.7.)
+    auto squares = [](uint4 u) {                       // of 16 bytes of a row; the eight are summed as a tree wherever they come from
+      const float2 f0 = unpack_half2(u.x), f1 = unpack_half2(u.y), f2 = unpack_half2(u.z), f3 = unpack_half2(u.w);
+      float t = f0.x * f0.x;
+      t = fmaf(f0.y, f0.y, t); t = fmaf(f1.x, f1.x, t); t = fmaf(f1.y, f1.y, t);
+      t = fmaf(f2.x, f2.x, t); t = fmaf(f2.y, f2.y, t); t = fmaf(f3.x, f3.x, t);
+      return fmaf(f3.y, f3.y, t);
+    };
+    float ss_first = 0.f;
+    if (ntile > 0) {
+      uint4 xr[8];                                     // eight lanes fetch a row, the warp four rows at a time
       int which;
-      const int row0 = i < ntile ? tile_row0(i, which) : 0;
-      const __half* src = (i < ntile && which) ? x2 : x;
+      const int64_t r0 = (int64_t)tile_row0(0, which) + quarter * 32 + (lane >> 3);
+      const __half* src = which ? x2 : x;
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        xr[j] = r0 + 4 * j < rows ? __ldg(reinterpret_cast<const uint4*>(src + ((size_t)(r0 + 4 * j) * H + h) * 64) + (lane & 7)) : make_uint4(0, 0, 0, 0);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const int64_t r = (int64_t)row0 + quarter * 32 + 4 * j + (lane >> 3);
-        xr[j] = i < ntile && r < rows ? __ldg(reinterpret_cast<const uint4*>(src + ((size_t)r * H + h) * 64) + (lane & 7)) : make_uint4(0, 0, 0, 0);
+        float t = squares(xr[j]);
+        t += __shfl_xor_sync(0xffffffffu, t, 1);
+        t += __shfl_xor_sync(0xffffffffu, t, 2);
+        t += __shfl_xor_sync(0xffffffffu, t, 4);
+        t = __shfl_sync(0xffffffffu, t, (lane & 3) * 8);
+        if ((lane >> 2) == j) ss_first = t;
       }
-    };
-    fetch(0);
+    }
     for (int i = 0; ok && i < ntile; ++i) {
       const int st = i & 1;
       int which;
       const int row0 = tile_row0(i, which);
       const uint8_t* mask = which ? row_mask2 : row_mask;
-      // |x|^2 of this thread's row: eight lanes hold each row that the warp fetched, four rows per fetch
-      float ss = 0.f;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const uint32_t xw[4] = {xr[j].x, xr[j].y, xr[j].z, xr[j].w};
-        float t = 0.f;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) { const float2 f = unpack_half2(xw[e]); t = fmaf(f.x, f.x, t); t = fmaf(f.y, f.y, t); }
-        t += __shfl_xor_sync(0xffffffffu, t, 1);
-        t += __shfl_xor_sync(0xffffffffu, t, 2);
-        t += __shfl_xor_sync(0xffffffffu, t, 4);
-        t = __shfl_sync(0xffffffffu, t, (lane & 3) * 8);
-        if ((lane >> 2) == j) ss = t;
-      }
-      const float inv = 1.f / (sqrtf(ss) + kNormEps);
+      if (!mbar_wait(&bars[bFull + st], (i >> 1) & 1)) { tc_fail(4); ok = false; break; }
       if (!mbar_wait(&bars[bU + st], (i >> 1) & 1)) { tc_fail(5); ok = false; break; }
       tc_fence_after_sync();
+      float ss = ss_first;                             // |x|^2 of this thread's row
+      if (i > 0) {
+        float t[8];
+#pragma unroll
+        for (int ch = 0; ch < 8; ++ch) t[ch] = squares(*reinterpret_cast<const uint4*>(sm + kX + st * kStage + row_chunk1(row, ch)));
+        ss = ((t[0] + t[1]) + (t[2] + t[3])) + ((t[4] + t[5]) + (t[6] + t[7]));
+      }
+      mbar_arrive(&bars[bEmpty + st]);
+      const float inv = 1.f / (sqrtf(ss) + kNormEps);
       uint32_t u[64];
       tmem_ld32(tmem + lane_addr + st * 64, u);
       tmem_ld32(tmem + lane_addr + st * 64 + 32, u + 32);
@@ -169,7 +180,6 @@ feature_map_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid
         *reinterpret_cast<uint4*>(sm + kOut + row_chunk1(row, ch)) = a;            // sin block
         *reinterpret_cast<uint4*>(sm + kOut + kBox + row_chunk1(row, ch)) = b;     // cos block
       }
-      fetch(i + 1);
       fence_async_smem();
       if (!epi_sync(&bars[bEpi], epi_phase)) { tc_fail(7); ok = false; break; }
       if (etid == 0) {
