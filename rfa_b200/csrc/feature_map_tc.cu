@@ -20,7 +20,7 @@ enum { bFull = 0, bEmpty = 2, bU = 4, bUFree = 6, bEpi = 8, bNum = 9 };
 __global__ void __launch_bounds__(fm::kThreads_, 3)
 feature_map_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_phi,
                           const __grid_constant__ CUtensorMap tm_x2, const __grid_constant__ CUtensorMap tm_phi2,
-                          const __half* __restrict__ x, const __half* __restrict__ x2, const float* __restrict__ w, const uint8_t* __restrict__ row_mask, const uint8_t* __restrict__ row_mask2,
+                          const float* __restrict__ w, const uint8_t* __restrict__ row_mask, const uint8_t* __restrict__ row_mask2,
                           int64_t rows, int H, float scale, int pair) {
   using namespace fm;
   extern __shared__ unsigned char fm_raw[];
@@ -104,55 +104,26 @@ feature_map_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
     uint32_t epi_phase = 0;
     bool ok = true;
-    // The rows of a CTA's first tile come from memory a second time (L2) for their norms, not from the staged tile: reads of it
-    // right after its barrier, and even right after the product that used it, saw 16-byte pieces that had not landed (the
-    // product never did) -- rows off by a few percent in one launch of 300 at two CTAs per SM, in every third at three, always in
-    // the first tile; what a neighbour's operand reads can hold back on shared memory is the likely reason, 3 us later all was
-    // well.  Later tiles land while the tile before them is worked on and are read after their product.  (All tiles from
-    // memory: 24.4 us a launch of 16384 x 16 rows, the first one only 21.4, none 20.7.)
-    auto squares = [](uint4 u) {                       // of 16 bytes of a row; the eight are summed as a tree wherever they come from
-      const float2 f0 = unpack_half2(u.x), f1 = unpack_half2(u.y), f2 = unpack_half2(u.z), f3 = unpack_half2(u.w);
-      float t = f0.x * f0.x;
-      t = fmaf(f0.y, f0.y, t); t = fmaf(f1.x, f1.x, t); t = fmaf(f1.y, f1.y, t);
-      t = fmaf(f2.x, f2.x, t); t = fmaf(f2.y, f2.y, t); t = fmaf(f3.x, f3.x, t);
-      return fmaf(f3.y, f3.y, t);
-    };
-    float ss_first = 0.f;
-    if (ntile > 0) {
-      uint4 xr[8];                                     // eight lanes fetch a row, the warp four rows at a time
-      int which;
-      const int64_t r0 = (int64_t)tile_row0(0, which) + quarter * 32 + (lane >> 3);
-      const __half* src = which ? x2 : x;
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-        xr[j] = r0 + 4 * j < rows ? __ldg(reinterpret_cast<const uint4*>(src + ((size_t)(r0 + 4 * j) * H + h) * 64) + (lane & 7)) : make_uint4(0, 0, 0, 0);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        float t = squares(xr[j]);
-        t += __shfl_xor_sync(0xffffffffu, t, 1);
-        t += __shfl_xor_sync(0xffffffffu, t, 2);
-        t += __shfl_xor_sync(0xffffffffu, t, 4);
-        t = __shfl_sync(0xffffffffu, t, (lane & 3) * 8);
-        if ((lane >> 2) == j) ss_first = t;
-      }
-    }
     for (int i = 0; ok && i < ntile; ++i) {
       const int st = i & 1;
       int which;
       const int row0 = tile_row0(i, which);
       const uint8_t* mask = which ? row_mask2 : row_mask;
       if (!mbar_wait(&bars[bFull + st], (i >> 1) & 1)) { tc_fail(4); ok = false; break; }
+      float ss = 0.f;                                  // |x|^2 of this thread's row, while the product is formed
+#pragma unroll
+      for (int ch = 0; ch < 8; ++ch) {
+        const uint4 u = *reinterpret_cast<const uint4*>(sm + kX + st * kStage + row_chunk1(row, ch));
+        float2 f;
+        f = unpack_half2(u.x); ss = fmaf(f.x, f.x, ss); ss = fmaf(f.y, f.y, ss);
+        f = unpack_half2(u.y); ss = fmaf(f.x, f.x, ss); ss = fmaf(f.y, f.y, ss);
+        f = unpack_half2(u.z); ss = fmaf(f.x, f.x, ss); ss = fmaf(f.y, f.y, ss);
+        f = unpack_half2(u.w); ss = fmaf(f.x, f.x, ss); ss = fmaf(f.y, f.y, ss);
+      }
+      mbar_release_stage(&bars[bEmpty + st]);
+      const float inv = 1.f / (sqrtf(ss) + kNormEps);
       if (!mbar_wait(&bars[bU + st], (i >> 1) & 1)) { tc_fail(5); ok = false; break; }
       tc_fence_after_sync();
-      float ss = ss_first;                             // |x|^2 of this thread's row
-      if (i > 0) {
-        float t[8];
-#pragma unroll
-        for (int ch = 0; ch < 8; ++ch) t[ch] = squares(*reinterpret_cast<const uint4*>(sm + kX + st * kStage + row_chunk1(row, ch)));
-        ss = ((t[0] + t[1]) + (t[2] + t[3])) + ((t[4] + t[5]) + (t[6] + t[7]));
-      }
-      mbar_arrive(&bars[bEmpty + st]);
-      const float inv = 1.f / (sqrtf(ss) + kNormEps);
       uint32_t u[64];
       tmem_ld32(tmem + lane_addr + st * 64, u);
       tmem_ld32(tmem + lane_addr + st * 64 + 32, u + 32);
@@ -210,7 +181,7 @@ int launch_feature_map_fwd_tc(const __half* x, const float* w, const uint8_t* ro
   int64_t gx = 3LL * sms / H;                    // three CTAs per SM, and never more CTAs than fit at once
   if (gx > ntile) gx = ntile;
   if (gx < 1) gx = 1;
-  launch_pdl(feature_map_fwd_tc_kernel, dim3((unsigned)gx, H), dim3(fm::kThreads_), fm::kSmem, st, tx, tp, tx2, tp2, x, pair ? x2 : x, w, row_mask, row_mask2,
+  launch_pdl(feature_map_fwd_tc_kernel, dim3((unsigned)gx, H), dim3(fm::kThreads_), fm::kSmem, st, tx, tp, tx2, tp2, w, row_mask, row_mask2,
              rows, H, scale, pair);
   return check_launch("rfa_feature_map_fwd");
 }
@@ -388,8 +359,6 @@ feature_map_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid
       // a masked row's features are constant zeros: no gradient flows through it
       const float scale_row = (mask && grow < rows && mask[grow]) ? 0.f : scale;
       if (!mbar_wait(&bars[bFull + sg], (i / kRing) & 1)) { tc_fail(16); break; }
-      if (!mbar_wait(&bars[bU + st], (i >> 1) & 1)) { tc_fail(17); break; }      // the norms after the product (see the forward)
-      tc_fence_after_sync();
       float ss = 0.f;                                  // |x|^2 of this thread's row
 #pragma unroll
       for (int ch = 0; ch < 8; ++ch) {
@@ -401,6 +370,8 @@ feature_map_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid
         f = unpack_half2(u.w); ss = fmaf(f.x, f.x, ss); ss = fmaf(f.y, f.y, ss);
       }
       const float n = sqrtf(ss), inv = 1.f / (n + kNormEps);
+      if (!mbar_wait(&bars[bU + st], (i >> 1) & 1)) { tc_fail(17); break; }
+      tc_fence_after_sync();
       uint32_t u[32];
       tmem_ld32(tmem + lane_addr + cU + st * 64 + half * 32, u);
       tmem_ld_wait();
@@ -427,9 +398,8 @@ feature_map_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid
         }
         *reinterpret_cast<uint4*>(sm + kGH + st * kBox + row_chunk1(row, ch)) = make_uint4(o[0], o[1], o[2], o[3]);
       }
-      fence_async_smem();
+      mbar_release_stage(&bars[bEmpty + sg]);          // this group's reads of the stage are done (the fence is the gh tile's, too)
       mbar_arrive(&bars[bGH + st]);
-      mbar_arrive(&bars[bEmpty + sg]);                 // this group's reads of the stage are done
     }
   } else {
     // ------------------------------------------------------------------ group 2: g_x
@@ -485,8 +455,7 @@ feature_map_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid
         }
         *reinterpret_cast<uint4*>(staging + row_chunk1(row, ch)) = make_uint4(o[0], o[1], o[2], o[3]);
       }
-      mbar_arrive(&bars[bEmpty + sg]);                 // this group's reads of the stage are done
-      fence_async_smem();
+      mbar_release_stage(&bars[bEmpty + sg]);          // this group's reads of the stage are done (the fence is the staging tile's, too)
       if (!epi_sync(&bars[bEpi], epi_phase)) { tc_fail(23); ok = false; break; }
       if (etid == 0) {
         tma_store_3d(which ? &tm_gx2 : &tm_gx, staging, 0, h, row0);

@@ -104,6 +104,16 @@ __device__ __forceinline__ void st_global_v8(void* p, const uint32_t (&v)[8]) {
 // ---- proxies / fences ---------------------------------------------------------
 // Generic-proxy writes to shared memory -> visible to the async proxy (TMA, UMMA).
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+// Give a staged tile back to the TMA producer, by a thread that has READ it with plain loads.  The refill is a write of the
+// async proxy, and an arrive alone does not keep this thread's plain reads in front of it: the loads may still sit in
+// the load/store queue, behind global loads of this or a neighbouring CTA, when the arrive has been counted and the
+// refill lands.  The proxy fence waits for them.  Without it the feature map's forward mixed 16-byte pieces of the tile two
+// further on into its row norms, in 6 to 20 of 100 launches (the refilled tile's values in every wrong row; 0 of 9600
+// launches with the fence, and 0 of 4800 with an arrive that depends on the loaded values).
+__device__ __forceinline__ void mbar_release_stage(uint64_t* bar) {
+  fence_async_smem();
+  mbar_arrive(bar);
+}
 __device__ __forceinline__ void tc_fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
