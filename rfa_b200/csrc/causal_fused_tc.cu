@@ -52,12 +52,11 @@ static_assert(kSmem <= 227 * 1024, "causal_fwd_fused: shared memory map");
 // TMEM columns
 constexpr uint32_t cA = 0, cN = 128, cS = 288, cUq = 368, cUk = 432;
 enum { xFull = 0, xEmpty = 2, vFull = 4, vEmpty = 6, uFull = 8, uFree = 9, phiFull = 10, phiFree = 11, aFull = 12, pFull = 13,
-       sDone = 14, nFull = 16, nFree = 18, bSt = 20, bCarry = 21, bNum = 22 };
+       sDone = 14, nFull = 16, nFree = 18, bSt = 20, bNum = 21 };
 // xFull/xEmpty: a raw stage (free once U has been formed from it and both feature groups have taken their rows' norms);
 // vFull/vEmpty: a V tile (free once P V and the state update have read it); uFull/uFree: the U accumulators;
 // phiFull/phiFree: the feature tiles (free = both issuers' products of the chunk are complete); aFull/pFull: scores
-// written / packed; sDone (per N buffer): issuer B's products complete; nFull/nFree: an N buffer; bSt: state tile exported;
-// bCarry: the state entering the sequence has been loaded (the producer starts after it).
+// written / packed; sDone (per N buffer): issuer B's products complete; nFull/nFree: an N buffer; bSt: state tile exported.
 }  // namespace fz
 
 __global__ void __launch_bounds__(fz::kThreads_, 1)
@@ -96,7 +95,6 @@ causal_fwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tm_xq, const __gr
     mbar_init(&bars[aFull], 1);
     mbar_init(&bars[pFull], 128);
     mbar_init(&bars[bSt], 128);
-    mbar_init(&bars[bCarry], 128);
     mbar_fence_init();
     tma_prefetch_desc(&tm_xq); tma_prefetch_desc(&tm_xk); tma_prefetch_desc(&tm_v);
   }
@@ -135,10 +133,6 @@ causal_fwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tm_xq, const __gr
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
-      // The state entering the sequence is fetched by the output/state group before the first TMA load is issued: with
-      // those global loads in flight while the first raw tiles landed, the feature warps' first reads of the tiles
-      // returned stale data in an earlier version of this kernel.
-      if (s_in && !mbar_wait(&bars[bCarry], 0)) tc_fail(20);
       for (int c = 0; c < nchunk; ++c) {
         const int st = c & 1;
         const int t0 = c * kTC;
@@ -292,13 +286,6 @@ causal_fwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tm_xq, const __gr
       r[64] = z_in ? __float_as_uint(z_in[row]) : 0u;
 #pragma unroll
       for (int n = 65; n < 80; ++n) r[n] = 0u;
-      if (s_in) {                       // every value has arrived (they are used below): the producer may start
-        uint32_t any = 0;
-#pragma unroll
-        for (int n = 0; n < 65; ++n) any |= r[n];
-        asm volatile("" ::"r"(any) : "memory");
-        mbar_arrive(&bars[bCarry]);
-      }
       store_state_row(s_tile, row, r);
 #pragma unroll
       for (int ch = 1; ch < 8; ++ch) *reinterpret_cast<uint4*>(s_tile + kBox + row_chunk1(row, ch)) = make_uint4(0, 0, 0, 0);
@@ -395,13 +382,11 @@ causal_fwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tm_xq, const __gr
       const unsigned char* raw = sm + st * kRaw + (is_key ? kXk : kXq);
       const int64_t t = (int64_t)c * kTC + row;
       if (!mbar_wait(&bars[xFull + st], (c >> 1) & 1)) { tc_fail(17); break; }
-      // the row's norm is taken only once U has been formed from the tile (see below): by then the tensor pipe has read
-      // every byte of it
       if (!mbar_wait(&bars[uFull], c & 1)) { tc_fail(18); break; }
       tc_fence_after_sync();
       uint32_t u[32];
       tmem_ld32(tmem + lane_addr + colU + 32 * half, u);
-      float ss = 0.f, ss_b = 0.f;                    // |x|^2 of this thread's row
+      float ss = 0.f, ss_b = 0.f;                    // |x|^2 of this thread's row, while U is on its way from tensor memory
 #pragma unroll
       for (int ch = 0; ch < 8; ++ch) {
         const uint4 xr = *reinterpret_cast<const uint4*>(raw + row_chunk1(row, ch));
@@ -411,7 +396,7 @@ causal_fwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tm_xq, const __gr
         f = unpack_half2(xr.z); ss = fmaf(f.x, f.x, ss); ss_b = fmaf(f.y, f.y, ss_b);
         f = unpack_half2(xr.w); ss = fmaf(f.x, f.x, ss); ss_b = fmaf(f.y, f.y, ss_b);
       }
-      mbar_arrive(&bars[xEmpty + st]);
+      mbar_release_stage(&bars[xEmpty + st]);
       const float inv = 1.f / (sqrtf(ss + ss_b) + kNormEps);
       // a key past the end of the sequence or masked as padding contributes nothing: all-zero features
       float sc = scale;

@@ -47,3 +47,17 @@ def test_feature_map(dev, pair):
     else:
         check(lambda: (ops.feature_map_fwd(x, w, 0.1),))
         check(lambda: ops.feature_map_bwd(x, w, g, 0.1, False)[:1])
+
+
+@pytest.mark.parametrize("carried", [False, True])
+def test_fused_forward(dev, carried):
+    """Feature map and attention in one kernel; the state carried in adds 64 global loads a thread in front of the first tiles."""
+    from rfa_b200 import ops
+    gen = torch.Generator("cuda").manual_seed(2)
+    B, H, T = 8, 16, 1024
+    w = torch.randn(H, 64, 64, generator=gen, device="cuda")
+    xq, xk = (tiles(gen, T, B, H, 64) for _ in range(2))
+    v = torch.randn(T, B, H, 64, generator=gen, device="cuda").half()
+    s = torch.randn(B * H, 128, 64, generator=gen, device="cuda") if carried else None
+    z = torch.rand(B * H, 128, generator=gen, device="cuda") if carried else None
+    check(lambda: ops.causal_fwd_fused(xq, xk, v, w, 0.1, s_in=s, z_in=z, return_state=True))
