@@ -156,7 +156,7 @@ cross_state_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid
         mbar_arrive(&bars[bReady + st]);
       }
       z_acc += column_sum2(stage + kK_, quarter, lane, nullptr);
-      mbar_arrive(&bars[bEmpty + st]);
+      mbar_release_stage(&bars[bEmpty + st]);
     }
     if (ok) {
       uint32_t r[64];

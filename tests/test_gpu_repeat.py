@@ -61,3 +61,18 @@ def test_fused_forward(dev, carried):
     s = torch.randn(B * H, 128, 64, generator=gen, device="cuda") if carried else None
     z = torch.rand(B * H, 128, generator=gen, device="cuda") if carried else None
     check(lambda: ops.causal_fwd_fused(xq, xk, v, w, 0.1, s_in=s, z_in=z, return_state=True))
+
+
+def test_cross(dev):
+    """Two CTAs per SM (256 sequences), padded rows that hold data."""
+    from rfa_b200 import ops
+    gen = torch.Generator("cuda").manual_seed(3)
+    T, B, H = 1024, 16, 16
+    phi = features(gen, T, B, H, 128)
+    v, g = tiles(gen, T, B, H, 64), torch.randn(T, B, H, 64, generator=gen, device="cuda").half()
+    pad = torch.arange(T, device="cuda")[None] >= torch.randint(T // 2, T + 1, (B, 1), generator=gen, device="cuda")
+    s, z = ops.cross_state_fwd(phi, v, pad)
+    check(lambda: ops.cross_state_fwd(phi, v, pad))
+    check(lambda: (ops.cross_query_fwd(phi, s, z),), 752)
+    check(lambda: ops.cross_query_bwd(phi, s, z, g), 752)
+    check(lambda: ops.cross_state_bwd(phi, v, pad, s, z), 752)
