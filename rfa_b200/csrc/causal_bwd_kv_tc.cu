@@ -281,7 +281,7 @@ causal_bwd_kv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
       if (!mbar_wait(&bars[vFullKQ + st], (i >> 1) & 1)) { tc_fail(16); break; }
       if (!mbar_wait(&bars[vG + st], (i >> 1) & 1)) { tc_fail(17); break; }
       dz_run += column_sum2(sm + st * kvStage + kvQ, quarter, lane, gz_buf + st * 128);
-      mbar_arrive(&bars[vEmpty + st]);             // this group's last read of the stage's tiles
+      mbar_release_stage(&bars[vEmpty + st]);      // this group's last read of the stage's tiles
       dzs[((i + 1) % 3) * 128 + row] = dz_run;
       mbar_arrive(&bars[vDz + (i + 1) % 3]);
     }

@@ -253,7 +253,7 @@ causal_bwd_q_saved_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __g
         if (!mbar_wait(&bars[sG + st], (c >> 1) & 1)) { tc_fail(11); break; }
         if (!mbar_wait(&bars[sFullK + st], (c >> 1) & 1)) { tc_fail(12); break; }
         if (dseg) dz_acc += column_sum2(sm + st * L::Stage + L::Q, quarter, lane, rg_buf + st * 128);
-        mbar_arrive(&bars[sEmpty + st]);
+        mbar_release_stage(&bars[sEmpty + st]);
       }
     }
     if (dseg) dz_seg[slot * kK + row] = dz_acc;       // (zero when the run has no tokens)
@@ -338,7 +338,7 @@ causal_bwd_q_saved_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __g
       //      group's epilogue of chunk c - 2) read it before it released dQ for chunk c - 1, which precedes this chunk's dA.
       if (!mbar_wait(&bars[sFullK + st], (c >> 1) & 1)) { tc_fail(15); break; }
       zrun += column_sum2(stage + L::K, quarter, lane, nullptr);
-      mbar_arrive(&bars[sEmpty + st]);             // this group's last read of the stage's tiles
+      mbar_release_stage(&bars[sEmpty + st]);      // this group's last read of the stage's tiles
       z_buf[((c + 1) % 3) * 128 + row] = zrun;
       mbar_arrive(&bars[sZ + (c + 1) % 3]);
     }
@@ -358,7 +358,7 @@ causal_bwd_q_saved_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __g
       //      the stage has been released
       if (!mbar_wait(&bars[sG + st], (c >> 1) & 1)) { tc_fail(17); ok = false; break; }
       const float gz = rg_buf[st * 128 + row];
-      mbar_arrive(&bars[sEmpty + st]);
+      mbar_release_stage(&bars[sEmpty + st]);
       if (!mbar_wait(&bars[sZ + c % 3], (c / 3) & 1)) { tc_fail(19); ok = false; break; }
       // ---- !WANT_DSEG: the staging tile of chunk c - 2 has been read out by its store
       if (!WANT_DSEG) {

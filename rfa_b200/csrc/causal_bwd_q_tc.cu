@@ -409,7 +409,7 @@ causal_bwd_q_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
       if (!mbar_wait(&bars[qG + st], (c >> 1) & 1)) { tc_fail(17); ok = false; break; }
       if (want_dseg) dz_acc += column_sum2(stage + bqQ, quarter, lane, gzs);      // dzseg += Q^T gz
       const float gz = gzs[row];
-      mbar_arrive(&bars[qEmpty + st]);             // this group's last read of the stage's tiles
+      mbar_release_stage(&bars[qEmpty + st]);      // this group's last read of the stage's tiles
       // ---- grad_q = dQ + gz z_prev^T -> fp16, written straight from registers (one 256-byte row per thread)
       if (!mbar_wait(&bars[qDQ + st], (c >> 1) & 1)) { tc_fail(18); ok = false; break; }
       tc_fence_after_sync();

@@ -76,3 +76,16 @@ def test_cross(dev):
     check(lambda: (ops.cross_query_fwd(phi, s, z),), 752)
     check(lambda: ops.cross_query_bwd(phi, s, z, g), 752)
     check(lambda: ops.cross_state_bwd(phi, v, pad, s, z), 752)
+
+
+@pytest.mark.parametrize("T,BH", [(1024, 128), (3072, 36)])
+def test_causal_backward(dev, T, BH):
+    """Both sweeps, from the saved output and recomputing, whole sequences and cut ones (with the segments' reverse totals)."""
+    from rfa_b200 import ops
+    gen = torch.Generator("cuda").manual_seed(T)
+    q, k = (features(gen, T, BH, 128) for _ in range(2))
+    v, g = tiles(gen, T, BH, 64), torch.randn(T, BH, 64, generator=gen, device="cuda").half()
+    out, ws, has = ops.causal_fwd_saved(q, k, v)
+    check(lambda: ops.causal_fwd_saved(q, k, v)[:1])
+    check(lambda: ops.causal_bwd_saved(q, k, v, g, out, ws, has))
+    check(lambda: ops.causal_bwd(q, k, v, g), 752)

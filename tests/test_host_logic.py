@@ -109,3 +109,21 @@ def test_matrix_sampling_with_a_generator_is_reproducible():
     x = sample_matrix_indices(num_layers=2, num_heads=2, bank_size=9)        # upstream's way: numpy's global RNG
     np.random.seed(3)
     assert x.tolist() == np.random.choice(9, size=4, replace=False).tolist()
+
+
+def test_staged_tiles_are_released_behind_the_proxy_fence():
+    """A stage that TMA refills is given back through ``mbar_release_stage`` (fence, then arrive): an arrive alone does not keep
+    the thread's plain reads of the tile in front of the refill.  Where a TMA store has read the stage, the wait for it does."""
+    import glob
+    import os
+    import re
+    root = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "rfa_b200", "csrc")
+    sites = 0
+    for path in sorted(glob.glob(os.path.join(root, "*.cu"))):
+        lines = open(path).read().splitlines()
+        for i, line in enumerate(lines):
+            if re.search(r"mbar_release_stage\(&bars\[\w*Empty", line):
+                sites += 1
+            if re.search(r"mbar_arrive\(&bars\[\w*Empty", line):
+                assert "tma_store_wait_read<0>()" in lines[i - 1], f"{os.path.basename(path)}:{i + 1}: {line.strip()}"
+    assert sites >= 9
