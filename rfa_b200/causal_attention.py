@@ -12,6 +12,7 @@ from typing import Dict, Optional
 
 import torch
 from torch import Tensor, nn
+from torch.autograd.forward_ad import unpack_dual
 from torch.nn import Parameter
 
 from . import ops
@@ -178,6 +179,14 @@ def fused_causal_rfa(*, q: Tensor, k: Tensor, v: Tensor, random_matrices: Tensor
     return attn.view(tgt_len, bsz, num_heads * head_dim)
 
 
+def _underived(*tensors: Optional[Tensor]) -> bool:
+    """Whether a call on these may go past the autograd functions: nothing is recorded and none carries a forward-mode
+    tangent (which those functions refuse, and a plain kernel call would drop)."""
+    if torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors):
+        return False
+    return all(t is None or unpack_dual(t).tangent is None for t in tensors)
+
+
 class CausalAttention(nn.Module):
     """Random feature causal self-attention layer (upstream causal_attention.py:154-280):
     q/k/v projections, per-head feature map with W' = sigma * W / tau, causal RFA,
@@ -258,9 +267,8 @@ class CausalAttention(nn.Module):
             # request (fuse_feature_map), because the backward then has to form the features again
             attn = fused_causal_rfa(q=q, k=k, v=v, random_matrices=w, key_padding_mask=key_padding_mask)
             return self.out_proj(attn.to(x.dtype))
-        if saved_state is not None and not (torch.is_grad_enabled() and any(
-                t is not None and t.requires_grad for t in (q, k, v, w, saved_state.get("prev_s"), saved_state.get("prev_z")))) \
-                and ops.decode_fused_supported(q, w):
+        if saved_state is not None and ops.decode_fused_supported(q, w) \
+                and _underived(q, k, v, w, saved_state.get("prev_s"), saved_state.get("prev_z")):
             assert tgt_len == 1
             attn = self._decode_step(q[0], k[0], v[0], w, saved_state)
             return self.out_proj(attn.reshape(1, bsz, embed_dim).to(x.dtype))

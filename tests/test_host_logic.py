@@ -3,6 +3,7 @@ and the upstream-generated fixtures."""
 import argparse
 
 import numpy as np
+import pytest
 import torch
 
 from conftest import golden
@@ -127,3 +128,27 @@ def test_staged_tiles_are_released_behind_the_proxy_fence():
             if re.search(r"mbar_arrive\(&bars\[\w*Empty", line):
                 assert "tma_store_wait_read<0>()" in lines[i - 1], f"{os.path.basename(path)}:{i + 1}: {line.strip()}"
     assert sites >= 9
+
+
+@pytest.mark.parametrize("what", ["x", "sigma"])
+def test_one_token_refuses_forward_mode(monkeypatch, what):
+    """A tangent reaches the feature map's autograd function, which has no forward-mode rule, instead of being dropped by the
+    fused decoding step (a plain kernel call)."""
+    import torch.autograd.forward_ad as fw
+    from rfa_b200 import CausalAttention, ops
+    monkeypatch.setattr(ops, "decode_fused_supported", lambda q, w: True)
+    monkeypatch.setattr(ops, "decode_step_fused", lambda q, k, v, w, scale, s, z: v.clone())
+    monkeypatch.setattr(ops, "feature_map_fwd", lambda x, w, scale, row_mask=None: torch.cat([x, x], dim=-1))
+    layer = CausalAttention(embed_dim=16, num_heads=2, head_dim=8, proj_dim=8)
+    x, w = torch.randn(1, 3, 16), torch.randn(2, 8, 8)
+    with torch.no_grad():
+        assert layer(x, w, saved_state={}).shape == x.shape
+        with fw.dual_level():
+            if what == "x":
+                x = fw.make_dual(x, torch.ones_like(x))
+            else:
+                sigma = layer.sigma.detach()
+                del layer.sigma
+                layer.sigma = fw.make_dual(sigma, torch.ones_like(sigma))
+            with pytest.raises(NotImplementedError, match="jvp"):
+                layer(x, w, saved_state={})
