@@ -21,12 +21,18 @@ using OptTensor = std::optional<Tensor>;
 
 namespace {
 
+// The calls run without the interpreter lock (see the module's end); what touches Python objects takes it.
 [[noreturn]] void raise(PyObject* type, const std::string& msg) {
+  py::gil_scoped_acquire lock;
   PyErr_SetString(type, msg.c_str());
   throw py::error_already_set();
 }
-std::string dtype_name(const Tensor& t) { return py::str(py::cast(t).attr("dtype")).cast<std::string>(); }
-std::string shape_name(const Tensor& t) { return py::str(py::cast(t).attr("shape")).cast<std::string>(); }
+std::string attr_name(const Tensor& t, const char* attr) {
+  py::gil_scoped_acquire lock;
+  return py::str(py::cast(t).attr(attr)).cast<std::string>();
+}
+std::string dtype_name(const Tensor& t) { return attr_name(t, "dtype"); }
+std::string shape_name(const Tensor& t) { return attr_name(t, "shape"); }
 
 void require_cuda(const Tensor& t) {
   if (!t.is_cuda())
@@ -118,7 +124,7 @@ OptTensor mask_bytes(const OptTensor& mask, int64_t n, const Tensor& like) {
 // ---- feature map ---------------------------------------------------------------------------------------------------------
 void check_feature_shapes(const Tensor& x, const Tensor& w) {
   rank(w, 3);
-  require(x.dim() >= 2 && x.size(-2) == w.size(0) && x.size(-1) == w.size(2), shapes(x, w));
+  if (!(x.dim() >= 2 && x.size(-2) == w.size(0) && x.size(-1) == w.size(2))) raise(PyExc_AssertionError, shapes(x, w));
 }
 Tensor phi_like(const Tensor& x, const Tensor& w, at::ScalarType dtype) {
   auto shape = x.sizes().vec();
@@ -157,7 +163,7 @@ std::tuple<Tensor, OptTensor> feature_map_bwd(Tensor x, Tensor w, Tensor g_phi, 
 }
 
 std::tuple<Tensor, Tensor> feature_map_fwd_pair(Tensor a, Tensor b, Tensor w, double scale, const OptTensor& mask_a, const OptTensor& mask_b) {
-  require(a.sizes() == b.sizes(), shapes(a, b));
+  if (a.sizes() != b.sizes()) raise(PyExc_AssertionError, shapes(a, b));
   check_feature_shapes(a, w);
   require_half(a, b);
   a = a.contiguous(); b = b.contiguous();
@@ -360,19 +366,22 @@ Tensor decode_step_fused(Tensor q, Tensor k, Tensor v, const Tensor& w, double s
 
 }  // namespace
 
+// Without the interpreter lock, as the foreign calls before them: an allocation, a launch on a full queue or the synchronisation
+// of an error report blocks this thread only.
 PYBIND11_MODULE(_native, m) {
-  m.def("feature_map_fwd", &feature_map_fwd);
-  m.def("feature_map_bwd", &feature_map_bwd);
-  m.def("feature_map_fwd_pair", &feature_map_fwd_pair);
-  m.def("feature_map_bwd_pair", &feature_map_bwd_pair);
-  m.def("causal_fwd", &causal_fwd);
-  m.def("causal_fwd_saved", &causal_fwd_saved);
-  m.def("causal_bwd_saved", &causal_bwd_saved);
-  m.def("causal_fwd_fused", &causal_fwd_fused);
-  m.def("cross_state_fwd", &cross_state_fwd);
-  m.def("cross_state_bwd", &cross_state_bwd);
-  m.def("cross_query_fwd", &cross_query_fwd);
-  m.def("cross_query_bwd", &cross_query_bwd);
-  m.def("decode_step", &decode_step);
-  m.def("decode_step_fused", &decode_step_fused);
+  const auto def = [&](const char* name, auto* f) { m.def(name, f, py::call_guard<py::gil_scoped_release>()); };
+  def("feature_map_fwd", &feature_map_fwd);
+  def("feature_map_bwd", &feature_map_bwd);
+  def("feature_map_fwd_pair", &feature_map_fwd_pair);
+  def("feature_map_bwd_pair", &feature_map_bwd_pair);
+  def("causal_fwd", &causal_fwd);
+  def("causal_fwd_saved", &causal_fwd_saved);
+  def("causal_bwd_saved", &causal_bwd_saved);
+  def("causal_fwd_fused", &causal_fwd_fused);
+  def("cross_state_fwd", &cross_state_fwd);
+  def("cross_state_bwd", &cross_state_bwd);
+  def("cross_query_fwd", &cross_query_fwd);
+  def("cross_query_bwd", &cross_query_bwd);
+  def("decode_step", &decode_step);
+  def("decode_step_fused", &decode_step_fused);
 }

@@ -152,3 +152,34 @@ def test_one_token_refuses_forward_mode(monkeypatch, what):
                 layer.sigma = fw.make_dual(sigma, torch.ones_like(sigma))
             with pytest.raises(NotImplementedError, match="jvp"):
                 layer(x, w, saved_state={})
+
+
+def test_native_calls_leave_the_interpreter_to_other_threads():
+    """The tensor-level calls run without the interpreter lock.  The time is that of a strided copy of the input, which
+    comes before the call finds that it is on the CPU."""
+    import threading
+    import time
+    from rfa_b200 import ops
+    x, w = torch.zeros(64, 1 << 20).t().unsqueeze(1), torch.zeros(1, 8, 64)
+    ticks, stop = [], threading.Event()
+
+    def tick():
+        while not stop.is_set():
+            ticks.append(time.perf_counter())
+            time.sleep(1e-3)
+    threads = torch.get_num_threads()
+    torch.set_num_threads(1)
+    other = threading.Thread(target=tick)
+    other.start()
+    try:
+        time.sleep(0.02)
+        t0 = time.perf_counter()
+        with pytest.raises(RuntimeError, match="CUDA tensors only"):
+            ops.feature_map_fwd(x, w, 0.1)
+        t1 = time.perf_counter()
+    finally:
+        stop.set()
+        other.join()
+        torch.set_num_threads(threads)
+    seen = [t0] + [t for t in ticks if t0 < t < t1] + [t1]
+    assert max(b - a for a, b in zip(seen, seen[1:])) < 0.5 * (t1 - t0), (len(seen), t1 - t0)
