@@ -203,6 +203,7 @@ std::tuple<Tensor, OptTensor, OptTensor> causal_fwd(Tensor q, Tensor k, Tensor v
   require(v.dim() >= 2 && k.sizes() == q.sizes() && v.size(0) == q.size(0) && v.size(1) == q.size(1));
   q = q.contiguous(); k = k.contiguous(); v = v.contiguous();
   const int64_t T = q.size(0), BH = q.size(1), K = q.size(2), d = v.size(-1);
+  if (s_in && !z_in) raise(PyExc_ValueError, "rfa_b200: a state is given as the pair (s, z), got s alone");
   Tensor out = fresh({T, BH, d}, q, at::kHalf);
   const OptTensor s = f32(s_in), z = f32(z_in);
   if (T == 0) {      // nothing to launch (empty tensors have no address); the state passes through

@@ -183,3 +183,11 @@ def test_native_calls_leave_the_interpreter_to_other_threads():
         torch.set_num_threads(threads)
     seen = [t0] + [t for t in ticks if t0 < t < t1] + [t1]
     assert max(b - a for a, b in zip(seen, seen[1:])) < 0.5 * (t1 - t0), (len(seen), t1 - t0)
+
+
+@pytest.mark.parametrize("T", [0, 3])
+def test_a_state_without_its_denominators_is_refused(T):
+    from rfa_b200 import ops
+    q, v = torch.zeros(T, 2, 128, dtype=torch.half), torch.zeros(T, 2, 64, dtype=torch.half)
+    with pytest.raises(ValueError, match="pair"):
+        ops.causal_fwd(q, q, v, torch.zeros(2, 128, 64), None, return_state=True)
