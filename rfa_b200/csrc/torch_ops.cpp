@@ -121,6 +121,11 @@ OptTensor mask_bytes(const OptTensor& mask, int64_t n, const Tensor& like) {
   return m;
 }
 
+// A padding mask [B, T] (any shape that views as one).
+OptTensor pad_bytes(const OptTensor& pad, int64_t B, int64_t T, const Tensor& like) {
+  return pad ? mask_bytes(pad->reshape({B, T}), B * T, like) : pad;
+}
+
 // ---- feature map ---------------------------------------------------------------------------------------------------------
 void check_feature_shapes(const Tensor& x, const Tensor& w) {
   rank(w, 3);
@@ -282,7 +287,7 @@ std::tuple<Tensor, Tensor> cross_state_fwd(Tensor phi_k, Tensor v, const OptTens
   rank(phi_k, 4);
   phi_k = phi_k.contiguous(); v = v.contiguous();
   const int64_t T = phi_k.size(0), B = phi_k.size(1), H = phi_k.size(2), K = phi_k.size(3), d = v.size(-1);
-  const OptTensor m = mask_bytes(pad, B * T, phi_k);
+  const OptTensor m = pad_bytes(pad, B, T, phi_k);
   Tensor s = fresh({B, H, K, d}, phi_k, at::kFloat), z = fresh({B, H, K}, phi_k, at::kFloat);
   Call c(phi_k);
   check(rfa_cross_state_fwd(ptr(phi_k), ptr(v), bptr(m), fptr(s), fptr(z), T, B, H, K, d, c.stream), "rfa_cross_state_fwd");
@@ -294,7 +299,7 @@ std::tuple<Tensor, Tensor> cross_state_bwd(Tensor phi_k, Tensor v, const OptTens
   phi_k = phi_k.contiguous(); v = v.contiguous();
   d_s = f32(d_s); d_z = f32(d_z);
   const int64_t T = phi_k.size(0), B = phi_k.size(1), H = phi_k.size(2), K = phi_k.size(3), d = v.size(-1);
-  const OptTensor m = mask_bytes(pad, B * T, phi_k);
+  const OptTensor m = pad_bytes(pad, B, T, phi_k);
   Tensor g_k = fresh_like(phi_k), g_v = fresh_like(v);
   Call c(phi_k);
   check(rfa_cross_state_bwd(ptr(phi_k), ptr(v), bptr(m), fptr(d_s), fptr(d_z), ptr(g_k), ptr(g_v), T, B, H, K, d, c.stream), "rfa_cross_state_bwd");

@@ -191,3 +191,12 @@ def test_a_state_without_its_denominators_is_refused(T):
     q, v = torch.zeros(T, 2, 128, dtype=torch.half), torch.zeros(T, 2, 64, dtype=torch.half)
     with pytest.raises(ValueError, match="pair"):
         ops.causal_fwd(q, q, v, torch.zeros(2, 128, 64), None, return_state=True)
+
+
+def test_a_padding_mask_of_another_size_raises_a_runtime_error():
+    from rfa_b200 import ops
+    phi, v = torch.zeros(4, 2, 3, 128, dtype=torch.half), torch.zeros(4, 2, 3, 64, dtype=torch.half)
+    with pytest.raises(RuntimeError, match="shape"):
+        ops.cross_state_fwd(phi, v, torch.zeros(3, 3))
+    with pytest.raises(RuntimeError, match="shape"):
+        ops.cross_state_bwd(phi, v, torch.zeros(3, 3), torch.zeros(2, 3, 128, 64), torch.zeros(2, 3, 128))
