@@ -24,8 +24,7 @@
  * all weights in fp32 where a chunk's tiles fit beside the state, else on
  * kernels that walk a sequence token by token, as upstream's do
  * (cuda/forward.cu:112-125); so do cross attention's query kernels and state
- * backward.  Of these geometries rfa_causal_fwd also takes a NULL workspace:
- * sequences are then not cut into segments.
+ * backward.
  * The packed-total / gathered-scan entry points of the sequence-sharded path and
  * rfa_causal_bwd_noalloc exist for K == 128, d == 64 only.  Unsupported
  * geometries are rejected with RFA_EUNSUPPORTED.  fp16 arrays are IEEE binary16.
@@ -152,6 +151,10 @@ int rfa_gather_random_matrices(const void* bank, int bank_dtype, int64_t n_bank,
  * tokens before this call's first token; s_out/z_out (may be NULL) receives
  * the state after its last token (prefill -> decode hand-off; segment carry).
  * workspace: rfa_causal_workspace_bytes(T,BH,K,d) bytes, 256-byte aligned.
+ * rfa_causal_fwd may be given none (NULL, or one that does not fit): sequences are
+ * then not cut into segments, which costs time where few long ones leave the GPU
+ * idle.  At K = 128, d = 64 that holds below 1024 tokens and above 74 (batch, head)
+ * pairs; from 1024 tokens on with at most 74 it is RFA_EWORKSPACE.
  * ---------------------------------------------------------------------- */
 size_t rfa_causal_workspace_bytes(int64_t T, int BH, int K, int d);
 

@@ -321,11 +321,13 @@ extern "C" int rfa_causal_fwd_staged(const void* q, const void* k, const void* v
     return launch_causal_generic_fwd((const __half*)q, (const __half*)k, (const __half*)v, (__half*)out, s_in, z_in, s_out, z_out,
                                      save_den ? gws.den : nullptr, T, BH, K, d, st);
   }
-  // a plain forward of these geometries asks for no workspace: without one the sequences stay whole
-  if (chunked && !save_den && (!workspace || ((uintptr_t)workspace & 255u) || workspace_bytes < carve_ws(nullptr, T, BH, K, d, p).bytes))
+  // Who has to bring a workspace is part of the interface and does not follow the plan: a forward that saves denominators, and at
+  // K = 128, d = 64 one of 1024 tokens and more with two or more segments to a wave.  Without one that fits the rest run whole.
+  const bool required = save_den || (is_tc(K, d) && T >= 1024 && kSms / BH >= 2);
+  if (!required && (!workspace || ((uintptr_t)workspace & 255u) || workspace_bytes < carve_ws(nullptr, T, BH, K, d, p).bytes))
     p = CausalPlan{1, cut_segments(T, kSegAlign, 1, 0).tseg};
   CausalWs ws{};
-  if (p.nseg > 1 || save_den)
+  if (p.nseg > 1 || required)
     if (int e = check_ws("causal_fwd", workspace, workspace_bytes, T, BH, K, d, p, &ws)) return e;
   if (p.nseg > 1) {
     if (!(ws_has & RFA_WS_PARTIALS) || chunked)      // (rfa_causal_shard_total, which leaves them, is not built for these)

@@ -583,6 +583,21 @@ def test_feature_map_pair_equals_two_single_launches(dev, rows, B, H, masked):
     assert_close(gxa, want_a, "g_x (pair, first array)")
 
 
+@pytest.mark.parametrize("T,BH,status", [(896, 2, 0), (900, 2, 0), (1000, 37, 0), (1023, 2, 0), (1024, 2, -4), (1024, 70, -4), (1024, 75, 0)])
+def test_forward_without_a_workspace(dev, T, BH, status):
+    """Whether the sequences would be cut or not: below 1024 tokens, or with less than two segments to a wave, none is needed; above
+    that one is, which is said before anything is launched.  The result is that of a forward with one up to the rounding
+    of sums in another order."""
+    import ctypes
+    from rfa_b200 import _lib, ops
+    q, k, v, _ = (t.half().to(dev) for t in generic_feats(T, BH, 128, 64, 3))
+    bare = torch.empty_like(v)
+    assert _lib.load().rfa_causal_fwd(*(t.data_ptr() for t in (q, k, v, bare)), None, None, None, None, None, ctypes.c_size_t(0),
+                                      T, BH, 128, 64, _lib.stream_of(q)) == status
+    if status == 0:
+        assert_close(bare, ops.causal_fwd(q, k, v), "out without a workspace")
+
+
 def test_feature_map_is_bit_stable(dev):
     """Repeated launches on the same inputs: the rows' norms must come from the tile that has landed, never from what the
     stage held before (a launch in three went wrong in a few rows of a CTA's first tile when they were read too early)."""
