@@ -19,6 +19,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(CSRC, "librfa_b200.so")
 NATIVE_SRC, NATIVE = os.path.join(CSRC, "torch_ops.cpp"), os.path.join(HERE, "_native.so")
+NATIVE_KEY = os.path.join(HERE, "_native.key")      # what the module was built for (see native_key)
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -68,9 +69,22 @@ def compile_one(src: str, verbose: bool) -> str:
     return obj
 
 
+def native_key() -> str:
+    """The interpreter and the torch an extension module is tied to."""
+    import torch
+    return f"torch {torch.__version__} cxx11-abi {int(torch._C._GLIBCXX_USE_CXX11_ABI)} python {sys.implementation.cache_tag}\n"
+
+
+def native_stale() -> bool:
+    if stale(NATIVE, [NATIVE_SRC, os.path.join(os.path.dirname(HERE), "include", "rfa_b200.h")]) or not os.path.exists(NATIVE_KEY):
+        return True
+    with open(NATIVE_KEY) as f:
+        return f.read() != native_key()
+
+
 def build_native() -> str:
     """The torch extension module: links the C-ABI library beside it (found through its own path)."""
-    if stale(NATIVE, [NATIVE_SRC, os.path.join(os.path.dirname(HERE), "include", "rfa_b200.h")]):
+    if native_stale():
         import sysconfig
 
         import torch
@@ -84,6 +98,8 @@ def build_native() -> str:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError("building _native.so failed:\n" + r.stdout + r.stderr)
+        with open(NATIVE_KEY, "w") as f:
+            f.write(native_key())
     return NATIVE
 
 

@@ -200,3 +200,22 @@ def test_a_padding_mask_of_another_size_raises_a_runtime_error():
         ops.cross_state_fwd(phi, v, torch.zeros(3, 3))
     with pytest.raises(RuntimeError, match="shape"):
         ops.cross_state_bwd(phi, v, torch.zeros(3, 3), torch.zeros(2, 3, 128, 64), torch.zeros(2, 3, 128))
+
+
+def test_the_native_module_is_rebuilt_for_another_torch(monkeypatch, tmp_path):
+    """The command that the import error names has to do something: a module newer than its sources but built for another torch
+    is stale."""
+    import os
+    from rfa_b200 import build
+    module, key = tmp_path / "_native.so", tmp_path / "_native.key"
+    monkeypatch.setattr(build, "NATIVE", str(module))
+    monkeypatch.setattr(build, "NATIVE_KEY", str(key))
+    assert build.native_stale()                      # nothing built
+    module.write_bytes(b"")
+    newest = max(os.path.getmtime(p) for p in (build.NATIVE_SRC, str(module)))
+    os.utime(module, (newest + 10, newest + 10))
+    assert build.native_stale()                      # built for nobody knows what
+    key.write_text(build.native_key())
+    assert not build.native_stale()
+    monkeypatch.setattr(torch, "__version__", "0.0")
+    assert build.native_stale()
