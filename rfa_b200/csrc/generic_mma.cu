@@ -4,8 +4,12 @@
 // d % 8 == 0, cuda/forward.cu:150-153); what does not fit stays on the token-at-a-time kernels of generic.cu.  Those keep
 // every number in fp32, and so do these: the state, the weights and the gradients' partial sums are fp32 in registers and
 // shared memory, and a product with such an operand is two mma.sync m16n8k8 tf32 products, of its leading 11 bits and
-// of the rest (hi = x rounded to tf32, lo = x - hi: 22 bits together); fp16 inputs are exact in tf32.  A product of two inputs is
-// one, and goes to m16n8k16 f16 with its operands straight from ldmatrix.  tf32 also has fp32's exponent range, which an fp16 split would not.  tcgen05's kind::tf32 would need operands
+// of the rest (hi = x rounded to tf32, lo = x - hi: 11 bits, a sign and 11 more); fp16 inputs are exact in tf32.  A product of two
+// inputs is one, and goes to m16n8k16 f16 with its operands straight from ldmatrix.  An accumulator inside an mma is
+// truncated, which over a chain of them is a bias: 16 terms of a sum are taken from zero, the sums of 16 added in fp32.
+// (Share of fp16 results that are not the rounded fp64 value at K = 256, d = 128, 130 tokens, a token at a time / one chain a
+// sum / sums of 16: out 0.04 / 0.46 / 0.05 %, gq 0.26 / 0.30 / 0.12, gk 0.13 / 0.33 / 0.10, gv 0.06 / 0.60 / 0.08.  The sums of 16
+// cost 1 to 3 % of the time; a third part of 2 bits changes none of these figures and costs 15 %.)  tf32 also has fp32's exponent range, which an fp16 split would not.  tcgen05's kind::tf32 would need operands
 // padded to its tiles and swizzled and the splits written back to shared memory; at these widths (32 to 256) the warps'
 // fragments read straight from fp32 tiles cost less.
 //
@@ -144,20 +148,22 @@ __device__ __forceinline__ void gm_exact(float (&acc)[2][4], GmTile x, int i0, G
     uint32_t a[4], b[4];
     gm_ldsm(a, pa + l);
     gm_ldsm(b, pb + l);
-    gm_mma16(acc[0], a, b[0], b[1]);
-    gm_mma16(acc[1], a, b[2], b[3]);
+    float part[2][4] = {};
+    gm_mma16(part[0], a, b[0], b[1]);
+    gm_mma16(part[1], a, b[2], b[3]);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) { acc[0][e] += part[0][e]; acc[1][e] += part[1][e]; }
   }
 }
 
-// acc (16 x 8 NT) += sum over l in [l0, l1) of A(i, l) B(l, j), one operand exact in tf32 and the other (SPLIT_A: A, else B) in two
+// acc (16 x 8 NT) += sum over l in [l0, l1) of A(i, l) B(l, j) (the outer loop: see the head of the file), one operand exact in tf32 and the other (SPLIT_A: A, else B) in two
 // parts.  The sum's order is free, so that slots t and t + 4 of a fragment's inner index stand for l = 2t and 2t + 1: a pair is one
 // 8-byte read of an fp32 operand stored along l, and one 8 x 8 block of ldmatrix (two halves a lane) of an fp16 operand,
 // whichever way it is stored (trans).  fa(l, a): A at rows g, g + 8 of column l + 2t, then of l + 2t + 1.  fb(l, b): b[n] = B at rows
 // l + 2t, l + 2t + 1 of column g of the n-th block of 8.
 template <int NT, bool SPLIT_A, class FA, class FB>
 __device__ __forceinline__ void gm_product(float (&acc)[NT][4], int nt, int l0, int l1, FA fa, FB fb) {
-#pragma unroll 2
-  for (int l = l0; l < l1; l += 8) {
+  const auto step = [&](int l, float (&part)[NT][4]) {
     float x[4];
     float2 b[NT];
     fa(l, x);
@@ -171,15 +177,24 @@ __device__ __forceinline__ void gm_product(float (&acc)[NT][4], int nt, int l0, 
     for (int n = 0; n < NT; ++n)
       if (n < nt) {
         if (SPLIT_A) {
-          gm_mma(acc[n], al, __float_as_uint(b[n].x), __float_as_uint(b[n].y));
-          gm_mma(acc[n], a, __float_as_uint(b[n].x), __float_as_uint(b[n].y));
+          gm_mma(part[n], al, __float_as_uint(b[n].x), __float_as_uint(b[n].y));
+          gm_mma(part[n], a, __float_as_uint(b[n].x), __float_as_uint(b[n].y));
         } else {
           uint32_t h0, l0_, h1, l1_;
           gm_split(b[n].x, h0, l0_); gm_split(b[n].y, h1, l1_);
-          gm_mma(acc[n], a, l0_, l1_);
-          gm_mma(acc[n], a, h0, h1);
+          gm_mma(part[n], a, l0_, l1_);
+          gm_mma(part[n], a, h0, h1);
         }
       }
+  };
+  for (int l = l0; l < l1; l += 16) {
+    float part[NT][4] = {};
+    step(l, part);
+    if (l + 8 < l1) step(l + 8, part);
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[n][e] += part[n][e];
   }
 }
 // operand readers for it
@@ -334,13 +349,7 @@ __device__ __forceinline__ void gm_update(float* S, float* z, const GmLayout& L,
           else b[n] = g == 0 ? wz : make_float2(0.f, 0.f);
       };
       const auto rows = gm_a_cols(x, i0);
-      for (int l = 0; l < C; l += 16) {        // as below
-        float part[2][4];
-        gm_zero(part);
-        gm_product<2, false>(part, nt, l, l + 16, rows, weighted);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) { acc[0][e] += part[0][e]; acc[1][e] += part[1][e]; }
-      }
+      gm_product<2, false>(acc, nt, 0, C, rows, weighted);
     } else {
       const __half *pa = x.p + i0 + gm_off_b(lane, x.pitch), *pb = y.p + j0 + gm_off_a(lane, y.pitch);
       const uint32_t ones = g == 0 ? 0x3C003C00u : 0u;         // column d of the z block
@@ -351,7 +360,6 @@ __device__ __forceinline__ void gm_update(float* S, float* z, const GmLayout& L,
         if (j0 < d) gm_ldsm_t(b, pb + l * y.pitch);
         else b[0] = b[1] = ones;
         if (j0 + 8 >= d) b[2] = b[3] = ones;
-        // 16 tokens summed from zero, the sums rounded to nearest: the accumulator inside an mma truncates
         float part[2][4];
         gm_zero(part);
         gm_mma16(part[0], a, b[0], b[1]);

@@ -55,6 +55,26 @@ def test_state_out_and_a_forward_without_workspace(dev, K, d, T):
     assert rel(bare, out.cpu().double()) < 4e-4
 
 
+@pytest.mark.parametrize("K,d,T", [(64, 32, 130), (256, 128, 130), (256, 128, 700), (128, 128, 300)])
+def test_results_are_rounded_from_fp32_sums(dev, K, d, T):
+    """How many fp16 results are not the fp64 value's rounding shows the error in front of that rounding, which the 2-norm hides.  With
+    a relative error of e the share is about 2^12 e: 2e-3 (3e-3 for gq, whose terms cancel) allows 8 (12) units of fp32's last place; chains of
+    truncating products had 0.5 % and more in out and gv."""
+    gen = torch.Generator("cuda").manual_seed(K + T)
+    x = torch.randn(2, T, 8, K // 2, generator=gen, device=dev, dtype=torch.float64)
+    w = torch.randn(K // 2, K // 2, generator=gen, device=dev, dtype=torch.float64)
+    u = (x / x.norm(dim=-1, keepdim=True)) @ w
+    q, k = (0.1 * torch.cat([u.sin(), u.cos()], dim=-1)).half()
+    v, g = torch.randn(2, T, 8, d, generator=gen, device=dev).half()
+    wide = [t.double() for t in (q, k, v, g)]
+    want = (RFA.forward_torch(*wide[:3]), *RFA.backward_torch(*wide))
+    leaves = [t.clone().requires_grad_() for t in (q, k, v)]
+    out = RFA.apply(*leaves)
+    out.backward(g)
+    share = [float((a != b.half()).double().mean()) for a, b in zip([out, *(t.grad for t in leaves)], want)]
+    assert all(s < gate for s, gate in zip(share, (2e-3, 3e-3, 2e-3, 2e-3))), share
+
+
 @pytest.mark.parametrize("which", [0, 1, 2])
 def test_no_token_sees_a_later_non_finite_one(dev, which):
     """A chunk's masked products multiply zeros with the tokens they mask; an infinity there must not reach earlier outputs."""
