@@ -75,6 +75,20 @@ def test_results_are_rounded_from_fp32_sums(dev, K, d, T):
     assert all(s < gate for s, gate in zip(share, (2e-3, 3e-3, 2e-3, 2e-3))), share
 
 
+@pytest.mark.parametrize("K,d", [(64, 32), (96, 40), (128, 128)])
+@pytest.mark.parametrize("T", [16, 45, 300])
+def test_the_reverse_state_is_an_fp32_sum(dev, K, d, T):
+    """Sum of q (x) (g / den): each term rounded twice (1 / den and its product with g, 2^-25 in the mean each), then fp32 sums of 8, and of
+    those: 9e-8 in the 2-norm at 16 tokens, and the square root of the number of sums more."""
+    from rfa_b200 import ops
+    q, k, v, g = (t.to(dev) for t in inputs(T, 8, K, d, T))
+    _, ds, _, _ = ops.causal_bwd_q(q, k, v, g, None, None, True)
+    Q, Kd, G = (t.double() for t in (q, k, g))
+    inv = 1 / (Q * torch.cumsum(Kd, 0)).sum(-1, keepdim=True).clamp_min(1)
+    want = torch.einsum("tbk,tbd->bkd", Q, G * inv)
+    assert float((ds - want).norm() / want.norm()) < 9e-8 * max(1.0, T / 16) ** 0.5
+
+
 @pytest.mark.parametrize("which", [0, 1, 2])
 def test_no_token_sees_a_later_non_finite_one(dev, which):
     """A chunk's masked products multiply zeros with the tokens they mask; an infinity there must not reach earlier outputs."""
