@@ -9,7 +9,7 @@
 
 namespace rfa {
 
-constexpr int kFmThreads = 256, kFmRows = 64;
+constexpr int kFmThreads = 256;
 // Bound by fp32 arithmetic at 64 x 64 (3 of 4 products' FMAs are in the backward) and by memory at 32 x 32.  The products are
 // register tiles of 4 x 4 fed by 16-byte shared-memory reads (8 reads, 12 wavefronts, per 64 FMAs and warp; one 4-byte
 // read per operand element kept the load/store unit busy twice as long as the FMA pipe), and what follows a product
@@ -18,46 +18,47 @@ constexpr int kFmThreads = 256, kFmRows = 64;
 //
 // A thread owns rows rg + 16 i (rg = tid / 16) and columns 4 (tid % 16) .. + 3 of each block of 64 columns.  Pitches are
 // the width + 4: rows one apart are 4 banks apart and stay 16-byte aligned.
-constexpr int kFmI = kFmRows / 16;
+//
+// NI rows a thread, 16 NI a tile: 64 of them, or 32 in a backward whose tiles of 64 would leave SMs idle (see its launch).
 
 struct FmSmem {
   float* Wt;   // [d][D + 4]   W transposed
-  float* X;    // [64][d + 4]  normalised rows
-  float* nrm;  // [64]
+  float* X;    // [rows][d + 4]  normalised rows
+  float* nrm;  // [rows]
   float* W;    // [D][d + 4]   (backward)
-  float* GU;   // [64][D + 4]  (backward)
-  float* c2;   // [64]         (backward) x_hat . g_xh
+  float* GU;   // [rows][D + 4]  (backward)
+  float* c2;   // [rows]         (backward) x_hat . g_xh
 };
-__host__ __device__ inline size_t fm_smem_floats(int D, int d, bool bwd) {
-  const size_t fwd = (size_t)d * (D + 4) + (size_t)kFmRows * (d + 4) + kFmRows;
-  return bwd ? fwd + (size_t)D * (d + 4) + (size_t)kFmRows * (D + 4) + kFmRows : fwd;
+__host__ __device__ inline size_t fm_smem_floats(int rows, int D, int d, bool bwd) {
+  const size_t fwd = (size_t)d * (D + 4) + (size_t)rows * (d + 4) + rows;
+  return bwd ? fwd + (size_t)D * (d + 4) + (size_t)rows * (D + 4) + rows : fwd;
 }
-__device__ __forceinline__ FmSmem fm_carve(float* base, int D, int d) {
+__device__ __forceinline__ FmSmem fm_carve(float* base, int rows, int D, int d) {
   FmSmem s;
   s.Wt = base;
   s.X = s.Wt + d * (D + 4);
-  s.nrm = s.X + kFmRows * (d + 4);
-  s.W = s.nrm + kFmRows;
+  s.nrm = s.X + rows * (d + 4);
+  s.W = s.nrm + rows;
   s.GU = s.W + D * (d + 4);
-  s.c2 = s.GU + kFmRows * (D + 4);
+  s.c2 = s.GU + rows * (D + 4);
   return s;
 }
 
-// Load + normalise 64 rows of this head into s.X (zero rows past the end): 16 lanes per row, all of a thread's loads issued
+// Load + normalise a tile of rows of this head into s.X (zero rows past the end): 16 lanes per row, all of a thread's loads issued
 // before the first sum.
-template <typename TX>
+template <int NI, typename TX>
 __device__ __forceinline__ void fm_load_rows(const FmSmem& s, const TX* __restrict__ x, int64_t row0, int64_t rows, int H, int h, int d) {
   const int rg = threadIdx.x >> 4, c = (threadIdx.x & 15) * 4;
-  float4 v[kFmI][2];
+  float4 v[NI][2];
 #pragma unroll
-  for (int i = 0; i < kFmI; ++i)
+  for (int i = 0; i < NI; ++i)
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const int64_t row = row0 + rg + 16 * i;
       v[i][u] = row < rows && c + 64 * u < d ? load4(x + ((size_t)row * H + h) * d + c + 64 * u) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 #pragma unroll
-  for (int i = 0; i < kFmI; ++i) {
+  for (int i = 0; i < NI; ++i) {
     float ss = 0.f;
 #pragma unroll
     for (int u = 0; u < 2; ++u) ss = fmaf(v[i][u].x, v[i][u].x, fmaf(v[i][u].y, v[i][u].y, fmaf(v[i][u].z, v[i][u].z, fmaf(v[i][u].w, v[i][u].w, ss))));
@@ -76,19 +77,20 @@ __device__ __forceinline__ void fm_axpy(float (&acc)[4], float a, float4 b) {
   acc[0] = fmaf(a, b.x, acc[0]); acc[1] = fmaf(a, b.y, acc[1]); acc[2] = fmaf(a, b.z, acc[2]); acc[3] = fmaf(a, b.w, acc[3]);
 }
 // acc[i][.] = sum_l A[rg + 16 i][l] B[l][col .. col + 3]
-__device__ __forceinline__ void fm_product(float (&acc)[kFmI][4], const float* A, int pa, const float* B, int pb, int L, int rg, int col) {
+template <int NI>
+__device__ __forceinline__ void fm_product(float (&acc)[NI][4], const float* A, int pa, const float* B, int pb, int L, int rg, int col) {
 #pragma unroll
-  for (int i = 0; i < kFmI; ++i)
+  for (int i = 0; i < NI; ++i)
 #pragma unroll
     for (int e = 0; e < 4; ++e) acc[i][e] = 0.f;
 #pragma unroll 2
   for (int l = 0; l < L; l += 4) {
-    float4 a[kFmI];
+    float4 a[NI];
 #pragma unroll
-    for (int i = 0; i < kFmI; ++i) a[i] = load4(A + (rg + 16 * i) * pa + l);
+    for (int i = 0; i < NI; ++i) a[i] = load4(A + (rg + 16 * i) * pa + l);
     const float4 b0 = load4(B + l * pb + col), b1 = load4(B + (l + 1) * pb + col), b2 = load4(B + (l + 2) * pb + col), b3 = load4(B + (l + 3) * pb + col);
 #pragma unroll
-    for (int i = 0; i < kFmI; ++i) {
+    for (int i = 0; i < NI; ++i) {
       fm_axpy(acc[i], a[i].x, b0); fm_axpy(acc[i], a[i].y, b1); fm_axpy(acc[i], a[i].z, b2); fm_axpy(acc[i], a[i].w, b3);
     }
   }
@@ -99,7 +101,8 @@ __global__ void __launch_bounds__(kFmThreads, 4)
 feature_map_fwd_kernel(const TX* __restrict__ x, const float* __restrict__ w, const uint8_t* __restrict__ row_mask,
                        TP* __restrict__ phi, int64_t rows, int H, int d, int D, float scale) {
   extern __shared__ __align__(16) float fm_smem[];
-  const FmSmem s = fm_carve(fm_smem, D, d);
+  constexpr int kFmI = 4, kFmRows = 16 * kFmI;
+  const FmSmem s = fm_carve(fm_smem, kFmRows, D, d);
   const int h = blockIdx.y, rg = threadIdx.x >> 4, cg = (threadIdx.x & 15) * 4;
   const float* wh = w + (size_t)h * D * d;
   for (int i = threadIdx.x; i < D * d; i += kFmThreads) s.Wt[(i % d) * (D + 4) + i / d] = wh[i];
@@ -107,7 +110,7 @@ feature_map_fwd_kernel(const TX* __restrict__ x, const float* __restrict__ w, co
   for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const int64_t row0 = tile * kFmRows;
     __syncthreads();
-    fm_load_rows(s, x, row0, rows, H, h, d);
+    fm_load_rows<kFmI>(s, x, row0, rows, H, h, d);
     __syncthreads();
     for (int col = cg; col < D; col += 64) {
       float u[kFmI][4];
@@ -130,13 +133,14 @@ feature_map_fwd_kernel(const TX* __restrict__ x, const float* __restrict__ w, co
 // Backward.  With g_u = scale * (g_sin * cos u - g_cos * sin u):
 //   g_xh = W^T g_u;  g_x = g_xh / (n + eps) - xh * (xh . g_xh) / n;  g_W += g_u (x) xh
 // GWT: 4 x 4 tiles of g_W per thread (D d <= 4096 GWT), summed per 64 rows from zero and kept in registers over the tiles.
-template <typename T, int GWT>
+template <typename T, int GWT, int NI>
 __global__ void __launch_bounds__(kFmThreads, GWT == 1 ? 2 : 1)
 feature_map_bwd_kernel(const T* __restrict__ x, const float* __restrict__ w, const uint8_t* __restrict__ row_mask,
                        const T* __restrict__ g_phi, T* __restrict__ g_x, float* __restrict__ g_w,
                        int64_t rows, int H, int d, int D, float scale) {
   extern __shared__ __align__(16) float fm_smem[];
-  const FmSmem s = fm_carve(fm_smem, D, d);
+  constexpr int kFmI = NI, kFmRows = 16 * NI;
+  const FmSmem s = fm_carve(fm_smem, kFmRows, D, d);
   const int h = blockIdx.y, rg = threadIdx.x >> 4, cg = (threadIdx.x & 15) * 4;
   const float* wh = w + (size_t)h * D * d;
   for (int i = threadIdx.x; i < D * d; i += kFmThreads) {
@@ -153,7 +157,7 @@ feature_map_bwd_kernel(const T* __restrict__ x, const float* __restrict__ w, con
   for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const int64_t row0 = tile * kFmRows;
     __syncthreads();
-    fm_load_rows(s, x, row0, rows, H, h, d);
+    fm_load_rows<kFmI>(s, x, row0, rows, H, h, d);
     __syncthreads();
     float dot[kFmI];
 #pragma unroll
@@ -247,11 +251,11 @@ static int fm_check(const void* x, const float* w, int64_t rows, int H, int d, i
 }
 
 // CTAs per head, so that the grid is one wave of the `ctas` that an SM holds
-static int fm_grid_x(int64_t rows, int H, int ctas) {
+static int fm_grid_x(int64_t rows, int tile, int H, int ctas) {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int64_t ntiles = (rows + kFmRows - 1) / kFmRows, fit = (int64_t)ctas * sms / H, want = fit < 1 ? 1 : fit;
+  const int64_t ntiles = (rows + tile - 1) / tile, fit = (int64_t)ctas * sms / H, want = fit < 1 ? 1 : fit;
   return (int)(ntiles < want ? ntiles : want);
 }
 static int fm_ctas(size_t smem, int most) {
@@ -276,8 +280,8 @@ extern "C" int rfa_feature_map_fwd_masked(const void* x, int x_dtype, const floa
     return launch_feature_map_fwd_tc((const __half*)x, w, row_mask, (__half*)phi, nullptr, nullptr, nullptr, rows, H, scale, sms,
                                      as_stream(stream));
   }
-  const size_t smem = fm_smem_floats(D, d, false) * sizeof(float);      // 100 KB at most (D, d <= 128)
-  const dim3 grid(fm_grid_x(rows, H, fm_ctas(smem, 4)), H);
+  const size_t smem = fm_smem_floats(64, D, d, false) * sizeof(float);      // 100 KB at most (D, d <= 128)
+  const dim3 grid(fm_grid_x(rows, 64, H, fm_ctas(smem, 4)), H);
   cudaStream_t st = as_stream(stream);
 #define RFA_LAUNCH(TX, TP)                                                                         \
   do {                                                                                             \
@@ -315,22 +319,31 @@ extern "C" int rfa_feature_map_bwd_masked(const void* x, int x_dtype, const floa
     return launch_feature_map_bwd_tc((const __half*)x, w, row_mask, (const __half*)g_phi, (__half*)g_x, nullptr, nullptr, nullptr,
                                      nullptr, g_w, rows, H, scale, sms, as_stream(stream));
   }
-  const size_t smem = fm_smem_floats(D, d, true) * sizeof(float);       // 199 KB at most (D, d <= 128)
   const bool small = D * d <= 4096;
-  const dim3 grid(fm_grid_x(rows, H, fm_ctas(smem, small ? 2 : 1)), H);
+  // Tiles of 32 rows where those of 64 would not give every SM one: a tile's three products follow one another, and so few
+  // CTAs are bound by that chain.  (128 x 128, 8 heads x 1, 64, 512 rows: 39, 42, 43 us in
+  // tiles of 64, 29, 30, 33 in tiles of 32; 64 x 64, 8 heads x 256 rows: 14.8 and 11.0.)
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int tile = (rows + 63) / 64 * H < sms ? 32 : 64;
+  const size_t smem = fm_smem_floats(tile, D, d, true) * sizeof(float);      // 199 KB at most (64 rows, D, d <= 128)
+  const dim3 grid(fm_grid_x(rows, tile, H, fm_ctas(smem, small ? 2 : 1)), H);
   cudaStream_t st = as_stream(stream);
-#define RFA_LAUNCH1(T, GWT)                                                                        \
+#define RFA_LAUNCH1(T, GWT, NI)                                                                    \
   do {                                                                                             \
-    cudaFuncSetAttribute(feature_map_bwd_kernel<T, GWT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-    feature_map_bwd_kernel<T, GWT><<<grid, kFmThreads, smem, st>>>((const T*)x, w, row_mask, (const T*)g_phi, (T*)g_x, g_w, rows, H, d, \
+    cudaFuncSetAttribute(feature_map_bwd_kernel<T, GWT, NI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    feature_map_bwd_kernel<T, GWT, NI><<<grid, kFmThreads, smem, st>>>((const T*)x, w, row_mask, (const T*)g_phi, (T*)g_x, g_w, rows, H, d, \
                                                                    D, scale);                      \
   } while (0)
-#define RFA_LAUNCH(T) do { if (small) RFA_LAUNCH1(T, 1); else RFA_LAUNCH1(T, 4); } while (0)
+#define RFA_LAUNCH2(T, GWT) do { if (tile == 32) RFA_LAUNCH1(T, GWT, 2); else RFA_LAUNCH1(T, GWT, 4); } while (0)
+#define RFA_LAUNCH(T) do { if (small) RFA_LAUNCH2(T, 1); else RFA_LAUNCH2(T, 4); } while (0)
   if (x_dtype == RFA_F16) RFA_LAUNCH(__half);
   else if (x_dtype == RFA_F32) RFA_LAUNCH(float);
   else return fail(RFA_EUNSUPPORTED, "feature_map_bwd: bad dtype %d", x_dtype);
 #undef RFA_LAUNCH
 #undef RFA_LAUNCH1
+#undef RFA_LAUNCH2
   return check_launch("rfa_feature_map_bwd");
 }
 

@@ -129,3 +129,22 @@ def test_feature_map_of_any_width_against_fp64(dev, dtype, rows, H, D, d):
     assert rel(phi, ref.detach()) < (2e-3 if tc else 4e-4 if half else 4e-7)
     assert rel(xg.grad, xd.grad) < (2e-3 if tc else 4e-4 if half else 1e-6)
     assert rel(wg.grad, wd.grad) < (2e-3 if tc else 2e-6)
+
+
+@pytest.mark.parametrize("D,d", [(32, 32), (72, 96), (128, 128)])
+@pytest.mark.parametrize("rows,H", [(33, 147), (33, 148), (148 * 64 - 64, 1), (148 * 64 - 63, 1)])
+def test_feature_map_backward_in_tiles_of_32_and_64(dev, rows, H, D, d):
+    """One SM to a tile of 64 rows is where the backward goes from tiles of 32 to tiles of 64.  fp32 as above; the gradient of the matrices
+    is a sum over up to 9409 rows, taken 32 or 64 at a time: 2e-6."""
+    from rfa_b200 import ops
+    gen = torch.Generator(dev).manual_seed(rows + H)
+    x, g = torch.randn(rows, H, d, generator=gen, device=dev), torch.randn(rows, H, 2 * D, generator=gen, device=dev)
+    w = torch.randn(H, D, d, generator=gen, device=dev)
+    mask = torch.rand(rows, generator=gen, device=dev) < 0.2
+    xd, wd = x.double().requires_grad_(), w.double().requires_grad_()
+    u = torch.einsum("thd,hkd->thk", xd / (xd.norm(dim=-1, keepdim=True) + 1e-3), wd)
+    (0.1 * torch.cat([u.sin(), u.cos()], dim=-1)).backward(g.double() * ~mask[:, None, None])
+    gx, gw = ops.feature_map_bwd(x, w, g, 0.1, True, row_mask=mask)
+    assert float((gx - xd.grad).norm() / xd.grad.norm()) < 1e-6
+    assert float((gw - wd.grad).norm() / wd.grad.norm()) < 2e-6
+    assert torch.equal(ops.feature_map_bwd(x, w, g, 0.1, False, row_mask=mask)[0], gx)
