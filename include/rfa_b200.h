@@ -151,10 +151,10 @@ int rfa_gather_random_matrices(const void* bank, int bank_dtype, int64_t n_bank,
  * tokens before this call's first token; s_out/z_out (may be NULL) receives
  * the state after its last token (prefill -> decode hand-off; segment carry).
  * workspace: rfa_causal_workspace_bytes(T,BH,K,d) bytes, 256-byte aligned.
- * rfa_causal_fwd may be given none (NULL, or one that does not fit): sequences are
- * then not cut into segments, which costs time where few long ones leave the GPU
- * idle.  At K = 128, d = 64 that holds below 1024 tokens and above 74 (batch, head)
- * pairs; from 1024 tokens on with at most 74 it is RFA_EWORKSPACE.
+ * rfa_causal_fwd needs none at K = 128, d = 64 below 1024 tokens or above 74
+ * (batch, head) pairs (from 1024 tokens on with at most 74 it is RFA_EWORKSPACE);
+ * other geometries may be given none (NULL, or one that does not fit) and then run
+ * sequences whole, which costs time where few long ones leave the GPU idle.
  * ---------------------------------------------------------------------- */
 size_t rfa_causal_workspace_bytes(int64_t T, int BH, int K, int d);
 

@@ -322,9 +322,11 @@ extern "C" int rfa_causal_fwd_staged(const void* q, const void* k, const void* v
                                      save_den ? gws.den : nullptr, T, BH, K, d, st);
   }
   // Who has to bring a workspace is part of the interface and does not follow the plan: a forward that saves denominators, and at
-  // K = 128, d = 64 one of 1024 tokens and more with two or more segments to a wave.  Without one that fits the rest run whole.
+  // K = 128, d = 64 one of 1024 tokens and more with two or more segments to a wave.  Below that a forward alone is not cut at
+  // all: its chunks take 1.45 us where the pre-pass and the scan take ten (whole / cut: 8 heads x 960 13.7 / 14.2, 36 heads 14.0 /
+  // 17.7).  Other geometries, whose chunks take 15, stay whole without a workspace that fits.
   const bool required = save_den || (is_tc(K, d) && T >= 1024 && kSms / BH >= 2);
-  if (!required && (!workspace || ((uintptr_t)workspace & 255u) || workspace_bytes < carve_ws(nullptr, T, BH, K, d, p).bytes))
+  if (!required && (is_tc(K, d) || !workspace || ((uintptr_t)workspace & 255u) || workspace_bytes < carve_ws(nullptr, T, BH, K, d, p).bytes))
     p = CausalPlan{1, cut_segments(T, kSegAlign, 1, 0).tseg};
   CausalWs ws{};
   if (p.nseg > 1 || required)

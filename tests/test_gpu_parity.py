@@ -585,9 +585,8 @@ def test_feature_map_pair_equals_two_single_launches(dev, rows, B, H, masked):
 
 @pytest.mark.parametrize("T,BH,status", [(896, 2, 0), (900, 2, 0), (1000, 37, 0), (1023, 2, 0), (1024, 2, -4), (1024, 70, -4), (1024, 75, 0)])
 def test_forward_without_a_workspace(dev, T, BH, status):
-    """Whether the sequences would be cut or not: below 1024 tokens, or with less than two segments to a wave, none is needed; above
-    that one is, which is said before anything is launched.  The result is that of a forward with one up to the rounding
-    of sums in another order."""
+    """Below 1024 tokens, or with less than two segments to a wave, none is needed, and one that is there is not used: a forward alone
+    runs sequences whole.  Above that one is needed, which is said before anything is launched."""
     import ctypes
     from rfa_b200 import _lib, ops
     q, k, v, _ = (t.half().to(dev) for t in generic_feats(T, BH, 128, 64, 3))
@@ -595,7 +594,8 @@ def test_forward_without_a_workspace(dev, T, BH, status):
     assert _lib.load().rfa_causal_fwd(*(t.data_ptr() for t in (q, k, v, bare)), None, None, None, None, None, ctypes.c_size_t(0),
                                       T, BH, 128, 64, _lib.stream_of(q)) == status
     if status == 0:
-        assert_close(bare, ops.causal_fwd(q, k, v), "out without a workspace")
+        assert torch.equal(bare, ops.causal_fwd(q, k, v))
+        assert_close(bare, O.causal_forward(*(t.float().cpu() for t in (q, k, v))), "out without a workspace")
 
 
 def test_feature_map_is_bit_stable(dev):
