@@ -20,8 +20,9 @@
  * d = head_dim.  The tensor-core attention kernels are built for K == 128 and
  * d == 64 (the only geometry upstream's benchmarks and checks use).  Any other
  * K % 8 == 0, d % 8 == 0 whose fp32 state [K][d+1] fits in shared memory (e.g.
- * K <= 256 with d <= 128) runs in chunks of 16 to 64 tokens with the state and
- * all weights in fp32 where a chunk's tiles fit beside the state, else on
+ * K <= 256 with d <= 128) runs in chunks of 16 to 64 tokens, state, weights and
+ * sums in fp32 (an fp32 operand of a product as two parts of 11 bits and a sign),
+ * where a chunk's tiles fit beside the state, else on
  * kernels that walk a sequence token by token, as upstream's do
  * (cuda/forward.cu:112-125); so do cross attention's query kernels and state
  * backward.

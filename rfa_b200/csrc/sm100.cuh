@@ -108,8 +108,8 @@ __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.a
 // async proxy, and an arrive alone does not keep this thread's plain reads in front of it: the loads may still sit in
 // the load/store queue, behind global loads of this or a neighbouring CTA, when the arrive has been counted and the
 // refill lands.  The proxy fence waits for them.  Without it the feature map's forward mixed 16-byte pieces of the tile two
-// further on into its row norms, in 6 to 20 of 100 launches (the refilled tile's values in every wrong row; 0 of 9600
-// launches with the fence, and 0 of 4800 with an arrive that depends on the loaded values).
+// further on into its row norms, in 5 to 21 of 100 launches (the refilled tile's values in every wrong row; 0 of 19200
+// launches with the fence, and 0 of 9600 with an arrive that depends on the loaded values).
 __device__ __forceinline__ void mbar_release_stage(uint64_t* bar) {
   fence_async_smem();
   mbar_arrive(bar);

@@ -599,8 +599,8 @@ def test_forward_without_a_workspace(dev, T, BH, status):
 
 
 def test_feature_map_is_bit_stable(dev):
-    """Repeated launches on the same inputs: the rows' norms must come from the tile that has landed, never from what the
-    stage held before (a launch in three went wrong in a few rows of a CTA's first tile when they were read too early)."""
+    """Repeated launches on the same inputs: the rows' norms must be read before the stage is refilled (test_gpu_repeat.py launches
+    each kernel more often, on tiles of different magnitude)."""
     from rfa_b200 import ops
     gen = torch.Generator().manual_seed(0)
     w = torch.randn(16, 64, 64, generator=gen).to(dev)

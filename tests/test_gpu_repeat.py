@@ -3,7 +3,7 @@
 What can go wrong is a stage refilled by TMA before a plain read of it has been made (a release without the proxy fence,
 ``mbar_release_stage``): the values of the tile that takes the stage next get into row norms, column sums or gradients.
 The rows of different tiles therefore differ in magnitude by powers of two, and launches follow one another without a
-gap, eight at a time: the fault was seen in 3 to 20 of 100 such launches, so that 1500 miss it only at rates far below.
+gap, eight at a time: the fault was seen in 1 to 21 of 100 such launches, and at rates down to one in 300, which 1500 miss in 7 of 1000 runs.
 """
 import pytest
 import torch
