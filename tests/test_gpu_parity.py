@@ -117,8 +117,8 @@ def generic_feats(T, BH, K, d, seed):
 
 
 @pytest.mark.parametrize("K,d", [(64, 32), (256, 128), (96, 40), (128, 128)])
-def test_other_geometries_run_on_the_generic_kernels(dev, K, d):
-    """Feature widths / head dims other than 128 / 64 (upstream accepts any K % 16 == 0, d % 8 == 0): causal forward,
+def test_other_geometries(dev, K, d):
+    """On the chunked kernels (test_gpu_token_kernels.py: what stays on the token-at-a-time ones).  Feature widths / head dims other than 128 / 64 (upstream accepts any K % 16 == 0, d % 8 == 0): causal forward,
     both backward forms (recomputing and RFA.apply's), state carries and the reverse-state total, against the oracle."""
     from rfa_b200 import ops
     from rfa_b200.rfa import RFA
