@@ -168,18 +168,22 @@ decode_step_fused_kernel(const TIn* __restrict__ q, const TIn* __restrict__ k,
     const int per = kDecodeThreads / D >= 16 ? 16 : (kDecodeThreads / D >= 8 ? 8 : (kDecodeThreads / D >= 4 ? 4 : (kDecodeThreads / D >= 2 ? 2 : 1)));
     const int rows_per_pass = kDecodeThreads / per;
     const int sub = tid % per;
-    for (int j = tid / per; j < D; j += rows_per_pass) {
+    // the same number of passes for every lane: a warp holds 32 / per rows, and the shuffles want all of them also where D ends
+    // inside one (D = 40, 56: with the loop left by some lanes the others waited for them, and they at the barrier below, for good)
+    for (int j0 = 0; j0 < D; j0 += rows_per_pass) {
+      const int j = j0 + tid / per;
       float uq = 0.f, uk = 0.f;
-      for (int i = sub * 4; i < d; i += per * 4) {
-        const float4 wv = *reinterpret_cast<const float4*>(wh + (size_t)j * d + i);
-        uq = fmaf(wv.x, xq[i], uq); uq = fmaf(wv.y, xq[i + 1], uq); uq = fmaf(wv.z, xq[i + 2], uq); uq = fmaf(wv.w, xq[i + 3], uq);
-        uk = fmaf(wv.x, xk[i], uk); uk = fmaf(wv.y, xk[i + 1], uk); uk = fmaf(wv.z, xk[i + 2], uk); uk = fmaf(wv.w, xk[i + 3], uk);
-      }
+      if (j < D)
+        for (int i = sub * 4; i < d; i += per * 4) {
+          const float4 wv = *reinterpret_cast<const float4*>(wh + (size_t)j * d + i);
+          uq = fmaf(wv.x, xq[i], uq); uq = fmaf(wv.y, xq[i + 1], uq); uq = fmaf(wv.z, xq[i + 2], uq); uq = fmaf(wv.w, xq[i + 3], uq);
+          uk = fmaf(wv.x, xk[i], uk); uk = fmaf(wv.y, xk[i + 1], uk); uk = fmaf(wv.z, xk[i + 2], uk); uk = fmaf(wv.w, xk[i + 3], uk);
+        }
       for (int o = per >> 1; o > 0; o >>= 1) {
         uq += __shfl_xor_sync(0xffffffffu, uq, o);
         uk += __shfl_xor_sync(0xffffffffu, uk, o);
       }
-      if (sub == 0) { us[j] = uq; us[D + j] = uk; }
+      if (sub == 0 && j < D) { us[j] = uq; us[D + j] = uk; }
     }
   }
   __syncthreads();

@@ -92,3 +92,42 @@ def test_layer_decode_step_against_the_differentiable_path(dev, head_dim, proj_d
     if head_dim != 24:
         assert rel(plain["prev_s"], recorded["prev_s"]) < 2e-3 and rel(plain["prev_z"], recorded["prev_z"]) < 2e-3
         assert plain["prev_s"].dtype == torch.float32
+
+
+@pytest.mark.parametrize("state_dtype,in_dtype", [(torch.float32, torch.float16), (torch.float16, torch.float16), (torch.float32, torch.float32)])
+@pytest.mark.parametrize("d", [4, 8, 32, 64, 128])
+@pytest.mark.parametrize("D", [8, 16, 24, 32, 40, 48, 56, 64, 72, 128, 136])
+def test_fused_decode_of_any_width(dev, D, d, in_dtype, state_dtype):
+    """Every way the projection is spread over a CTA's lanes (16 lanes a row at D = 8 down to one from D = 72 on), with D ending inside
+    a warp's rows at 40 and 56; against fp64.  fp16 features and state are rounded once (2^-11, 2.9e-4 in the 2-norm) and their errors add up
+    over an output's features: 1e-3; fp32: sums of d and 2 D terms, 2e-6."""
+    B, H = 2, 3
+    gen = torch.Generator().manual_seed(D + d)
+    q, k, v = (torch.randn(B, H, d, generator=gen).to(in_dtype) for _ in range(3))
+    w = torch.randn(H, D, d, generator=gen)
+    s, z = (torch.randn(B, H, 2 * D, d, generator=gen) * 0.1).to(state_dtype), torch.rand(B, H, 2 * D, generator=gen).to(state_dtype)
+
+    def phi(x):
+        x = x.double()
+        u = torch.einsum("bhd,hkd->bhk", x / (x.norm(dim=-1, keepdim=True) + 1e-3), w.double())
+        return 0.1 * torch.cat([u.sin(), u.cos()], dim=-1)
+    pq, pk = phi(q), phi(k)
+    S, Z = s.double() + pk[..., None] * v.double()[..., None, :], z.double() + pk
+    want = torch.einsum("bhk,bhkd->bhd", pq, S) / (pq * Z).sum(-1, keepdim=True).clamp_min(1)
+    sg, zg = s.to(dev), z.to(dev)
+    out = ops.decode_step_fused(q.to(dev), k.to(dev), v.to(dev), w.to(dev), 0.1, sg, zg)
+    gate = 2e-6 if in_dtype == torch.float32 else 1e-3
+    assert rel(out.cpu(), want) < gate and rel(sg.cpu(), S) < gate and rel(zg.cpu(), Z) < gate
+
+
+@pytest.mark.parametrize("proj_dim", [40, 56])
+def test_layer_decodes_with_a_proj_dim_that_ends_inside_a_warp(dev, proj_dim):
+    """CausalAttention, one token at a time, against the same layer over the whole sequence."""
+    from rfa_b200 import CausalAttention
+    torch.manual_seed(proj_dim)
+    layer = CausalAttention(embed_dim=64, num_heads=2, head_dim=32, proj_dim=proj_dim).to(dev).half()
+    x, w = torch.randn(5, 3, 64, device=dev).half(), torch.randn(2, proj_dim, 32, device=dev).half()
+    saved = {}
+    with torch.no_grad():
+        steps = torch.cat([layer(x[t:t + 1], w, saved_state=saved) for t in range(5)])
+        assert_close(steps, layer(x, w), "decoded")
