@@ -165,20 +165,20 @@ decode_step_fused_kernel(const TIn* __restrict__ q, const TIn* __restrict__ k,
   float* us = xk + d;
   const float* wh = w + (size_t)h * D * d;
   {
-    const int per = kDecodeThreads / D >= 16 ? 16 : (kDecodeThreads / D >= 8 ? 8 : (kDecodeThreads / D >= 4 ? 4 : (kDecodeThreads / D >= 2 ? 2 : 1)));
-    const int rows_per_pass = kDecodeThreads / per;
-    const int sub = tid % per;
-    // the same number of passes for every lane: a warp holds 32 / per rows, and the shuffles want all of them also where D ends
-    // inside one (D = 40, 56: with the loop left by some lanes the others waited for them, and they at the barrier below, for good)
-    for (int j0 = 0; j0 < D; j0 += rows_per_pass) {
-      const int j = j0 + tid / per;
+    const int fit = kDecodeThreads / D, lg = fit >= 16 ? 4 : fit >= 8 ? 3 : fit >= 4 ? 2 : fit >= 2 ? 1 : 0;
+    const int per = 1 << lg, rows_per_pass = kDecodeThreads >> lg, rows_per_warp = 32 >> lg, sub = tid & (per - 1);
+    // The shuffles want all lanes of a warp also where D ends inside its rows (D = 40, 56): those past the end go over the
+    // last row once more.  (With the loop left by some lanes the others waited for them, and they at the barrier below,
+    // for good.)
+    const int end = (D + rows_per_warp - 1) & ~(rows_per_warp - 1);
+    for (int j = tid >> lg; j < end; j += rows_per_pass) {
+      const float* wj = wh + (size_t)min(j, D - 1) * d;
       float uq = 0.f, uk = 0.f;
-      if (j < D)
-        for (int i = sub * 4; i < d; i += per * 4) {
-          const float4 wv = *reinterpret_cast<const float4*>(wh + (size_t)j * d + i);
-          uq = fmaf(wv.x, xq[i], uq); uq = fmaf(wv.y, xq[i + 1], uq); uq = fmaf(wv.z, xq[i + 2], uq); uq = fmaf(wv.w, xq[i + 3], uq);
-          uk = fmaf(wv.x, xk[i], uk); uk = fmaf(wv.y, xk[i + 1], uk); uk = fmaf(wv.z, xk[i + 2], uk); uk = fmaf(wv.w, xk[i + 3], uk);
-        }
+      for (int i = sub * 4; i < d; i += per * 4) {
+        const float4 wv = *reinterpret_cast<const float4*>(wj + i);
+        uq = fmaf(wv.x, xq[i], uq); uq = fmaf(wv.y, xq[i + 1], uq); uq = fmaf(wv.z, xq[i + 2], uq); uq = fmaf(wv.w, xq[i + 3], uq);
+        uk = fmaf(wv.x, xk[i], uk); uk = fmaf(wv.y, xk[i + 1], uk); uk = fmaf(wv.z, xk[i + 2], uk); uk = fmaf(wv.w, xk[i + 3], uk);
+      }
       for (int o = per >> 1; o > 0; o >>= 1) {
         uq += __shfl_xor_sync(0xffffffffu, uq, o);
         uk += __shfl_xor_sync(0xffffffffu, uk, o);
