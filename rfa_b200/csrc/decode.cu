@@ -146,6 +146,8 @@ decode_step_fused_kernel(const TIn* __restrict__ q, const TIn* __restrict__ k,
   const size_t bh = blockIdx.x;
   const int h = (int)(bh % H);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  pdl_wait();                // q, k, v and w come from the launch before it in a layer, the state from the step before that
+  pdl_launch_dependents();
   float4 buf[kDecodePrefetch];
   decode_prefetch(S + bh * (size_t)K * d, K, d, buf);
   for (int i = tid; i < d; i += kDecodeThreads) vs[i] = to_f(v[bh * d + i]);
@@ -321,6 +323,9 @@ decode_stream_fused_kernel(const TIn* __restrict__ q, const TIn* __restrict__ k,
     mbar_fence_init();
   }
   __syncthreads();
+  pdl_wait();                // the state of the step before, 1 to 3 us of whose drain the launch and the lines above now overlap:
+                             // 4096 heads, one step after another, 51.7 -> 48.6 us (5.7 TB/s)
+  pdl_launch_dependents();
   full += grp * kStages;
   done += grp * kStages;
 
@@ -501,8 +506,8 @@ extern "C" int rfa_decode_step_fused(const void* q, const void* k, const void* v
     const cudaError_t e = cudaFuncSetAttribute(decode_stream_fused_kernel<TI, TS>, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
                                                (int)dst::Layout<TI, TS>::Smem);                                                  \
     if (e != cudaSuccess) return fail((int)e, "decode_fused: cannot reserve shared memory: %s", cudaGetErrorString(e));          \
-    decode_stream_fused_kernel<TI, TS><<<sms, dst::kThreads_, dst::Layout<TI, TS>::Smem, st>>>(                                  \
-        (const TI*)q, (const TI*)k, (const TI*)v, w, scale, (TS*)s, (TS*)z, (TI*)out, BH, H);                                    \
+    launch_pdl(decode_stream_fused_kernel<TI, TS>, dim3(sms), dim3(dst::kThreads_), dst::Layout<TI, TS>::Smem, st,               \
+               (const TI*)q, (const TI*)k, (const TI*)v, w, scale, (TS*)s, (TS*)z, (TI*)out, BH, H);                             \
   } while (0)
     if (in_dtype == RFA_F16 && state_dtype == RFA_F32) RFA_LAUNCH(__half, float);
     else if (in_dtype == RFA_F16) RFA_LAUNCH(__half, __half);
@@ -511,8 +516,8 @@ extern "C" int rfa_decode_step_fused(const void* q, const void* k, const void* v
     return check_launch("rfa_decode_step_fused (streaming)");
   }
 #define RFA_LAUNCH(TI, TS)                                                                        \
-  decode_step_fused_kernel<TI, TS><<<BH, kDecodeThreads, smem, st>>>(                             \
-      (const TI*)q, (const TI*)k, (const TI*)v, w, scale, (TS*)s, (TS*)z, (TI*)out, H, D, d)
+  launch_pdl(decode_step_fused_kernel<TI, TS>, dim3(BH), dim3(kDecodeThreads), smem, st,          \
+             (const TI*)q, (const TI*)k, (const TI*)v, w, scale, (TS*)s, (TS*)z, (TI*)out, H, D, d)
   if (in_dtype == RFA_F16 && state_dtype == RFA_F32) RFA_LAUNCH(__half, float);
   else if (in_dtype == RFA_F16 && state_dtype == RFA_F16) RFA_LAUNCH(__half, __half);
   else if (in_dtype == RFA_F32 && state_dtype == RFA_F32) RFA_LAUNCH(float, float);
