@@ -328,6 +328,20 @@ int rfa_decode_step_fused(const void* q, const void* k, const void* v, int in_dt
                           void* s, void* z, int state_dtype, void* out,
                           int BH, int H, int D, int d, rfa_stream_t stream);
 
+/* Projections of n rows (a batch's one token each) by `count` (1 to 3) matrices
+ * of one shape:  y[m] = x w[m]^T + b[m];  x [n, in], w[m] [out, in], b[m] [out]
+ * (or NULL), y[m] [n, out] fp16, sums in fp32; in, out multiples of 8.  w, b, y
+ * are HOST arrays of device pointers.
+ * rm != NULL: the same launch forms the step's random matrices for
+ * rfa_decode_step_fused,  w_eff [H, D, d] fp32 = (sigma * rm) * inv_tau from fp16
+ * rm [H, D, d] and sigma [H, d] (or NULL), each product rounded to fp16.
+ * replaces nn.Linear on one token and build_random_matrices,
+ * causal_attention.py:222-248, utils.py:90-97. */
+int rfa_linear_rows(const void* x, const void* const* w, const void* const* b,
+                    void* const* y, int count, int n, int in, int out,
+                    const void* rm, const void* sigma, float inv_tau, float* w_eff,
+                    int H, int D, int d, rfa_stream_t stream);
+
 /* One decoding step of cross attention for all L layers in one launch:
  *   out[l] = phi_q[l] . s_l / max(|phi_q[l] . z_l|, 1)
  * phi_q [L,BH,K], out [L,BH,d] of in_dtype; s_ptrs / z_ptrs: DEVICE arrays of L

@@ -14,8 +14,10 @@ import torch
 from torch import Tensor, nn
 from torch.autograd import forward_ad
 from torch.nn import Parameter
+from torch.nn.modules import module as module_hooks
 
 from . import ops
+from ._plain import plain_tensors
 from .rfa import RFA
 from .utils import (EPS, SCALE, build_random_matrices, normalize_attn_weights, random_project, random_project_pair,
                     upgrade_state_dict_named)
@@ -189,6 +191,23 @@ def _underived(*tensors: Optional[Tensor]) -> bool:
     return all(t is None or forward_ad.unpack_dual(t).tangent is None for t in tensors)
 
 
+_LINEAR_FORWARD = nn.Linear.forward
+
+
+def _plain_call(tensors, linears) -> bool:
+    """Whether calling ``linears`` on these tensors is nothing but x W^T + b, so that a kernel may take its place: a plain context and
+    plain tensors, no autocast, no subclass of ``nn.Linear``, no hook that would see the call."""
+    if not plain_tensors(*tensors):
+        return False
+    if torch.is_autocast_enabled("cuda") or module_hooks._has_any_global_hook() or nn.Linear.forward is not _LINEAR_FORWARD:
+        return False
+    for lin in linears:
+        if type(lin) is not nn.Linear or "forward" in lin.__dict__ or lin._forward_hooks or lin._forward_pre_hooks \
+                or lin._backward_hooks or lin._backward_pre_hooks:
+            return False
+    return True
+
+
 class CausalAttention(nn.Module):
     """Random feature causal self-attention layer (upstream causal_attention.py:154-280):
     q/k/v projections, per-head feature map with W' = sigma * W / tau, causal RFA,
@@ -236,17 +255,43 @@ class CausalAttention(nn.Module):
     def _heads(self, t: Tensor) -> Tensor:
         return t.contiguous().view(t.size(0), t.size(1), self.num_heads, self.head_dim)
 
-    def _decode_step(self, q: Tensor, k: Tensor, v: Tensor, w: Tensor, saved_state: Dict[str, Optional[Tensor]]) -> Tensor:
-        """One token from the raw per-head vectors [bsz, num_heads, head_dim]: ``incremental_rfa`` with the feature map inside
-        the kernel, the state updated in place."""
+    @staticmethod
+    def _state(saved_state: Dict[str, Optional[Tensor]], bsz: int, w: Tensor):
+        """The running state of a decoding call, zeros on first use.  w ``[num_heads, proj_dim, head_dim]``."""
         s, z = saved_state.get("prev_s"), saved_state.get("prev_z")
         assert (s is None) == (z is None)
         if s is None:
-            s = torch.zeros(*q.shape[:2], 2 * w.size(1), q.size(2), device=v.device, dtype=torch.float32)
-            z = torch.zeros(*q.shape[:2], 2 * w.size(1), device=v.device, dtype=torch.float32)
+            s = torch.zeros(bsz, w.size(0), 2 * w.size(1), w.size(2), device=w.device, dtype=torch.float32)
+            z = torch.zeros(bsz, w.size(0), 2 * w.size(1), device=w.device, dtype=torch.float32)
+        return s, z
+
+    def _decode_step(self, q: Tensor, k: Tensor, v: Tensor, w: Tensor, saved_state: Dict[str, Optional[Tensor]]) -> Tensor:
+        """One token from the raw per-head vectors [bsz, num_heads, head_dim]: ``incremental_rfa`` with the feature map inside
+        the kernel, the state updated in place."""
+        s, z = self._state(saved_state, q.size(0), w)
         attn = ops.decode_step_fused(q, k, v, w.float().contiguous(), SCALE, s, z)
         saved_state["prev_s"], saved_state["prev_z"] = s, z
         return attn
+
+    def _decode_layer(self, x: Tensor, random_matrices: Tensor, saved_state: Dict[str, Optional[Tensor]]) -> Optional[Tensor]:
+        """One token through the whole layer in three launches (host time is what a small decoding call consists of); None, and
+        nothing done, where the call is to go module by module."""
+        if not (x.is_cuda and x.dtype is torch.float16 and random_matrices.dim() == 3 and random_matrices.is_cuda):
+            return None
+        linears = (self.q_proj, self.k_proj, self.v_proj, self.out_proj)
+        sigma = self.sigma if self.reparam_proj else None
+        s, z = saved_state.get("prev_s"), saved_state.get("prev_z")
+        if not _plain_call((x, random_matrices, sigma, s, z), linears):
+            return None
+        weights = [t for lin in linears for t in (lin.weight, lin.bias)]
+        if not all(t is None or type(t) is Parameter for t in weights) or not _underived(x, random_matrices, sigma, s, z, *weights):
+            return None
+        if s is None and z is None:
+            s, z = self._state(saved_state, x.size(1), random_matrices)
+        y = ops.layer_decode(x, *linears, random_matrices, sigma, self.tau, SCALE, s, z)
+        if y is not None:
+            saved_state["prev_s"], saved_state["prev_z"] = s, z
+        return y
 
     def forward(self, x: Tensor, random_matrices: Tensor, key_padding_mask: Optional[Tensor] = None,
                 attn_mask: Optional[Tensor] = None,
@@ -257,6 +302,10 @@ class CausalAttention(nn.Module):
         and tgt_len must be 1; masks are ignored there, as upstream does."""
         tgt_len, bsz, embed_dim = x.size()
         assert embed_dim == self.embed_dim
+        if saved_state is not None and tgt_len == 1:
+            y = self._decode_layer(x, random_matrices, saved_state)
+            if y is not None:
+                return y
         q, k, v = self._heads(self.q_proj(x)), self._heads(self.k_proj(x)), self._heads(self.v_proj(x))
         w = build_random_matrices(random_matrices=random_matrices, tau=self.tau,
                                   sigma=self.sigma if self.reparam_proj else None,

@@ -370,6 +370,46 @@ Tensor decode_step_fused(Tensor q, Tensor k, Tensor v, const Tensor& w, double s
   return out;
 }
 
+// One token [1, B, E] through a whole self-attention layer: the three projections and the step's random matrices in one launch, the
+// decoding step, the output projection.  Null where a launch here would not be what the separate tensor calls do (dtype,
+// layout, a broadcast shape, a batch that the library GEMMs serve better): nothing has been done then.
+OptTensor layer_decode(const Tensor& x, const Tensor& wq, const OptTensor& bq, const Tensor& wk, const OptTensor& bk, const Tensor& wv,
+                       const OptTensor& bv, const Tensor& wo, const OptTensor& bo, const Tensor& rm, const OptTensor& sigma, double tau,
+                       double scale, const OptTensor& s, const OptTensor& z) {
+  constexpr int64_t kMaxBatch = 128;      // the largest batch that was measured faster than the library GEMMs
+  if (!x.is_cuda() || x.dim() != 3 || x.size(0) != 1 || rm.dim() != 3) return std::nullopt;
+  const int64_t B = x.size(1), E = x.size(2), H = rm.size(0), D = rm.size(1), d = rm.size(2);
+  const auto plain = [&](const Tensor& t, at::IntArrayRef shape, at::ScalarType type) {
+    return t.scalar_type() == type && t.sizes() == shape && t.device() == x.device() && t.layout() == at::kStrided && t.is_contiguous() &&
+           !t.is_conj() && !t.is_neg() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
+  };
+  const auto bias = [&](const OptTensor& b) { return !b || plain(*b, {E}, at::kHalf); };
+  const bool width = D > 0 && D % 8 == 0 && D <= 128 && (d == 8 || d == 16 || d == 32 || d == 64 || d == 128);
+  if (B < 1 || B > kMaxBatch || !width || H < 1 || H * d != E || !plain(x, {1, B, E}, at::kHalf)) return std::nullopt;
+  for (const Tensor* w : {&wq, &wk, &wv, &wo})
+    if (!plain(*w, {E, E}, at::kHalf)) return std::nullopt;
+  if (!bias(bq) || !bias(bk) || !bias(bv) || !bias(bo) || !plain(rm, {H, D, d}, at::kHalf)) return std::nullopt;
+  if (sigma && !plain(*sigma, {H, 1, d}, at::kHalf)) return std::nullopt;
+  if (!s || !z || !plain(*s, {B, H, 2 * D, d}, s->scalar_type()) || !plain(*z, {B, H, 2 * D}, s->scalar_type())) return std::nullopt;
+  if (s->scalar_type() != at::kFloat && s->scalar_type() != at::kHalf) return std::nullopt;
+  Tensor qkv = fresh({4, B, E}, x, at::kHalf), w_eff = fresh({H, D, d}, x, at::kFloat), y = fresh({1, B, E}, x, at::kHalf);
+  char* base = static_cast<char*>(qkv.data_ptr());
+  const int64_t step = B * E * 2;                    // 8 | E: every part is aligned
+  const void *w3[3] = {wq.data_ptr(), wk.data_ptr(), wv.data_ptr()}, *b3[3] = {ptr(bq), ptr(bk), ptr(bv)};
+  void* y3[3] = {base, base + step, base + 2 * step};
+  void* attn = base + 3 * step;
+  Call c(x);
+  check(rfa_linear_rows(x.data_ptr(), w3, b3, y3, 3, B, E, E, rm.data_ptr(), ptr(sigma), static_cast<float>(1.0 / tau), fptr(w_eff), H, D, d, c.stream),
+        "rfa_linear_rows");
+  check(rfa_decode_step_fused(y3[0], y3[1], y3[2], RFA_F16, fptr(w_eff), scale, s->data_ptr(), z->data_ptr(), dtype_code(*s), attn, B * H, H, D, d,
+                              c.stream),
+        "rfa_decode_step_fused");
+  const void *wo1[1] = {wo.data_ptr()}, *bo1[1] = {ptr(bo)};
+  void* yo1[1] = {y.data_ptr()};
+  check(rfa_linear_rows(attn, wo1, bo1, yo1, 1, B, E, E, nullptr, nullptr, 1.f, nullptr, 0, 0, 0, c.stream), "rfa_linear_rows");
+  return y;
+}
+
 }  // namespace
 
 // Without the interpreter lock, as the foreign calls before them: an allocation, a launch on a full queue or the synchronisation
@@ -390,4 +430,5 @@ PYBIND11_MODULE(_native, m) {
   def("cross_query_bwd", &cross_query_bwd);
   def("decode_step", &decode_step);
   def("decode_step_fused", &decode_step_fused);
+  def("layer_decode", &layer_decode);
 }

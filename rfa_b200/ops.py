@@ -307,6 +307,14 @@ def decode_fused_supported(q: Tensor, w: Tensor) -> bool:
             and w.dim() == 3 and w.shape[0] == q.shape[-2] and d == q.shape[-1])
 
 
+def layer_decode(x: Tensor, q_proj, k_proj, v_proj, out_proj, random_matrices: Tensor, sigma: Optional[Tensor], tau: float,
+                 scale: float, s: Optional[Tensor], z: Optional[Tensor]) -> Optional[Tensor]:
+    """One token x [1, B, E] through a layer's projections (``nn.Linear`` modules) and its decoding step in three launches, the
+    state updated IN PLACE; None, with nothing done, where the tensors are not ones the kernels take (then: module by module)."""
+    return native().layer_decode(x, q_proj.weight, q_proj.bias, k_proj.weight, k_proj.bias, v_proj.weight, v_proj.bias,
+                                 out_proj.weight, out_proj.bias, random_matrices, sigma, tau, scale, s, z)
+
+
 class CrossDecodeStates:
     """The cross-attention states of all layers of a decoder, gathered once per sequence for ``cross_decode_step``:
     device arrays of pointers to each layer's ``s [B,H,K,d]`` and ``z [B,H,K]`` (fp32, contiguous).  The states are
