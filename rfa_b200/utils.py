@@ -9,6 +9,8 @@ import torch
 from torch import Tensor
 
 from . import ops
+from ._lib import native
+from ._plain import plain_tensors
 
 EPS = 1.0
 SCALE = 0.1
@@ -196,6 +198,8 @@ def random_project_pair(*, x_a: Tensor, x_b: Tensor, random_matrices: Tensor, sc
     if key_padding_mask_b is not None and key_padding_mask_b.dim() > 0:
         assert key_padding_mask_b.shape == (x_b.size(1), x_b.size(0)), (key_padding_mask_b.shape, x_b.shape)
         row_mask = key_padding_mask_b.to(torch.bool).t().contiguous()
+    if plain_tensors(x_a, x_b, random_matrices, row_mask):
+        return native().feature_map_pair_node(x_a, x_b, random_matrices, scale, None, row_mask)
     return _FeatureMapPair.apply(x_a, x_b, random_matrices, scale, None, row_mask)
 
 
@@ -212,6 +216,8 @@ def random_project(*, x: Tensor, random_matrices: Tensor, scale: float = SCALE,
     if key_padding_mask is not None and key_padding_mask.dim() > 0:
         assert key_padding_mask.shape == (x.size(1), x.size(0)), (key_padding_mask.shape, x.shape)
         row_mask = key_padding_mask.to(torch.bool).t().contiguous()          # [seq_len, bsz]: one entry per row of x
+    if plain_tensors(x, random_matrices, row_mask):
+        return native().feature_map_node(x, random_matrices, scale, row_mask)
     return _FeatureMap.apply(x, random_matrices, scale, row_mask)
 
 

@@ -219,3 +219,33 @@ def test_the_native_module_is_rebuilt_for_another_torch(monkeypatch, tmp_path):
     assert not build.native_stale()
     monkeypatch.setattr(torch, "__version__", "0.0")
     assert build.native_stale()
+
+
+def test_what_a_native_short_cut_leaves_to_the_tensor_expressions():
+    """CPU tensors, subclasses and every context that wants to see a call: compiling, a transform, a mode, a forward-mode level; a caller
+    that is compiled reaches the function as before (here: its refusal of CPU tensors)."""
+    import torch.autograd.forward_ad as fw
+    from rfa_b200 import _plain
+    from rfa_b200.rfa import RFA
+    from torch.overrides import TorchFunctionMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Function(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    class Dispatch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+    assert _plain.plain_context() and not _plain.plain_tensors(torch.zeros(1))
+    for context in (Function, Dispatch, fw.dual_level):
+        with context():
+            assert not _plain.plain_context()
+    seen = []
+    torch.func.vmap(lambda x: (seen.append(_plain.plain_context()), x)[1])(torch.zeros(2))
+    torch.jit.trace(lambda x: (seen.append(_plain.plain_context()), x + 1)[1], torch.zeros(2), check_trace=False)
+    assert seen and not any(seen)
+    assert torch.compile(lambda x: x + 1 if _plain.plain_context() else x + 2, backend="eager")(torch.zeros(1)).item() == 2
+    q = torch.zeros(4, 1, 128, dtype=torch.half)
+    with pytest.raises(RuntimeError, match="no CPU path"):
+        torch.compile(lambda q, v: RFA.apply(q, q, v) * 2, backend="eager")(q, q[..., :64])
