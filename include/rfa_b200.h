@@ -376,6 +376,17 @@ int rfa_causal_fwd_fused(const void* x_q, const void* x_k, const void* v,
                          int64_t T, int B, int H, int d, int D,
                          int save_den, rfa_stream_t stream);
 
+/* The same forward for a layer's evaluation pass, from what the layer holds: the
+ * matrices as fp16 rm [H, D, d] with sigma [H, d] (or NULL) and 1 / tau, each
+ * product rounded to fp16 as build_random_matrices does (utils.py:90-97), and the
+ * padding mask as the layer gets it, pad_mask [B, T] bytes (or NULL).  No state
+ * in or out, nothing kept for a backward. */
+int rfa_causal_fwd_fused_layer(const void* x_q, const void* x_k, const void* v,
+                               const void* rm, const void* sigma, float inv_tau,
+                               const uint8_t* pad_mask, float scale, void* out,
+                               int64_t T, int B, int H, int d, int D,
+                               rfa_stream_t stream);
+
 /* Measurement aid, no upstream counterpart: streams in [T, BH, 64*nb] fp16 through
  * shared memory with the tile pattern of the causal kernels (one CTA per (batch,
  * head), chunks of 128 tokens, nb boxes of 128 rows x 128 bytes per chunk, two

@@ -293,6 +293,17 @@ class CausalAttention(nn.Module):
             saved_state["prev_s"], saved_state["prev_z"] = s, z
         return y
 
+    def _fused_layer_pass(self, q: Tensor, k: Tensor, v: Tensor, random_matrices: Tensor, mask: Optional[Tensor]) -> bool:
+        """Whether a pass without gradients may hand the layer's own matrices and mask to the fused forward: what the tensor
+        expressions around it would make of them, it makes of them (the mul, the conversion and the mask's transpose are three
+        launches and 10 us of the 188 that a pass over 8 x 2048 tokens of 16 heads takes)."""
+        sigma = self.sigma if self.reparam_proj else None
+        half = torch.float16
+        return (ops.fused_forward_supported(q, random_matrices) and q.dtype is k.dtype is v.dtype is half
+                and tuple(random_matrices.shape) == (self.num_heads, 64, 64) and random_matrices.dtype is half
+                and (sigma is None or (sigma.dtype is half and tuple(sigma.shape) == (self.num_heads, 1, 64)))
+                and plain_tensors(q, k, v, random_matrices, sigma, mask) and _underived(q, k, v, random_matrices, sigma))
+
     def forward(self, x: Tensor, random_matrices: Tensor, key_padding_mask: Optional[Tensor] = None,
                 attn_mask: Optional[Tensor] = None,
                 saved_state: Optional[Dict[str, Optional[Tensor]]] = None) -> Tensor:
@@ -307,6 +318,14 @@ class CausalAttention(nn.Module):
             if y is not None:
                 return y
         q, k, v = self._heads(self.q_proj(x)), self._heads(self.k_proj(x)), self._heads(self.v_proj(x))
+        if saved_state is None and self.cuda_causal_rfa and self._fused_layer_pass(q, k, v, random_matrices, key_padding_mask):
+            # head_dim 64, proj_dim 64, fp16, no gradient: features, matrices and padding mask formed inside the kernel
+            if key_padding_mask is not None and key_padding_mask.dim() == 0:
+                key_padding_mask = None
+            assert key_padding_mask is None or key_padding_mask.shape == (bsz, tgt_len)
+            attn = ops.causal_fwd_fused(q, k, v, random_matrices, SCALE, sigma=self.sigma if self.reparam_proj else None, tau=self.tau,
+                                        pad_mask=key_padding_mask)
+            return self.out_proj(attn.view(tgt_len, bsz, embed_dim))
         w = build_random_matrices(random_matrices=random_matrices, tau=self.tau,
                                   sigma=self.sigma if self.reparam_proj else None,
                                   reparam_proj=self.reparam_proj)

@@ -59,10 +59,17 @@ enum { xFull = 0, xEmpty = 2, vFull = 4, vEmpty = 6, uFull = 8, uFree = 9, phiFu
 // written / packed; sDone (per N buffer): issuer B's products complete; nFull/nFree: an N buffer; bSt: state tile exported.
 }  // namespace fz
 
+// the heads' matrices: w [H][64][64] fp32 as they are, or sigma * rm * inv_tau of fp16 rm [H][64][64] and sigma [H][64] (null: rm)
+struct FusedMatrices {
+  const float* w;
+  const __half *rm, *sigma;
+  float inv_tau;
+};
+
 __global__ void __launch_bounds__(fz::kThreads_, 1)
 causal_fwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_constant__ CUtensorMap tm_xk,
-                           const __grid_constant__ CUtensorMap tm_v, const float* __restrict__ w,
-                           const uint8_t* __restrict__ row_mask, __half* __restrict__ out,
+                           const __grid_constant__ CUtensorMap tm_v, const FusedMatrices m,
+                           const uint8_t* __restrict__ row_mask, int64_t mask_t, int64_t mask_b, __half* __restrict__ out,
                            const float* __restrict__ s_in, const float* __restrict__ z_in,
                            float* __restrict__ s_out, float* __restrict__ z_out, float* __restrict__ den_out,
                            int64_t T, int BH, int H, float scale) {
@@ -114,10 +121,24 @@ causal_fwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tm_xq, const __gr
   // W_h -> fp16 K-major operand tile [64 rows j][64 i]
   for (int i = tid; i < 64 * 8; i += kThreads_) {
     const int j = i >> 3, ch = i & 7;
-    const float4 a = *reinterpret_cast<const float4*>(w + ((size_t)h * 64 + j) * 64 + ch * 8);
-    const float4 b = *reinterpret_cast<const float4*>(w + ((size_t)h * 64 + j) * 64 + ch * 8 + 4);
     uint4 u;
-    u.x = pack_half2(a.x, a.y); u.y = pack_half2(a.z, a.w); u.z = pack_half2(b.x, b.y); u.w = pack_half2(b.z, b.w);
+    if (m.rm) {                 // sigma * W / tau from fp16, rounded after each as the tensor expressions round
+      float f[8];
+      load8(m.rm + ((size_t)h * 64 + j) * 64 + ch * 8, f);
+      if (m.sigma) {
+        float s[8];
+        load8(m.sigma + h * 64 + ch * 8, s);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] = __half2float(__float2half_rn(f[e] * s[e]));
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) f[e] *= m.inv_tau;
+      u.x = pack_half2(f[0], f[1]); u.y = pack_half2(f[2], f[3]); u.z = pack_half2(f[4], f[5]); u.w = pack_half2(f[6], f[7]);
+    } else {
+      const float4 a = *reinterpret_cast<const float4*>(m.w + ((size_t)h * 64 + j) * 64 + ch * 8);
+      const float4 b = *reinterpret_cast<const float4*>(m.w + ((size_t)h * 64 + j) * 64 + ch * 8 + 4);
+      u.x = pack_half2(a.x, a.y); u.y = pack_half2(a.z, a.w); u.z = pack_half2(b.x, b.y); u.w = pack_half2(b.z, b.w);
+    }
     *reinterpret_cast<uint4*>(sm + kW + row_chunk1(j, ch)) = u;
   }
   fence_async_smem();
@@ -376,7 +397,6 @@ causal_fwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tm_xq, const __gr
     const int half = ((warp - 12) >> 2) & 1;       // which 32 of the 64 projected columns
     const uint32_t colU = is_key ? cUk : cUq;
     unsigned char* tile = sm + (is_key ? kPhiK : kPhiQ);
-    const int nb = BH / H;                           // batch size: row_mask is [T][batch]
     for (int c = 0; c < nchunk; ++c) {
       const int st = c & 1;
       const unsigned char* raw = sm + st * kRaw + (is_key ? kXk : kXq);
@@ -400,7 +420,7 @@ causal_fwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tm_xq, const __gr
       const float inv = 1.f / (sqrtf(ss + ss_b) + kNormEps);
       // a key past the end of the sequence or masked as padding contributes nothing: all-zero features
       float sc = scale;
-      if (is_key && (t >= T || (row_mask && row_mask[t * nb + bh / H]))) sc = 0.f;
+      if (is_key && (t >= T || (row_mask && row_mask[t * mask_t + bh / H * mask_b]))) sc = 0.f;
       tmem_ld_wait();
       tc_fence_before_sync();
       mbar_arrive(&bars[uFree]);
@@ -430,17 +450,18 @@ causal_fwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tm_xq, const __gr
   if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
-// x_q, x_k, v, out [T][BH][64] fp16 (BH = batch * H, head index fastest); w [H][64][64] fp32; row_mask [T][batch] or null
-int launch_causal_fwd_fused_tc(const __half* xq, const __half* xk, const __half* v, const float* w, const uint8_t* row_mask,
-                               __half* out, const float* s_in, const float* z_in, float* s_out, float* z_out, float* den_out,
+// x_q, x_k, v, out [T][BH][64] fp16 (BH = batch * H, head index fastest); w [H][64][64] fp32, or null: rm, sigma and inv_tau as in
+// FusedMatrices; row_mask: byte t * mask_t + b * mask_b marks key t of sequence b, or null
+int launch_causal_fwd_fused_tc(const __half* xq, const __half* xk, const __half* v, const float* w, const __half* rm, const __half* sigma,
+                               float inv_tau, const uint8_t* row_mask, int64_t mask_t, int64_t mask_b, __half* out, const float* s_in, const float* z_in, float* s_out, float* z_out, float* den_out,
                                int64_t T, int BH, int H, float scale, cudaStream_t st) {
   CUtensorMap tq, tk, tv;
   if (make_tmap_rows(&tq, xq, T, BH, kD, kTC) || make_tmap_rows(&tk, xk, T, BH, kD, kTC) || make_tmap_rows(&tv, v, T, BH, kD, kTC))
     return fail(RFA_EDEVICE, "causal_fwd_fused: cuTensorMapEncodeTiled failed or is unavailable");
   cudaError_t e = cudaFuncSetAttribute(causal_fwd_fused_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fz::kSmem);
   if (e != cudaSuccess) return fail((int)e, "causal_fwd_fused: cannot reserve %u bytes of shared memory: %s", fz::kSmem, cudaGetErrorString(e));
-  launch_pdl(causal_fwd_fused_tc_kernel, dim3(BH), dim3(fz::kThreads_), fz::kSmem, st, tq, tk, tv, w, row_mask, out, s_in, z_in, s_out,
-             z_out, den_out, T, BH, H, scale);
+  launch_pdl(causal_fwd_fused_tc_kernel, dim3(BH), dim3(fz::kThreads_), fz::kSmem, st, tq, tk, tv, FusedMatrices{w, rm, sigma, inv_tau},
+             row_mask, mask_t, mask_b, out, s_in, z_in, s_out, z_out, den_out, T, BH, H, scale);
   return check_launch("rfa_causal_fwd_fused");
 }
 

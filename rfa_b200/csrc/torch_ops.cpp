@@ -284,6 +284,28 @@ std::tuple<Tensor, OptTensor, OptTensor, OptTensor> causal_fwd_fused(Tensor xq, 
   return {out, s_out, z_out, ws};
 }
 
+// The same without state or workspace, from the layer's own fp16 matrices (and sigma, tau) and its padding mask [B, T].
+Tensor causal_fwd_fused_layer(Tensor xq, Tensor xk, Tensor v, Tensor rm, OptTensor sigma, double tau, double scale, const OptTensor& pad) {
+  require_half(xq, xk, v, rm);
+  rank(xq, 4);
+  rank(rm, 3);
+  xq = xq.contiguous(); xk = xk.contiguous(); v = v.contiguous(); rm = rm.contiguous();
+  const int64_t T = xq.size(0), B = xq.size(1), H = xq.size(2), d = xq.size(3), D = rm.size(1);
+  require(xk.sizes() == xq.sizes() && v.sizes() == xq.sizes() && rm.size(0) == H && rm.size(2) == d);
+  if (sigma) {
+    require_half(*sigma);
+    require(sigma->numel() == H * d);
+    sigma = sigma->contiguous();
+  }
+  Tensor out = fresh({T, B * H, d}, xq, at::kHalf);
+  const OptTensor m = pad_bytes(pad, B, T, xq);
+  Call c(xq);
+  check(rfa_causal_fwd_fused_layer(ptr(xq), ptr(xk), ptr(v), ptr(rm), ptr(sigma), static_cast<float>(1.0 / tau), bptr(m), scale, ptr(out), T, B, H, d,
+                                   D, c.stream),
+        "rfa_causal_fwd_fused_layer");
+  return out;
+}
+
 // ---- cross ---------------------------------------------------------------------------------------------------------------
 std::tuple<Tensor, Tensor> cross_state_fwd(Tensor phi_k, Tensor v, const OptTensor& pad) {
   require_half(phi_k, v);
@@ -526,6 +548,7 @@ PYBIND11_MODULE(_native, m) {
   def("causal_fwd_saved", &causal_fwd_saved);
   def("causal_bwd_saved", &causal_bwd_saved);
   def("causal_fwd_fused", &causal_fwd_fused);
+  def("causal_fwd_fused_layer", &causal_fwd_fused_layer);
   def("cross_state_fwd", &cross_state_fwd);
   def("cross_state_bwd", &cross_state_bwd);
   def("cross_query_fwd", &cross_query_fwd);

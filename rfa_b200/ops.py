@@ -144,11 +144,18 @@ def fused_forward_supported(x: Tensor, w: Tensor) -> bool:
 
 def causal_fwd_fused(x_q: Tensor, x_k: Tensor, v: Tensor, w: Tensor, scale: float, row_mask: Optional[Tensor] = None,
                      s_in: Optional[Tensor] = None, z_in: Optional[Tensor] = None, return_state: bool = False,
-                     save_den: bool = False):
+                     save_den: bool = False, *, sigma: Optional[Tensor] = None, tau: Optional[float] = None,
+                     pad_mask: Optional[Tensor] = None):
     """Causal RFA forward from the raw per-head vectors: x_q, x_k, v [T, B, H, 64] fp16, w [H, 64, 64] fp32; the features
     scale * [sin | cos]((W x) / (|x| + 1e-3)) of q and k are formed inside the kernel.  row_mask [T, B] (or [T * B]) marks
     padded keys.  Returns out [T, B*H, 64] and, as asked, the final state (s, z) and the workspace holding the raw
-    denominators for ``causal_bwd_saved(..., ws_has=WS_DEN)``: (out[, s, z][, ws])."""
+    denominators for ``causal_bwd_saved(..., ws_has=WS_DEN)``: (out[, s, z][, ws]).
+
+    With ``tau`` given, w is the layer's own fp16 bank [H, 64, 64], taken as sigma * w / tau (``sigma`` [H, 1, 64] fp16 or None), and
+    ``pad_mask`` [B, T] its padding mask: out alone, and no launch but this one."""
+    if tau is not None:
+        assert row_mask is None and s_in is None and z_in is None and not return_state and not save_den
+        return native().causal_fwd_fused_layer(x_q, x_k, v, w, sigma, tau, scale, pad_mask)
     out, s_out, z_out, ws = native().causal_fwd_fused(x_q, x_k, v, w, scale, row_mask, s_in, z_in, return_state, save_den)
     res = (out,)
     if return_state:

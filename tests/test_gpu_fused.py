@@ -162,3 +162,32 @@ def test_causal_attention_module_uses_the_fused_forward(dev, monkeypatch):
     names = ["out", "g_x", "g_w"] + ["g_" + k for k, _ in layer.named_parameters()]
     for a, b, name in zip(fused, two, names):
         assert_close(a, b, "module " + name, rel=2e-3)
+
+
+@pytest.mark.parametrize("T,B", [(1, 1), (77, 3), (300, 2)])
+@pytest.mark.parametrize("tau,reparam,mask", [(1.0, True, "ragged"), (0.7, True, None), (2.0, False, "ragged"), (1.0, False, "scalar"), (1.0, True, "floats")])
+def test_layer_pass_from_its_own_matrices_and_mask(dev, T, B, tau, reparam, mask):
+    """A pass without gradients hands the kernel sigma, W, tau and the padding mask as they are; inside a dispatch mode the tensor
+    expressions form them: the same roundings, so the same bits (1 / tau is rounded once more at most: 2^-10 of the features)."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    from rfa_b200 import CausalAttention
+
+    class Seen(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+    torch.manual_seed(T)
+    layer = CausalAttention(embed_dim=128, num_heads=2, head_dim=64, proj_dim=64, tau=tau, reparam_proj=reparam).to(dev).half()
+    if reparam:
+        torch.nn.init.uniform_(layer.sigma, 0.5, 1.5)
+    w, x = torch.randn(2, 64, 64, device=dev).half(), torch.randn(T, B, 128, device=dev).half()
+    pad = torch.arange(T, device=dev)[None, :] >= torch.randint((T + 1) // 2, T + 1, (B, 1), device=dev)
+    pad = {"ragged": pad, "floats": pad.float(), "scalar": torch.tensor(False, device=dev), None: None}[mask]
+    with torch.no_grad():
+        got = layer(x, w, key_padding_mask=pad)
+        with Seen():
+            want = layer(x, w, key_padding_mask=pad)
+        assert torch.equal(got, want) if tau in (1.0, 2.0) else float((got - want).float().norm() / want.float().norm()) < 2e-3
+        if mask == "ragged":
+            with pytest.raises(AssertionError):
+                layer(x, w, key_padding_mask=torch.zeros(B + 1, T, dtype=torch.bool, device=dev))
