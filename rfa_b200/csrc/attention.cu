@@ -59,7 +59,7 @@ int launch_causal_short_fwd(const __half* q, const __half* k, const __half* v, _
 int launch_causal_short_bwd(const __half* q, const __half* k, const __half* v, const __half* g, const __half* out, const float* den, __half* gq,
                             __half* gk, __half* gv, int64_t T, int BH, cudaStream_t st);
 
-// chunked tensor-core kernels for other geometries (generic_mma.cu)
+// chunked tensor-core kernels for other geometries (generic_split.cu, generic_mma.cu)
 int generic_chunk(int K, int d, int* ctas);
 int launch_causal_chunked_fwd(const __half* q, const __half* k, const __half* v, __half* out, const float* s_seg, const float* z_seg,
                               float* s_out, float* z_out, float* den_out, int64_t T, int BH, int nseg, int64_t tseg, int K, int d,
@@ -109,7 +109,7 @@ static CausalPlan cut_segments(int64_t T, int64_t chunk, int64_t fit, int64_t mi
 }
 static CausalPlan plan_causal(int64_t T, int BH) { return cut_segments(T, kSegAlign, kSms / BH, 6); }
 
-// Which kernels serve a geometry: the tcgen05 ones (K = 128, d = 64), the chunked ones of generic_mma.cu, or the
+// Which kernels serve a geometry: the tcgen05 ones (K = 128, d = 64), the chunked ones of generic_split.cu and generic_mma.cu, or the
 // token-at-a-time ones of generic.cu.
 static bool is_tc(int K, int d) { return K == kK && d == kD; }
 static bool is_chunked(int K, int d) { return !is_tc(K, d) && generic_chunk(K, d, nullptr) > 0; }
@@ -119,8 +119,8 @@ static CausalPlan plan_geometry(int64_t T, int BH, int K, int d) {
   int ctas = 1;
   const int chunk = generic_chunk(K, d, &ctas);
   if (!chunk) return CausalPlan{1, T};
-  // A chunk takes these kernels 20 us and more, a cut's pre-pass and scans 15: any cut that one wave holds.  Forward + backward in
-  // us at (K, d, heads x batch, tokens), whole / cut: (64, 32, 32, 200) 109 / 47, (128, 128, 32, 200) 361 / 137,
+  // A chunk takes these kernels 10 us and more, a cut's pre-pass and scans 10: any cut that one wave holds.  Forward + backward of
+  // generic_mma.cu's kernels in us at (K, d, heads x batch, tokens), whole / cut: (64, 32, 32, 200) 109 / 47, (128, 128, 32, 200) 361 / 137,
   // (256, 128, 8, 128) 357 / 152, (64, 32, 8, 512) 217 / 46.
   return cut_segments(T, chunk, kSms * ctas / BH, 1);
 }

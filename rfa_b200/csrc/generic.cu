@@ -1,5 +1,5 @@
 // Causal and cross RFA for the geometries neither the tcgen05 kernels (K = 128, d = 64) nor the chunked ones
-// (generic_mma.cu: the causal path and the state reduction, where a chunk's tiles fit beside the state) serve: any K % 8 == 0,
+// (generic_split.cu, generic_mma.cu: the causal path and the state reduction, where a chunk's tiles fit beside the state) serve: any K % 8 == 0,
 // d % 8 == 0 whose fp32 state [K][d + 1] fits in shared memory.
 // Upstream's kernels accept any K % 16 == 0, d % 8 == 0 (cuda/forward.cu:150-153, cuda/backward.cu:560-562) and its
 // cross attention is einsums of any size (cross_attention.py:97-104, 266-269); these kernels keep that reach.

@@ -1,7 +1,8 @@
 // Causal RFA and the state reduction for geometries other than K = 128, d = 64, in chunks on the tensor cores.
 //
 // Any K % 8 == 0, d % 8 == 0 whose fp32 state and one chunk's tiles fit in shared memory (upstream takes any K % 16 == 0,
-// d % 8 == 0, cuda/forward.cu:150-153); what does not fit stays on the token-at-a-time kernels of generic.cu.  Those keep
+// d % 8 == 0, cuda/forward.cu:150-153); what does not fit stays on the token-at-a-time kernels of generic.cu, and those whose
+// state fits a second time, as an operand, are on the faster kernels of generic_split.cu: here it is K = 256, d = 128 and the like.  Those of generic.cu keep
 // every number in fp32, and so do these: the state, the weights and the gradients' partial sums are fp32 in registers and
 // shared memory, and a product with such an operand is two mma.sync m16n8k8 tf32 products, of its leading 11 bits and
 // of the rest (hi = x rounded to tf32, lo = x - hi: 11 bits, a sign and 11 more); fp16 inputs are exact in tf32.  A product of two
@@ -9,7 +10,8 @@
 // truncated, which over a chain of them is a bias: 16 terms of a sum are taken from zero, the sums of 16 added in fp32.
 // (Share of fp16 results that are not the rounded fp64 value at K = 256, d = 128, 130 tokens, a token at a time / one chain a
 // sum / sums of 16: out 0.04 / 0.46 / 0.05 %, gq 0.26 / 0.30 / 0.12, gk 0.13 / 0.33 / 0.10, gv 0.06 / 0.60 / 0.08.  The sums of 16
-// cost 1 to 3 % of the time; a third part of 2 bits changes none of these figures and costs 15 %.)  tf32 also has fp32's exponent range, which an fp16 split would not.  tcgen05's kind::tf32 would need operands
+// cost 1 to 3 % of the time; a third part of 2 bits changes none of these figures and costs 15 %.)  tf32 also has fp32's exponent range, for
+// which an fp16 split wants a factor per block and so a place in shared memory.  tcgen05's kind::tf32 would need operands
 // padded to its tiles and swizzled and the splits written back to shared memory; at these widths (32 to 256) the warps'
 // fragments read straight from fp32 tiles cost less.
 //
@@ -26,15 +28,11 @@
 // A masked product multiplies zeros with the tokens it masks, and 0 * inf is NaN: a chunk whose second operand holds a
 // non-finite value takes the masked products element by element, over the unmasked tokens only, so that what a
 // token makes of its predecessors never depends on its successors.
-#include <math_constants.h>
-
-#include "common.cuh"
+#include "generic_mma.cuh"
 
 namespace rfa {
 
 constexpr int kGmRegs = 80;      // three CTAs of 256 threads on an SM, or one of 512
-
-__host__ __device__ inline int gm_round16(int x) { return (x + 15) & ~15; }
 
 // Shared-memory layout (bytes), the same on host and device.  Row pitches: fp16 tiles + 8 and fp32 arrays + 4 elements, which
 // keep the fragment reads below (rows 8 apart in g, pairs of columns in t, and their transposes) free of bank conflicts or
@@ -59,58 +57,11 @@ __host__ __device__ inline GmLayout gm_layout(int C, int K, int d, int stages, i
   L.total = L.tile + (uint32_t)stages * (nx * L.x_bytes + ny * L.y_bytes);
   return L;
 }
-__host__ __device__ inline int gm_groups32(int K) { return (K + 31) / 32; }
 // per-row fp32 arrays of each kernel
 __host__ __device__ inline int gm_rows_fwd(int C) { return C / 16 + 1; }                                   // rs, qz
 __host__ __device__ inline int gm_rows_bwd_q(int C, int K) { return 2 * (C / 16) + gm_groups32(K) + 3; }   // rs, pg, wq, qz, inv, gz
 constexpr int kGmRowsKv = 2, kGmRowsState = 2;                                                             // inv, gz
 
-struct GmTile { const __half* p; int pitch; };
-
-// ---- loads ---------------------------------------------------------------------------------------------------------------
-__device__ __forceinline__ void gm_cp16(void* dst, const void* src, bool live) {
-  const uint32_t s = (uint32_t)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(src), "r"(live ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ void gm_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void gm_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// f(row, first column) of this thread's 16-byte pieces of a tile of C rows of `width` halves; one division for all of them
-template <class F>
-__device__ __forceinline__ void gm_each16(int C, int width, F f) {
-  const int w8 = width >> 3, dr = blockDim.x / w8, dc = blockDim.x - dr * w8;
-  int r = threadIdx.x / w8, c = threadIdx.x - r * w8;
-  while (r < C) {
-    f(r, c * 8);
-    r += dr;
-    c += dc;
-    if (c >= w8) { c -= w8; ++r; }
-  }
-}
-// C rows of `width` halves, token t0 + r of sequence bh; rows from `valid` on, and masked ones, come out as zeros
-__device__ __forceinline__ void gm_load(__half* dst, int pitch, const __half* src, int C, int width, int64_t t0, int valid, int BH,
-                                        int bh, const uint8_t* mrow) {
-  const size_t row = (size_t)BH * width;
-  src += ((size_t)t0 * BH + bh) * width;
-  gm_each16(C, width, [&](int r, int c) {
-    const bool live = r < valid && !(mrow && mrow[t0 + r]);
-    gm_cp16(dst + r * pitch + c, src + (live ? r * row + c : 0), live);
-  });
-}
-// has any of this thread's own chunks of the tile a non-finite value?  (after its cp.async have landed)
-__device__ __forceinline__ bool gm_odd(const __half* tile, int pitch, int C, int width) {
-  bool odd = false;
-  gm_each16(C, width, [&](int r, int c) {
-    const uint4 u = *reinterpret_cast<const uint4*>(tile + r * pitch + c);
-    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-    for (int e = 0; e < 4; ++e) odd |= (w[e] & 0x7C00u) == 0x7C00u || (w[e] & 0x7C000000u) == 0x7C000000u;
-  });
-  return odd;
-}
-
-// ---- products --------------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void gm_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
@@ -122,40 +73,6 @@ __device__ __forceinline__ void gm_split(float x, uint32_t& hi, uint32_t& lo) {
   lo = __float_as_uint(x - __uint_as_float(hi)) + 0x1000u;
   if (!(fabsf(x) < CUDART_INF_F)) { hi = __float_as_uint(x); lo = 0u; }      // infinities and NaN stay what they are
 }
-__device__ __forceinline__ void gm_mma16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void gm_ldsm(uint32_t (&r)[4], const __half* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
-}
-__device__ __forceinline__ void gm_ldsm_t(uint32_t (&r)[4], const __half* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
-}
-// The lane's row and column offset for the four 8 x 8 blocks of a 16 x 16 fragment: A by rows or B by rows of the inner index
-// (trans) take `a`, B by rows of its columns or A by rows of the inner index (trans) take `b`.
-__device__ __forceinline__ int gm_off_a(int lane, int pitch) { return (lane & 15) * pitch + (lane >> 4) * 8; }
-__device__ __forceinline__ int gm_off_b(int lane, int pitch) { return ((lane & 7) + (lane >> 4) * 8) * pitch + ((lane >> 3) & 1) * 8; }
-// acc (16 x 16, rows i0, columns j0) = X Y^T of two fp16 tiles stored along the inner index, `width` (rounded up to 16: zeros) long
-__device__ __forceinline__ void gm_exact(float (&acc)[2][4], GmTile x, int i0, GmTile y, int j0, int width) {
-  const int lane = threadIdx.x & 31;
-  const __half *pa = x.p + i0 * x.pitch + gm_off_a(lane, x.pitch), *pb = y.p + j0 * y.pitch + gm_off_b(lane, y.pitch);
-#pragma unroll 4
-  for (int l = 0; l < width; l += 16) {
-    uint32_t a[4], b[4];
-    gm_ldsm(a, pa + l);
-    gm_ldsm(b, pb + l);
-    float part[2][4] = {};
-    gm_mma16(part[0], a, b[0], b[1]);
-    gm_mma16(part[1], a, b[2], b[3]);
-#pragma unroll
-    for (int e = 0; e < 4; ++e) { acc[0][e] += part[0][e]; acc[1][e] += part[1][e]; }
-  }
-}
-
 // acc (16 x 8 NT) += sum over l in [l0, l1) of A(i, l) B(l, j) (the outer loop: see the head of the file), one operand exact in tf32 and the other (SPLIT_A: A, else B) in two
 // parts.  The sum's order is free, so that slots t and t + 4 of a fragment's inner index stand for l = 2t and 2t + 1: a pair is one
 // 8-byte read of an fp32 operand stored along l, and one 8 x 8 block of ldmatrix (two halves a lane) of an fp16 operand,
@@ -267,46 +184,6 @@ __device__ __forceinline__ auto gm_b_frows(const float* s, int pitch, int j0, in
     for (int n = 0; n < NT; ++n) b[n] = n < nt ? *reinterpret_cast<const float2*>(p + 8 * n * pitch + l) : make_float2(0.f, 0.f);
   };
 }
-// The same product where A is triangular (SA) and B holds a non-finite value: element by element, only over the l that
-// ok(i, l) admits.
-template <int NT, class LA, class LB, class OK>
-__device__ __noinline__ void gm_product_masked(float (&acc)[NT][4], int i0, int j0, int nt, int l0, int l1, LA la, LB lb, OK ok) {
-  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  for (int l = l0; l < l1; l += 2)
-    for (int r = 0; r < 2; ++r) {
-      const int i = i0 + g + 8 * r;
-      const float2 a = la(i, l);
-#pragma unroll
-      for (int n = 0; n < NT; ++n)
-        if (n < nt)
-          for (int e = 0; e < 2; ++e) {
-            const float2 b = lb(l, j0 + 8 * n + 2 * t + e);
-            if (ok(i, l)) acc[n][2 * r + e] = fmaf(a.x, b.x, acc[n][2 * r + e]);
-            if (ok(i, l + 1)) acc[n][2 * r + e] = fmaf(a.y, b.y, acc[n][2 * r + e]);
-          }
-    }
-}
-template <int NT>
-__device__ __forceinline__ void gm_zero(float (&acc)[NT][4]) {
-#pragma unroll
-  for (int n = 0; n < NT; ++n)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) acc[n][e] = 0.f;
-}
-// single elements of operands
-__device__ __forceinline__ float2 gm_row(GmTile x, int i, int l) {          // fp16 tile stored along l: x[i][l], x[i][l + 1]
-  return __half22float2(*reinterpret_cast<const __half2*>(x.p + i * x.pitch + l));
-}
-__device__ __forceinline__ float2 gm_col(GmTile x, int l, int j) {          // fp16 tile stored across l: x[l][j], x[l + 1][j]
-  return make_float2(__half2float(x.p[l * x.pitch + j]), __half2float(x.p[(l + 1) * x.pitch + j]));
-}
-__device__ __forceinline__ float2 gm_frow(const float* s, int pitch, int i, int l) { return *reinterpret_cast<const float2*>(s + i * pitch + l); }
-__device__ __forceinline__ float2 gm_fcol(const float* s, int pitch, int l, int j) { return make_float2(s[l * pitch + j], s[(l + 1) * pitch + j]); }
-__device__ __forceinline__ float gm_quad(float v) {
-  v += __shfl_xor_sync(0xffffffffu, v, 1);
-  return v + __shfl_xor_sync(0xffffffffu, v, 2);
-}
-
 // ---- shared steps ------------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void gm_state_in(float* S, float* z, const GmLayout& L, const float* s_in, const float* z_in, int K, int d) {
   for (int e = threadIdx.x; e < L.Kp * d; e += blockDim.x) {
@@ -321,12 +198,6 @@ __device__ __forceinline__ void gm_state_out(const float* S, const float* z, con
     s_out[e] = S[kk * L.ps + n];
   }
   for (int i = threadIdx.x; i < K; i += blockDim.x) z_out[i] = z[i];
-}
-// zero the pad columns that gm_exact reads, once: the loads never touch them
-__device__ __forceinline__ void gm_pad(GmTile tile, int C, int width) {
-  const int w = gm_round16(width) - width;         // 0 or 8
-  if (w)
-    for (int i = threadIdx.x; i < C; i += blockDim.x) *reinterpret_cast<uint4*>(const_cast<__half*>(tile.p) + i * tile.pitch + width) = make_uint4(0, 0, 0, 0);
 }
 // S += X^T (wy Y), z += X^T wz over a chunk: summed in registers from zero, then added to the fp32 state with one rounding.
 // WEIGHTED: per-row factors inv (of Y) and gz (of z); else 1.
@@ -386,22 +257,6 @@ __device__ __forceinline__ void gm_update(float* S, float* z, const GmLayout& L,
     }
   }
 }
-// qz[row] = q[row] . z, four threads per row
-template <int C>
-__device__ __forceinline__ void gm_qz(float* qz, GmTile q, const float* z, int K) {
-  const int row = threadIdx.x >> 2;
-  if (row < C) {                                       // whole warps: C is a multiple of 8
-    float s = 0.f;
-    for (int l = 2 * (threadIdx.x & 3); l < K; l += 8) {
-      const float2 a = gm_row(q, row, l);
-      s = fmaf(a.x, z[l], fmaf(a.y, z[l + 1], s));
-    }
-    s = gm_quad(s);
-    if ((threadIdx.x & 3) == 0) qz[row] = s;
-  }
-}
-__device__ __forceinline__ void gm_store2(__half* p, float a, float b) { *reinterpret_cast<__half2*>(p) = __floats2half2_rn(a, b); }
-
 // ===========================================================================================================================
 // forward.  grid (BH, nseg); s_seg / z_seg: the state entering each segment (null = zero)
 // ===========================================================================================================================
@@ -423,13 +278,14 @@ gm_causal_fwd_kernel(const __half* __restrict__ q, const __half* __restrict__ k,
     unsigned char* b = gm_raw + L.tile + (uint32_t)(STAGES == 2 ? c & 1 : 0) * (2 * L.x_bytes + L.y_bytes);
     return GmTile{(const __half*)(b + which * L.x_bytes), which < 2 ? L.px : L.py};
   };
+  const GmWalk walk_x = gm_walk(K), walk_y = gm_walk(d);
   auto load = [&](int c) {
     if (c < nchunk) {
       const int64_t t0 = t_begin + (int64_t)c * C;
       const int valid = (int)min((int64_t)C, t_end - t0);
-      gm_load((__half*)tile(c, 0).p, L.px, q, C, K, t0, valid, BH, bh, nullptr);
-      gm_load((__half*)tile(c, 1).p, L.px, k, C, K, t0, valid, BH, bh, nullptr);
-      gm_load((__half*)tile(c, 2).p, L.py, v, C, d, t0, valid, BH, bh, nullptr);
+      gm_load((__half*)tile(c, 0).p, L.px, q, C, K, walk_x, t0, valid, BH, bh, nullptr);
+      gm_load((__half*)tile(c, 1).p, L.px, k, C, K, walk_x, t0, valid, BH, bh, nullptr);
+      gm_load((__half*)tile(c, 2).p, L.py, v, C, d, walk_y, t0, valid, BH, bh, nullptr);
     }
     gm_commit();
   };
@@ -442,7 +298,7 @@ gm_causal_fwd_kernel(const __half* __restrict__ q, const __half* __restrict__ k,
     const GmTile tq = tile(c, 0), tk = tile(c, 1), tv = tile(c, 2);
     const int64_t t0 = t_begin + (int64_t)c * C;
     const int valid = (int)min((int64_t)C, t_end - t0);
-    const bool odd = __syncthreads_or(gm_odd(tv.p, tv.pitch, C, d)) != 0;
+    const bool odd = __syncthreads_or(gm_odd(tv.p, tv.pitch, C, walk_y)) != 0;
     // P = tril(Q K^T), its row sums per 16 columns, q . z
     constexpr int MT = C / 16;
     for (int w = warp; w < MT * MT; w += blockDim.x >> 5) {
@@ -528,14 +384,15 @@ gm_causal_bwd_q_kernel(const __half* __restrict__ q, const __half* __restrict__ 
     unsigned char* b = gm_raw + L.tile + (uint32_t)(STAGES == 2 ? c & 1 : 0) * (2 * L.x_bytes + 2 * L.y_bytes);
     return GmTile{(const __half*)(b + (which < 2 ? which * L.x_bytes : 2 * L.x_bytes + (which - 2) * L.y_bytes)), which < 2 ? L.px : L.py};
   };
+  const GmWalk walk_x = gm_walk(K), walk_y = gm_walk(d);
   auto load = [&](int c) {
     if (c < nchunk) {
       const int64_t t0 = t_begin + (int64_t)c * C;
       const int valid = (int)min((int64_t)C, t_end - t0);
-      gm_load((__half*)tile(c, 0).p, L.px, q, C, K, t0, valid, BH, bh, nullptr);
-      gm_load((__half*)tile(c, 1).p, L.px, k, C, K, t0, valid, BH, bh, nullptr);
-      gm_load((__half*)tile(c, 2).p, L.py, v, C, d, t0, valid, BH, bh, nullptr);
-      gm_load((__half*)tile(c, 3).p, L.py, gr, C, d, t0, valid, BH, bh, nullptr);
+      gm_load((__half*)tile(c, 0).p, L.px, q, C, K, walk_x, t0, valid, BH, bh, nullptr);
+      gm_load((__half*)tile(c, 1).p, L.px, k, C, K, walk_x, t0, valid, BH, bh, nullptr);
+      gm_load((__half*)tile(c, 2).p, L.py, v, C, d, walk_y, t0, valid, BH, bh, nullptr);
+      gm_load((__half*)tile(c, 3).p, L.py, gr, C, d, walk_y, t0, valid, BH, bh, nullptr);
     }
     gm_commit();
   };
@@ -548,7 +405,7 @@ gm_causal_bwd_q_kernel(const __half* __restrict__ q, const __half* __restrict__ 
     const GmTile tq = tile(c, 0), tk = tile(c, 1), tv = tile(c, 2), tg = tile(c, 3);
     const int64_t t0 = t_begin + (int64_t)c * C;
     const int valid = (int)min((int64_t)C, t_end - t0);
-    const bool odd = __syncthreads_or(gm_odd(tk.p, tk.pitch, C, K)) != 0;
+    const bool odd = __syncthreads_or(gm_odd(tk.p, tk.pitch, C, walk_x)) != 0;
     // G = g V^T on and below the diagonal; per 16 columns the row sums of P and of P o G
     for (int w = warp; w < MT * MT; w += blockDim.x >> 5) {
       const int mi = w / MT, ni = w % MT, i0 = mi * 16, j0 = ni * 16;
@@ -649,15 +506,6 @@ gm_causal_bwd_q_kernel(const __half* __restrict__ q, const __half* __restrict__ 
   }
 }
 
-// inv and gz of a chunk's rows, from what sweep 1 left
-__device__ __forceinline__ void gm_row_scalars(float* inv, float* gz, const float* ws_den, const float* ws_gz, int C, size_t base, int valid) {
-  const int i = threadIdx.x;
-  if (i < C) {
-    inv[i] = i < valid ? 1.f / fmaxf(ws_den[base + i], kEps) : 0.f;
-    gz[i] = i < valid ? ws_gz[base + i] : 0.f;
-  }
-}
-
 // ===========================================================================================================================
 // backward, sweep 2 (chunks in reverse): gk, gv
 // ===========================================================================================================================
@@ -681,14 +529,15 @@ gm_causal_bwd_kv_kernel(const __half* __restrict__ q, const __half* __restrict__
     unsigned char* b = gm_raw + L.tile + (uint32_t)(STAGES == 2 ? c & 1 : 0) * (2 * L.x_bytes + 2 * L.y_bytes);
     return GmTile{(const __half*)(b + (which < 2 ? which * L.x_bytes : 2 * L.x_bytes + (which - 2) * L.y_bytes)), which < 2 ? L.px : L.py};
   };
+  const GmWalk walk_x = gm_walk(K), walk_y = gm_walk(d);
   auto load = [&](int c) {                   // c counts down to 0
     if (c >= 0) {
       const int64_t t0 = t_begin + (int64_t)c * C;
       const int valid = (int)min((int64_t)C, t_end - t0);
-      gm_load((__half*)tile(c, 0).p, L.px, q, C, K, t0, valid, BH, bh, nullptr);
-      gm_load((__half*)tile(c, 1).p, L.px, k, C, K, t0, valid, BH, bh, nullptr);
-      gm_load((__half*)tile(c, 2).p, L.py, v, C, d, t0, valid, BH, bh, nullptr);
-      gm_load((__half*)tile(c, 3).p, L.py, gr, C, d, t0, valid, BH, bh, nullptr);
+      gm_load((__half*)tile(c, 0).p, L.px, q, C, K, walk_x, t0, valid, BH, bh, nullptr);
+      gm_load((__half*)tile(c, 1).p, L.px, k, C, K, walk_x, t0, valid, BH, bh, nullptr);
+      gm_load((__half*)tile(c, 2).p, L.py, v, C, d, walk_y, t0, valid, BH, bh, nullptr);
+      gm_load((__half*)tile(c, 3).p, L.py, gr, C, d, walk_y, t0, valid, BH, bh, nullptr);
     }
     gm_commit();
   };
@@ -702,7 +551,7 @@ gm_causal_bwd_kv_kernel(const __half* __restrict__ q, const __half* __restrict__
     gm_row_scalars(inv, gz, ws_den, ws_gz, C, (size_t)bh * T + t0, valid);
     if (STAGES == 2) { load(c - 1); gm_wait<1>(); } else gm_wait<0>();
     const GmTile tq = tile(c, 0), tk = tile(c, 1), tv = tile(c, 2), tg = tile(c, 3);
-    const bool odd = __syncthreads_or(gm_odd(tq.p, tq.pitch, C, K) || gm_odd(tg.p, tg.pitch, C, d)) != 0;
+    const bool odd = __syncthreads_or(gm_odd(tq.p, tq.pitch, C, walk_x) || gm_odd(tg.p, tg.pitch, C, walk_y)) != 0;
     // P' = inv tril(Q K^T), D = tril(inv g V^T + gz)
     for (int w = warp; w < MT * MT; w += blockDim.x >> 5) {
       const int mi = w / MT, ni = w % MT, i0 = mi * 16, j0 = ni * 16;
@@ -799,12 +648,13 @@ gm_state_kernel(const __half* __restrict__ x, const __half* __restrict__ y, cons
     unsigned char* b = gm_raw + L.tile + (uint32_t)(STAGES == 2 ? c & 1 : 0) * (L.x_bytes + L.y_bytes);
     return GmTile{(const __half*)(b + which * L.x_bytes), which < 1 ? L.px : L.py};
   };
+  const GmWalk walk_x = gm_walk(K), walk_y = gm_walk(d);
   auto load = [&](int c) {
     if (c < nchunk) {
       const int64_t t0 = t_begin + (int64_t)c * C;
       const int valid = (int)min((int64_t)C, t_end - t0);
-      gm_load((__half*)tile(c, 0).p, L.px, x, C, K, t0, valid, BH, bh, mrow);
-      gm_load((__half*)tile(c, 1).p, L.py, y, C, d, t0, valid, BH, bh, mrow);
+      gm_load((__half*)tile(c, 0).p, L.px, x, C, K, walk_x, t0, valid, BH, bh, mrow);
+      gm_load((__half*)tile(c, 1).p, L.py, y, C, d, walk_y, t0, valid, BH, bh, mrow);
     }
     gm_commit();
   };
@@ -848,9 +698,22 @@ static GmShape gm_shape(int K, int d) {
   return GmShape{0, 0, 0, 0};
 }
 
+// the kernels whose operands are split into fp16 tiles once (generic_split.cu), where they fit
+int split_chunk(int K, int d, int* ctas);
+int launch_causal_split_fwd(const __half* q, const __half* k, const __half* v, __half* out, const float* s_seg, const float* z_seg, float* s_out,
+                            float* z_out, float* den_out, int64_t T, int BH, int nseg, int64_t tseg, int K, int d, cudaStream_t st);
+int launch_causal_split_bwd_q(const __half* q, const __half* k, const __half* v, const __half* g, __half* gq, const float* s_seg, const float* z_seg,
+                              float* ws_den, float* ws_gz, int64_t T, int BH, int nseg, int64_t tseg, int K, int d, cudaStream_t st);
+int launch_causal_split_bwd_kv(const __half* q, const __half* k, const __half* v, const __half* g, __half* gk, __half* gv, const float* ws_den,
+                               const float* ws_gz, const float* ds_seg, const float* dz_seg, int64_t T, int BH, int nseg, int64_t tseg, int K,
+                               int d, cudaStream_t st);
+int launch_state_split(const __half* x, const __half* y, const uint8_t* pad_mask, const float* ws_den, const float* ws_gz, float* s, float* z,
+                       int64_t T, int BH, int H, int nseg, int64_t tseg, int runs, int K, int d, cudaStream_t st);
+
 // Tokens per chunk of the chunked kernels for this geometry, 0 when it does not fit them; *ctas = how many of their CTAs
 // one SM holds.
 int generic_chunk(int K, int d, int* ctas) {
+  if (const int chunk = split_chunk(K, d, ctas)) return chunk;
   if (K <= 0 || d <= 0 || K % 8 || d % 8 || K > 1024 || d > 1024) return 0;
   const GmShape s = gm_shape(K, d);
   if (ctas) *ctas = s.ctas;
@@ -867,7 +730,7 @@ static int gm_launch(KERNEL kernel, const char* what, int threads, uint32_t smem
 #define RFA_GM_DISPATCH(shape, CALL)                                  \
   do {                                                                \
     const GmShape gs_ = (shape);                                      \
-    if (gs_.C == 64) { if (gs_.stages == 2) { CALL(64, 2); } else { CALL(64, 1); } } \
+    if (gs_.C == 64) { CALL(64, 1); }                                 \
     if (gs_.C == 32) { if (gs_.stages == 2) { CALL(32, 2); } else { CALL(32, 1); } } \
     if (gs_.stages == 2) { CALL(16, 2); } else { CALL(16, 1); }       \
   } while (0)
@@ -875,6 +738,7 @@ static int gm_launch(KERNEL kernel, const char* what, int threads, uint32_t smem
 int launch_causal_chunked_fwd(const __half* q, const __half* k, const __half* v, __half* out, const float* s_seg, const float* z_seg,
                               float* s_out, float* z_out, float* den_out, int64_t T, int BH, int nseg, int64_t tseg, int K, int d,
                               cudaStream_t st) {
+  if (split_chunk(K, d, nullptr)) return launch_causal_split_fwd(q, k, v, out, s_seg, z_seg, s_out, z_out, den_out, T, BH, nseg, tseg, K, d, st);
 #define RFA_GM_CALL(C, N) return gm_launch(gm_causal_fwd_kernel<C, N>, "rfa_causal_fwd (chunked)", gs_.threads, gm_layout(C, K, d, N, 2, 1, 1, gm_rows_fwd(C)).total, \
                                            dim3(BH, nseg), st, q, k, v, out, s_seg, z_seg, s_out, z_out, den_out, T, BH, tseg, K, d)
   RFA_GM_DISPATCH(gm_shape(K, d), RFA_GM_CALL);
@@ -884,6 +748,7 @@ int launch_causal_chunked_fwd(const __half* q, const __half* k, const __half* v,
 int launch_causal_chunked_bwd_q(const __half* q, const __half* k, const __half* v, const __half* g, __half* gq, const float* s_seg,
                                 const float* z_seg, float* ws_den, float* ws_gz, int64_t T, int BH, int nseg, int64_t tseg, int K, int d,
                                 cudaStream_t st) {
+  if (split_chunk(K, d, nullptr)) return launch_causal_split_bwd_q(q, k, v, g, gq, s_seg, z_seg, ws_den, ws_gz, T, BH, nseg, tseg, K, d, st);
 #define RFA_GM_CALL(C, N) return gm_launch(gm_causal_bwd_q_kernel<C, N>, "rfa_causal_bwd_q (chunked)", gs_.threads, gm_layout(C, K, d, N, 2, 2, 1, gm_rows_bwd_q(C, K)).total, \
                                            dim3(BH, nseg), st, q, k, v, g, gq, s_seg, z_seg, ws_den, ws_gz, T, BH, tseg, K, d)
   RFA_GM_DISPATCH(gm_shape(K, d), RFA_GM_CALL);
@@ -893,6 +758,7 @@ int launch_causal_chunked_bwd_q(const __half* q, const __half* k, const __half* 
 int launch_causal_chunked_bwd_kv(const __half* q, const __half* k, const __half* v, const __half* g, __half* gk, __half* gv,
                                  const float* ws_den, const float* ws_gz, const float* ds_seg, const float* dz_seg, int64_t T, int BH,
                                  int nseg, int64_t tseg, int K, int d, cudaStream_t st) {
+  if (split_chunk(K, d, nullptr)) return launch_causal_split_bwd_kv(q, k, v, g, gk, gv, ws_den, ws_gz, ds_seg, dz_seg, T, BH, nseg, tseg, K, d, st);
 #define RFA_GM_CALL(C, N) return gm_launch(gm_causal_bwd_kv_kernel<C, N>, "rfa_causal_bwd_kv (chunked)", gs_.threads, gm_layout(C, K, d, N, 2, 2, 2, kGmRowsKv).total, \
                                            dim3(BH, nseg), st, q, k, v, g, gk, gv, ws_den, ws_gz, ds_seg, dz_seg, T, BH, tseg, K, d)
   RFA_GM_DISPATCH(gm_shape(K, d), RFA_GM_CALL);
@@ -902,6 +768,7 @@ int launch_causal_chunked_bwd_kv(const __half* q, const __half* k, const __half*
 // the first `runs` of nseg runs of tokens; ws_den / ws_gz null: sums of k (x) v and k; else of q (x) (g / den) and gz q
 int launch_state_chunked(const __half* x, const __half* y, const uint8_t* pad_mask, const float* ws_den, const float* ws_gz, float* s,
                          float* z, int64_t T, int BH, int H, int nseg, int64_t tseg, int runs, int K, int d, cudaStream_t st) {
+  if (split_chunk(K, d, nullptr)) return launch_state_split(x, y, pad_mask, ws_den, ws_gz, s, z, T, BH, H, nseg, tseg, runs, K, d, st);
 #define RFA_GM_CALL(C, N)                                                                                                             \
   return ws_den ? gm_launch(gm_state_kernel<C, N, true>, "state reduction (chunked)", gs_.threads, gm_layout(C, K, d, N, 1, 1, 0, kGmRowsState).total, \
                             dim3(BH, runs), st, x, y, pad_mask, ws_den, ws_gz, s, z, T, BH, H, nseg, tseg, K, d)                             \

@@ -1,4 +1,4 @@
-"""The chunked kernels of the geometries other than K = 128, d = 64 (csrc/generic_mma.cu) against the PyTorch twins in fp64.
+"""The chunked kernels of the geometries other than K = 128, d = 64 (csrc/generic_split.cu, generic_mma.cu) against the PyTorch twins in fp64.
 
 Results are fp16, so that a correct one is within half a unit in the last place of the fp64 value: 2^-11 = 4.9e-4 relative at
 worst, 2.9e-4 in the 2-norm of evenly spread significands; the gate is 4e-4 in the 2-norm.  Below fp16's smallest normal number
@@ -106,6 +106,26 @@ def test_no_token_sees_a_later_non_finite_one(dev, which):
     if which == 0:       # q of a token reaches the key gradients of itself and of earlier tokens only
         _, gk, gv = RFA.backward_cuda(q, k, v, g)
         assert torch.isfinite(gk[cut + 1:]).all() and torch.isfinite(gv[cut + 1:]).all()
+
+
+@pytest.mark.parametrize("K,d", [(64, 32), (96, 40), (72, 24)])
+@pytest.mark.parametrize("T", [33, 200])
+def test_columns_and_tokens_of_very_different_magnitude(dev, K, d, T):
+    """A split operand has one power of two per 16 x 16 block: columns of v and g from 2^-9 to 2^9 and tokens of q and k from 2^-8 to 1
+    share blocks, and every column of out and gv (a product with those columns alone) still has fp16's rounding error and no more."""
+    q, k, v, g = inputs(T, 2, K, d, T)
+    gen = torch.Generator().manual_seed(K)
+    tokens = 2.0 ** torch.randint(-8, 1, (T, 1, 1), generator=gen)
+    columns = 2.0 ** torch.linspace(-9, 9, d).round()
+    q, k, v, g = (q * tokens).half(), (k * tokens.flip(0)).half(), (v * columns).half(), (g * columns.flip(0)).half()
+    want = RFA.forward_torch(*(t.double() for t in (q, k, v)))
+    gq, gk, gv = RFA.backward_torch(*(t.double() for t in (q, k, v, g)))
+    leaves = [t.to(dev).requires_grad_() for t in (q, k, v)]
+    out = RFA.apply(*leaves)
+    out.backward(g.to(dev))
+    for j in range(d):
+        assert rel(out[..., j], want[..., j], 2.0 ** -24) < 4e-4 and rel(leaves[2].grad[..., j], gv[..., j], 2.0 ** -24) < 4e-4, j
+    assert rel(leaves[0].grad, gq, 2.0 ** -24) < 4e-4 and rel(leaves[1].grad, gk, 2.0 ** -24) < 4e-4
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
