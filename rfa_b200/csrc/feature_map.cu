@@ -1,4 +1,5 @@
-// Fused random feature map and its gradient.
+// Fused random feature map and its gradient on register tiles: widths above 64, and few rows (the rest: feature_map_mma.cu,
+// feature_map_tc.cu).
 //
 //   n = |x|_2,  xh = x / (n + 1e-3),  u = W_h xh,  phi = scale * [sin u | cos u]
 // (upstream utils.py:100-120, one pass instead of norm/div/einsum/sin/cos/cat/mul).
@@ -6,6 +7,7 @@
 // tiles of 64 rows with that head's W resident in shared memory; each x element is
 // read once and each phi element written once.
 #include "common.cuh"
+#include "trig.cuh"
 
 namespace rfa {
 
@@ -121,7 +123,7 @@ feature_map_fwd_kernel(const TX* __restrict__ x, const float* __restrict__ w, co
         if (row >= rows) continue;
         const float sc = (row_mask && row_mask[row]) ? 0.f : scale;     // a masked row gets all-zero features
         float4 sn, cs;
-        sincosf(u[i][0], &sn.x, &cs.x); sincosf(u[i][1], &sn.y, &cs.y); sincosf(u[i][2], &sn.z, &cs.z); sincosf(u[i][3], &sn.w, &cs.w);
+        fm_sincos(u[i][0], sn.x, cs.x); fm_sincos(u[i][1], sn.y, cs.y); fm_sincos(u[i][2], sn.z, cs.z); fm_sincos(u[i][3], sn.w, cs.w);
         TP* dst = phi + ((size_t)row * H + h) * 2 * D + col;
         store4(dst, make_float4(sn.x * sc, sn.y * sc, sn.z * sc, sn.w * sc));
         store4(dst + D, make_float4(cs.x * sc, cs.y * sc, cs.z * sc, cs.w * sc));
@@ -178,10 +180,10 @@ feature_map_bwd_kernel(const T* __restrict__ x, const float* __restrict__ w, con
       for (int i = 0; i < kFmI; ++i) {
         float4 gu;
         float sn, cs;
-        sincosf(u[i][0], &sn, &cs); gu.x = scale * (gs[i].x * cs - gc[i].x * sn);
-        sincosf(u[i][1], &sn, &cs); gu.y = scale * (gs[i].y * cs - gc[i].y * sn);
-        sincosf(u[i][2], &sn, &cs); gu.z = scale * (gs[i].z * cs - gc[i].z * sn);
-        sincosf(u[i][3], &sn, &cs); gu.w = scale * (gs[i].w * cs - gc[i].w * sn);
+        fm_sincos(u[i][0], sn, cs); gu.x = scale * (gs[i].x * cs - gc[i].x * sn);
+        fm_sincos(u[i][1], sn, cs); gu.y = scale * (gs[i].y * cs - gc[i].y * sn);
+        fm_sincos(u[i][2], sn, cs); gu.z = scale * (gs[i].z * cs - gc[i].z * sn);
+        fm_sincos(u[i][3], sn, cs); gu.w = scale * (gs[i].w * cs - gc[i].w * sn);
         dot[i] = fmaf(gu.x, u[i][0], fmaf(gu.y, u[i][1], fmaf(gu.z, u[i][2], fmaf(gu.w, u[i][3], dot[i]))));
         store4(s.GU + (rg + 16 * i) * (D + 4) + col, gu);
       }
@@ -240,6 +242,14 @@ int launch_feature_map_bwd_tc(const __half* x, const float* w, const uint8_t* ro
                               const __half* x2, const uint8_t* row_mask2, const __half* g_phi2, __half* g_x2, float* g_w,
                               int64_t rows, int H, float scale, int sms, cudaStream_t st);
 
+// split operands on the tensor cores for widths up to 64 (feature_map_mma.cu)
+template <typename TX, typename TP>
+int launch_feature_map_mma_fwd(const TX* x, const float* w, const uint8_t* row_mask, TP* phi, int64_t rows, int H, int d, int D, float scale,
+                               int sms, cudaStream_t st);
+template <typename T>
+int launch_feature_map_mma_bwd(const T* x, const float* w, const uint8_t* row_mask, const T* g_phi, T* g_x, float* g_w, int64_t rows, int H,
+                               int d, int D, float scale, int sms, cudaStream_t st);
+
 static int fm_check(const void* x, const float* w, int64_t rows, int H, int d, int D) {
   RFA_REQUIRE(x && w, RFA_EINVAL, "feature_map: null pointer");
   RFA_REQUIRE(rows >= 0 && H > 0 && d > 0 && D > 0, RFA_EINVAL, "feature_map: rows=%lld H=%d d=%d D=%d",
@@ -249,6 +259,13 @@ static int fm_check(const void* x, const float* w, int64_t rows, int H, int d, i
   RFA_REQUIRE(H <= 65535, RFA_EUNSUPPORTED, "feature_map: H=%d exceeds 65535", H);
   return 0;
 }
+
+// Whether the tensor-core kernels take it: a warp of theirs owns 16 rows, and below four of those to an SM its chain through
+// products and sines is longer than what the register tiles here take with a whole CTA to 64 (32) rows.  us, here / there: fp32 64 x 64,
+// 8 heads x 16, 256, 1024, 1536, 2048, 3072 rows forward 6.1 / 7.0, 7.3 / 7.1, 7.4 / 8.1, 10.2 / 8.4, 10.2 / 8.4, 13.6 / 10.4, backward
+// 10.5 / 14.1, 10.8 / 14.7, 16.4 / 18.0, 21.5 / 18.7, 22.5 / 19.4, 37.3 / 22.4; 32 x 32, 16 x 512 5.9 / 5.6 and 9.9 / 10.6, 8 x 1536 7.2 / 5.8
+// and 13.6 / 11.3.
+static bool fm_mma(int64_t rows, int H, int d, int D, int sms) { return d <= 64 && D <= 64 && (rows + 15) / 16 * H > 4 * sms; }
 
 // CTAs per head, so that the grid is one wave of the `ctas` that an SM holds
 static int fm_grid_x(int64_t rows, int tile, int H, int ctas) {
@@ -273,12 +290,19 @@ extern "C" int rfa_feature_map_fwd_masked(const void* x, int x_dtype, const floa
   RFA_REQUIRE(phi, RFA_EINVAL, "feature_map_fwd: null output");
   RFA_REQUIRE(aligned16(x) && aligned16(w) && aligned16(phi), RFA_EALIGN, "feature_map_fwd: 16-byte alignment required");
   if (rows == 0) return 0;
-  if (x_dtype == RFA_F16 && phi_dtype == RFA_F16 && d == 64 && D == 64) {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (x_dtype == RFA_F16 && phi_dtype == RFA_F16 && d == 64 && D == 64)
     return launch_feature_map_fwd_tc((const __half*)x, w, row_mask, (__half*)phi, nullptr, nullptr, nullptr, rows, H, scale, sms,
                                      as_stream(stream));
+  if (fm_mma(rows, H, d, D, sms)) {
+#define RFA_MMA(TX, TP) return launch_feature_map_mma_fwd<TX, TP>((const TX*)x, w, row_mask, (TP*)phi, rows, H, d, D, scale, sms, as_stream(stream))
+    if (x_dtype == RFA_F16 && phi_dtype == RFA_F16) RFA_MMA(__half, __half);
+    if (x_dtype == RFA_F32 && phi_dtype == RFA_F32) RFA_MMA(float, float);
+    if (x_dtype == RFA_F16 && phi_dtype == RFA_F32) RFA_MMA(__half, float);
+    if (x_dtype == RFA_F32 && phi_dtype == RFA_F16) RFA_MMA(float, __half);
+#undef RFA_MMA
   }
   const size_t smem = fm_smem_floats(64, D, d, false) * sizeof(float);      // 100 KB at most (D, d <= 128)
   const dim3 grid(fm_grid_x(rows, 64, H, fm_ctas(smem, 4)), H);
@@ -312,20 +336,22 @@ extern "C" int rfa_feature_map_bwd_masked(const void* x, int x_dtype, const floa
   RFA_REQUIRE(x_dtype == g_dtype && x_dtype == gx_dtype, RFA_EUNSUPPORTED,
               "feature_map_bwd: x, g_phi and g_x must share one dtype");
   if (rows == 0) return 0;
-  if (x_dtype == RFA_F16 && d == 64 && D == 64) {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (x_dtype == RFA_F16 && d == 64 && D == 64)
     return launch_feature_map_bwd_tc((const __half*)x, w, row_mask, (const __half*)g_phi, (__half*)g_x, nullptr, nullptr, nullptr,
                                      nullptr, g_w, rows, H, scale, sms, as_stream(stream));
+  if (fm_mma(rows, H, d, D, sms)) {
+    if (x_dtype == RFA_F16) return launch_feature_map_mma_bwd((const __half*)x, w, row_mask, (const __half*)g_phi, (__half*)g_x, g_w, rows, H, d, D,
+                                                              scale, sms, as_stream(stream));
+    if (x_dtype == RFA_F32) return launch_feature_map_mma_bwd((const float*)x, w, row_mask, (const float*)g_phi, (float*)g_x, g_w, rows, H, d, D,
+                                                              scale, sms, as_stream(stream));
   }
   const bool small = D * d <= 4096;
   // Tiles of 32 rows where those of 64 would not give every SM one: a tile's three products follow one another, and so few
   // CTAs are bound by that chain.  (128 x 128, 8 heads x 1, 64, 512 rows: 39, 42, 43 us in
   // tiles of 64, 29, 30, 33 in tiles of 32; 64 x 64, 8 heads x 256 rows: 14.8 and 11.0.)
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int tile = (rows + 63) / 64 * H < sms ? 32 : 64;
   const size_t smem = fm_smem_floats(tile, D, d, true) * sizeof(float);      // 199 KB at most (64 rows, D, d <= 128)
   const dim3 grid(fm_grid_x(rows, tile, H, fm_ctas(smem, small ? 2 : 1)), H);

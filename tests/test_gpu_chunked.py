@@ -151,6 +151,64 @@ def test_feature_map_of_any_width_against_fp64(dev, dtype, rows, H, D, d):
     assert rel(wg.grad, wd.grad) < (2e-3 if tc else 2e-6)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("D,d", [(64, 64), (32, 32), (48, 40), (8, 64), (56, 8)])
+@pytest.mark.parametrize("rows,H", [(197 * 16, 3), (197 * 16 + 1, 3), (131, 148), (16, 1000), (9601, 1)])
+def test_feature_map_on_split_operands(dev, dtype, rows, H, D, d):
+    """csrc/feature_map_mma.cu from more than four groups of 16 rows to an SM on (the first case has one too few): ragged groups,
+    shares of unequal length, CTAs with one group, widths that end inside a block of 16 or 32.  Gates as for the other fp32 kernels; a row
+    of zeros, one of 1e4 and one with an infinity, whose results are NaN and touch no other row."""
+    if dtype == torch.float16 and (D, d) == (64, 64):
+        pytest.skip("the tensor-core kernel for fp16 operands")
+    from rfa_b200 import ops
+    gen = torch.Generator(dev).manual_seed(rows + D)
+    x, g = torch.randn(rows, H, d, generator=gen, device=dev).to(dtype), torch.randn(rows, H, 2 * D, generator=gen, device=dev).to(dtype)
+    w = torch.randn(H, D, d, generator=gen, device=dev) * 2
+    x[3], x[5] = 0, x[5] * 1e4
+    mask = torch.rand(rows, generator=gen, device=dev) < 0.2
+    mask[3] = mask[5] = False
+    xd, wd = x.double().requires_grad_(), w.double().requires_grad_()
+    u = torch.einsum("thd,hkd->thk", xd / (xd.norm(dim=-1, keepdim=True) + 1e-3), wd)
+    ref = 0.1 * torch.cat([u.sin(), u.cos()], dim=-1) * ~mask[:, None, None]
+    ref.backward(g.double())
+    ref_gx = torch.nan_to_num(xd.grad)                       # the norm's gradient at a row of zeros
+    phi = ops.feature_map_fwd(x, w, 0.1, row_mask=mask)
+    gx, gw = ops.feature_map_bwd(x, w, g, 0.1, True, row_mask=mask)
+    err = lambda a, b: float((a.double() - b).norm() / b.norm())
+    half = dtype == torch.float16
+    keep = [i for i in range(rows) if i != 3]
+    assert err(phi, ref.detach()) < (4e-4 if half else 4e-7)
+    assert err(gx[keep], ref_gx[keep]) < (4e-4 if half else 1e-6) and err(gw, wd.grad) < 2e-6
+    assert torch.equal(ops.feature_map_bwd(x, w, g, 0.1, False, row_mask=mask)[0], gx)
+    x[7, 0, 0] = float("inf")
+    bad = ops.feature_map_fwd(x, w, 0.1, row_mask=mask)
+    assert not torch.isfinite(bad[7, 0]).any() or bool(mask[7])
+    assert torch.equal(bad[:7], phi[:7]) and torch.equal(bad[8:], phi[8:])
+    g[9, 0, 0] = float("inf")
+    mask[9] = False
+    x[7, 0, 0] = 0
+    bx, _ = ops.feature_map_bwd(x, w, g, 0.1, True, row_mask=mask)
+    assert not torch.isfinite(bx[9, 0]).any() and torch.equal(bx[16:], gx[16:])
+    assert torch.isfinite(bx[:9]).all() and torch.isfinite(bx[10:16]).all()
+    assert err(bx[10:16], ref_gx[10:16]) < (4e-4 if half else 1e-6)      # rows that share its 16 are summed element by element
+
+
+def test_sines_of_every_size(dev):
+    """csrc/trig.cuh through the feature map: one product a column, so that u is w to a rounding.  2e-7 absolute up to 8000, where the reduction
+    is its own, and beyond, where it is the library's."""
+    from rfa_b200 import ops
+    n = 4 * 148 * 16 + 16
+    w = torch.zeros(1, 64, 8, device=dev)
+    w[0, :, 0] = torch.cat([torch.linspace(-10, 10, 32, device=dev), 10 ** torch.linspace(1, 6, 32, device=dev)])
+    x = torch.zeros(n, 1, 8, device=dev)
+    x[:, 0, 0] = 1e4 * (1 + torch.rand(n, device=dev))
+    for rows in (n, 64):
+        phi = ops.feature_map_fwd(x[:rows], w, 1.0)[:, 0].double()
+        u = (x[:rows, 0, :1].double() / (x[:rows, 0, :1].double() + 1e-3)) * w[0, :, 0].double()
+        bound = 2e-7 + 2.0 ** -21 * u.abs()               # u itself is rounded: 22 bits of x and of w
+        assert ((phi[:, :64] - u.sin()).abs() <= bound).all() and ((phi[:, 64:] - u.cos()).abs() <= bound).all()
+
+
 @pytest.mark.parametrize("D,d", [(32, 32), (72, 96), (128, 128)])
 @pytest.mark.parametrize("rows,H", [(33, 147), (33, 148), (148 * 64 - 64, 1), (148 * 64 - 63, 1)])
 def test_feature_map_backward_in_tiles_of_32_and_64(dev, rows, H, D, d):
