@@ -342,6 +342,22 @@ int rfa_linear_rows(const void* x, const void* const* w, const void* const* b,
                     const void* rm, const void* sigma, float inv_tau, float* w_eff,
                     int H, int D, int d, rfa_stream_t stream);
 
+/* The small parts of a layer's training step, fp16 with fp32 sums.
+ * rfa_column_sums: out[m][c] = sum over rows of g[m][row][c] for `count` (1 to 3)
+ * arrays [rows, cols], cols a multiple of 8 (bias gradients); g, out are HOST
+ * arrays of device pointers.
+ * rfa_layer_matrices: w_eff [H, D, d] fp32 = (sigma * rm) * inv_tau as in
+ * rfa_linear_rows; pad_mask != NULL: row_mask [T, B] = pad_mask [B, T] transposed.
+ * rfa_layer_matrices_bwd: from g_w [H, D, d] fp32, g_sigma [H, d] and / or
+ * g_rm [H, D, d] (NULL: not wanted; sigma NULL: 1), d at most 256.
+ * replace what autograd makes of nn.Linear and build_random_matrices,
+ * causal_attention.py:222-248, utils.py:90-97. */
+int rfa_column_sums(const void* const* g, void* const* out, int count, int64_t rows, int cols, rfa_stream_t stream);
+int rfa_layer_matrices(const void* rm, const void* sigma, float inv_tau, float* w_eff, int H, int D, int d,
+                       const uint8_t* pad_mask, uint8_t* row_mask, int64_t T, int B, rfa_stream_t stream);
+int rfa_layer_matrices_bwd(const float* g_w, const void* rm, const void* sigma, float inv_tau, void* g_sigma, void* g_rm,
+                           int H, int D, int d, rfa_stream_t stream);
+
 /* One decoding step of cross attention for all L layers in one launch:
  *   out[l] = phi_q[l] . s_l / max(|phi_q[l] . z_l|, 1)
  * phi_q [L,BH,K], out [L,BH,d] of in_dtype; s_ptrs / z_ptrs: DEVICE arrays of L

@@ -59,6 +59,9 @@ SIGNATURES = {
     "rfa_stream_probe": (_int, [_vp, _vp, _i64, _int, _int, _int, _vp]),
     "rfa_cross_decode_step": (_int, [_vp, _int, _vp, _vp, _vp, _int, _int, _int, _int, _vp]),
     "rfa_linear_rows": (_int, [_vp] * 4 + [_int] * 4 + [_vp, _vp, _f32, _vp, _int, _int, _int, _vp]),
+    "rfa_column_sums": (_int, [_vp, _vp, _int, _i64, _int, _vp]),
+    "rfa_layer_matrices": (_int, [_vp, _vp, _f32, _vp, _int, _int, _int, _vp, _vp, _i64, _int, _vp]),
+    "rfa_layer_matrices_bwd": (_int, [_vp, _vp, _vp, _f32, _vp, _vp, _int, _int, _int, _vp]),
     "rfa_decode_step_fused": (_int, [_vp, _vp, _vp, _int, _vp, _f32, _vp, _vp, _int, _vp, _int, _int, _int, _int, _vp]),
 }
 

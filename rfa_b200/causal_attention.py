@@ -293,6 +293,25 @@ class CausalAttention(nn.Module):
             saved_state["prev_s"], saved_state["prev_z"] = s, z
         return y
 
+    def _train_layer(self, x: Tensor, random_matrices: Tensor, mask: Optional[Tensor]) -> Optional[Tensor]:
+        """The pass with gradients as native autograd nodes, whose biases', matrices' and mask's small launches are one each: 22 launches
+        where module by module takes 35 (24 x 150 tokens in 8 heads, which is host time: 698 us, so 465; 8 x 2048 tokens in 16 heads
+        858, 757).  None, and nothing done, where the call is to go module by module."""
+        sigma = self.sigma if self.reparam_proj else None
+        if not (torch.is_grad_enabled() and x.is_cuda and x.dtype is torch.float16 and random_matrices.dtype is torch.float16):
+            return None
+        if not (x.requires_grad or random_matrices.requires_grad or self.q_proj.weight.requires_grad
+                or (sigma is not None and sigma.requires_grad)):
+            return None                                   # nothing that the attention's own choice of kernels counts as recording
+        linears = (self.q_proj, self.k_proj, self.v_proj, self.out_proj)
+        if mask is not None and mask.dim() == 0:
+            mask = None
+        if not _plain_call((x, random_matrices, sigma, mask), linears):
+            return None
+        if not all(t is None or type(t) is Parameter or type(t) is Tensor for lin in linears for t in (lin.weight, lin.bias)):
+            return None
+        return ops.layer_train(x, *linears, random_matrices, sigma, self.tau, SCALE, mask)
+
     def _fused_layer_pass(self, q: Tensor, k: Tensor, v: Tensor, random_matrices: Tensor, mask: Optional[Tensor]) -> bool:
         """Whether a pass without gradients may hand the layer's own matrices and mask to the fused forward: what the tensor
         expressions around it would make of them, it makes of them (the mul, the conversion and the mask's transpose are three
@@ -315,6 +334,10 @@ class CausalAttention(nn.Module):
         assert embed_dim == self.embed_dim
         if saved_state is not None and tgt_len == 1:
             y = self._decode_layer(x, random_matrices, saved_state)
+            if y is not None:
+                return y
+        if saved_state is None and self.cuda_causal_rfa and not self.fuse_feature_map:
+            y = self._train_layer(x, random_matrices, key_padding_mask)
             if y is not None:
                 return y
         q, k, v = self._heads(self.q_proj(x)), self._heads(self.k_proj(x)), self._heads(self.v_proj(x))

@@ -14,7 +14,7 @@
 // first product.  tcgen05 would stage both through shared memory for M = 128 rows of which a batch of 8 fills 8.
 // The warps' sums meet in shared memory in fp32, so that a chain inside the mma's truncating accumulators is 1/8 (1/4) of
 // the inner index.
-#include "common.cuh"
+#include "matrices.cuh"
 #include "sm100.cuh"
 
 namespace rfa {
@@ -24,36 +24,10 @@ struct LrArgs {
   const __half *w[kLrMax], *b[kLrMax];
   __half* y[kLrMax];
 };
-// the random matrices of the step: w_eff[h][j][l] = round(sigma[h][l] * rm[h][j][l]) (sigma null: rm) * inv_tau, rounded again where
-// inv_tau is not 1 -- the fp16 roundings of the tensor expressions they replace
-struct LrMatrices {
-  const __half *rm, *sigma;
-  float* w_eff;
-  float inv_tau;
-  int n, Dd, d;      // elements in all, per head, per row
-};
 
 __device__ __forceinline__ void lr_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-__device__ __forceinline__ void lr_matrices(const LrMatrices& m, int block, int blocks) {
-  for (int i = (block * kLrThreads + threadIdx.x) * 8; i < m.n; i += blocks * kLrThreads * 8) {      // 8 | d: a piece is of one row
-    float w[8];
-    load8(m.rm + i, w);
-    if (m.sigma) {
-      float s[8];
-      load8(m.sigma + (size_t)(i / m.Dd) * m.d + i % m.d, s);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) w[e] = __half2float(__float2half_rn(w[e] * s[e]));
-    }
-    if (m.inv_tau != 1.f)
-#pragma unroll
-      for (int e = 0; e < 8; ++e) w[e] = __half2float(__float2half_rn(w[e] * m.inv_tau));
-    store4(m.w_eff + i, make_float4(w[0], w[1], w[2], w[3]));
-    store4(m.w_eff + i + 4, make_float4(w[4], w[5], w[6], w[7]));
-  }
 }
 
 // grid (matrix blocks + count * row tiles, token groups).  KS: parts the inner index is split into; the other 8 / KS warps take
@@ -67,7 +41,7 @@ linear_rows_kernel(const __half* __restrict__ x, const __grid_constant__ LrArgs 
   sm100::pdl_wait();
   sm100::pdl_launch_dependents();
   if (blockIdx.x < (unsigned)m_blocks) {
-    if (blockIdx.y == 0) lr_matrices(m, blockIdx.x, m_blocks);
+    if (blockIdx.y == 0) lr_matrices<kLrThreads>(m, blockIdx.x, m_blocks);
     return;
   }
   const int tile = blockIdx.x - m_blocks, which = tile / tiles, row0 = (tile % tiles) * kRows, tok0 = blockIdx.y * kTok;

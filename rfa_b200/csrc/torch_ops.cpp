@@ -521,6 +521,136 @@ struct CrossQueryBackward : torch::autograd::Function<CrossQueryBackward> {
   }
 };
 
+// y_m = x W_m^T + b_m for one to three matrices, and their gradients: nn.Linear's graph with one launch for the biases, and with the input's
+// gradient summed by the products themselves.  y_m takes `shape`, whatever its view of [rows, out]: no view nodes around it.
+struct Shape3 { int64_t n[3]; };                       // (an array of them would be taken for several arguments)
+struct ProjectBackward : torch::autograd::Function<ProjectBackward> {
+  static Tensor rows(const Tensor& t, int64_t width) { return t.reshape({-1, width}); }
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& w0, const OptTensor& w1, const OptTensor& w2, const OptTensor& b0,
+                               const OptTensor& b1, const OptTensor& b2, Shape3 shape) {
+    const OptTensor w[3] = {w0, w1, w2}, b[3] = {b0, b1, b2};
+    const Tensor x2 = x.view({-1, w0.size(1)});
+    bool need_x = false;                               // what autograd keeps for nn.Linear: x for W's gradient, W for x's
+    variable_list y, keep{Tensor()};
+    std::vector<int64_t> bias;
+    for (int m = 0; m < 3 && w[m]; ++m) {
+      y.push_back(at::_unsafe_view(at::linear(x2, *w[m], b[m]), shape.n));
+      keep.push_back(x.requires_grad() ? *w[m] : Tensor());
+      need_x |= w[m]->requires_grad();
+      bias.push_back(b[m].has_value());
+    }
+    if (need_x) keep[0] = x;
+    ctx->save_for_backward(keep);
+    ctx->saved_data["bias"] = bias;
+    ctx->saved_data["in"] = w0.size(1);
+    ctx->saved_data["out"] = w0.size(0);
+    ctx->saved_data["x_shape"] = x.sizes().vec();
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, const variable_list& g) {
+    const variable_list s = ctx->get_saved_variables();
+    const auto bias = ctx->saved_data["bias"].toIntVector();
+    const int64_t in = ctx->saved_data["in"].toInt(), out = ctx->saved_data["out"].toInt();
+    const int n = static_cast<int>(bias.size());
+    const bool recorded = at::GradMode::is_enabled();  // a backward that is itself differentiated: tensor expressions throughout
+    variable_list r(8), g2(n);
+    for (int m = 0; m < n; ++m) g2[m] = rows(g[m], out);
+    if (ctx->needs_input_grad(0)) {
+      Tensor gx = at::mm(g2[0], s[1]);
+      for (int m = 1; m < n; ++m) recorded ? gx = gx + at::mm(g2[m], s[1 + m]) : gx.addmm_(g2[m], s[1 + m]);
+      r[0] = at::_unsafe_view(gx, ctx->saved_data["x_shape"].toIntVector());
+    }
+    for (int m = 0; m < n; ++m)
+      if (ctx->needs_input_grad(1 + m)) r[1 + m] = at::mm(g2[m].t(), rows(s[0], in));
+    int edge = 1 + n, count = 0;                       // absent biases have no edge
+    const void* from[3];
+    void* to[3];
+    for (int m = 0; m < n; ++m) {
+      if (!bias[m] || !ctx->needs_input_grad(edge++)) continue;
+      if (!recorded) g2[m] = g2[m].contiguous();
+      if (recorded || out % 8 || reinterpret_cast<uintptr_t>(g2[m].data_ptr()) % 16) {
+        r[4 + m] = g2[m].sum(0);
+        continue;
+      }
+      r[4 + m] = fresh({out}, g2[m], at::kHalf);
+      from[count] = g2[m].data_ptr();
+      to[count++] = r[4 + m].data_ptr();
+    }
+    if (count) {
+      Call c(g2[0]);
+      check(rfa_column_sums(from, to, count, g2[0].size(0), out, c.stream), "rfa_column_sums");
+    }
+    return r;
+  }
+};
+
+// The layer's random matrices in fp32 from fp16 ones and sigma (build_random_matrices); `mask`, if any, is filled from `pad` on the way.
+struct MatricesBackward : torch::autograd::Function<MatricesBackward> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& rm, const OptTensor& sigma, double tau, const OptTensor& pad, const OptTensor& mask) {
+    const int64_t H = rm.size(0), D = rm.size(1), d = rm.size(2);
+    Tensor w = fresh({H, D, d}, rm, at::kFloat);
+    ctx->save_for_backward({sigma && sigma->requires_grad() ? rm : Tensor(), sigma && rm.requires_grad() ? *sigma : Tensor()});
+    ctx->saved_data["tau"] = tau;
+    ctx->saved_data["sigma"] = sigma.has_value();
+    Call c(rm);
+    check(rfa_layer_matrices(ptr(rm), ptr(sigma), static_cast<float>(1.0 / tau), fptr(w), H, D, d, bptr(pad),
+                             mask ? static_cast<uint8_t*>(mask->data_ptr()) : nullptr, pad ? pad->size(1) : 0, pad ? pad->size(0) : 0, c.stream),
+          "rfa_layer_matrices");
+    return w;
+  }
+  static variable_list backward(AutogradContext* ctx, const variable_list& g) {
+    const variable_list s = ctx->get_saved_variables();
+    const double tau = ctx->saved_data["tau"].toDouble();
+    const bool sigma = ctx->saved_data["sigma"].toBool(), need_rm = ctx->needs_input_grad(0), need_sigma = sigma && ctx->needs_input_grad(1);
+    Tensor g_rm, g_sigma;
+    if (at::GradMode::is_enabled()) {
+      const Tensor gt = g[0] / tau;
+      if (need_rm) g_rm = (sigma ? gt * s[1] : gt).to(at::kHalf);
+      if (need_sigma) g_sigma = (gt * s[0]).sum(1, true).to(at::kHalf);
+    } else {
+      const Tensor gw = g[0].contiguous();
+      const int64_t H = gw.size(0), D = gw.size(1), d = gw.size(2);
+      if (need_rm) g_rm = fresh({H, D, d}, gw, at::kHalf);
+      if (need_sigma) g_sigma = fresh({H, 1, d}, gw, at::kHalf);
+      Call c(gw);
+      check(rfa_layer_matrices_bwd(fptr(gw), need_sigma ? ptr(s[0]) : nullptr, sigma && need_rm ? ptr(s[1]) : nullptr, static_cast<float>(1.0 / tau),
+                                   need_sigma ? ptr(g_sigma) : nullptr, need_rm ? ptr(g_rm) : nullptr, H, D, d, c.stream),
+            "rfa_layer_matrices_bwd");
+    }
+    return {g_rm, g_sigma, Tensor(), Tensor(), Tensor()};
+  }
+};
+
+// A layer's pass with gradients, x [T, B, E] -> y [T, B, E].  Null, with nothing done, where the nodes are not what the separate calls do.
+OptTensor layer_train(const Tensor& x, const Tensor& wq, const OptTensor& bq, const Tensor& wk, const OptTensor& bk, const Tensor& wv,
+                      const OptTensor& bv, const Tensor& wo, const OptTensor& bo, const Tensor& rm, const OptTensor& sigma, double tau,
+                      double scale, const OptTensor& pad) {
+  if (!x.is_cuda() || x.dim() != 3 || rm.dim() != 3 || x.numel() == 0) return std::nullopt;
+  const int64_t T = x.size(0), B = x.size(1), E = x.size(2), H = rm.size(0), D = rm.size(1), d = rm.size(2);
+  const auto plain = [&](const Tensor& t, at::IntArrayRef shape, at::ScalarType type) {
+    return t.scalar_type() == type && t.sizes() == shape && t.device() == x.device() && t.layout() == at::kStrided && t.is_contiguous() &&
+           !t.is_conj() && !t.is_neg() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
+  };
+  if (H < 1 || D < 8 || D % 8 || D > 128 || d < 8 || d % 8 || d > 128 || H * d != E || H > 65535 || !plain(x, {T, B, E}, at::kHalf)) return std::nullopt;
+  for (const Tensor* w : {&wq, &wk, &wv, &wo})
+    if (!plain(*w, {E, E}, at::kHalf)) return std::nullopt;
+  for (const OptTensor* b : {&bq, &bk, &bv, &bo})
+    if (*b && !plain(**b, {E}, at::kHalf)) return std::nullopt;
+  if (!plain(rm, {H, D, d}, at::kHalf) || (sigma && !plain(*sigma, {H, 1, d}, at::kHalf))) return std::nullopt;
+  if (pad && !(pad->scalar_type() == at::kBool && pad->sizes() == at::IntArrayRef({B, T}) && pad->device() == x.device() && pad->is_contiguous()))
+    return std::nullopt;
+  OptTensor mask;
+  if (pad) mask = fresh({T, B}, x, at::kBool);
+  const variable_list p = ProjectBackward::apply(x, wq, OptTensor(wk), OptTensor(wv), bq, bk, bv, Shape3{{T, B * H, d}});
+  const Tensor w = MatricesBackward::apply(rm, sigma, tau, pad, mask);
+  variable_list phi;
+  const Tensor q = p[0].view({T, B, H, d}), k = p[1].view({T, B, H, d});
+  if (D == 64 && d == 64) phi = FeatureMapPairBackward::apply(q, k, w, scale, OptTensor(), mask);
+  else phi = {FeatureMapBackward::apply(q, w, scale, OptTensor()), FeatureMapBackward::apply(k, w, scale, mask)};
+  const Tensor attn = RFABackward::apply(phi[0].view({T, B * H, 2 * D}), phi[1].view({T, B * H, 2 * D}), p[2]);
+  return ProjectBackward::apply(attn, wo, OptTensor(), OptTensor(), bo, OptTensor(), OptTensor(), Shape3{{T, B, E}})[0];
+}
+
 Tensor rfa_node(const Tensor& q, const Tensor& k, const Tensor& v) { return RFABackward::apply(q, k, v); }
 Tensor feature_map_node(const Tensor& x, const Tensor& w, double scale, const OptTensor& mask) { return FeatureMapBackward::apply(x, w, scale, mask); }
 std::tuple<Tensor, Tensor> feature_map_pair_node(const Tensor& a, const Tensor& b, const Tensor& w, double scale, const OptTensor& mask_a,
@@ -556,6 +686,7 @@ PYBIND11_MODULE(_native, m) {
   def("decode_step", &decode_step);
   def("decode_step_fused", &decode_step_fused);
   def("layer_decode", &layer_decode);
+  def("layer_train", &layer_train);
   def("rfa_node", &rfa_node);
   def("feature_map_node", &feature_map_node);
   def("feature_map_pair_node", &feature_map_pair_node);

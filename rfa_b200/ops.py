@@ -322,6 +322,14 @@ def layer_decode(x: Tensor, q_proj, k_proj, v_proj, out_proj, random_matrices: T
                                  out_proj.weight, out_proj.bias, random_matrices, sigma, tau, scale, s, z)
 
 
+def layer_train(x: Tensor, q_proj, k_proj, v_proj, out_proj, random_matrices: Tensor, sigma: Optional[Tensor], tau: float,
+                scale: float, pad_mask: Optional[Tensor]) -> Optional[Tensor]:
+    """A layer's pass with gradients, x [T, B, E], as five native autograd nodes (the projections, the random matrices, the features, the
+    attention, the output projection); pad_mask [B, T] bool.  None, with nothing done, where the tensors are not ones they take."""
+    return native().layer_train(x, q_proj.weight, q_proj.bias, k_proj.weight, k_proj.bias, v_proj.weight, v_proj.bias,
+                                out_proj.weight, out_proj.bias, random_matrices, sigma, tau, scale, pad_mask)
+
+
 class CrossDecodeStates:
     """The cross-attention states of all layers of a decoder, gathered once per sequence for ``cross_decode_step``:
     device arrays of pointers to each layer's ``s [B,H,K,d]`` and ``z [B,H,K]`` (fp32, contiguous).  The states are
