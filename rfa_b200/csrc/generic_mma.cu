@@ -29,6 +29,7 @@
 // non-finite value takes the masked products element by element, over the unmasked tokens only, so that what a
 // token makes of its predecessors never depends on its successors.
 #include "generic_mma.cuh"
+#include "sm100.cuh"
 
 namespace rfa {
 
@@ -291,9 +292,11 @@ gm_causal_fwd_kernel(const __half* __restrict__ q, const __half* __restrict__ k,
   };
   for (int s = 0; s < STAGES; ++s)
     for (int i = 0; i < 3; ++i) gm_pad(tile(s, i), C, i < 2 ? K : d);
+  sm100::pdl_wait();            // everything above overlaps the tail of the previous kernel in the stream
   load(0);
   gm_state_in(S, z, L, s_seg ? s_seg + slot * K * d : nullptr, z_seg ? z_seg + slot * K : nullptr, K, d);
   for (int c = 0; c < nchunk; ++c) {
+    if (c == nchunk - 1) sm100::pdl_launch_dependents();
     if (STAGES == 2) { load(c + 1); gm_wait<1>(); } else gm_wait<0>();
     const GmTile tq = tile(c, 0), tk = tile(c, 1), tv = tile(c, 2);
     const int64_t t0 = t_begin + (int64_t)c * C;
@@ -398,9 +401,11 @@ gm_causal_bwd_q_kernel(const __half* __restrict__ q, const __half* __restrict__ 
   };
   for (int s = 0; s < STAGES; ++s)
     for (int i = 0; i < 4; ++i) gm_pad(tile(s, i), C, i < 2 ? K : d);
+  sm100::pdl_wait();            // everything above overlaps the tail of the previous kernel in the stream
   load(0);
   gm_state_in(S, z, L, s_seg ? s_seg + slot * K * d : nullptr, z_seg ? z_seg + slot * K : nullptr, K, d);
   for (int c = 0; c < nchunk; ++c) {
+    if (c == nchunk - 1) sm100::pdl_launch_dependents();
     if (STAGES == 2) { load(c + 1); gm_wait<1>(); } else gm_wait<0>();
     const GmTile tq = tile(c, 0), tk = tile(c, 1), tv = tile(c, 2), tg = tile(c, 3);
     const int64_t t0 = t_begin + (int64_t)c * C;
@@ -543,9 +548,11 @@ gm_causal_bwd_kv_kernel(const __half* __restrict__ q, const __half* __restrict__
   };
   for (int s = 0; s < STAGES; ++s)
     for (int i = 0; i < 4; ++i) gm_pad(tile(s, i), C, i < 2 ? K : d);
+  sm100::pdl_wait();            // everything above overlaps the tail of the previous kernel in the stream
   load(nchunk - 1);
   gm_state_in(S, z, L, ds_seg ? ds_seg + slot * K * d : nullptr, dz_seg ? dz_seg + slot * K : nullptr, K, d);
   for (int c = nchunk - 1; c >= 0; --c) {
+    if (c == 0) sm100::pdl_launch_dependents();
     const int64_t t0 = t_begin + (int64_t)c * C;
     const int valid = (int)min((int64_t)C, t_end - t0);
     gm_row_scalars(inv, gz, ws_den, ws_gz, C, (size_t)bh * T + t0, valid);
@@ -658,9 +665,11 @@ gm_state_kernel(const __half* __restrict__ x, const __half* __restrict__ y, cons
     }
     gm_commit();
   };
+  sm100::pdl_wait();            // everything above overlaps the tail of the previous kernel in the stream
   load(0);
   gm_state_in(S, z, L, nullptr, nullptr, K, d);
   for (int c = 0; c < nchunk; ++c) {
+    if (c == nchunk - 1) sm100::pdl_launch_dependents();
     const int64_t t0 = t_begin + (int64_t)c * C;
     if (WEIGHTED) gm_row_scalars(inv, gz, ws_den, ws_gz, C, (size_t)bh * T + t0, (int)min((int64_t)C, t_end - t0));
     if (STAGES == 2) { load(c + 1); gm_wait<1>(); } else gm_wait<0>();
@@ -724,7 +733,7 @@ template <class KERNEL, class... Args>
 static int gm_launch(KERNEL kernel, const char* what, int threads, uint32_t smem, dim3 grid, cudaStream_t st, Args... args) {
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return fail((int)e, "%s: cannot reserve %u bytes of shared memory: %s", what, smem, cudaGetErrorString(e));
-  kernel<<<grid, threads, smem, st>>>(args...);
+  sm100::launch_pdl(kernel, grid, dim3(threads), smem, st, args...);      // (K, d) = (256, 128), 32 x 512: 422.6 -> 415.4 us a step, 128 x 512 1115 -> 1107
   return check_launch(what);
 }
 #define RFA_GM_DISPATCH(shape, CALL)                                  \

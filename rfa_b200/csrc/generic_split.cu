@@ -9,10 +9,16 @@
 // tensor pipe 12 %, a third of the stalls at the chunk's barriers): forward + backward kernels 185 -> 141 us at (K, d) = (64, 32), 64 heads x
 // 1024 tokens, 138 -> 92 at (96, 40), 64 x 300, 392 -> 323 at (128, 128), 64 x 512, 123 -> 57 at (128, 128), 8 x 200.
 #include "generic_split.cuh"
+#include "sm100.cuh"
 
 namespace rfa {
 
 constexpr int kGsRegs = 80;      // 24 warps on an SM: three CTAs of 256 threads, two of 384 or one of 768
+// Whether launches may be placed while the previous kernel drains: segments of at most four chunks.  A step is five to seven launches then, and
+// their gaps a good part of it; longer kernels lose more to the CTAs' uneven placement than the gaps cost.  us a step without / with: (64, 32), 64
+// heads x 1024 tokens (4 chunks) 145.4 / 136.2, 128 x 512 (4) 143.6 / 136.5; (96, 40), 64 x 300 (3) 96.8 / 90.2, 128 x 512 (8) 219 / 231; (128, 128),
+// 64 x 512 (8) 322.8 / 320.5, 128 x 512 (16) 491 / 501.
+__host__ __device__ inline bool gs_pdl(int64_t tseg, int C) { return tseg <= 4 * C; }
 
 struct GsLayout {
   int Kp, dp, px, py, ps, ph, pc;      // K and d rounded up to 16; pitches of X tiles (q, k), Y tiles (v, g), the fp32 state, [.][d] and [C][C] split matrices
@@ -327,9 +333,11 @@ gs_causal_fwd_kernel(const __half* __restrict__ q, const __half* __restrict__ k,
     gm_commit();
   };
   for (int i = 0; i < 3; ++i) gm_pad(tile(i), C, i < 2 ? K : d);
+  sm100::pdl_wait();            // everything above overlaps the tail of the previous kernel in the stream
   load(0);
   gs_state_in<true>(S, z, L, op, s_seg ? s_seg + slot * K * d : nullptr, z_seg ? z_seg + slot * K : nullptr, K, d);
   for (int c = 0; c < nchunk; ++c) {
+    if (c == nchunk - 1 && gs_pdl(tseg, C)) sm100::pdl_launch_dependents();
     gm_wait<0>();
     const GmTile tq = tile(0), tk = tile(1), tv = tile(2);
     const int64_t t0 = t_begin + (int64_t)c * C;
@@ -433,9 +441,11 @@ gs_causal_bwd_q_kernel(const __half* __restrict__ q, const __half* __restrict__ 
     gm_commit();
   };
   for (int i = 0; i < 4; ++i) gm_pad(tile(i), C, i < 2 ? K : d);
+  sm100::pdl_wait();            // everything above overlaps the tail of the previous kernel in the stream
   load(0);
   gs_state_in<true>(S, z, L, op, s_seg ? s_seg + slot * K * d : nullptr, z_seg ? z_seg + slot * K : nullptr, K, d);
   for (int c = 0; c < nchunk; ++c) {
+    if (c == nchunk - 1 && gs_pdl(tseg, C)) sm100::pdl_launch_dependents();
     gm_wait<0>();
     const GmTile tq = tile(0), tk = tile(1), tv = tile(2), tg = tile(3);
     const int64_t t0 = t_begin + (int64_t)c * C;
@@ -601,9 +611,11 @@ gs_causal_bwd_kv_kernel(const __half* __restrict__ q, const __half* __restrict__
     gm_commit();
   };
   for (int i = 0; i < 4; ++i) gm_pad(tile(i), C, i < 2 ? K : d);
+  sm100::pdl_wait();            // everything above overlaps the tail of the previous kernel in the stream
   load(nchunk - 1);
   gs_state_in<true>(S, z, L, op, ds_seg ? ds_seg + slot * K * d : nullptr, dz_seg ? dz_seg + slot * K : nullptr, K, d);
   for (int c = nchunk - 1; c >= 0; --c) {
+    if (c == 0 && gs_pdl(tseg, C)) sm100::pdl_launch_dependents();
     const int64_t t0 = t_begin + (int64_t)c * C;
     const int valid = (int)min((int64_t)C, t_end - t0);
     gs_row_scalars(rows, ws_den, ws_gz, C, (size_t)bh * T + t0, valid);
@@ -715,9 +727,11 @@ gs_state_kernel(const __half* __restrict__ x, const __half* __restrict__ y, cons
     gm_commit();
   };
   for (int i = 0; i < 2; ++i) gm_pad(tile(i), C, i < 1 ? K : d);
+  sm100::pdl_wait();            // everything above overlaps the tail of the previous kernel in the stream
   load(0);
   gs_state_in<false>(S, z, L, Gs, nullptr, nullptr, K, d);
   for (int c = 0; c < nchunk; ++c) {
+    if (c == nchunk - 1 && gs_pdl(tseg, C)) sm100::pdl_launch_dependents();
     const int64_t t0 = t_begin + (int64_t)c * C;
     if (WEIGHTED) gs_row_scalars(rows, ws_den, ws_gz, C, (size_t)bh * T + t0, (int)min((int64_t)C, t_end - t0));
     gm_wait<0>();
@@ -764,10 +778,11 @@ int split_chunk(int K, int d, int* ctas) {
 }
 
 template <class KERNEL, class... Args>
-static int gs_launch(KERNEL kernel, const char* what, int threads, uint32_t smem, dim3 grid, cudaStream_t st, Args... args) {
+static int gs_launch(KERNEL kernel, const char* what, bool pdl, int threads, uint32_t smem, dim3 grid, cudaStream_t st, Args... args) {
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return fail((int)e, "%s: cannot reserve %u bytes of shared memory: %s", what, smem, cudaGetErrorString(e));
-  kernel<<<grid, threads, smem, st>>>(args...);
+  if (pdl) sm100::launch_pdl(kernel, grid, dim3(threads), smem, st, args...);
+  else kernel<<<grid, threads, smem, st>>>(args...);
   return check_launch(what);
 }
 #define RFA_GS_DISPATCH(shape, CALL)            \
@@ -780,14 +795,14 @@ static int gs_launch(KERNEL kernel, const char* what, int threads, uint32_t smem
 
 int launch_causal_split_fwd(const __half* q, const __half* k, const __half* v, __half* out, const float* s_seg, const float* z_seg, float* s_out,
                             float* z_out, float* den_out, int64_t T, int BH, int nseg, int64_t tseg, int K, int d, cudaStream_t st) {
-#define RFA_GS_CALL(C) return gs_launch(gs_causal_fwd_kernel<C>, "rfa_causal_fwd (chunked)", gs_.threads, gs_layout_fwd(C, K, d).total, \
+#define RFA_GS_CALL(C) return gs_launch(gs_causal_fwd_kernel<C>, "rfa_causal_fwd (chunked)", gs_pdl(tseg, C), gs_.threads, gs_layout_fwd(C, K, d).total, \
                                         dim3(BH, nseg), st, q, k, v, out, s_seg, z_seg, s_out, z_out, den_out, T, BH, tseg, K, d)
   RFA_GS_DISPATCH(gs_shape(K, d), RFA_GS_CALL);
 #undef RFA_GS_CALL
 }
 int launch_causal_split_bwd_q(const __half* q, const __half* k, const __half* v, const __half* g, __half* gq, const float* s_seg, const float* z_seg,
                               float* ws_den, float* ws_gz, int64_t T, int BH, int nseg, int64_t tseg, int K, int d, cudaStream_t st) {
-#define RFA_GS_CALL(C) return gs_launch(gs_causal_bwd_q_kernel<C>, "rfa_causal_bwd_q (chunked)", gs_.threads, gs_layout_q(C, K, d).total, \
+#define RFA_GS_CALL(C) return gs_launch(gs_causal_bwd_q_kernel<C>, "rfa_causal_bwd_q (chunked)", gs_pdl(tseg, C), gs_.threads, gs_layout_q(C, K, d).total, \
                                         dim3(BH, nseg), st, q, k, v, g, gq, s_seg, z_seg, ws_den, ws_gz, T, BH, tseg, K, d)
   RFA_GS_DISPATCH(gs_shape(K, d), RFA_GS_CALL);
 #undef RFA_GS_CALL
@@ -795,7 +810,7 @@ int launch_causal_split_bwd_q(const __half* q, const __half* k, const __half* v,
 int launch_causal_split_bwd_kv(const __half* q, const __half* k, const __half* v, const __half* g, __half* gk, __half* gv, const float* ws_den,
                                const float* ws_gz, const float* ds_seg, const float* dz_seg, int64_t T, int BH, int nseg, int64_t tseg, int K,
                                int d, cudaStream_t st) {
-#define RFA_GS_CALL(C) return gs_launch(gs_causal_bwd_kv_kernel<C>, "rfa_causal_bwd_kv (chunked)", gs_.threads, gs_layout_kv(C, K, d).total, \
+#define RFA_GS_CALL(C) return gs_launch(gs_causal_bwd_kv_kernel<C>, "rfa_causal_bwd_kv (chunked)", gs_pdl(tseg, C), gs_.threads, gs_layout_kv(C, K, d).total, \
                                         dim3(BH, nseg), st, q, k, v, g, gk, gv, ws_den, ws_gz, ds_seg, dz_seg, T, BH, tseg, K, d)
   RFA_GS_DISPATCH(gs_shape(K, d), RFA_GS_CALL);
 #undef RFA_GS_CALL
@@ -803,9 +818,9 @@ int launch_causal_split_bwd_kv(const __half* q, const __half* k, const __half* v
 int launch_state_split(const __half* x, const __half* y, const uint8_t* pad_mask, const float* ws_den, const float* ws_gz, float* s, float* z,
                        int64_t T, int BH, int H, int nseg, int64_t tseg, int runs, int K, int d, cudaStream_t st) {
 #define RFA_GS_CALL(C)                                                                                                                \
-  return ws_den ? gs_launch(gs_state_kernel<C, true>, "state reduction (chunked)", gs_.threads, gs_layout_state(C, K, d, true).total, \
+  return ws_den ? gs_launch(gs_state_kernel<C, true>, "state reduction (chunked)", gs_pdl(tseg, C), gs_.threads, gs_layout_state(C, K, d, true).total, \
                             dim3(BH, runs), st, x, y, pad_mask, ws_den, ws_gz, s, z, T, BH, H, nseg, tseg, K, d)                      \
-                : gs_launch(gs_state_kernel<C, false>, "state reduction (chunked)", gs_.threads, gs_layout_state(C, K, d, false).total, \
+                : gs_launch(gs_state_kernel<C, false>, "state reduction (chunked)", gs_pdl(tseg, C), gs_.threads, gs_layout_state(C, K, d, false).total, \
                             dim3(BH, runs), st, x, y, pad_mask, ws_den, ws_gz, s, z, T, BH, H, nseg, tseg, K, d)
   RFA_GS_DISPATCH(gs_shape(K, d), RFA_GS_CALL);
 #undef RFA_GS_CALL
