@@ -61,6 +61,12 @@ void require_half(const T&... ts) {
   for (const Tensor* t : {&ts...})
     if (t->scalar_type() != at::kHalf) raise(PyExc_TypeError, "rfa_b200: this kernel is fp16-only, got " + dtype_name(*t));
 }
+// A kernel launched on x's device must not be handed another device's addresses.
+void require_device(const Tensor& x, std::initializer_list<const Tensor*> others) {
+  for (const Tensor* t : others)
+    if (t->device() != x.device())
+      raise(PyExc_RuntimeError, "rfa_b200: expected all tensors on " + x.device().str() + ", got one on " + t->device().str());
+}
 void require(bool ok, const std::string& msg = "") {
   if (!ok) raise(PyExc_AssertionError, msg);
 }
@@ -289,6 +295,7 @@ Tensor causal_fwd_fused_layer(Tensor xq, Tensor xk, Tensor v, Tensor rm, OptTens
   require_half(xq, xk, v, rm);
   rank(xq, 4);
   rank(rm, 3);
+  require_device(xq, {&xk, &v, &rm, sigma ? &*sigma : &xq});
   xq = xq.contiguous(); xk = xk.contiguous(); v = v.contiguous(); rm = rm.contiguous();
   const int64_t T = xq.size(0), B = xq.size(1), H = xq.size(2), d = xq.size(3), D = rm.size(1);
   require(xk.sizes() == xq.sizes() && v.sizes() == xq.sizes() && rm.size(0) == H && rm.size(2) == d);

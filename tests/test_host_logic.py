@@ -249,3 +249,27 @@ def test_what_a_native_short_cut_leaves_to_the_tensor_expressions():
     q = torch.zeros(4, 1, 128, dtype=torch.half)
     with pytest.raises(RuntimeError, match="no CPU path"):
         torch.compile(lambda q, v: RFA.apply(q, q, v) * 2, backend="eager")(q, q[..., :64])
+
+
+@pytest.fixture
+def layer_pass(monkeypatch):
+    """A layer, its q, k, v and matrices, in place of whose CUDA tensors CPU ones stand; which of them a pass hands to the kernel."""
+    from rfa_b200 import CausalAttention, causal_attention, ops
+    monkeypatch.setattr(ops, "fused_forward_supported", lambda *_: True)
+    monkeypatch.setattr(causal_attention, "plain_tensors", lambda *_: True)
+    layer = CausalAttention(embed_dim=128, num_heads=2, head_dim=64, proj_dim=64).half().requires_grad_(False)
+    qkv = list(torch.zeros(3, 5, 1, 2, 64, dtype=torch.half))
+    return layer, qkv, torch.zeros(2, 64, 64, dtype=torch.half)
+
+
+def test_a_layer_pass_keeps_matrices_of_another_device_from_the_kernel(layer_pass):
+    """`meta` stands for another GPU: the tensor expressions refuse it, and so does the native call itself, before anything is launched."""
+    from rfa_b200._lib import native
+    layer, (q, k, v), w = layer_pass
+    assert layer._fused_layer_pass(q, k, v, w, None)
+    assert not layer._fused_layer_pass(q, k, v, w.to("meta"), None)
+    layer.sigma = torch.nn.Parameter(layer.sigma.to("meta"), requires_grad=False)
+    assert not layer._fused_layer_pass(q, k, v, w, None)
+    for sigma, rm in ((None, w.to("meta")), (layer.sigma, w)):
+        with pytest.raises(RuntimeError, match="expected all tensors on cpu, got one on meta"):
+            native().causal_fwd_fused_layer(q, k, v, rm, sigma, 1.0, 0.1, None)
