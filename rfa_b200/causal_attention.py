@@ -318,8 +318,8 @@ class CausalAttention(nn.Module):
         launches and 10 us of the 188 that a pass over 8 x 2048 tokens of 16 heads takes)."""
         sigma = self.sigma if self.reparam_proj else None
         half = torch.float16
-        if any(t is not None and t.device != q.device for t in (random_matrices, sigma)):
-            return False                                  # the tensor expressions refuse operands of two devices
+        if any(t is not None and (t.device != q.device or t.data_ptr() % 16) for t in (random_matrices, sigma)):
+            return False           # the tensor expressions refuse operands of two devices and make aligned ones of a view at any offset
         return (ops.fused_forward_supported(q, random_matrices) and q.dtype is k.dtype is v.dtype is half
                 and tuple(random_matrices.shape) == (self.num_heads, 64, 64) and random_matrices.dtype is half
                 and (sigma is None or (sigma.dtype is half and tuple(sigma.shape) == (self.num_heads, 1, 64)))

@@ -191,3 +191,19 @@ def test_layer_pass_from_its_own_matrices_and_mask(dev, T, B, tau, reparam, mask
         if mask == "ragged":
             with pytest.raises(AssertionError):
                 layer(x, w, key_padding_mask=torch.zeros(B + 1, T, dtype=torch.bool, device=dev))
+
+
+@pytest.mark.parametrize("which", ["matrices", "sigma", "both"])
+def test_layer_pass_from_views_at_odd_offsets(dev, which):
+    """Slices of a flat buffer whose address is a multiple of 2 bytes only: what aligned copies of them give."""
+    from rfa_b200 import CausalAttention
+    torch.manual_seed(0)
+    layer = CausalAttention(embed_dim=128, num_heads=2, head_dim=64, proj_dim=64).to(dev).half().requires_grad_(False)
+    torch.nn.init.uniform_(layer.sigma, 0.5, 1.5)
+    w, x = torch.randn(2, 64, 64, device=dev).half(), torch.randn(40, 3, 128, device=dev).half()
+    odd = lambda t: torch.cat([t.new_zeros(3), t.flatten()])[3:].view(t.shape)
+    want = layer(x, w)
+    if which != "matrices":
+        layer.sigma = torch.nn.Parameter(odd(layer.sigma.data), requires_grad=False)
+        assert layer.sigma.data_ptr() % 16
+    assert torch.equal(layer(x, odd(w) if which != "sigma" else w), want)

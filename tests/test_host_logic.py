@@ -273,3 +273,11 @@ def test_a_layer_pass_keeps_matrices_of_another_device_from_the_kernel(layer_pas
     for sigma, rm in ((None, w.to("meta")), (layer.sigma, w)):
         with pytest.raises(RuntimeError, match="expected all tensors on cpu, got one on meta"):
             native().causal_fwd_fused_layer(q, k, v, rm, sigma, 1.0, 0.1, None)
+
+
+def test_a_layer_pass_keeps_matrices_at_odd_addresses_from_the_kernel(layer_pass):
+    layer, (q, k, v), w = layer_pass
+    odd = lambda t: torch.cat([t.new_zeros(3), t.flatten()])[3:].view(t.shape)
+    assert not layer._fused_layer_pass(q, k, v, odd(w), None)
+    layer.sigma = torch.nn.Parameter(odd(layer.sigma.data), requires_grad=False)
+    assert not layer._fused_layer_pass(q, k, v, w, None)
