@@ -273,10 +273,15 @@ class CausalAttention(nn.Module):
         saved_state["prev_s"], saved_state["prev_z"] = s, z
         return attn
 
+    def _own_heads(self, random_matrices: Tensor) -> bool:
+        """Whether the matrices are for this layer's heads.  A native pass takes the split of the features into heads from them, and others may
+        divide embed_dim too, which the module-by-module call refuses."""
+        return random_matrices.dim() == 3 and random_matrices.size(0) == self.num_heads and random_matrices.size(2) == self.head_dim
+
     def _decode_layer(self, x: Tensor, random_matrices: Tensor, saved_state: Dict[str, Optional[Tensor]]) -> Optional[Tensor]:
         """One token through the whole layer in three launches (host time is what a small decoding call consists of); None, and
         nothing done, where the call is to go module by module."""
-        if not (x.is_cuda and x.dtype is torch.float16 and random_matrices.dim() == 3 and random_matrices.is_cuda):
+        if not (x.is_cuda and x.dtype is torch.float16 and random_matrices.is_cuda and self._own_heads(random_matrices)):
             return None
         linears = (self.q_proj, self.k_proj, self.v_proj, self.out_proj)
         sigma = self.sigma if self.reparam_proj else None
@@ -298,7 +303,8 @@ class CausalAttention(nn.Module):
         where module by module takes 35 (24 x 150 tokens in 8 heads, which is host time: 698 us, so 465; 8 x 2048 tokens in 16 heads
         858, 757).  None, and nothing done, where the call is to go module by module."""
         sigma = self.sigma if self.reparam_proj else None
-        if not (torch.is_grad_enabled() and x.is_cuda and x.dtype is torch.float16 and random_matrices.dtype is torch.float16):
+        if not (torch.is_grad_enabled() and x.is_cuda and x.dtype is torch.float16 and random_matrices.dtype is torch.float16
+                and self._own_heads(random_matrices)):
             return None
         if not (x.requires_grad or random_matrices.requires_grad or self.q_proj.weight.requires_grad
                 or (sigma is not None and sigma.requires_grad)):

@@ -157,3 +157,23 @@ def test_what_goes_module_by_module(dev):
     with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(t.shape) or t, lambda t: t):
         layer(x, rm).sum().backward()
     assert packed
+
+
+@pytest.mark.parametrize("heads,head_dim,proj_dim", [(16, 32, 64), (4, 128, 32), (8, 64, 64)])
+def test_matrices_of_another_split_into_heads_are_refused(dev, heads, head_dim, proj_dim):
+    """A layer of 8 heads of 64 without sigma: matrices of 16 heads of 32 divide its features too, and are refused as they are module by module."""
+    layer = CausalAttention(embed_dim=512, num_heads=8, head_dim=64, proj_dim=64, reparam_proj=False).to(dev).half()
+    rm = torch.randn(heads, proj_dim, head_dim, device=dev).half()
+    train = lambda: layer(torch.randn(20, 2, 512, device=dev).half().requires_grad_(), rm)
+    state = {}
+
+    def decode():
+        with torch.no_grad():
+            return layer(torch.randn(1, 2, 512, device=dev).half(), rm, saved_state=state)
+    for call in (train, decode):
+        if heads == 8:
+            call()
+            continue
+        with pytest.raises((AssertionError, ValueError, RuntimeError)):
+            call()
+        assert not state
