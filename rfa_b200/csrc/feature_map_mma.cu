@@ -1,13 +1,13 @@
 // Feature map and its gradient for widths up to 64 that are not the fp16 64 x 64 of feature_map_tc.cu: fp32 rows, and fp16 rows of
 // other widths (formulas in feature_map.cu).
 //
-// fp32 throughout, on the tensor cores: both operands of a product are split into two fp16 tiles under a power of two per block
+// fp32 throughout, on the tensor cores: both operands of a product are split into two fp16 tiles under a power of two per block or row
 // (generic_split.cuh; normalised rows are below 1 and share one), 22 bits each, and three mma.sync m16n8k16 make the product, lo hi,
 // hi lo, hi hi; what is left out is 2^-22 of a term.  16 terms at a time from zero, those sums scaled and added in fp32.
 // Register tiles on the FMA pipe (feature_map.cu) read 16 bytes of shared memory for every 8 FMAs, which bounded them, and the sines
 // of CUDA's library are 75 instructions a pair (trig.cuh); splits into tf32 at every read (6 mma per 16 terms instead of 3, and 5
 // instructions an element and read) were no faster than those.  What bounds it now is instructions issued (issue slots 60 %).
-// fp32, 64 x 64, 4096 rows of 16 heads: forward 30.1 -> 18.2 us, backward 67.6 -> 40.5; 32 x 32, 4096 rows of 8 heads 11.8 -> 6.9 and 23.7 -> 14.5.
+// fp32, 64 x 64, 4096 rows of 16 heads: forward 30.1 -> 18.2 us, backward 67.6 -> 42.4 (40.2 with one factor a block); 32 x 32, 4096 rows of 8 heads 11.8 -> 6.8 and 23.7 -> 14.0.
 // Errors against fp64 (phi, g_x, g_W): 1.62, 2.27, 2.42e-7 -> 1.27, 1.72, 1.95e-7, from shorter chains of fp32 sums.
 //
 // A warp owns 16 rows: it loads, normalises and splits them, and their products, sines and results stay within the warp
@@ -23,14 +23,15 @@ constexpr int kThreads = 256, kWarps = kThreads / 32, kMax = 64, kRows = 16 * kW
 constexpr int kP = kMax + 8;                        // pitch in halves: 8 rows start in 8 different 16-byte banks
 constexpr float kXs = 16384.f, kXi = 1.f / kXs;     // the factor of normalised rows
 constexpr uint32_t kW = 0, kX = kW + 2 * kMax * kP * 2, kWf = kX + 2 * kRows * kP * 2, kNrm = kWf + 16 * 4, kFwdBytes = kNrm + kRows * 4,
-                   kG = kFwdBytes, kGf = kG + 2 * kRows * kP * 2, kBwdBytes = kGf + kWarps * 4 * 4;
+                   kG = kFwdBytes, kGf = kG + 2 * kRows * kP * 2, kBwdBytes = kGf + kRows * 4 * 4;
 constexpr int kCtas = 2;                            // on an SM (three of the forward, at 80 registers a thread: 22.6 us instead of 18.2)
 static_assert(kCtas * (kBwdBytes + 1024) <= 228 * 1024 && kG % 16 == 0, "feature_map_mma: shared memory");
 
+__device__ __forceinline__ float2 both(float f) { return make_float2(f, f); }
 // ---- products ------------------------------------------------------------------------------------------------------------------
 // acc (16 x 32, nt blocks of 8 columns) = A B of two split operands, L terms: pa, pb the lane's shared-memory addresses of the first
 // fragments, da, db their steps per 16 terms and dn B's per 16 columns, (TA, TB) whether the fragments are transposed; f(l, n): the factor
-// of the sums over terms 16 l .. for columns 16 n ..
+// of the sums over terms 16 l .. for columns 16 n .., in rows g and g + 8
 template <bool TA, bool TB, class F>
 __device__ __forceinline__ void product(float (&acc)[4][4], int nt, int L, uint32_t pa, uint32_t a_lo, uint32_t da, uint32_t pb, uint32_t b_lo,
                                         uint32_t db, uint32_t dn, F f) {
@@ -53,9 +54,11 @@ __device__ __forceinline__ void product(float (&acc)[4][4], int nt, int L, uint3
         gm_mma16(p[1], ah, bl[2], bl[3]);
         gm_mma16(p[0], ah, bh[0], bh[1]);
         gm_mma16(p[1], ah, bh[2], bh[3]);
-        const float sc = f(l, n);
-        gs_add(acc[2 * n], p[0], sc);
-        gs_add(acc[2 * n + 1], p[1], sc);
+        const float2 sc = f(l, n);
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[2 * n + m][e] = fmaf(p[m][e], e < 2 ? sc.x : sc.y, acc[2 * n + m][e]);
       }
   }
 }
@@ -121,14 +124,15 @@ __device__ __forceinline__ Share share_of(int64_t rows) {
   return Share{units * blockIdx.x / gridDim.x, units * (blockIdx.x + 1) / gridDim.x};
 }
 struct Tiles {
-  GsSplit W, G;             // W [j][l] and g_u [row][j]
+  GsSplit W;                // [j][l]
   __half *xh, *xl;          // normalised rows
+  GsByRow G;                // g_u [row][j]
   float* nrm;
 };
 __device__ __forceinline__ Tiles tiles_at(unsigned char* base) {
   Tiles s;
   s.W = GsSplit{(__half*)(base + kW), (__half*)(base + kW) + kMax * kP, (float*)(base + kWf), kP, 4};
-  s.G = GsSplit{(__half*)(base + kG), (__half*)(base + kG) + kRows * kP, (float*)(base + kGf), kP, 4};
+  s.G = GsByRow{(__half*)(base + kG), (__half*)(base + kG) + kRows * kP, (float*)(base + kGf), kP, 4, 1};
   s.xh = (__half*)(base + kX); s.xl = s.xh + kRows * kP;
   s.nrm = (float*)(base + kNrm);
   return s;
@@ -137,7 +141,50 @@ __device__ __forceinline__ Tiles tiles_at(unsigned char* base) {
 __device__ __forceinline__ void project(float (&u)[4][4], int nt, const Tiles& s, int row, int c, int d, int lane) {
   const float* f = s.W.inv_s + 2 * c * 4;
   product<false, false>(u, nt, (d + 15) / 16, gm_addr(s.xh + row * kP + gm_off_a(lane, kP)), 2 * kRows * kP, 32,
-                        gm_addr(s.W.hi + 32 * c * kP + gm_off_b(lane, kP)), 2 * kMax * kP, 32, 32 * kP, [&](int l, int n) { return f[n * 4 + l] * kXi; });
+                        gm_addr(s.W.hi + 32 * c * kP + gm_off_b(lane, kP)), 2 * kMax * kP, 32, 32 * kP, [&](int l, int n) { return both(f[n * 4 + l] * kXi); });
+}
+
+// g_u.  g_x = g_u W is a product for each row by itself, so that a row must not lose bits to a larger one beside it: where a row of a block is
+// below 2^-kEven of another, each has a factor of its own there (2^-27 of the row's largest element is the most that a shared one costs it).  g_W sums
+// over rows, where one factor a block is what can be taken out of the sum: such blocks are split again for it (even_rows).
+constexpr uint32_t kEven = 12;
+static __device__ __noinline__ bool put_g_faded(GsByRow m, int r0, int j0, float4 x, float4 y, uint32_t line) {
+  const float a[2][4] = {{x.x, x.y, x.z, x.w}, {y.x, y.y, y.z, y.w}};
+  uint32_t mag[2];
+  gs_row_mags<true>(mag, a);
+  const bool own = __any_sync(0xffffffffu, mag[0] - 1 < line || mag[1] - 1 < line);      // 0 is not: it has no bits to lose
+  if (!own) mag[0] = mag[1] = __reduce_max_sync(0xffffffffu, max(mag[0], mag[1]));
+  gs_put_rows_as<true>(m, r0, j0, a, mag);
+  return own;
+}
+// -> whether the block's rows have factors of their own
+__device__ __forceinline__ bool put_g(const GsByRow& m, int r0, int j0, const float (&a)[2][4]) {
+  uint32_t mag[2] = {0, 0};                            // this lane's part of a row: one that has not faded in any lane has not faded
+#pragma unroll
+  for (int e = 0; e < 8; ++e) mag[e >> 1 & 1] = max(mag[e >> 1 & 1], gs_mag(a[e >> 2][e & 3]));
+  const uint32_t most = __reduce_max_sync(0xffffffffu, max(mag[0], mag[1])), exponent = most & kGsInf;
+  const uint32_t line = most >= kGsInf ? ~0u : exponent > (kEven << 23) ? exponent - (kEven << 23) : 0u;
+  if (__any_sync(0xffffffffu, mag[0] - 1 < line || mag[1] - 1 < line))
+    return put_g_faded(m, r0, j0, make_float4(a[0][0], a[0][1], a[0][2], a[0][3]), make_float4(a[1][0], a[1][1], a[1][2], a[1][3]), line);
+  const uint32_t all[2] = {most, most};
+  gs_put_rows_as<false>(m, r0, j0, a, all);
+  return false;
+}
+// the warp's blocks (bits of `own`) of finite numbers with one factor each again
+static __device__ __noinline__ void even_rows(GsByRow m, int r0, uint32_t own) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  for (int b = 0; b < 4; ++b) {
+    if (!(own >> b & 1)) continue;
+    float a[2][4];
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) a[n][e] = gs_at(m, r0 + g + 8 * (e >> 1), 16 * b + 8 * n + 2 * t + (e & 1));
+    uint32_t mag[2];
+    gs_row_mags<false>(mag, a);
+    mag[0] = mag[1] = __reduce_max_sync(0xffffffffu, max(mag[0], mag[1]));
+    gs_put_rows_as<false>(m, r0, 16 * b, a, mag);      // every lane has read what it writes; the factors were read before the reduction
+  }
 }
 
 template <typename TX, typename TP>
@@ -203,6 +250,7 @@ feature_map_mma_bwd_kernel(const T* __restrict__ x, const float* __restrict__ w,
     const int active = (int)min((int64_t)kWarps, sh.end - at);
     __syncthreads();                                  // W is there; the tile before has been read
     bool odd = false;
+    uint32_t own = 0;                                 // blocks of g_u whose rows have factors of their own
     if (warp < active) {
       put_rows(v, s.xh + r0 * kP, s.xl + r0 * kP, s.nrm + r0, d, lane);
       __syncwarp();
@@ -247,7 +295,7 @@ feature_map_mma_bwd_kernel(const T* __restrict__ x, const float* __restrict__ w,
                 dot[r] = fmaf(a[m][2 * r], n < nt ? u[n][2 * r] : 0.f, fmaf(a[m][2 * r + 1], n < nt ? u[n][2 * r + 1] : 0.f, dot[r]));
                 odd |= !(fabsf(a[m][2 * r]) < CUDART_INF_F) | !(fabsf(a[m][2 * r + 1]) < CUDART_INF_F);
               }
-            gs_put(s.G, r0, 32 * c + 16 * b, a);
+            own |= (uint32_t)put_g(s.G, r0, 32 * c + 16 * b, a) << (2 * c + b);
           }
       }
       float c2[2], inv[2];
@@ -275,9 +323,10 @@ feature_map_mma_bwd_kernel(const T* __restrict__ x, const float* __restrict__ w,
                 for (int j = 0; j < D; ++j) a[n][e] = fmaf(gs_at(s.G, r0 + g + 8 * (e >> 1), j), wh[j * d + 32 * c + 8 * n + 2 * t + (e & 1)], a[n][e]);
             }
         } else {
-          const float *fg = s.G.inv_s + warp * 4, *fw = s.W.inv_s + 2 * c;
+          const float *fg = s.G.inv_s + (r0 + g) * 4, *fw = s.W.inv_s + 2 * c;
           product<false, true>(a, nt, (D + 15) / 16, gm_addr(s.G.hi + r0 * kP + gm_off_a(lane, kP)), 2 * kRows * kP, 32,
-                               gm_addr(s.W.hi + 32 * c + gm_off_a(lane, kP)), 2 * kMax * kP, 32 * kP, 32, [&](int l, int n) { return fg[l] * fw[4 * l + n]; });
+                               gm_addr(s.W.hi + 32 * c + gm_off_a(lane, kP)), 2 * kMax * kP, 32 * kP, 32,
+                               [&](int l, int n) { return make_float2(fg[l] * fw[4 * l + n], fg[32 + l] * fw[4 * l + n]); });
         }
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
@@ -292,6 +341,7 @@ feature_map_mma_bwd_kernel(const T* __restrict__ x, const float* __restrict__ w,
             }
         }
       }
+      if (own && g_w && !scalar) even_rows(s.G, r0, own);
     }
     const bool scalar = __syncthreads_or(odd) != 0;
     if (warp < (int)min((int64_t)kWarps, sh.end - at - kWarps)) ask_rows(v, x, (at + kWarps + warp) * 16, rows, H, h, d, lane);
@@ -313,7 +363,7 @@ feature_map_mma_bwd_kernel(const T* __restrict__ x, const float* __restrict__ w,
       } else {
         const float* fg = s.G.inv_s + (j0 >> 4);
         product<true, true>(a, lt, active, gm_addr(s.G.hi + j0 + gm_off_b(lane, kP)), 2 * kRows * kP, 32 * kP,
-                            gm_addr(s.xh + l0 + gm_off_a(lane, kP)), 2 * kRows * kP, 32 * kP, 32, [&](int l, int) { return fg[4 * l] * kXi; });
+                            gm_addr(s.xh + l0 + gm_off_a(lane, kP)), 2 * kRows * kP, 32 * kP, 32, [&](int l, int) { return both(fg[64 * l] * kXi); });
       }
 #pragma unroll
       for (int n = 0; n < 4; ++n)

@@ -75,9 +75,68 @@ __device__ __forceinline__ void gs_put(const GsSplit& m, int i0, int j0, const f
   if (mag < kGsInf) gs_put_as<false>(m, i0, j0, a, mag);
   else gs_put_odd(m, i0, j0, make_float4(a[0][0], a[0][1], a[0][2], a[0][3]), make_float4(a[1][0], a[1][1], a[1][2], a[1][3]));
 }
+
+// ---- with a factor for each row of a block -----------------------------------------------------------------------------------
+// For products whose results are of one row each: a row does not lose bits to a larger one beside it.
+struct GsByRow {
+  __half *hi, *lo;
+  float* inv_s;      // [row fr + column / 16 fc]
+  int pitch, fr, fc;
+};
+// the largest (ODD: finite) magnitudes of rows g and g + 8, in all four lanes of a row
+template <bool ODD>
+__device__ __forceinline__ void gs_row_mags(uint32_t (&mag)[2], const float (&a)[2][4]) {
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    mag[r] = 0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const uint32_t b = gs_mag(a[e >> 1][2 * r + (e & 1)]);
+      if (!ODD || b < kGsInf) mag[r] = max(mag[r], b);
+    }
+    mag[r] = max(mag[r], __shfl_xor_sync(0xffffffffu, mag[r], 1));
+    mag[r] = max(mag[r], __shfl_xor_sync(0xffffffffu, mag[r], 2));
+  }
+}
+template <bool ODD>
+__device__ __forceinline__ void gs_put_rows_as(const GsByRow& m, int i0, int j0, const float (&a)[2][4], const uint32_t (&mag)[2]) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const int row = i0 + g + 8 * r, at = row * m.pitch + j0 + 2 * t;
+    float s, inv_s;
+    gs_factors(mag[r], s, inv_s);
+    if (t == 0) m.inv_s[row * m.fr + (j0 >> 4) * m.fc] = inv_s;
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+      uint32_t hi, lo;
+      gs_parts<ODD>(a[n][2 * r], a[n][2 * r + 1], s, hi, lo);
+      *reinterpret_cast<uint32_t*>(m.hi + at + 8 * n) = hi;
+      *reinterpret_cast<uint32_t*>(m.lo + at + 8 * n) = lo;
+    }
+  }
+}
+static __device__ __noinline__ void gs_put_rows_odd(GsByRow m, int i0, int j0, float4 x, float4 y) {
+  const float a[2][4] = {{x.x, x.y, x.z, x.w}, {y.x, y.y, y.z, y.w}};
+  uint32_t mag[2];
+  gs_row_mags<true>(mag, a);
+  gs_put_rows_as<true>(m, i0, j0, a, mag);
+}
+__device__ __forceinline__ void gs_put_rows(const GsByRow& m, int i0, int j0, const float (&a)[2][4]) {
+  uint32_t mag[2];
+  gs_row_mags<false>(mag, a);
+  if (__any_sync(0xffffffffu, max(mag[0], mag[1]) >= kGsInf))
+    gs_put_rows_odd(m, i0, j0, make_float4(a[0][0], a[0][1], a[0][2], a[0][3]), make_float4(a[1][0], a[1][1], a[1][2], a[1][3]));
+  else gs_put_rows_as<false>(m, i0, j0, a, mag);
+}
+
+// ---- reading -------------------------------------------------------------------------------------------------------------------
 // an element put together again, for the element-by-element products
 __device__ __forceinline__ float gs_at(const GsSplit& m, int i, int l) {
   return (__half2float(m.hi[i * m.pitch + l]) + __half2float(m.lo[i * m.pitch + l])) * m.inv_s[(i >> 4) * m.sp + (l >> 4)];
+}
+__device__ __forceinline__ float gs_at(const GsByRow& m, int i, int l) {
+  return (__half2float(m.hi[i * m.pitch + l]) + __half2float(m.lo[i * m.pitch + l])) * m.inv_s[i * m.fr + (l >> 4) * m.fc];
 }
 __device__ __forceinline__ void gs_add(float (&acc)[4], const float (&p)[4], float f) {
 #pragma unroll

@@ -226,3 +226,27 @@ def test_feature_map_backward_in_tiles_of_32_and_64(dev, rows, H, D, d):
     assert float((gx - xd.grad).norm() / xd.grad.norm()) < 1e-6
     assert float((gw - wd.grad).norm() / wd.grad.norm()) < 2e-6
     assert torch.equal(ops.feature_map_bwd(x, w, g, 0.1, False, row_mask=mask)[0], gx)
+
+
+@pytest.mark.parametrize("D,d", [(64, 64), (32, 32), (48, 40)])
+@pytest.mark.parametrize("step", [1, 3, -3])
+def test_feature_map_backward_of_faded_rows(dev, D, d, step):
+    """csrc/feature_map_mma.cu: the gradients of 16 neighbouring rows fall by 2^step from row to row, to 2^-45 of the largest; each row of g_x has the
+    error that a row by itself has (22 bits of W and of g_u, fp32 sums: 3e-7; 1e-6 allowed), and g_W that of a sum over all rows."""
+    from rfa_b200 import ops
+    gen = torch.Generator(dev).manual_seed(D + step)
+    rows, H = 41, 250
+    x, w = torch.randn(rows, H, d, generator=gen, device=dev), torch.randn(H, D, d, generator=gen, device=dev)
+    g = torch.randn(rows, H, 2 * D, generator=gen, device=dev)
+    g *= 2.0 ** -(torch.arange(rows, device=dev) % 16 * step % 48).float()[:, None, None]
+    g[20] = 0
+    xd, wd = x.double().requires_grad_(), w.double().requires_grad_()
+    u = torch.einsum("thd,hkd->thk", xd / (xd.norm(dim=-1, keepdim=True) + 1e-3), wd)
+    (0.1 * torch.cat([u.sin(), u.cos()], dim=-1)).backward(g.double())
+    gx, gw = ops.feature_map_bwd(x, w, g, 0.1, True)
+    assert (gx[20] == 0).all()
+    keep = [i for i in range(rows) if i != 20]
+    per_row = (gx.double() - xd.grad).norm(dim=(1, 2))[keep] / xd.grad.norm(dim=(1, 2))[keep]
+    assert float(per_row.max()) < 1e-6, per_row
+    assert float((gw - wd.grad).norm() / wd.grad.norm()) < 2e-6
+    assert torch.equal(ops.feature_map_bwd(x, w, g, 0.1, False)[0], gx)
