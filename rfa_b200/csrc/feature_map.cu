@@ -265,7 +265,18 @@ static int fm_check(const void* x, const float* w, int64_t rows, int H, int d, i
 // 8 heads x 16, 256, 1024, 1536, 2048, 3072 rows forward 6.1 / 7.0, 7.3 / 7.1, 7.4 / 8.1, 10.2 / 8.4, 10.2 / 8.4, 13.6 / 10.4, backward
 // 10.5 / 14.1, 10.8 / 14.7, 16.4 / 18.0, 21.5 / 18.7, 22.5 / 19.4, 37.3 / 22.4; 32 x 32, 16 x 512 5.9 / 5.6 and 9.9 / 10.6, 8 x 1536 7.2 / 5.8
 // and 13.6 / 11.3.
-static bool fm_mma(int64_t rows, int H, int d, int D, int sms) { return d <= 64 && D <= 64 && (rows + 15) / 16 * H > 4 * sms; }
+// The line is higher
+//  - where D > 32 and d <= 32, as the products are a small part there: 64 x 8, 16 heads x 600, 900, 1300 rows forward 5.7 / 7.0, 5.7 / 7.2, 7.2 / 7.7,
+//    64 heads x 500 9.0 / 8.8; backward 13.1 / 13.2, 13.6 / 13.8, 22.1 / 14.9;
+//  - for the backward of few heads, whose CTAs all add to the same matrices: 64 x 64, 1 head x 9600, 14400, 20800 rows 21.2 / 24.7, 24.1 / 25.5, 32.6 / 26.7;
+//  - where the heads are more than the CTAs that the SMs hold, each of which has W to split: 64 x 64, 400 heads x 24, 52, 80 rows forward 12.1 / 15.0,
+//    13.1 / 14.9, 21.6 / 15.7, 64 x 8, 400 heads x 160 17.0 / 21.3.
+static bool fm_mma(int64_t rows, int H, int d, int D, int sms, bool backward) {
+  if (d > 64 || D > 64) return false;
+  const bool lean = D > 32 && d <= 32;
+  const int64_t a_head = (rows + 15) / 16, line = lean ? (backward ? 8 : 12) : backward && H < 8 ? 8 : 4;
+  return a_head * H > line * sms && (H <= 2 * sms || a_head >= (lean && !backward ? 32 : 5));
+}
 
 // CTAs per head, so that the grid is one wave of the `ctas` that an SM holds
 static int fm_grid_x(int64_t rows, int tile, int H, int ctas) {
@@ -296,7 +307,7 @@ extern "C" int rfa_feature_map_fwd_masked(const void* x, int x_dtype, const floa
   if (x_dtype == RFA_F16 && phi_dtype == RFA_F16 && d == 64 && D == 64)
     return launch_feature_map_fwd_tc((const __half*)x, w, row_mask, (__half*)phi, nullptr, nullptr, nullptr, rows, H, scale, sms,
                                      as_stream(stream));
-  if (fm_mma(rows, H, d, D, sms)) {
+  if (fm_mma(rows, H, d, D, sms, false)) {
 #define RFA_MMA(TX, TP) return launch_feature_map_mma_fwd<TX, TP>((const TX*)x, w, row_mask, (TP*)phi, rows, H, d, D, scale, sms, as_stream(stream))
     if (x_dtype == RFA_F16 && phi_dtype == RFA_F16) RFA_MMA(__half, __half);
     if (x_dtype == RFA_F32 && phi_dtype == RFA_F32) RFA_MMA(float, float);
@@ -342,7 +353,7 @@ extern "C" int rfa_feature_map_bwd_masked(const void* x, int x_dtype, const floa
   if (x_dtype == RFA_F16 && d == 64 && D == 64)
     return launch_feature_map_bwd_tc((const __half*)x, w, row_mask, (const __half*)g_phi, (__half*)g_x, nullptr, nullptr, nullptr,
                                      nullptr, g_w, rows, H, scale, sms, as_stream(stream));
-  if (fm_mma(rows, H, d, D, sms)) {
+  if (fm_mma(rows, H, d, D, sms, true)) {
     if (x_dtype == RFA_F16) return launch_feature_map_mma_bwd((const __half*)x, w, row_mask, (const __half*)g_phi, (__half*)g_x, g_w, rows, H, d, D,
                                                               scale, sms, as_stream(stream));
     if (x_dtype == RFA_F32) return launch_feature_map_mma_bwd((const float*)x, w, row_mask, (const float*)g_phi, (float*)g_x, g_w, rows, H, d, D,

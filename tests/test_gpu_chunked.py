@@ -250,3 +250,12 @@ def test_feature_map_backward_of_faded_rows(dev, D, d, step):
     assert float(per_row.max()) < 1e-6, per_row
     assert float((gw - wd.grad).norm() / wd.grad.norm()) < 2e-6
     assert torch.equal(ops.feature_map_bwd(x, w, g, 0.1, False)[0], gx)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("D,d", [(64, 64), (32, 32), (48, 40), (64, 24), (56, 8)])
+@pytest.mark.parametrize("rows,H", [(3 * 16, 198), (8 * 16 + 3, 132), (222 * 16, 8), (395 * 16 + 1, 3), (1184 * 16 + 5, 1), (33 * 16, 297), (5 * 16, 297), (16, 1000)])
+def test_feature_map_around_its_lines(dev, dtype, rows, H, D, d):
+    """Both sides of the lines in csrc/feature_map.cu between its kernels and those of feature_map_mma.cu: 4, 8 or 12 groups of 16 rows to an SM,
+    more heads than CTAs.  The gates are those of either."""
+    test_feature_map_on_split_operands(dev, dtype, rows, H, D, d)
