@@ -8,6 +8,7 @@
 // the states at their boundaries come from a reduction pre-pass plus an exclusive scan, the
 // same primitive a multi-device split of the sequence uses.
 #include "common.cuh"
+#include "segments.cuh"
 #include "sm100.cuh"
 
 namespace rfa {
@@ -16,11 +17,6 @@ namespace rfa {
 // segment planning (host) -- depends on (T, BH) only, so that the workspace size
 // query and every launch agree.
 // ---------------------------------------------------------------------------
-struct CausalPlan {
-  int nseg;        // segments per (batch, head)
-  int64_t tseg;    // tokens per segment (multiple of every kernel's chunk length)
-};
-
 constexpr int kSegAlign = 128;
 
 // tensor-core forward (causal_tc.cu)
@@ -60,7 +56,7 @@ int launch_causal_short_bwd(const __half* q, const __half* k, const __half* v, c
                             __half* gk, __half* gv, int64_t T, int BH, cudaStream_t st);
 
 // chunked tensor-core kernels for other geometries (generic_split.cu, generic_mma.cu)
-int generic_chunk(int K, int d, int* ctas);
+int generic_chunk(int64_t T, int BH, int K, int d, int* ctas);
 int launch_causal_chunked_fwd(const __half* q, const __half* k, const __half* v, __half* out, const float* s_seg, const float* z_seg,
                               float* s_out, float* z_out, float* den_out, int64_t T, int BH, int nseg, int64_t tseg, int K, int d,
                               cudaStream_t st);
@@ -98,30 +94,21 @@ int launch_state_generic_bwd(const __half* k, const __half* v, const uint8_t* pa
 // that one wave of SMs holds: (8, 512) 36 / 37, (16, 600) 43 / 39, (36, 700) 50 / 50, (64, 1024) 67 / 69, (8, 1024) 64 / 38,
 // (72, 2000) 125 / 116, (36, 1531) 93 / 60, (8, 2048) 121 / 46, (4, 4096) 235 / 48, (32, 16384) 915 / 363.  A forward alone
 // at (8, 1024) takes 14 us either way and is slower cut below that, hence 6 chunks saved as the line.
-constexpr int64_t kSms = 148;
-static CausalPlan cut_segments(int64_t T, int64_t chunk, int64_t fit, int64_t min_saved) {
-  const int64_t n = (T + chunk - 1) / chunk;
-  if (fit >= 2 && n >= 2) {
-    const int64_t s = fit < n ? fit : n, m = (n + s - 1) / s;
-    if (n - m >= min_saved) return CausalPlan{(int)((n + m - 1) / m), m * chunk};
-  }
-  return CausalPlan{1, n * chunk};
-}
 static CausalPlan plan_causal(int64_t T, int BH) { return cut_segments(T, kSegAlign, kSms / BH, 6); }
 
 // Which kernels serve a geometry: the tcgen05 ones (K = 128, d = 64), the chunked ones of generic_split.cu and generic_mma.cu, or the
 // token-at-a-time ones of generic.cu.
 static bool is_tc(int K, int d) { return K == kK && d == kD; }
-static bool is_chunked(int K, int d) { return !is_tc(K, d) && generic_chunk(K, d, nullptr) > 0; }
+static bool is_chunked(int K, int d) { return !is_tc(K, d) && generic_chunk(1, 1, K, d, nullptr) > 0; }
 
 static CausalPlan plan_geometry(int64_t T, int BH, int K, int d) {
   if (is_tc(K, d)) return plan_causal(T, BH);
   int ctas = 1;
-  const int chunk = generic_chunk(K, d, &ctas);
+  const int chunk = generic_chunk(T, BH, K, d, &ctas);
   if (!chunk) return CausalPlan{1, T};
-  // A chunk takes these kernels 10 us and more, a cut's pre-pass and scans 10: any cut that one wave holds.  Forward + backward of
-  // generic_mma.cu's kernels in us at (K, d, heads x batch, tokens), whole / cut: (64, 32, 32, 200) 109 / 47, (128, 128, 32, 200) 361 / 137,
-  // (256, 128, 8, 128) 357 / 152, (64, 32, 8, 512) 217 / 46.
+  // A chunk takes these kernels 10 us and more, a cut's pre-pass and scans about as much: any cut that one wave holds.  Forward + backward in us, whole /
+  // cut, at (K, d, heads x batch, tokens): (64, 32, 32, 200) 75 / 39, (128, 128, 32, 200) 205 / 88, (96, 96, 8, 512) 264 / 48, (64, 32, 8, 512) 152 / 30,
+  // (64, 32, 64, 1024) 300 / 134, and of generic_mma.cu's (256, 128, 8, 128) 273 / 154.
   return cut_segments(T, chunk, kSms * ctas / BH, 1);
 }
 

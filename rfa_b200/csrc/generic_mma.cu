@@ -29,6 +29,7 @@
 // non-finite value takes the masked products element by element, over the unmasked tokens only, so that what a
 // token makes of its predecessors never depends on its successors.
 #include "generic_mma.cuh"
+#include "segments.cuh"
 #include "sm100.cuh"
 
 namespace rfa {
@@ -708,7 +709,7 @@ static GmShape gm_shape(int K, int d) {
 }
 
 // the kernels whose operands are split into fp16 tiles once (generic_split.cu), where they fit
-int split_chunk(int K, int d, int* ctas);
+int split_chunk(int64_t T, int BH, int K, int d, bool whole, int* ctas);
 int launch_causal_split_fwd(const __half* q, const __half* k, const __half* v, __half* out, const float* s_seg, const float* z_seg, float* s_out,
                             float* z_out, float* den_out, int64_t T, int BH, int nseg, int64_t tseg, int K, int d, cudaStream_t st);
 int launch_causal_split_bwd_q(const __half* q, const __half* k, const __half* v, const __half* g, __half* gq, const float* s_seg, const float* z_seg,
@@ -719,11 +720,26 @@ int launch_causal_split_bwd_kv(const __half* q, const __half* k, const __half* v
 int launch_state_split(const __half* x, const __half* y, const uint8_t* pad_mask, const float* ws_den, const float* ws_gz, float* s, float* z,
                        int64_t T, int BH, int H, int nseg, int64_t tseg, int runs, int K, int d, cudaStream_t st);
 
-// Tokens per chunk of the chunked kernels for this geometry, 0 when it does not fit them; *ctas = how many of their CTAs
+// Whether those take the call.  Where only their chunks of 16 fit, one CTA makes a 16 x 16 block of scores at a time, and the longer chunks here
+// are faster as soon as several follow one another: a token here costs 7/8 of one there (half of it at d = 8, which is padded to 16
+// there), a call one chunk of 16 more.  us forward + backward, here / there: (160, 128), 8 heads x 512 tokens 152 / 92, 64 x 512 495 / 550,
+// 128 x 1024 1519 / 1765; (512, 32) 122 / 99, 644 / 639, 2046 / 2125; (520, 24), 16 x 512 185 / 175; (896, 8), 8 x 64 99 / 60, 8 x 512 110 / 119,
+// 64 x 512 722 / 853.
+static bool takes_split(int64_t T, int BH, int K, int d, bool whole) {
+  int ctas = 1;
+  const int chunk = split_chunk(T, BH, K, d, whole, &ctas);
+  if (chunk != 16) return chunk > 0;
+  const GmShape here = gm_shape(K, d);
+  if (here.C <= 16) return true;
+  const auto chunks = [&](int C, int n) { return cut_segments(T, C, whole ? 1 : kSms * n / BH, 1).tseg / C; };      // one after another
+  return (d < 16 ? 32 : 16) * chunks(16, ctas) < 7 * here.C * chunks(here.C, here.ctas) / 8 + 16;
+}
+
+// Tokens per chunk of the chunked kernels for these calls, 0 when the geometry does not fit them; *ctas = how many of their CTAs
 // one SM holds.
-int generic_chunk(int K, int d, int* ctas) {
-  if (const int chunk = split_chunk(K, d, ctas)) return chunk;
+int generic_chunk(int64_t T, int BH, int K, int d, int* ctas) {
   if (K <= 0 || d <= 0 || K % 8 || d % 8 || K > 1024 || d > 1024) return 0;
+  if (takes_split(T, BH, K, d, false)) return split_chunk(T, BH, K, d, false, ctas);
   const GmShape s = gm_shape(K, d);
   if (ctas) *ctas = s.ctas;
   return s.C;
@@ -747,7 +763,7 @@ static int gm_launch(KERNEL kernel, const char* what, int threads, uint32_t smem
 int launch_causal_chunked_fwd(const __half* q, const __half* k, const __half* v, __half* out, const float* s_seg, const float* z_seg,
                               float* s_out, float* z_out, float* den_out, int64_t T, int BH, int nseg, int64_t tseg, int K, int d,
                               cudaStream_t st) {
-  if (split_chunk(K, d, nullptr)) return launch_causal_split_fwd(q, k, v, out, s_seg, z_seg, s_out, z_out, den_out, T, BH, nseg, tseg, K, d, st);
+  if (takes_split(T, BH, K, d, nseg == 1)) return launch_causal_split_fwd(q, k, v, out, s_seg, z_seg, s_out, z_out, den_out, T, BH, nseg, tseg, K, d, st);
 #define RFA_GM_CALL(C, N) return gm_launch(gm_causal_fwd_kernel<C, N>, "rfa_causal_fwd (chunked)", gs_.threads, gm_layout(C, K, d, N, 2, 1, 1, gm_rows_fwd(C)).total, \
                                            dim3(BH, nseg), st, q, k, v, out, s_seg, z_seg, s_out, z_out, den_out, T, BH, tseg, K, d)
   RFA_GM_DISPATCH(gm_shape(K, d), RFA_GM_CALL);
@@ -757,7 +773,7 @@ int launch_causal_chunked_fwd(const __half* q, const __half* k, const __half* v,
 int launch_causal_chunked_bwd_q(const __half* q, const __half* k, const __half* v, const __half* g, __half* gq, const float* s_seg,
                                 const float* z_seg, float* ws_den, float* ws_gz, int64_t T, int BH, int nseg, int64_t tseg, int K, int d,
                                 cudaStream_t st) {
-  if (split_chunk(K, d, nullptr)) return launch_causal_split_bwd_q(q, k, v, g, gq, s_seg, z_seg, ws_den, ws_gz, T, BH, nseg, tseg, K, d, st);
+  if (takes_split(T, BH, K, d, nseg == 1)) return launch_causal_split_bwd_q(q, k, v, g, gq, s_seg, z_seg, ws_den, ws_gz, T, BH, nseg, tseg, K, d, st);
 #define RFA_GM_CALL(C, N) return gm_launch(gm_causal_bwd_q_kernel<C, N>, "rfa_causal_bwd_q (chunked)", gs_.threads, gm_layout(C, K, d, N, 2, 2, 1, gm_rows_bwd_q(C, K)).total, \
                                            dim3(BH, nseg), st, q, k, v, g, gq, s_seg, z_seg, ws_den, ws_gz, T, BH, tseg, K, d)
   RFA_GM_DISPATCH(gm_shape(K, d), RFA_GM_CALL);
@@ -767,7 +783,7 @@ int launch_causal_chunked_bwd_q(const __half* q, const __half* k, const __half* 
 int launch_causal_chunked_bwd_kv(const __half* q, const __half* k, const __half* v, const __half* g, __half* gk, __half* gv,
                                  const float* ws_den, const float* ws_gz, const float* ds_seg, const float* dz_seg, int64_t T, int BH,
                                  int nseg, int64_t tseg, int K, int d, cudaStream_t st) {
-  if (split_chunk(K, d, nullptr)) return launch_causal_split_bwd_kv(q, k, v, g, gk, gv, ws_den, ws_gz, ds_seg, dz_seg, T, BH, nseg, tseg, K, d, st);
+  if (takes_split(T, BH, K, d, nseg == 1)) return launch_causal_split_bwd_kv(q, k, v, g, gk, gv, ws_den, ws_gz, ds_seg, dz_seg, T, BH, nseg, tseg, K, d, st);
 #define RFA_GM_CALL(C, N) return gm_launch(gm_causal_bwd_kv_kernel<C, N>, "rfa_causal_bwd_kv (chunked)", gs_.threads, gm_layout(C, K, d, N, 2, 2, 2, kGmRowsKv).total, \
                                            dim3(BH, nseg), st, q, k, v, g, gk, gv, ws_den, ws_gz, ds_seg, dz_seg, T, BH, tseg, K, d)
   RFA_GM_DISPATCH(gm_shape(K, d), RFA_GM_CALL);
@@ -777,7 +793,7 @@ int launch_causal_chunked_bwd_kv(const __half* q, const __half* k, const __half*
 // the first `runs` of nseg runs of tokens; ws_den / ws_gz null: sums of k (x) v and k; else of q (x) (g / den) and gz q
 int launch_state_chunked(const __half* x, const __half* y, const uint8_t* pad_mask, const float* ws_den, const float* ws_gz, float* s,
                          float* z, int64_t T, int BH, int H, int nseg, int64_t tseg, int runs, int K, int d, cudaStream_t st) {
-  if (split_chunk(K, d, nullptr)) return launch_state_split(x, y, pad_mask, ws_den, ws_gz, s, z, T, BH, H, nseg, tseg, runs, K, d, st);
+  if (takes_split(T, BH, K, d, nseg == 1)) return launch_state_split(x, y, pad_mask, ws_den, ws_gz, s, z, T, BH, H, nseg, tseg, runs, K, d, st);
 #define RFA_GM_CALL(C, N)                                                                                                             \
   return ws_den ? gm_launch(gm_state_kernel<C, N, true>, "state reduction (chunked)", gs_.threads, gm_layout(C, K, d, N, 1, 1, 0, kGmRowsState).total, \
                             dim3(BH, runs), st, x, y, pad_mask, ws_den, ws_gz, s, z, T, BH, H, nseg, tseg, K, d)                             \

@@ -9,6 +9,7 @@
 // tensor pipe 12 %, a third of the stalls at the chunk's barriers): forward + backward kernels 185 -> 141 us at (K, d) = (64, 32), 64 heads x
 // 1024 tokens, 138 -> 92 at (96, 40), 64 x 300, 392 -> 323 at (128, 128), 64 x 512, 123 -> 57 at (128, 128), 8 x 200.
 #include "generic_split.cuh"
+#include "segments.cuh"
 #include "sm100.cuh"
 
 namespace rfa {
@@ -753,26 +754,42 @@ gs_state_kernel(const __half* __restrict__ x, const __half* __restrict__ y, cons
 // ---------------------------------------------------------------------------------------------------------------------------
 constexpr uint32_t kGsSmemMax = 227 * 1024;
 struct GsShape { int C, ctas, threads; };
-// The longest chunk of which two CTAs fit an SM, else the longest that fits: a longer chunk shares the state's products, its update and the
-// barriers among more tokens, and the second CTA works while one waits at its barriers or for its tiles (a second stage of tiles
-// in its place was slower).  24 warps in all.  Forward + backward kernels in us, chunks of 64 / 32 / 16 tokens: (K, d) = (64, 32), 64
-// heads x 1024 tokens 141 / 152 / 198, 8 x 512 37 / 33 / 37; (96, 40), 64 x 300 104 (one CTA) / 92 / 111; (128, 128), 64 x 512 - / 323 / 541.
-static GsShape gs_shape(int K, int d) {
-  GsShape one{0, 0, 0};
-  for (int C : {64, 32, 16}) {
-    const uint32_t a = gs_layout_q(C, K, d).total, b = gs_layout_kv(C, K, d).total, need = a > b ? a : b;
-    if (need > kGsSmemMax) continue;
+// Which chunk.  A longer one shares the state's products, its update and the barriers among more tokens; shorter ones leave room for
+// more CTAs on an SM, one of which works while another waits, and cut a sequence into more segments.  24 warps in all.
+//
+// Chunks of 64 wherever two of their CTAs fit an SM: us forward + backward, 64 / 32 / 16 tokens, (K, d) = (64, 32), 64 heads x 512 tokens 71 / 80 / 111,
+// 128 x 1024 256 / 243 / 363, 64 x 45 21 / 27 / 27.  Where one fits, against those of 32 (of which one to three do), gs_cost decides; in units of an
+// uncut chunk of 64 (23 to 40 us) it is a fit to 500 calls of 11 geometries, 0.4 % over the better of the two in the mean and 16 % at most:
+// (64, 96), 148 heads x 1024 459 / 533, 96 x 1024 444 / 364, 64 x 512 144 / 145, 8 x 256 40 / 33, 64 x 45 28 / 42; (96, 96), 64 x 512 174 / 227 / 247,
+// 128 x 1024 555 / 732 / 964; (64, 128) 175 / 227 / 239, 551 / 732 / 923.
+// Chunks of 16 where two CTAs fit and only one of 32, and all of them at half of the SMs: (192, 48), 4 heads x 128 51 / 38 / 33, 16 x 128 52 / 39 / 46; and
+// where nothing longer fits (there generic_mma.cu decides).
+static float gs_cost(int C, int ctas, int64_t T, int BH, bool whole) {
+  const CausalPlan p = cut_segments(T, C, whole ? 1 : kSms * ctas / BH, 1);
+  const int64_t n = (int64_t)BH * p.nseg, fit = kSms * ctas, waves = (n + fit - 1) / fit, per_sm = (n + kSms - 1) / kSms;
+  const float m = (float)(p.tseg / C);
+  if (C == 64) return waves * (p.nseg == 1 ? m : 0.2f + 1.16f * m);      // a cut one makes the pre-pass too
+  const float w = per_sm == 1 ? 0.75f : per_sm == 2 || ctas == 2 ? 1.1f : 1.42f;
+  return waves * (p.nseg == 1 ? 0.82f * w * m : 0.35f + w * m);
+}
+// whole: the sequences are not cut (a call without a workspace, a state reduction alone)
+static GsShape gs_shape(int64_t T, int BH, int K, int d, bool whole) {
+  int ctas[3];                  // how many CTAs of chunks of 64, 32, 16 an SM holds
+  for (int i = 0; i < 3; ++i) {
+    const uint32_t a = gs_layout_q(64 >> i, K, d).total, b = gs_layout_kv(64 >> i, K, d).total, need = a > b ? a : b;
     const int n = (int)(kGsSmemMax / (need + 1024));
-    if (n >= 2) return GsShape{C, n > 3 ? 3 : n, n == 2 ? 384 : 256};
-    if (!one.C) one = GsShape{C, 1, 768};
+    ctas[i] = need > kGsSmemMax ? 0 : n < 1 ? 1 : n > 3 ? 3 : n;
   }
-  return one;
+  int i = ctas[0] ? 0 : ctas[1] ? 1 : 2;
+  if (ctas[0] == 1 && ctas[1] && gs_cost(32, ctas[1], T, BH, whole) < gs_cost(64, 1, T, BH, whole)) i = 1;
+  if (ctas[0] < 2 && ctas[1] < 2 && ctas[2] > 1 && (T <= 16 || (!whole && (T + 15) / 16 * BH <= kSms / 2))) i = 2;
+  return GsShape{ctas[i] ? 64 >> i : 0, ctas[i], ctas[i] == 3 ? 256 : ctas[i] == 2 ? 384 : 768};
 }
 
-// Tokens per chunk of these kernels for this geometry, 0 when it does not fit them; *ctas = how many of their CTAs one SM holds
-int split_chunk(int K, int d, int* ctas) {
+// Tokens per chunk of these kernels, 0 when the geometry does not fit them; *ctas = how many of their CTAs one SM holds
+int split_chunk(int64_t T, int BH, int K, int d, bool whole, int* ctas) {
   if (K <= 0 || d <= 0 || K % 8 || d % 8 || K > 1024 || d > 1024) return 0;
-  const GsShape s = gs_shape(K, d);
+  const GsShape s = gs_shape(T, BH, K, d, whole);
   if (ctas) *ctas = s.ctas;
   return s.C;
 }
@@ -797,14 +814,14 @@ int launch_causal_split_fwd(const __half* q, const __half* k, const __half* v, _
                             float* z_out, float* den_out, int64_t T, int BH, int nseg, int64_t tseg, int K, int d, cudaStream_t st) {
 #define RFA_GS_CALL(C) return gs_launch(gs_causal_fwd_kernel<C>, "rfa_causal_fwd (chunked)", gs_pdl(tseg, C), gs_.threads, gs_layout_fwd(C, K, d).total, \
                                         dim3(BH, nseg), st, q, k, v, out, s_seg, z_seg, s_out, z_out, den_out, T, BH, tseg, K, d)
-  RFA_GS_DISPATCH(gs_shape(K, d), RFA_GS_CALL);
+  RFA_GS_DISPATCH(gs_shape(T, BH, K, d, nseg == 1), RFA_GS_CALL);
 #undef RFA_GS_CALL
 }
 int launch_causal_split_bwd_q(const __half* q, const __half* k, const __half* v, const __half* g, __half* gq, const float* s_seg, const float* z_seg,
                               float* ws_den, float* ws_gz, int64_t T, int BH, int nseg, int64_t tseg, int K, int d, cudaStream_t st) {
 #define RFA_GS_CALL(C) return gs_launch(gs_causal_bwd_q_kernel<C>, "rfa_causal_bwd_q (chunked)", gs_pdl(tseg, C), gs_.threads, gs_layout_q(C, K, d).total, \
                                         dim3(BH, nseg), st, q, k, v, g, gq, s_seg, z_seg, ws_den, ws_gz, T, BH, tseg, K, d)
-  RFA_GS_DISPATCH(gs_shape(K, d), RFA_GS_CALL);
+  RFA_GS_DISPATCH(gs_shape(T, BH, K, d, nseg == 1), RFA_GS_CALL);
 #undef RFA_GS_CALL
 }
 int launch_causal_split_bwd_kv(const __half* q, const __half* k, const __half* v, const __half* g, __half* gk, __half* gv, const float* ws_den,
@@ -812,7 +829,7 @@ int launch_causal_split_bwd_kv(const __half* q, const __half* k, const __half* v
                                int d, cudaStream_t st) {
 #define RFA_GS_CALL(C) return gs_launch(gs_causal_bwd_kv_kernel<C>, "rfa_causal_bwd_kv (chunked)", gs_pdl(tseg, C), gs_.threads, gs_layout_kv(C, K, d).total, \
                                         dim3(BH, nseg), st, q, k, v, g, gk, gv, ws_den, ws_gz, ds_seg, dz_seg, T, BH, tseg, K, d)
-  RFA_GS_DISPATCH(gs_shape(K, d), RFA_GS_CALL);
+  RFA_GS_DISPATCH(gs_shape(T, BH, K, d, nseg == 1), RFA_GS_CALL);
 #undef RFA_GS_CALL
 }
 int launch_state_split(const __half* x, const __half* y, const uint8_t* pad_mask, const float* ws_den, const float* ws_gz, float* s, float* z,
@@ -822,7 +839,7 @@ int launch_state_split(const __half* x, const __half* y, const uint8_t* pad_mask
                             dim3(BH, runs), st, x, y, pad_mask, ws_den, ws_gz, s, z, T, BH, H, nseg, tseg, K, d)                      \
                 : gs_launch(gs_state_kernel<C, false>, "state reduction (chunked)", gs_pdl(tseg, C), gs_.threads, gs_layout_state(C, K, d, false).total, \
                             dim3(BH, runs), st, x, y, pad_mask, ws_den, ws_gz, s, z, T, BH, H, nseg, tseg, K, d)
-  RFA_GS_DISPATCH(gs_shape(K, d), RFA_GS_CALL);
+  RFA_GS_DISPATCH(gs_shape(T, BH, K, d, nseg == 1), RFA_GS_CALL);
 #undef RFA_GS_CALL
 }
 

@@ -14,7 +14,7 @@ from rfa_b200.rfa import RFA
 
 pytestmark = pytest.mark.gpu
 
-GEOMETRIES = [(64, 32), (96, 40), (128, 128), (256, 128), (72, 24), (8, 8), (512, 64)]      # chunks of 64, 32 and 16 tokens
+GEOMETRIES = [(64, 32), (96, 40), (128, 128), (256, 128), (72, 24), (8, 8), (512, 64)]      # the kernels they reach have chunks of 64 and 32 tokens
 
 
 def inputs(T, BH, K, d, seed):
@@ -259,3 +259,39 @@ def test_feature_map_around_its_lines(dev, dtype, rows, H, D, d):
     """Both sides of the lines in csrc/feature_map.cu between its kernels and those of feature_map_mma.cu: 4, 8 or 12 groups of 16 rows to an SM,
     more heads than CTAs.  The gates are those of either."""
     test_feature_map_on_split_operands(dev, dtype, rows, H, D, d)
+
+
+# (K, d, tokens, heads) -> which kernels, chunk, CTAs on an SM: each that the dispatch can reach, with several chunks after one another where it makes any
+REACHED = [(8, 8, 131, 150),        # generic_split.cu: 64, three
+           (64, 32, 131, 150),      # 64, two
+           (64, 96, 131, 148),      # 64, one
+           (64, 64, 131, 150),      # 32, three
+           (64, 96, 131, 150),      # 32, two
+           (128, 128, 131, 150),    # 32, one
+           (192, 48, 131, 2),       # 16, two
+           (160, 128, 131, 20),     # 16, one, in segments
+           (160, 128, 112, 148),    # 16, one, whole
+           (160, 128, 128, 148),    # generic_mma.cu from here on: 64, one stage of tiles
+           (192, 128, 131, 150),
+           (896, 8, 131, 40),       # 32, one stage
+           (160, 176, 131, 40),     # 32, two stages
+           (208, 208, 70, 40),      # 16, one stage
+           (224, 184, 70, 40)]      # 16, two stages
+
+
+@pytest.mark.parametrize("K,d,T,BH", REACHED)
+def test_every_chunked_kernel_against_fp64(dev, K, d, T, BH):
+    from rfa_b200 import _lib
+    q, k, v, g = (t.to(dev) for t in inputs(T, BH, K, d, K + d + T))
+    want = RFA.forward_torch(*(t.double() for t in (q, k, v))).cpu()
+    grads = [t.cpu() for t in RFA.backward_torch(*(t.double() for t in (q, k, v, g)))]
+    leaves = [t.clone().requires_grad_() for t in (q, k, v)]
+    out = RFA.apply(*leaves)
+    out.backward(g)
+    assert rel(out, want, 2.0 ** -24) < 4e-4
+    for name, leaf, ref in zip("qkv", leaves, grads):
+        assert rel(leaf.grad, ref, 2.0 ** -24) < 4e-4, name
+    bare = torch.empty_like(out)                       # no workspace: sequences stay whole
+    assert _lib.load().rfa_causal_fwd(*(t.data_ptr() for t in (q, k, v, bare)), None, None, None, None, None,
+                                      ctypes.c_size_t(0), T, BH, K, d, _lib.stream_of(q)) == 0
+    assert rel(bare, want, 2.0 ** -24) < 4e-4
