@@ -12,6 +12,7 @@
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/extension.h>
 
+#include <algorithm>
 #include <atomic>
 #include <string>
 #include <tuple>
@@ -402,13 +403,27 @@ Tensor decode_step_fused(Tensor q, Tensor k, Tensor v, const Tensor& w, double s
   return out;
 }
 
+// The largest batch for which one token through a layer of E features is faster by these kernels than by the library GEMMs module by module, at most 128.
+// linear_rows.cu reads x once for every 16 or 32 rows of W and W once for every 64 tokens, so that the products lose as E and the batch grow, while
+// the launches that are saved cost 60 us of host time.  us a layer with weights from HBM, here / module by module: E = 1024, 128 rows 48 / 101; 2048, 32, 33, 128
+// rows 36 / 98, 55 / 98, 96 / 98; 2560, 48, 64 rows 88 / 99, 101 / 98; 4096, 16, 32 rows 53 / 100, 106 / 100; 8192, 8, 16 rows 115 / 133, 253 / 148.  In a CUDA
+// graph only the kernels count: 47.0 / 47.4; 36 / 44, 54 / 44, 95 / 79; 86 / 57, 100 / 62; 52 / 63, 100 / 73; 114 / 121, 215 / 135.
+int64_t most_rows(int64_t E, bool captured) {
+  if (captured) return E <= 1024 ? 128 : E <= 2048 ? 32 : E <= 4096 ? 16 : 8;
+  return E <= 2048 ? 128 : std::clamp<int64_t>((300 << 20) / (E * E), 8, 128);
+}
+bool capturing(const Tensor& x) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  C10_CUDA_CHECK(cudaStreamIsCapturing(c10::cuda::getCurrentCUDAStream(x.device().index()).stream(), &status));
+  return status != cudaStreamCaptureStatusNone;
+}
+
 // One token [1, B, E] through a whole self-attention layer: the three projections and the step's random matrices in one launch, the
 // decoding step, the output projection.  Null where a launch here would not be what the separate tensor calls do (dtype,
 // layout, a broadcast shape, a batch that the library GEMMs serve better): nothing has been done then.
 OptTensor layer_decode(const Tensor& x, const Tensor& wq, const OptTensor& bq, const Tensor& wk, const OptTensor& bk, const Tensor& wv,
                        const OptTensor& bv, const Tensor& wo, const OptTensor& bo, const Tensor& rm, const OptTensor& sigma, double tau,
                        double scale, const OptTensor& s, const OptTensor& z) {
-  constexpr int64_t kMaxBatch = 128;      // the largest batch that was measured faster than the library GEMMs
   if (!x.is_cuda() || x.dim() != 3 || x.size(0) != 1 || rm.dim() != 3) return std::nullopt;
   const int64_t B = x.size(1), E = x.size(2), H = rm.size(0), D = rm.size(1), d = rm.size(2);
   const auto plain = [&](const Tensor& t, at::IntArrayRef shape, at::ScalarType type) {
@@ -417,7 +432,7 @@ OptTensor layer_decode(const Tensor& x, const Tensor& wq, const OptTensor& bq, c
   };
   const auto bias = [&](const OptTensor& b) { return !b || plain(*b, {E}, at::kHalf); };
   const bool width = D > 0 && D % 8 == 0 && D <= 128 && (d == 8 || d == 16 || d == 32 || d == 64 || d == 128);
-  if (B < 1 || B > kMaxBatch || !width || H < 1 || H * d != E || !plain(x, {1, B, E}, at::kHalf)) return std::nullopt;
+  if (B < 1 || B > most_rows(E, capturing(x)) || !width || H < 1 || H * d != E || !plain(x, {1, B, E}, at::kHalf)) return std::nullopt;
   for (const Tensor* w : {&wq, &wk, &wv, &wo})
     if (!plain(*w, {E, E}, at::kHalf)) return std::nullopt;
   if (!bias(bq) || !bias(bk) || !bias(bv) || !bias(bo) || !plain(rm, {H, D, d}, at::kHalf)) return std::nullopt;

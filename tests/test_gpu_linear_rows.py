@@ -79,3 +79,37 @@ def test_layer_call_takes_what_it_took(dev):
         layer.out_proj = Doubled(128, 128).to(dev).half()
         layer.out_proj.load_state_dict(out_proj.state_dict())
         assert rel(layer(x, w, saved_state={}), 2 * base) < 3e-3
+
+
+@pytest.mark.parametrize("heads,batch,eager,captured", [(16, 128, True, True), (32, 32, True, True), (32, 33, True, False), (40, 48, True, False),
+                                                        (40, 49, False, False), (64, 16, True, True), (64, 18, True, False), (64, 19, False, False)])
+def test_the_largest_batch_of_a_layer_call(dev, monkeypatch, heads, batch, eager, captured):
+    """Which batches the launch takes depends on the width, and in a CUDA graph, where the host does not count, on less of it; either way the result is the
+    layer's."""
+    from rfa_b200 import ops
+    torch.manual_seed(heads)
+    E = 64 * heads
+    layer = CausalAttention(embed_dim=E, num_heads=heads, head_dim=64, proj_dim=64).to(dev).half().requires_grad_(False)
+    w, x = torch.randn(heads, 64, 64, device=dev).half(), torch.randn(1, batch, E, device=dev).half()
+    took, decode = [], ops.layer_decode
+
+    def seen(*args):
+        y = decode(*args)
+        took.append(y is not None)
+        return y
+    monkeypatch.setattr(ops, "layer_decode", seen)
+    state = lambda: dict(prev_s=torch.zeros(batch, heads, 128, 64, device=dev), prev_z=torch.zeros(batch, heads, 128, device=dev))
+    hook = layer.v_proj.register_forward_hook(lambda *args: None)
+    want = layer(x, w, saved_state=state())
+    hook.remove()
+    assert not took
+    got, held = layer(x, w, saved_state=state()), state()
+    assert took == [eager]
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        replayed = layer(x, w, saved_state=held)
+    assert took == [eager, captured]
+    graph.replay()
+    for y in (got, replayed):
+        assert ((y - want).float().norm() / want.float().norm()).item() < 3e-3
