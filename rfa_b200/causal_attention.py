@@ -273,15 +273,16 @@ class CausalAttention(nn.Module):
         saved_state["prev_s"], saved_state["prev_z"] = s, z
         return attn
 
-    def _own_heads(self, random_matrices: Tensor) -> bool:
+    def _own_matrices(self, random_matrices: Tensor) -> bool:
         """Whether the matrices are for this layer's heads.  A native pass takes the split of the features into heads from them, and others may
-        divide embed_dim too, which the module-by-module call refuses."""
-        return random_matrices.dim() == 3 and random_matrices.size(0) == self.num_heads and random_matrices.size(2) == self.head_dim
+        divide embed_dim too, which the module-by-module call refuses.  (A tau that is a tensor, which may want a gradient, stays with the tensor
+        expressions too.)"""
+        return isinstance(self.tau, (int, float)) and random_matrices.dim() == 3 and random_matrices.size(0) == self.num_heads and random_matrices.size(2) == self.head_dim
 
     def _decode_layer(self, x: Tensor, random_matrices: Tensor, saved_state: Dict[str, Optional[Tensor]]) -> Optional[Tensor]:
         """One token through the whole layer in three launches (host time is what a small decoding call consists of); None, and
         nothing done, where the call is to go module by module."""
-        if not (x.is_cuda and x.dtype is torch.float16 and random_matrices.is_cuda and self._own_heads(random_matrices)):
+        if not (x.is_cuda and x.dtype is torch.float16 and random_matrices.is_cuda and self._own_matrices(random_matrices)):
             return None
         linears = (self.q_proj, self.k_proj, self.v_proj, self.out_proj)
         sigma = self.sigma if self.reparam_proj else None
@@ -304,7 +305,7 @@ class CausalAttention(nn.Module):
         858, 757).  None, and nothing done, where the call is to go module by module."""
         sigma = self.sigma if self.reparam_proj else None
         if not (torch.is_grad_enabled() and x.is_cuda and x.dtype is torch.float16 and random_matrices.dtype is torch.float16
-                and self._own_heads(random_matrices)):
+                and self._own_matrices(random_matrices)):
             return None
         if not (x.requires_grad or random_matrices.requires_grad or self.q_proj.weight.requires_grad
                 or (sigma is not None and sigma.requires_grad)):
@@ -326,7 +327,7 @@ class CausalAttention(nn.Module):
         half = torch.float16
         if any(t is not None and (t.device != q.device or t.data_ptr() % 16) for t in (random_matrices, sigma)):
             return False           # the tensor expressions refuse operands of two devices and make aligned ones of a view at any offset
-        return (ops.fused_forward_supported(q, random_matrices) and q.dtype is k.dtype is v.dtype is half
+        return (self._own_matrices(random_matrices) and ops.fused_forward_supported(q, random_matrices) and q.dtype is k.dtype is v.dtype is half
                 and tuple(random_matrices.shape) == (self.num_heads, 64, 64) and random_matrices.dtype is half
                 and (sigma is None or (sigma.dtype is half and tuple(sigma.shape) == (self.num_heads, 1, 64)))
                 and plain_tensors(q, k, v, random_matrices, sigma, mask) and _underived(q, k, v, random_matrices, sigma))

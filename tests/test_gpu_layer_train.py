@@ -177,3 +177,19 @@ def test_matrices_of_another_split_into_heads_are_refused(dev, heads, head_dim, 
         with pytest.raises((AssertionError, ValueError, RuntimeError)):
             call()
         assert not state
+
+
+def test_a_temperature_that_is_a_tensor(dev):
+    """Its gradient, and the results of the number that it holds."""
+    torch.manual_seed(0)
+    layer, rm = make(dev)
+    x = torch.randn(20, 2, 512, device=dev).half()
+    layer.tau = 2.0
+    want, first = layer(x, rm), layer(x[:1], rm, saved_state={})
+    layer.tau = torch.nn.Parameter(torch.tensor(2.0, device=dev))
+    got = layer(x, rm)
+    got.sum().backward()
+    assert layer.tau.grad is not None and torch.isfinite(layer.tau.grad) and layer.tau.grad != 0
+    near = lambda a, b: ((a - b).float().norm() / b.float().norm()).item() < 3e-3
+    with torch.no_grad():
+        assert near(got, want) and near(layer(x, rm), want) and near(layer(x[:1], rm, saved_state={}), first)

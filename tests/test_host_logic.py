@@ -281,3 +281,10 @@ def test_a_layer_pass_keeps_matrices_at_odd_addresses_from_the_kernel(layer_pass
     assert not layer._fused_layer_pass(q, k, v, odd(w), None)
     layer.sigma = torch.nn.Parameter(odd(layer.sigma.data), requires_grad=False)
     assert not layer._fused_layer_pass(q, k, v, w, None)
+
+
+def test_a_layer_pass_leaves_a_temperature_that_is_a_tensor_to_the_tensor_expressions(layer_pass):
+    layer, (q, k, v), w = layer_pass
+    assert layer._fused_layer_pass(q, k, v, w, None)
+    layer.tau = torch.tensor(2.0)
+    assert not layer._fused_layer_pass(q, k, v, w, None)
