@@ -295,3 +295,25 @@ def test_every_chunked_kernel_against_fp64(dev, K, d, T, BH):
     assert _lib.load().rfa_causal_fwd(*(t.data_ptr() for t in (q, k, v, bare)), None, None, None, None, None,
                                       ctypes.c_size_t(0), T, BH, K, d, _lib.stream_of(q)) == 0
     assert rel(bare, want, 2.0 ** -24) < 4e-4
+
+
+@pytest.mark.parametrize("rows", [720, 16])
+def test_sines_of_exact_arguments(dev, rows):
+    """csrc/trig.cuh (720 rows of 40 heads) and CUDA's sines (16 rows) where u is w to the bit: the normalised entry is 1, values of one octave share a block
+    of 16, and 22 significant bits survive the split.  From 2^-6 to 2^20, on both sides of where the reduction becomes the library's,
+    every other one next to a multiple of pi / 2.  1.6 units of fp32's last place at 1 and the library's 2: 1.2e-7."""
+    from rfa_b200 import ops
+    H, D, d = 40, 64, 8
+    gen = torch.Generator().manual_seed(rows)
+    lowest = 2.0 ** torch.linspace(-6, 19, H * D // 16).double()
+    u = (lowest[:, None] * (1 + torch.rand(len(lowest), 16, generator=gen, dtype=torch.double))).view(H, D)
+    near = (u[:, ::2] / (torch.pi / 2)).round().clamp_min(1) * (torch.pi / 2)
+    u[:, ::2] = torch.where(u[:, ::2] > 1.6, near, u[:, ::2])
+    mantissa, exponent = torch.frexp(u)
+    u = torch.ldexp((mantissa * 2 ** 22).round() / 2 ** 22, exponent)
+    w = torch.zeros(H, D, d, dtype=torch.double)
+    w[:, :, 0] = u
+    x = torch.zeros(rows, H, d, device=dev)
+    x[:, :, 0] = 2.0 ** 40
+    phi = ops.feature_map_fwd(x, w.float().to(dev), 1.0).cpu().double()
+    assert ((phi[..., :D] - u.sin()).abs() <= 1.2e-7).all() and ((phi[..., D:] - u.cos()).abs() <= 1.2e-7).all()
