@@ -26,7 +26,7 @@ struct GsLayout {
   uint32_t x_bytes, y_bytes;
   uint32_t S, z, s_hi, s_f, P, p_f, D, d_f, G, g_f, row, tile, total;
 };
-enum { kGsState = 1, kGsP = 2, kGsD = 4, kGsG = 8 };      // which split matrices a kernel holds
+enum { kGsState = 1, kGsP = 2, kGsD = 4, kGsG = 8, kGsByRow = 16 };      // which split matrices a kernel holds; P with a factor a row
 __host__ __device__ inline GsLayout gs_layout(int C, int K, int d, int nx, int ny, int has, int row_floats) {
   GsLayout L;
   L.Kp = gm_round16(K); L.dp = gm_round16(d);
@@ -39,11 +39,11 @@ __host__ __device__ inline GsLayout gs_layout(int C, int K, int d, int nx, int n
   L.s_hi = take(has & kGsState ? (uint32_t)L.Kp * L.ph * 4 : 0);
   L.s_f = take(has & kGsState ? (uint32_t)(L.Kp / 16) * (L.dp / 16) * 4 : 0);
   L.P = take(has & kGsP ? (uint32_t)C * L.pc * 4 : 0);
-  L.p_f = take(has & kGsP ? (uint32_t)(C / 16) * (C / 16) * 4 : 0);
+  L.p_f = take(has & kGsP ? (uint32_t)(C / 16) * (has & kGsByRow ? C : C / 16) * 4 : 0);
   L.D = take(has & kGsD ? (uint32_t)C * L.pc * 4 : 0);
   L.d_f = take(has & kGsD ? (uint32_t)(C / 16) * (C / 16) * 4 : 0);
   L.G = take(has & kGsG ? (uint32_t)C * L.ph * 4 : 0);
-  L.g_f = take(has & kGsG ? (uint32_t)(C / 16) * (L.dp / 16) * 4 : 0);
+  L.g_f = take(has & kGsG ? (uint32_t)(C / 16) * L.dp * 2 : 0);
   L.row = take((uint32_t)row_floats * 4);
   L.tile = at;
   L.total = at + nx * L.x_bytes + ny * L.y_bytes;
@@ -57,27 +57,26 @@ __device__ __forceinline__ GsSplit gs_split_at(unsigned char* base, uint32_t hi,
 __host__ __device__ inline int gs_rows_fwd(int C) { return (C / 16 + 1) * C; }                                  // rs, qz
 __host__ __device__ inline int gs_rows_q(int C, int K) { return (2 * (C / 16) + gm_groups32(K) + 3) * C; }      // rs, pg, wq, qz, inv, gz
 __host__ __device__ inline int gs_rows_w(int C) { return 3 * C + 16; }                                          // inv, gz, gz in two fp16 parts, its factors
-__host__ __device__ inline GsLayout gs_layout_fwd(int C, int K, int d) { return gs_layout(C, K, d, 2, 1, kGsState | kGsP, gs_rows_fwd(C)); }
+__host__ __device__ inline GsLayout gs_layout_fwd(int C, int K, int d) { return gs_layout(C, K, d, 2, 1, kGsState | kGsP | kGsByRow, gs_rows_fwd(C)); }
 __host__ __device__ inline GsLayout gs_layout_q(int C, int K, int d) { return gs_layout(C, K, d, 2, 2, kGsState | kGsD, gs_rows_q(C, K)); }
 __host__ __device__ inline GsLayout gs_layout_kv(int C, int K, int d) { return gs_layout(C, K, d, 2, 2, kGsState | kGsP | kGsD | kGsG, gs_rows_w(C)); }
 __host__ __device__ inline GsLayout gs_layout_state(int C, int K, int d, bool w) { return gs_layout(C, K, d, 1, 1, w ? kGsG : 0, w ? gs_rows_w(C) : 0); }
 
 // ---- products ------------------------------------------------------------------------------------------------------------------
-// acc (16 x 8 NT) += sum over l in [l0, l1) of A(i, l) B(l, j): A rows i0.. (TRANS: columns i0..) of a split matrix, B columns j0.. of an
-// fp16 tile stored along j
-template <int NT, bool TRANS>
-__device__ __forceinline__ void gs_product_a(float (&acc)[NT][4], int nt, int l0, int l1, const GsSplit& A, int i0, GmTile y, int j0) {
+// acc (16 x 8 NT) += sum over l in [l0, l1) of A(i, l) B(l, j), B columns j0.. of an fp16 tile stored along j.  f: a lane's factors (rows g, g + 8) for
+// the first 16 terms, df to the next
+template <int NT, bool TRANS, class F>
+__device__ __forceinline__ void gs_product(float (&acc)[NT][4], int nt, int l0, int l1, const __half* hi, const __half* lo_, int at, uint32_t da, GmTile y,
+                                           int j0, F f) {
   const int lane = threadIdx.x & 31;
-  const int at = TRANS ? i0 + gm_off_b(lane, A.pitch) + l0 * A.pitch : i0 * A.pitch + gm_off_a(lane, A.pitch) + l0;
-  uint32_t ph = gm_addr(A.hi + at), pb = gm_addr(y.p + j0 + gm_off_a(lane, y.pitch) + l0 * y.pitch);
-  const uint32_t lo = (uint32_t)((const char*)A.lo - (const char*)A.hi), da = TRANS ? 32u * A.pitch : 32u, db = 32u * y.pitch;
-  const float* f = A.inv_s + (TRANS ? (i0 >> 4) + (l0 >> 4) * A.sp : (i0 >> 4) * A.sp + (l0 >> 4));
+  uint32_t ph = gm_addr(hi + at), pb = gm_addr(y.p + j0 + gm_off_a(lane, y.pitch) + l0 * y.pitch);
+  const uint32_t lo = (uint32_t)((const char*)lo_ - (const char*)hi), db = 32u * y.pitch;
 #pragma unroll 1
-  for (int l = l0; l < l1; l += 16, ph += da, pb += db, f += TRANS ? A.sp : 1) {
+  for (int l = l0; l < l1; l += 16, ph += da, pb += db) {
     uint32_t h[4], o[4];
     if (TRANS) { gm_ldsm_t(h, ph); gm_ldsm_t(o, ph + lo); }
     else { gm_ldsm(h, ph); gm_ldsm(o, ph + lo); }
-    const float sc = *f;
+    const float2 sc = f();
 #pragma unroll
     for (int n = 0; n < NT; n += 2)
       if (n < nt) {
@@ -88,10 +87,34 @@ __device__ __forceinline__ void gs_product_a(float (&acc)[NT][4], int nt, int l0
         gm_mma16_0(p[1], o, b[2], b[3]);
         gm_mma16(p[0], h, b[0], b[1]);
         gm_mma16(p[1], h, b[2], b[3]);
-        gs_add(acc[n], p[0], sc);
-        gs_add(acc[n + 1], p[1], sc);
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[n + m][e] = fmaf(p[m][e], e < 2 ? sc.x : sc.y, acc[n + m][e]);
       }
   }
+}
+// A rows i0.. of a matrix with a factor for each row; (TRANS: columns i0..) of one with a factor a block
+template <int NT>
+__device__ __forceinline__ void gs_product_rows(float (&acc)[NT][4], int nt, int l0, int l1, const GsByRow& A, int i0, GmTile y, int j0) {
+  const int lane = threadIdx.x & 31;
+  const float* f = A.inv_s + (i0 + (lane >> 2)) * A.fr + (l0 >> 4) * A.fc;
+  gs_product<NT, false>(acc, nt, l0, l1, A.hi, A.lo, i0 * A.pitch + gm_off_a(lane, A.pitch) + l0, 32u, y, j0, [&] {
+    const float2 r = make_float2(f[0], f[8 * A.fr]);
+    f += A.fc;
+    return r;
+  });
+}
+template <int NT, bool TRANS>
+__device__ __forceinline__ void gs_product_a(float (&acc)[NT][4], int nt, int l0, int l1, const GsSplit& A, int i0, GmTile y, int j0) {
+  const int lane = threadIdx.x & 31;
+  const float* f = A.inv_s + (TRANS ? (i0 >> 4) + (l0 >> 4) * A.sp : (i0 >> 4) * A.sp + (l0 >> 4));
+  gs_product<NT, TRANS>(acc, nt, l0, l1, A.hi, A.lo, TRANS ? i0 + gm_off_b(lane, A.pitch) + l0 * A.pitch : i0 * A.pitch + gm_off_a(lane, A.pitch) + l0,
+                        TRANS ? 32u * A.pitch : 32u, y, j0, [&] {
+                          const float r = *f;
+                          f += TRANS ? A.sp : 1;
+                          return make_float2(r, r);
+                        });
 }
 // the same with A rows i0.. of an fp16 tile stored along l and B the split matrix, stored along j (ALONG_J) or along l
 template <int NT, bool ALONG_J>
@@ -199,10 +222,13 @@ __device__ __forceinline__ void gs_row_scalars(const GsRows& r, const float* ws_
     if ((i & 15) == 0) r.z_f[i >> 4] = inv_s;
   }
 }
-// inv g as operand, blocks of 16 x 16 from item `w0` on in steps of `dw`
+// inv g as operand, blocks of 16 x 16 from item `w0` on in steps of `dw`; a factor for each column of a block, which is one column of the fp32 state
+// that it is summed into.  The factors are powers of two, whose lower 16 bits are zero: a word holds two columns' (floats would take (128, 96) its
+// chunks of 64)
+__device__ __forceinline__ uint32_t* gs_col_factors(const GsSplit& G, int i0, int j) { return reinterpret_cast<uint32_t*>(G.inv_s) + ((i0 >> 4) * G.sp + j) / 2; }
 template <int C>
 __device__ __forceinline__ void gs_scale_rows(const GsSplit& G, GmTile y, const float* inv, int d, int w0, int dw) {
-  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, nb = G.sp;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, nb = G.sp / 16;
   const GsDiv by(nb);
   for (int w = w0; w < (C / 16) * nb; w += dw) {
     int i0, j0;
@@ -217,7 +243,27 @@ __device__ __forceinline__ void gs_scale_rows(const GsSplit& G, GmTile y, const 
         const float2 v = j < d ? gm_row(y, i, j) : make_float2(0.f, 0.f);
         a[n][2 * r] = v.x * inv[i]; a[n][2 * r + 1] = v.y * inv[i];
       }
-    gs_put(G, i0, j0, a);
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+      float f[2], inv_f[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const uint32_t x = gs_mag(a[n][e]), y = gs_mag(a[n][2 + e]);
+        uint32_t mag = max(x < kGsInf ? x : 0u, y < kGsInf ? y : 0u);
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) mag = max(mag, __shfl_xor_sync(0xffffffffu, mag, o));
+        gs_factors(mag, f[e], inv_f[e]);
+      }
+      const int j = j0 + 8 * n + 2 * t;
+      if (g == 0) *gs_col_factors(G, i0, j) = __float_as_uint(inv_f[0]) >> 16 | __float_as_uint(inv_f[1]);
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        uint32_t hi, lo;
+        gs_parts<true>(a[n][2 * r] * f[0], a[n][2 * r + 1] * f[1], 1.f, hi, lo);
+        *reinterpret_cast<uint32_t*>(G.hi + (i0 + g + 8 * r) * G.pitch + j) = hi;
+        *reinterpret_cast<uint32_t*>(G.lo + (i0 + g + 8 * r) * G.pitch + j) = lo;
+      }
+    }
   }
 }
 __device__ __forceinline__ uint32_t gs_pair(const __half* p) { return *reinterpret_cast<const uint32_t*>(p); }
@@ -249,9 +295,12 @@ __device__ __forceinline__ void gs_update(float* S, float* z, const GsLayout& L,
         gm_mma16_0(p[1], a, o[2], o[3]);
         gm_mma16(p[0], a, b[0], b[1]);
         gm_mma16(p[1], a, b[2], b[3]);
-        const float sc = G.inv_s[(l >> 4) * nb + (j0 >> 4)];
-        gs_add(acc[0], p[0], sc);
-        gs_add(acc[1], p[1], sc);
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+          const uint32_t sc = *gs_col_factors(G, l, j0 + 8 * n + 2 * t);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[n][e] = fmaf(p[n][e], __uint_as_float(e & 1 ? sc & 0xFFFF0000u : sc << 16), acc[n][e]);
+        }
         if (j0 == 0) {
           const uint32_t h0 = g == 0 ? gs_pair(rows.z_hi + l + 2 * t) : 0u, h1 = g == 0 ? gs_pair(rows.z_hi + l + 8 + 2 * t) : 0u;
           const uint32_t o0 = g == 0 ? gs_pair(rows.z_lo + l + 2 * t) : 0u, o1 = g == 0 ? gs_pair(rows.z_lo + l + 8 + 2 * t) : 0u;
@@ -311,7 +360,9 @@ gs_causal_fwd_kernel(const __half* __restrict__ q, const __half* __restrict__ k,
   const GsLayout L = gs_layout_fwd(C, K, d);
   constexpr int MT = C / 16;
   float *S = (float*)(gs_raw + L.S), *z = (float*)(gs_raw + L.z), *rs = (float*)(gs_raw + L.row), *qz = rs + MT * C;
-  const GsSplit op = gs_split_at(gs_raw, L.s_hi, L.s_f, L.Kp, L.ph, L.dp / 16), P = gs_split_at(gs_raw, L.P, L.p_f, C, L.pc, MT);
+  const GsSplit op = gs_split_at(gs_raw, L.s_hi, L.s_f, L.Kp, L.ph, L.dp / 16);
+  // a token's output is divided by its own denominator: weights of another in its block may be any times larger than its own
+  const GsByRow P{(__half*)(gs_raw + L.P), (__half*)(gs_raw + L.P) + C * L.pc, (float*)(gs_raw + L.p_f), L.pc, 1, C};
   const int bh = blockIdx.x, seg = blockIdx.y, nseg = gridDim.y;
   const int64_t t_begin = seg * tseg, t_end = min(T, t_begin + tseg);
   const int nchunk = (int)((t_end - t_begin + C - 1) / C);
@@ -360,7 +411,7 @@ gs_causal_fwd_kernel(const __half* __restrict__ q, const __half* __restrict__ k,
           if (j0 + 8 * n + 2 * t + (e & 1) > i0 + g + 8 * (e >> 1)) acc[n][e] = 0.f;
           r[e >> 1] += acc[n][e];
         }
-      gs_put(P, i0, j0, acc);
+      gs_put_rows(P, i0, j0, acc);
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         r[e] = gm_quad(r[e]);
@@ -378,7 +429,7 @@ gs_causal_fwd_kernel(const __half* __restrict__ q, const __half* __restrict__ k,
       gm_zero(acc);
       if (odd) gm_product_masked<2>(acc, i0, j0, nt, 0, i0 + 16, [=](int i, int l) { return make_float2(gs_at(P, i, l), gs_at(P, i, l + 1)); },
                                     [=](int l, int j) { return gm_col(tv, l, j); }, [](int i, int l) { return l <= i; });
-      else gs_product_a<2, false>(acc, nt, 0, i0 + 16, P, i0, tv, j0);
+      else gs_product_rows<2>(acc, nt, 0, i0 + 16, P, i0, tv, j0);
       gs_product_b<2, true>(acc, nt, K, tq, i0, op, j0);
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
@@ -588,7 +639,7 @@ gs_causal_bwd_kv_kernel(const __half* __restrict__ q, const __half* __restrict__
   float *S = (float*)(gs_raw + L.S), *z = (float*)(gs_raw + L.z);
   const GsRows rows = gs_rows_at((float*)(gs_raw + L.row), C);
   const GsSplit op = gs_split_at(gs_raw, L.s_hi, L.s_f, L.Kp, L.ph, L.dp / 16), P = gs_split_at(gs_raw, L.P, L.p_f, C, L.pc, MT),
-                D = gs_split_at(gs_raw, L.D, L.d_f, C, L.pc, MT), Gs = gs_split_at(gs_raw, L.G, L.g_f, C, L.ph, L.dp / 16);
+                D = gs_split_at(gs_raw, L.D, L.d_f, C, L.pc, MT), Gs = gs_split_at(gs_raw, L.G, L.g_f, C, L.ph, L.dp);
   const int bh = blockIdx.x, seg = blockIdx.y, nseg = gridDim.y;
   const int64_t t_begin = seg * tseg, t_end = min(T, t_begin + tseg);
   const int nchunk = (int)((t_end - t_begin + C - 1) / C);
@@ -710,7 +761,7 @@ gs_state_kernel(const __half* __restrict__ x, const __half* __restrict__ y, cons
   const GsLayout L = gs_layout_state(C, K, d, WEIGHTED);
   float *S = (float*)(gs_raw + L.S), *z = (float*)(gs_raw + L.z);
   const GsRows rows = gs_rows_at((float*)(gs_raw + L.row), C);
-  const GsSplit Gs = gs_split_at(gs_raw, L.G, L.g_f, C, L.ph, L.dp / 16);
+  const GsSplit Gs = gs_split_at(gs_raw, L.G, L.g_f, C, L.ph, L.dp);
   const int bh = blockIdx.x, seg = blockIdx.y;
   const int64_t t_begin = seg * tseg, t_end = min(T, t_begin + tseg);
   const int nchunk = t_end > t_begin ? (int)((t_end - t_begin + C - 1) / C) : 0;

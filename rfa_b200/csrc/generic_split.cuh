@@ -1,4 +1,5 @@
-// fp32 matrices as operands of mma.sync m16n8k16 f16: two fp16 tiles and a power of two per 16 x 16 block.
+// fp32 matrices as operands of mma.sync m16n8k16 f16: two fp16 tiles and a power of two per 16 x 16 block, or for each of a block's rows or columns
+// where they are results that must not lose bits to one another.
 //
 // x is held as hi = fp16(s x) and lo = fp16(s x - hi): 22 bits.  s takes the block's largest finite element to [2^14, 2^15), so that
 // fp16's range costs nothing: an element down to 2^-17 of its block's largest keeps all 22 bits, and what a smaller one loses

@@ -317,3 +317,35 @@ def test_sines_of_exact_arguments(dev, rows):
     x[:, :, 0] = 2.0 ** 40
     phi = ops.feature_map_fwd(x, w.float().to(dev), 1.0).cpu().double()
     assert ((phi[..., :D] - u.sin()).abs() <= 1.2e-7).all() and ((phi[..., D:] - u.cos()).abs() <= 1.2e-7).all()
+
+
+@pytest.mark.parametrize("K,d", [(64, 32), (96, 40), (128, 128), (160, 128)])
+@pytest.mark.parametrize("T", [16, 45])
+def test_a_token_beside_a_much_larger_one(dev, K, d, T):
+    """Queries of 2^15 and of 2^-14 in one block of 16: each output is divided by its own token's denominator, so that the small one's (which the clamp
+    leaves at 1) must not have the error of the large one's weights.  Every token has fp16's rounding error and no more."""
+    gen = torch.Generator().manual_seed(K + T)
+    q, k = (torch.rand(T, 3, K, generator=gen) * 0.3 + 0.02 for _ in range(2))
+    v = torch.randn(T, 3, d, generator=gen) * 1024
+    q = q * torch.where(torch.arange(T) % 2 == 0, 2.0 ** 15, 2.0 ** -14)[:, None, None]
+    q, k, v = q.half(), k.half(), v.half()
+    want = RFA.forward_torch(*(t.double() for t in (q, k, v)))
+    out = RFA.forward_cuda(*(t.to(dev) for t in (q, k, v)))
+    for t in range(T):
+        assert rel(out[t], want[t], 2.0 ** -24) < 4e-4, t
+
+
+@pytest.mark.parametrize("K,d", [(64, 32), (96, 40), (128, 128), (160, 128)])
+@pytest.mark.parametrize("T", [16, 45, 300])
+def test_a_column_of_the_reverse_state_beside_a_much_larger_one(dev, K, d, T):
+    """As above for every column by itself, with gradients whose columns fall from 2^8 to 2^-14 within a block."""
+    from rfa_b200 import ops
+    q, k, v, g = inputs(T, 8, K, d, T)
+    g = (g * 2.0 ** torch.linspace(8, -14, 16).round().repeat(d // 16 + 1)[:d]).half()
+    q, k, v, g = (t.to(dev) for t in (q, k, v, g))
+    _, ds, _, _ = ops.causal_bwd_q(q, k, v, g, None, None, True)
+    Q, Kd, G = (t.double() for t in (q, k, g))
+    inv = 1 / (Q * torch.cumsum(Kd, 0)).sum(-1, keepdim=True).clamp_min(1)
+    want = torch.einsum("tbk,tbd->bkd", Q, G * inv)
+    error = (ds - want).norm(dim=(0, 1)) / want.norm(dim=(0, 1))
+    assert float(error.max()) < 1.2e-7 * max(1.0, T / 16) ** 0.5, error
