@@ -325,12 +325,13 @@ class CausalAttention(nn.Module):
         launches and 10 us of the 188 that a pass over 8 x 2048 tokens of 16 heads takes)."""
         sigma = self.sigma if self.reparam_proj else None
         half = torch.float16
-        if any(t is not None and (t.device != q.device or t.data_ptr() % 16) for t in (random_matrices, sigma)):
-            return False           # the tensor expressions refuse operands of two devices and make aligned ones of a view at any offset
-        return (self._own_matrices(random_matrices) and ops.fused_forward_supported(q, random_matrices) and q.dtype is k.dtype is v.dtype is half
+        if not (self._own_matrices(random_matrices) and ops.fused_forward_supported(q, random_matrices) and q.dtype is k.dtype is v.dtype is half
                 and tuple(random_matrices.shape) == (self.num_heads, 64, 64) and random_matrices.dtype is half
                 and (sigma is None or (sigma.dtype is half and tuple(sigma.shape) == (self.num_heads, 1, 64)))
-                and plain_tensors(q, k, v, random_matrices, sigma, mask) and _underived(q, k, v, random_matrices, sigma))
+                and plain_tensors(q, k, v, random_matrices, sigma, mask) and _underived(q, k, v, random_matrices, sigma)):
+            return False
+        # the tensor expressions refuse operands of two devices and make aligned ones of a view at any offset
+        return all(t is None or (t.device == q.device and t.data_ptr() % 16 == 0) for t in (random_matrices, sigma))
 
     def forward(self, x: Tensor, random_matrices: Tensor, key_padding_mask: Optional[Tensor] = None,
                 attn_mask: Optional[Tensor] = None,

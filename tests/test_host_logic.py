@@ -288,3 +288,12 @@ def test_a_layer_pass_leaves_a_temperature_that_is_a_tensor_to_the_tensor_expres
     assert layer._fused_layer_pass(q, k, v, w, None)
     layer.tau = torch.tensor(2.0)
     assert not layer._fused_layer_pass(q, k, v, w, None)
+
+
+def test_a_layer_pass_asks_for_no_address_while_it_is_traced(layer_pass, monkeypatch):
+    """A tensor that only stands for one while a call is traced or compiled has none."""
+    from rfa_b200 import causal_attention
+    layer, (q, k, v), w = layer_pass
+    monkeypatch.setattr(causal_attention, "plain_tensors", lambda *_: False)
+    monkeypatch.setattr(torch.Tensor, "data_ptr", lambda self: pytest.fail("asked for an address"))
+    assert not layer._fused_layer_pass(q, k, v, w, None)
