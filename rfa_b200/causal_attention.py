@@ -192,6 +192,7 @@ def _underived(*tensors: Optional[Tensor]) -> bool:
 
 
 _LINEAR_FORWARD = nn.Linear.forward
+_NUMBER = (int, float)                                    # a tau that is a tensor may want a gradient: the native passes leave it alone
 
 
 def _plain_call(tensors, linears) -> bool:
@@ -273,16 +274,10 @@ class CausalAttention(nn.Module):
         saved_state["prev_s"], saved_state["prev_z"] = s, z
         return attn
 
-    def _own_matrices(self, random_matrices: Tensor) -> bool:
-        """Whether the matrices are for this layer's heads.  A native pass takes the split of the features into heads from them, and others may
-        divide embed_dim too, which the module-by-module call refuses.  (A tau that is a tensor, which may want a gradient, stays with the tensor
-        expressions too.)"""
-        return isinstance(self.tau, (int, float)) and random_matrices.dim() == 3 and random_matrices.size(0) == self.num_heads and random_matrices.size(2) == self.head_dim
-
     def _decode_layer(self, x: Tensor, random_matrices: Tensor, saved_state: Dict[str, Optional[Tensor]]) -> Optional[Tensor]:
         """One token through the whole layer in three launches (host time is what a small decoding call consists of); None, and
         nothing done, where the call is to go module by module."""
-        if not (x.is_cuda and x.dtype is torch.float16 and random_matrices.is_cuda and self._own_matrices(random_matrices)):
+        if not (x.is_cuda and x.dtype is torch.float16 and random_matrices.dim() == 3 and random_matrices.is_cuda and isinstance(self.tau, _NUMBER)):
             return None
         linears = (self.q_proj, self.k_proj, self.v_proj, self.out_proj)
         sigma = self.sigma if self.reparam_proj else None
@@ -294,7 +289,7 @@ class CausalAttention(nn.Module):
             return None
         if s is None and z is None:
             s, z = self._state(saved_state, x.size(1), random_matrices)
-        y = ops.layer_decode(x, *linears, random_matrices, sigma, self.tau, SCALE, s, z)
+        y = ops.layer_decode(x, *linears, random_matrices, sigma, self.tau, SCALE, s, z, self.num_heads)
         if y is not None:
             saved_state["prev_s"], saved_state["prev_z"] = s, z
         return y
@@ -305,8 +300,8 @@ class CausalAttention(nn.Module):
         858, 757).  None, and nothing done, where the call is to go module by module."""
         sigma = self.sigma if self.reparam_proj else None
         if not (torch.is_grad_enabled() and x.is_cuda and x.dtype is torch.float16 and random_matrices.dtype is torch.float16
-                and self._own_matrices(random_matrices)):
-            return None
+                and random_matrices.dim() == 3 and random_matrices.size(0) == self.num_heads and isinstance(self.tau, _NUMBER)):
+            return None                                   # (matrices for another number of heads may divide embed_dim too: refused module by module)
         if not (x.requires_grad or random_matrices.requires_grad or self.q_proj.weight.requires_grad
                 or (sigma is not None and sigma.requires_grad)):
             return None                                   # nothing that the attention's own choice of kernels counts as recording
@@ -325,7 +320,7 @@ class CausalAttention(nn.Module):
         launches and 10 us of the 188 that a pass over 8 x 2048 tokens of 16 heads takes)."""
         sigma = self.sigma if self.reparam_proj else None
         half = torch.float16
-        if not (self._own_matrices(random_matrices) and ops.fused_forward_supported(q, random_matrices) and q.dtype is k.dtype is v.dtype is half
+        if not (isinstance(self.tau, _NUMBER) and ops.fused_forward_supported(q, random_matrices) and q.dtype is k.dtype is v.dtype is half
                 and tuple(random_matrices.shape) == (self.num_heads, 64, 64) and random_matrices.dtype is half
                 and (sigma is None or (sigma.dtype is half and tuple(sigma.shape) == (self.num_heads, 1, 64)))
                 and plain_tensors(q, k, v, random_matrices, sigma, mask) and _underived(q, k, v, random_matrices, sigma)):

@@ -20,8 +20,8 @@
 // state update); 3 = issuer U (the projections: issuing a product costs its thread about as long as the tensor pipe takes
 // to run it, so the three chains are issued by three threads); 4..7 = score group; 8..11 = output/state group; 12..19 =
 // query features, 20..27 = key features (two warpgroups each: thread <-> row, and half of the 64 projected columns per
-// warpgroup -- the sines and cosines are the longest step of a chunk and bound by the special-function unit, which
-// sixteen warps keep busier than eight).  Register budgets differ by role (setmaxnreg): issuers 64, score group 96,
+// warpgroup -- the sines and cosines are the longest step of a chunk, a chain of waits more than the special-function unit's time
+// (it is 35 % busy), of which sixteen warps hide more than eight: 58 -> 55 us at 8 x 16 x 2048).  Register budgets differ by role (setmaxnreg): issuers 64, score group 96,
 // output/state group 104, feature warps 56.  Within a group thread <-> TMEM lane <-> token row / state row.  All waits
 // are bounded.
 #include <type_traits>

@@ -6,7 +6,8 @@
 // hi lo, hi hi; what is left out is 2^-22 of a term.  16 terms at a time from zero, those sums scaled and added in fp32.
 // Register tiles on the FMA pipe (feature_map.cu) read 16 bytes of shared memory for every 8 FMAs, which bounded them, and the sines
 // of CUDA's library are 75 instructions a pair (trig.cuh); splits into tf32 at every read (6 mma per 16 terms instead of 3, and 5
-// instructions an element and read) were no faster than those.  What bounds it now is instructions issued (issue slots 60 %).
+// instructions an element and read) were no faster than those.  What bounds it now is issue slots and fixed latencies at 16 warps an SM (slots
+// 57 % forward, 49 % backward, no pipe above 33 %).
 // fp32, 64 x 64, 4096 rows of 16 heads: forward 30.1 -> 18.2 us, backward 67.6 -> 42.4 (40.2 with one factor a block); 32 x 32, 4096 rows of 8 heads 11.8 -> 6.8 and 23.7 -> 14.0.
 // Errors against fp64 (phi, g_x, g_W): 1.62, 2.27, 2.42e-7 -> 1.27, 1.72, 1.95e-7, from shorter chains of fp32 sums.
 //

@@ -5,9 +5,9 @@
 // State, weights and partial sums are fp32; as operands they are split into two fp16 tiles (generic_split.cuh), once, by the warp that
 // made them.
 // The kernels of generic_mma.cu split into tf32 in registers, at every read: 28 instructions a fragment of A, and four mma per 16 terms
-// where there are two here.  Both are bound by instructions issued, not by memory or the tensor pipe (issue slots 50 %, ALU 38 %,
-// tensor pipe 12 %, a third of the stalls at the chunk's barriers): forward + backward kernels 185 -> 141 us at (K, d) = (64, 32), 64 heads x
-// 1024 tokens, 138 -> 92 at (96, 40), 64 x 300, 392 -> 323 at (128, 128), 64 x 512, 123 -> 57 at (128, 128), 8 x 200.
+// where there are two here.  Both are bound by issue slots and a chunk's chain of phases, not by memory or the tensor pipe (slots 50 %, ALU 35 %,
+// tensor pipe 12 %, a third of a warp's wait at the chunk's barriers): forward + backward kernels 185 -> 137 us at (K, d) = (64, 32), 64 heads x
+// 1024 tokens, 138 -> 90 at (96, 40), 64 x 300, 392 -> 317 at (128, 128), 64 x 512, 123 -> 57 at (128, 128), 8 x 200.
 #include "generic_split.cuh"
 #include "segments.cuh"
 #include "sm100.cuh"

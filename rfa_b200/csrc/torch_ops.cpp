@@ -423,7 +423,7 @@ bool capturing(const Tensor& x) {
 // layout, a broadcast shape, a batch that the library GEMMs serve better): nothing has been done then.
 OptTensor layer_decode(const Tensor& x, const Tensor& wq, const OptTensor& bq, const Tensor& wk, const OptTensor& bk, const Tensor& wv,
                        const OptTensor& bv, const Tensor& wo, const OptTensor& bo, const Tensor& rm, const OptTensor& sigma, double tau,
-                       double scale, const OptTensor& s, const OptTensor& z) {
+                       double scale, const OptTensor& s, const OptTensor& z, int64_t heads) {
   if (!x.is_cuda() || x.dim() != 3 || x.size(0) != 1 || rm.dim() != 3) return std::nullopt;
   const int64_t B = x.size(1), E = x.size(2), H = rm.size(0), D = rm.size(1), d = rm.size(2);
   const auto plain = [&](const Tensor& t, at::IntArrayRef shape, at::ScalarType type) {
@@ -432,7 +432,7 @@ OptTensor layer_decode(const Tensor& x, const Tensor& wq, const OptTensor& bq, c
   };
   const auto bias = [&](const OptTensor& b) { return !b || plain(*b, {E}, at::kHalf); };
   const bool width = D > 0 && D % 8 == 0 && D <= 128 && (d == 8 || d == 16 || d == 32 || d == 64 || d == 128);
-  if (B < 1 || B > most_rows(E, capturing(x)) || !width || H < 1 || H * d != E || !plain(x, {1, B, E}, at::kHalf)) return std::nullopt;
+  if (B < 1 || B > most_rows(E, false) || (B > most_rows(E, true) && capturing(x)) || !width || H < 1 || H * d != E || (heads && H != heads) || !plain(x, {1, B, E}, at::kHalf)) return std::nullopt;
   for (const Tensor* w : {&wq, &wk, &wv, &wo})
     if (!plain(*w, {E, E}, at::kHalf)) return std::nullopt;
   if (!bias(bq) || !bias(bk) || !bias(bv) || !bias(bo) || !plain(rm, {H, D, d}, at::kHalf)) return std::nullopt;

@@ -315,11 +315,12 @@ def decode_fused_supported(q: Tensor, w: Tensor) -> bool:
 
 
 def layer_decode(x: Tensor, q_proj, k_proj, v_proj, out_proj, random_matrices: Tensor, sigma: Optional[Tensor], tau: float,
-                 scale: float, s: Optional[Tensor], z: Optional[Tensor]) -> Optional[Tensor]:
+                 scale: float, s: Optional[Tensor], z: Optional[Tensor], num_heads: int = 0) -> Optional[Tensor]:
     """One token x [1, B, E] through a layer's projections (``nn.Linear`` modules) and its decoding step in three launches, the
-    state updated IN PLACE; None, with nothing done, where the tensors are not ones the kernels take (then: module by module)."""
+    state updated IN PLACE; None, with nothing done, where the tensors are not ones the kernels take (then: module by module), or the
+    matrices are not ``num_heads`` (0: any)."""
     return native().layer_decode(x, q_proj.weight, q_proj.bias, k_proj.weight, k_proj.bias, v_proj.weight, v_proj.bias,
-                                 out_proj.weight, out_proj.bias, random_matrices, sigma, tau, scale, s, z)
+                                 out_proj.weight, out_proj.bias, random_matrices, sigma, tau, scale, s, z, num_heads)
 
 
 def layer_train(x: Tensor, q_proj, k_proj, v_proj, out_proj, random_matrices: Tensor, sigma: Optional[Tensor], tau: float,
