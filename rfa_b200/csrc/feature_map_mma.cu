@@ -8,7 +8,7 @@
 // of CUDA's library are 75 instructions a pair (trig.cuh); splits into tf32 at every read (6 mma per 16 terms instead of 3, and 5
 // instructions an element and read) were no faster than those.  What bounds it now is issue slots and fixed latencies at 16 warps an SM (slots
 // 57 % forward, 49 % backward, no pipe above 33 %).
-// fp32, 64 x 64, 4096 rows of 16 heads: forward 30.1 -> 18.2 us, backward 67.6 -> 42.4 (40.2 with one factor a block); 32 x 32, 4096 rows of 8 heads 11.8 -> 6.8 and 23.7 -> 14.0.
+// fp32, 64 x 64, 4096 rows of 16 heads: forward 30.1 -> 18.2 us, backward 67.6 -> 41.8 (40.2 with one factor a block, 46.6 with faded rows in every one); 32 x 32, 4096 rows of 8 heads 11.8 -> 6.8 and 23.7 -> 14.4.
 // Errors against fp64 (phi, g_x, g_W): 1.62, 2.27, 2.42e-7 -> 1.27, 1.72, 1.95e-7, from shorter chains of fp32 sums.
 //
 // A warp owns 16 rows: it loads, normalises and splits them, and their products, sines and results stay within the warp
@@ -31,14 +31,15 @@ static_assert(kCtas * (kBwdBytes + 1024) <= 228 * 1024 && kG % 16 == 0, "feature
 __device__ __forceinline__ float2 both(float f) { return make_float2(f, f); }
 // ---- products ------------------------------------------------------------------------------------------------------------------
 // acc (16 x 32, nt blocks of 8 columns) = A B of two split operands, L terms: pa, pb the lane's shared-memory addresses of the first
-// fragments, da, db their steps per 16 terms and dn B's per 16 columns, (TA, TB) whether the fragments are transposed; f(l, n): the factor
-// of the sums over terms 16 l .. for columns 16 n .., in rows g and g + 8
-template <bool TA, bool TB, class F>
+// fragments, da, db their steps per 16 terms and dn B's per 16 columns, (TA, TB) whether the fragments are transposed; the sums over terms 16 l .. have
+// the factors r(l), of rows g and g + 8, and f(l, n), of columns 16 n ..
+template <bool TA, bool TB, class R, class F>
 __device__ __forceinline__ void product(float (&acc)[4][4], int nt, int L, uint32_t pa, uint32_t a_lo, uint32_t da, uint32_t pb, uint32_t b_lo,
-                                        uint32_t db, uint32_t dn, F f) {
+                                        uint32_t db, uint32_t dn, R r, F f) {
   gm_zero(acc);
 #pragma unroll 1
   for (int l = 0; l < L; ++l, pa += da, pb += db) {
+    const float2 fr = r(l);
     uint32_t ah[4], al[4];
     if (TA) { gm_ldsm_t(ah, pa); gm_ldsm_t(al, pa + a_lo); }
     else { gm_ldsm(ah, pa); gm_ldsm(al, pa + a_lo); }
@@ -55,7 +56,8 @@ __device__ __forceinline__ void product(float (&acc)[4][4], int nt, int L, uint3
         gm_mma16(p[1], ah, bl[2], bl[3]);
         gm_mma16(p[0], ah, bh[0], bh[1]);
         gm_mma16(p[1], ah, bh[2], bh[3]);
-        const float2 sc = f(l, n);
+        const float fn = f(l, n);
+        const float2 sc = make_float2(fr.x * fn, fr.y * fn);
 #pragma unroll
         for (int m = 0; m < 2; ++m)
 #pragma unroll
@@ -142,7 +144,7 @@ __device__ __forceinline__ Tiles tiles_at(unsigned char* base) {
 __device__ __forceinline__ void project(float (&u)[4][4], int nt, const Tiles& s, int row, int c, int d, int lane) {
   const float* f = s.W.inv_s + 2 * c * 4;
   product<false, false>(u, nt, (d + 15) / 16, gm_addr(s.xh + row * kP + gm_off_a(lane, kP)), 2 * kRows * kP, 32,
-                        gm_addr(s.W.hi + 32 * c * kP + gm_off_b(lane, kP)), 2 * kMax * kP, 32, 32 * kP, [&](int l, int n) { return both(f[n * 4 + l] * kXi); });
+                        gm_addr(s.W.hi + 32 * c * kP + gm_off_b(lane, kP)), 2 * kMax * kP, 32, 32 * kP, [](int) { return both(kXi); }, [&](int l, int n) { return f[n * 4 + l]; });
 }
 
 // g_u.  g_x = g_u W is a product for each row by itself, so that a row must not lose bits to a larger one beside it: where a row of a block is
@@ -327,7 +329,7 @@ feature_map_mma_bwd_kernel(const T* __restrict__ x, const float* __restrict__ w,
           const float *fg = s.G.inv_s + (r0 + g) * 4, *fw = s.W.inv_s + 2 * c;
           product<false, true>(a, nt, (D + 15) / 16, gm_addr(s.G.hi + r0 * kP + gm_off_a(lane, kP)), 2 * kRows * kP, 32,
                                gm_addr(s.W.hi + 32 * c + gm_off_a(lane, kP)), 2 * kMax * kP, 32 * kP, 32,
-                               [&](int l, int n) { return make_float2(fg[l] * fw[4 * l + n], fg[32 + l] * fw[4 * l + n]); });
+                               [&](int l) { return make_float2(fg[l], fg[32 + l]); }, [&](int l, int n) { return fw[4 * l + n]; });
         }
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
@@ -364,7 +366,7 @@ feature_map_mma_bwd_kernel(const T* __restrict__ x, const float* __restrict__ w,
       } else {
         const float* fg = s.G.inv_s + (j0 >> 4);
         product<true, true>(a, lt, active, gm_addr(s.G.hi + j0 + gm_off_b(lane, kP)), 2 * kRows * kP, 32 * kP,
-                            gm_addr(s.xh + l0 + gm_off_a(lane, kP)), 2 * kRows * kP, 32 * kP, 32, [&](int l, int) { return both(fg[64 * l] * kXi); });
+                            gm_addr(s.xh + l0 + gm_off_a(lane, kP)), 2 * kRows * kP, 32 * kP, 32, [&](int l) { return both(fg[64 * l]); }, [](int, int) { return kXi; });
       }
 #pragma unroll
       for (int n = 0; n < 4; ++n)
