@@ -349,3 +349,15 @@ def test_a_column_of_the_reverse_state_beside_a_much_larger_one(dev, K, d, T):
     want = torch.einsum("tbk,tbd->bkd", Q, G * inv)
     error = (ds - want).norm(dim=(0, 1)) / want.norm(dim=(0, 1))
     assert float(error.max()) < 1.2e-7 * max(1.0, T / 16) ** 0.5, error
+
+
+@pytest.mark.parametrize("K,d,T,B,H", [(64, 96, 200, 2, 2), (192, 48, 200, 2, 2), (192, 48, 16, 3, 1), (160, 128, 64, 2, 2), (160, 128, 300, 2, 2), (64, 64, 150, 50, 3)])
+def test_state_reductions_alone(dev, K, d, T, B, H):
+    """Sequences that are not cut have a choice of chunks of their own: fp32 sums of exact products, 2e-6, padded keys left out."""
+    from rfa_b200 import ops
+    gen = torch.Generator(dev).manual_seed(K + T)
+    k, v = torch.randn(T, B, H, K, generator=gen, device=dev).half(), torch.randn(T, B, H, d, generator=gen, device=dev).half()
+    pad = torch.rand(B, T, generator=gen, device=dev) < 0.3
+    s, z = ops.cross_state_fwd(k, v, pad)
+    kd = k.double() * ~pad.t()[:, :, None, None]
+    assert rel(s, torch.einsum("tbhk,tbhd->bhkd", kd, v.double()).cpu()) < 2e-6 and rel(z, kd.sum(0).cpu()) < 2e-6
